@@ -1,0 +1,547 @@
+// Linear layers for several activations on the fifth-generation tensor cores (tcgen05.mma kind::i8, accumulators in
+// tensor memory): the exact integer arithmetic of linear.cu as a GEMM, weights [rows x columns] times the four base-256
+// digits ("limbs") of every activation, 4 B columns.
+//
+// xprep_tc_kernel turns the activations into digits once, with one power-of-two scale per activation, and lays them out as
+// the operand image: per block of 128 columns NC rows of 128 bytes, swizzled. linear_tc_kernel is a cluster of S blocks per
+// run of up to 256 weight rows; block r of the cluster takes the r-th part of the columns. Per 128-column block of its part
+// TMA brings the weights of all rows of the run (one box, rows the tensor lacks are not fetched) and one bulk copy the
+// digits. INT8 weights are the A operand as they land. INT4 nibbles go to tensor memory as bytes (worker warps: four
+// 16-byte shared-memory reads, two masks per word, one tcgen05.st per row and block) and the MMA takes A from there: writing
+// the widened bytes back to shared memory for the MMA to read again would cost four times the bytes of the nibbles there,
+// and shared-memory bandwidth is what an M = 128 integer MMA of 128 columns uses up first.
+// All digit sums are exact int32, recombined to one int64 per (row, activation); the S parts of a run meet in the blocks'
+// shared memory (distributed shared memory, every block finishes the activations b = rank mod S), are added as integers and
+// converted once: the result does not depend on S or on how the rows are dealt.
+//   warps 0-7: INT4 widening, then epilogue    warp 8: weights (TMA)    warp 9: digits (bulk copies)    warp 10: MMA issue
+// The weights do not depend on the kernel ahead: their ring fills before the dependency wait. With at most 128 rows per run a
+// block takes no more than half of an SM's shared memory and tensor memory, so that the next launch's blocks move in beside it
+// and have their weights under way while this launch ends.
+#include "common.cuh"
+#include "tc_common.cuh"
+#include "xconvert.cuh"
+#include <cudaTypedefs.h>
+
+bool ibcu_push_match(ibcu_ctx* ctx, float* const* outs, int n);      // comm.cu
+void ibcu_push_fill(ibcu_ctx* ctx, GatherPush* gp, size_t bytes);
+
+namespace {
+
+constexpr int TQ_WORKERS = 8, TQ_A_WARP = 8, TQ_B_WARP = 9, TQ_MMA_WARP = 10, TQ_THREADS = 11 * 32;
+constexpr int TQ_MAX_STAGES = 8;
+constexpr int TQ_MAX_B = 32;
+
+struct alignas(64) TqMaps { CUtensorMap m[4]; };
+
+struct TqParams {
+    LinTensor t[4];
+    int n_tensors, run_start[5];               // runs of tensor i are [run_start[i], run_start[i + 1])
+    int R, NC, B, nkb, S;                      // rows per run (a multiple of 8), MMA columns, activations, 128-column blocks per row, cluster size
+    int sa, sb, a_stage;                       // ring depths, bytes of a weight stage
+    int tmem_cols, xparts;
+    const int8_t* xtiles;                      // digit image [nkb][NC][128]
+    const float* xscale;                       // [B][xparts], equal over the parts
+    const int* xsum;                           // [B][xparts][4] digit sums (INT4 bias)
+    GatherPush gp;
+    int* err;
+};
+
+struct TqShared {
+    unsigned long long full_a[TQ_MAX_STAGES], empty_a[TQ_MAX_STAGES];    // TMA -> MMA or widening warps, and back
+    unsigned long long full_b[TQ_MAX_STAGES], empty_b[TQ_MAX_STAGES];
+    unsigned long long full_t[4], empty_t[4];                            // INT4: widened blocks in tensor memory
+    unsigned long long full_acc, empty_acc, drained;
+    uint32_t tmem_base;
+    int abort_flag;
+    float back[TQ_MAX_B];
+    long long bias[TQ_MAX_B];
+};
+
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory"); }
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// shared-memory matrix descriptor, K-major with the 128-byte swizzle: 8-row atoms of 1024 bytes follow one another; the K
+// offset inside the 128-byte rows is part of the start address
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                 :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+                    "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// the four digit sums of one (row, activation) as one integer
+__device__ __forceinline__ long long join_limbs(const uint32_t* a) {
+    return (((long long)(int)a[3] * 256 + (int)a[2]) * 256 + (int)a[1]) * 256 + (int)a[0];
+}
+__device__ __forceinline__ float row_scale(const LinTensor& W, int row) {
+    return W.scales_fp32 ? reinterpret_cast<const float*>(W.scales)[row] : __half2float(reinterpret_cast<const __half*>(W.scales)[row]);
+}
+
+// grid (parts, B): digits of one activation (or of one part of its columns when the caller knows the maximum)
+template <int T>
+__global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, int part_cols, int all_cols, int nc, int perm8, int8_t* __restrict__ xtiles,
+                                                     float* __restrict__ xscale, int* __restrict__ xsum, const GatherWait gw) {
+    __shared__ XScratch sc;
+    pdl_launch_dependents();
+    pdl_wait();
+    gather_wait(gw);
+    const int part = blockIdx.x, b = blockIdx.y, c0 = part * part_cols;
+    const XTiles dst = { xtiles, nc, b * LIN_LIMBS, c0 };
+    xconvert_any(src, N, b, c0, min(part_cols, all_cols - c0), dst, perm8, sc, xscale + b * gridDim.x + part, xsum + ((size_t)b * gridDim.x + part) * LIN_LIMBS);
+}
+
+// BITS 4 or 8; T: 128-row tiles per run
+template <int BITS, int T>
+__global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
+    extern __shared__ __align__(1024) unsigned char tq_smem[];
+    constexpr int NT = T == 1 ? 4 : 2;                         // widened blocks in tensor memory
+    constexpr int TW = T == 1 ? 4 : 8;                         // worker warps that share a widened block
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int S = p.S, rank = (int)blockIdx.x % S, cl = (int)blockIdx.x / S, ncl = (int)gridDim.x / S;
+    const int nruns = p.run_start[p.n_tensors];
+    const int k0 = (int)((long)p.nkb * rank / S), k1 = (int)((long)p.nkb * (rank + 1) / S);
+    unsigned char* ringA = tq_smem;
+    unsigned char* ringB = tq_smem + (((size_t)p.sa * p.a_stage + 1023) & ~(size_t)1023);
+    const int b_stage = p.NC * 128;
+    size_t ring_bytes = (size_t)(ringB - tq_smem) + (size_t)p.sb * b_stage;
+    if (BITS == 8 && ring_bytes < (size_t)p.sa * p.a_stage + T * 16384) ring_bytes = (size_t)p.sa * p.a_stage + T * 16384;   // an MMA reads 128 rows whatever the run has
+    TqShared* sh = reinterpret_cast<TqShared*>(tq_smem + ((ring_bytes + 15) & ~(size_t)15));
+    volatile int* abort_flag = &sh->abort_flag;
+    pdl_launch_dependents();
+
+    if (tid == 0) {
+        for (int s = 0; s < TQ_MAX_STAGES; s++) {
+            mbar_init(smem_u32(&sh->full_a[s]), 1); mbar_init(smem_u32(&sh->empty_a[s]), BITS == 8 ? 1 : TW);
+            mbar_init(smem_u32(&sh->full_b[s]), 1); mbar_init(smem_u32(&sh->empty_b[s]), 1);
+        }
+        for (int s = 0; s < 4; s++) { mbar_init(smem_u32(&sh->full_t[s]), TW); mbar_init(smem_u32(&sh->empty_t[s]), 1); }
+        mbar_init(smem_u32(&sh->full_acc), 1); mbar_init(smem_u32(&sh->empty_acc), TQ_WORKERS); mbar_init(smem_u32(&sh->drained), 1);
+        sh->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+
+    auto tensor_of = [&](int run, int& ti, int& row0) {
+        ti = 0;
+#pragma unroll
+        for (int i = 1; i < 4; i++) if (i < p.n_tensors && run >= p.run_start[i]) ti = i;
+        row0 = (run - p.run_start[ti]) * p.R;
+    };
+
+    // weights: the ring fills at once, before tensor memory is there and before the kernel ahead has ended
+    if (warp == TQ_A_WARP) {
+        if (lane == 0) {
+            int s = 0; uint32_t ph = 1;                         // a fresh ring is free
+            bool ok = true;
+            for (int run = cl; run < nruns && ok; run += ncl) {
+                int ti, row0;
+                tensor_of(run, ti, row0);
+                for (int kb = k0; kb < k1; kb++) {
+                    ok = mbar_wait(smem_u32(&sh->empty_a[s]), ph, abort_flag, 1);
+                    if (!ok) break;
+                    mbar_expect_tx(smem_u32(&sh->full_a[s]), (uint32_t)p.R * (BITS == 8 ? 128u : 64u));
+                    tma_load_2d(smem_u32(ringA + (size_t)s * p.a_stage), &maps.m[ti], kb * (BITS == 8 ? 128 : 64), row0, smem_u32(&sh->full_a[s]));
+                    if (++s == p.sa) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (warp == TQ_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)p.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    // everyone but the weight warp, which is still filling its ring, needs the tensor-memory address
+    if (warp != TQ_A_WARP) asm volatile("bar.sync 1, %0;" :: "n"(TQ_THREADS - 32) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = warp == TQ_A_WARP ? 0u : sh->tmem_base;
+    const uint32_t tmem_a = tmem_base + (uint32_t)(T * p.NC);                          // INT4: NT blocks of T x 32 columns
+
+    if (warp == TQ_B_WARP) {
+        pdl_wait();
+        if (lane == 0) {
+            int s = 0; uint32_t ph = 1;
+            bool ok = true;
+            for (int run = cl; run < nruns && ok; run += ncl)
+                for (int kb = k0; kb < k1; kb++) {
+                    ok = mbar_wait(smem_u32(&sh->empty_b[s]), ph, abort_flag, 2);
+                    if (!ok) break;
+                    mbar_expect_tx(smem_u32(&sh->full_b[s]), (uint32_t)b_stage);
+                    bulk_load(smem_u32(ringB + (size_t)s * b_stage), p.xtiles + (size_t)kb * b_stage, (uint32_t)b_stage, smem_u32(&sh->full_b[s]));
+                    if (++s == p.sb) { s = 0; ph ^= 1; }
+                }
+        }
+        __syncwarp();
+    } else if (warp == TQ_MMA_WARP) {
+        if (lane == 0) {
+            // s32 accumulators; A unsigned bytes for widened nibbles, signed for INT8; B signed digits
+            const uint32_t idesc = (2u << 4) | ((BITS == 8 ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(p.NC >> 3) << 17) | (8u << 24);
+            int sA = 0, sB = 0, sT = 0;
+            uint32_t phA = 0, phB = 0, phT = 0;
+            bool ok = true;
+            int j = 0;
+            for (int run = cl; run < nruns && ok; run += ncl, j++) {
+                ok = mbar_wait(smem_u32(&sh->empty_acc), (uint32_t)((j & 1) ^ 1), abort_flag, 3);
+                for (int kb = k0; kb < k1 && ok; kb++) {
+                    ok = mbar_wait(smem_u32(&sh->full_b[sB]), phB, abort_flag, 4) &&
+                         (BITS == 8 ? mbar_wait(smem_u32(&sh->full_a[sA]), phA, abort_flag, 5) : mbar_wait(smem_u32(&sh->full_t[sT]), phT, abort_flag, 6));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t b0 = smem_u32(ringB + (size_t)sB * b_stage), a0 = smem_u32(ringA + (size_t)sA * p.a_stage);
+#pragma unroll
+                    for (int m = 0; m < 4; m++) {
+                        const uint64_t bd = smem_desc_sw128(b0 + m * 32);
+#pragma unroll
+                        for (int tt = 0; tt < T; tt++) {
+                            const uint32_t d = tmem_base + (uint32_t)(tt * p.NC);
+                            if (BITS == 8) mma_i8_ss(d, smem_desc_sw128(a0 + tt * 16384 + m * 32), bd, idesc, (kb > k0 || m) ? 1u : 0u);
+                            else mma_i8_ts(d, tmem_a + (uint32_t)((sT * T + tt) * 32 + m * 8), bd, idesc, (kb > k0 || m) ? 1u : 0u);
+                        }
+                    }
+                    mma_commit(smem_u32(&sh->empty_b[sB]));
+                    if (++sB == p.sb) { sB = 0; phB ^= 1; }
+                    if (BITS == 8) { mma_commit(smem_u32(&sh->empty_a[sA])); if (++sA == p.sa) { sA = 0; phA ^= 1; } }
+                    else { mma_commit(smem_u32(&sh->empty_t[sT])); if (++sT == NT) { sT = 0; phT ^= 1; } }
+                }
+                if (ok) mma_commit(smem_u32(&sh->full_acc));
+            }
+            mma_commit(smem_u32(&sh->drained));
+            mbar_wait(smem_u32(&sh->drained), 0u, abort_flag, 7);                      // nothing of this block is left in the tensor pipe
+        }
+        __syncwarp();
+    } else if (warp < TQ_WORKERS) {
+        const int q = warp & 3, h = warp >> 2;                                         // tensor-memory quarter; T == 1: which blocks / activations, T == 2: which tile
+        int s = 0, sT = 0, j = 0;
+        uint32_t phA = 0, phT = 1;
+        bool alive = true, staged = false;
+        for (int run = cl; run < nruns && alive; run += ncl, j++) {
+            int ti, row0;
+            tensor_of(run, ti, row0);
+            const LinTensor& W = p.t[ti];
+            const int rows = min(p.R, W.M - row0);
+            const int rt = T == 1 ? 0 : h;                                              // tile of this warp
+            const int rl = rt * 128 + q * 32 + lane;                                    // this thread's row of the run
+            if (BITS == 4) {
+                const uint32_t rawrow = (uint32_t)rl * 64u, sw = (uint32_t)((rl >> 1) & 3);
+                const bool have = rt * 128 + q * 32 < p.R;                              // the box has rows for this warp
+                for (int kb = k0; kb < k1; kb++) {
+                    if (T == 2 || ((kb - k0) & 1) == h) {
+                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_a[s]), phA, abort_flag, 8))) { alive = false; break; }
+                        uint32_t o[32];
+                        if (have) {
+                            const unsigned char* raw = ringA + (size_t)s * p.a_stage + (rl < p.R ? rawrow : 0u);
+#pragma unroll
+                            for (int c = 0; c < 4; c++) {                              // the 64-byte swizzle: piece c of row r at piece c ^ (r / 2 % 4)
+                                const uint4 v = *reinterpret_cast<const uint4*>(raw + (((uint32_t)c ^ sw) << 4));
+                                const uint32_t w[4] = { v.x, v.y, v.z, v.w };
+#pragma unroll
+                                for (int u = 0; u < 4; u++) { o[c * 8 + 2 * u] = w[u] & 0x0F0F0F0Fu; o[c * 8 + 2 * u + 1] = (w[u] >> 4) & 0x0F0F0F0Fu; }
+                            }
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&sh->empty_a[s]));          // the nibbles are in registers
+                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_t[sT]), phT, abort_flag, 9))) { alive = false; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (have) {
+                            tmem_st32(tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)((sT * T + rt) * 32), o);
+                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        }
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[sT]));
+                    }
+                    if (++s == p.sa) { s = 0; phA ^= 1; }
+                    if (++sT == NT) { sT = 0; phT ^= 1; }
+                }
+                if (!alive) break;
+            }
+            if (!staged) {
+                // what the preparation kernel left: 2^-s and 8 x the digit sum of every activation
+                pdl_wait();
+                if (tid < p.B) {
+                    sh->back[tid] = p.xscale[tid * p.xparts];
+                    long long sum = 0;
+                    if (BITS == 4)
+                        for (int part = 0; part < p.xparts; part++) sum += join_limbs(reinterpret_cast<const uint32_t*>(p.xsum) + ((size_t)tid * p.xparts + part) * LIN_LIMBS);
+                    sh->bias[tid] = 8 * sum;
+                }
+                asm volatile("bar.sync 2, %0;" :: "n"(TQ_WORKERS * 32) : "memory");
+                staged = true;
+            }
+            if (S == 1) {
+                const bool have = rl < rows;
+                const int row = row0 + rl;
+                const float sc = have ? row_scale(W, row) : 0.0f;
+                const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc), (uint32_t)(j & 1), abort_flag, 10))) { alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int g0 = T == 1 ? h : 0, gstep = T == 1 ? 2 : 1;
+                for (int g = g0; g * 4 < p.B; g += gstep) {
+                    uint32_t acc[16];
+                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
+                    float* o = W.out + (size_t)(g * 4) * W.out_stride + row;
+                    float old[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+                    if (W.epilogue == IBCU_EPI_ADD) {
+#pragma unroll
+                        for (int u = 0; u < 4; u++) if (have && g * 4 + u < p.B) old[u] = o[(size_t)u * W.out_stride];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int b = g * 4 + u;
+                        if (b >= p.B || !have) continue;
+                        const long long V = join_limbs(acc + 4 * u) - (BITS == 4 ? sh->bias[b] : 0ll);
+                        const float y = (float)((double)V * (double)sh->back[b]);
+                        const float v = W.epilogue == IBCU_EPI_ADD ? old[u] + y * sc : y * sc;
+                        o[(size_t)u * W.out_stride] = v;
+                        if (p.gp.world) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->empty_acc));                   // the tensor cores may overwrite the accumulators
+            } else {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc), 0u, abort_flag, 10))) { alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+        }
+    }
+    if (S > 1) {
+        // one run per cluster: the parts of the columns meet. Rings are free once every block's MMAs are done; block b mod S takes activation b.
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        const int BL = (p.B + S - 1) / S;                                               // activations per block
+        constexpr int RP = T * 128;
+        int ti, row0;
+        tensor_of(cl, ti, row0);
+        const LinTensor& W = p.t[ti];
+        const int rows = min(p.R, W.M - row0);
+        const uint32_t recv = smem_u32(tq_smem);                                        // [source block][activation][row] int64
+        if (warp < TQ_WORKERS && !*abort_flag) {
+            const int q = warp & 3, h = warp >> 2, rt = T == 1 ? 0 : h, rl = rt * 128 + q * 32 + lane;
+            const int g0 = T == 1 ? h : 0, gstep = T == 1 ? 2 : 1;
+            if (rt * 128 + q * 32 < rows) {
+                for (int g = g0; g * 4 < p.B; g += gstep) {
+                    uint32_t acc[16];
+                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int b = g * 4 + u;
+                        if (b >= p.B) continue;
+                        const uint32_t mine = recv + (uint32_t)(((rank * BL + b / S) * RP + rl) * 8);
+                        uint32_t remote;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(mine), "r"(b % S));
+                        asm volatile("st.shared::cluster.u64 [%0], %1;" :: "r"(remote), "l"(join_limbs(acc + 4 * u)) : "memory");
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp < TQ_WORKERS && !*abort_flag) {
+            const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
+            const long long* rv = reinterpret_cast<const long long*>(tq_smem);
+            const int nb = (p.B - rank + S - 1) / S;
+            for (int e = tid; e < nb * RP; e += TQ_WORKERS * 32) {
+                const int rl = e % RP, bl = e / RP, b = bl * S + rank;
+                if (rl >= rows) continue;
+                const int row = row0 + rl;
+                const float sc = row_scale(W, row);
+                float* o = W.out + (size_t)b * W.out_stride + row;
+                const float old = W.epilogue == IBCU_EPI_ADD ? *o : 0.0f;
+                long long V = BITS == 4 ? -sh->bias[b] : 0ll;
+                for (int k = 0; k < S; k++) V += rv[(size_t)(k * BL + bl) * RP + rl];
+                const float y = (float)((double)V * (double)sh->back[b]);
+                const float v = W.epilogue == IBCU_EPI_ADD ? old + y * sc : y * sc;
+                *o = v;
+                if (p.gp.world) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
+            }
+        }
+    }
+    // ── the end: tensor memory back, a wait that ran out reported ──
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == TQ_MMA_WARP) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
+    }
+    if (tid == 0 && sh->abort_flag) {
+        *p.err = 100 + sh->abort_flag;
+        for (int i = 0; i < 1000; i++) __nanosleep(1000);      // copies still on their way into this block's shared memory land before it goes
+    }
+}
+
+// ── host ──
+using EncodeFn = PFN_cuTensorMapEncodeTiled_v12000;
+EncodeFn encode_fn() {
+    static EncodeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) { cudaGetLastError(); f = nullptr; }
+        return (EncodeFn)f;
+    }();
+    return fn;
+}
+
+template <int BITS, int T>
+int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
+    auto kern = linear_tc_kernel<BITS, T>;
+    static size_t allowed[64];
+    size_t& have = allowed[ctx->device & 63];
+    if (smem > have) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(linear_tc_kernel, smem=%zu): %s", smem, cudaGetErrorString(e));
+        have = smem;
+    }
+    return ibcu_launch(ctx, kern, dim3(grid), dim3(TQ_THREADS), smem, p.S, true, maps, p);
+}
+
+}  // namespace
+
+// The call as the preparation kernel and the tcgen05 kernel. Returns IBCU_ERR_STATE without touching the context's error when
+// the call is not its own (the caller takes the other kernels).
+int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, const float* x, int N, int B, int bits, const ibcu_prologue_t* pro, int op) {
+    EncodeFn encode = encode_fn();
+    const int rowbytes = bits == 8 ? N : N / 2;
+    if (!encode || rowbytes % 16 || B > TQ_MAX_B) return IBCU_ERR_STATE;
+    long total_rows = 0;
+    for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
+    if (total_rows == 0) return IBCU_OK;
+    TqParams p;
+    memset(&p, 0, sizeof p);
+    p.n_tensors = n_tensors; p.B = B; p.nkb = (N + 127) / 128;
+    p.NC = (B * LIN_LIMBS + 15) / 16 * 16;
+    // Columns over S blocks of a cluster: enough rows per block that the digits every block fetches stay few against the
+    // weights, and no more than 256 of them.
+    int S = 1;
+    const int slots_of[4] = { ctx->sm_count, ctx->sm_count / 2, ctx->sm_count * 9 / 40, ctx->sm_count / 9 };
+    int lg = 0;
+    while (lg < 3 && total_rows / slots_of[lg] < 80 && p.nkb >= (4 << lg)) lg++;
+    while (lg > 0 && (p.nkb < (1 << lg) || total_rows > 256L * slots_of[lg])) lg--;
+    S = 1 << lg;
+    const int slots = slots_of[lg];
+    int R = (int)((total_rows + slots - 1) / slots);
+    if (R > 256) R = 256;
+    R = (R + 7) & ~7;
+    for (; R < 256; R += 8) {
+        int n = 0;
+        for (int i = 0; i < n_tensors; i++) n += (tensors[i].M + R - 1) / R;
+        if (n <= slots) break;
+    }
+    const int T = R > 128 ? 2 : 1;
+    p.R = R; p.S = S;
+    int nruns = 0;
+    for (int i = 0, row = 0; i < n_tensors; i++) {
+        p.t[i] = { (const uint8_t*)tensors[i].w, tensors[i].scales, tensors[i].out, tensors[i].M,
+                   tensors[i].out_stride, tensors[i].scales_fp32, tensors[i].epilogue, row, 0, 0, -1 };
+        p.run_start[i] = nruns;
+        nruns += (tensors[i].M + R - 1) / R;
+        row += tensors[i].M;
+    }
+    for (int i = n_tensors; i <= 4; i++) p.run_start[i] = nruns;
+    if (S > 1 && nruns > slots) return IBCU_ERR_STATE;
+    // shared memory: half an SM's for runs of one tile, so that consecutive launches overlap; tensor memory likewise
+    const int tcols = T * p.NC + (bits == 4 ? 128 : 0);
+    p.tmem_cols = 32;
+    while (p.tmem_cols < tcols) p.tmem_cols *= 2;
+    const size_t cap = (T == 1 ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
+    const size_t b_stage = (size_t)p.NC * 128;
+    p.a_stage = R * (bits == 8 ? 128 : 64);
+    const int nk = (p.nkb + S - 1) / S;
+    p.sb = T == 1 ? (p.NC > 96 ? 3 : 4) : 4;
+    if (p.sb > nk) p.sb = nk;
+    const int sa = (int)((cap - p.sb * b_stage - (bits == 8 ? 16384 : 0)) / p.a_stage);
+    p.sa = sa > TQ_MAX_STAGES ? TQ_MAX_STAGES : sa;
+    if (p.sa > nk && nruns <= slots) p.sa = nk;
+    auto ring_of = [&]() {
+        size_t r = (((size_t)p.sa * p.a_stage + 1023) & ~(size_t)1023) + (size_t)p.sb * b_stage;
+        if (bits == 8 && r < (size_t)p.sa * p.a_stage + T * 16384) r = (size_t)p.sa * p.a_stage + T * 16384;
+        return r;
+    };
+    const size_t recv = S > 1 ? (size_t)S * ((B + S - 1) / S) * T * 128 * 8 : 0;
+    while (p.sa < TQ_MAX_STAGES && recv > ring_of()) p.sa++;                             // few digits and a short ring: the meeting place needs the room
+    if (recv > ring_of() || p.sa < 1) return IBCU_ERR_STATE;
+    const size_t smem = ((ring_of() + 15) & ~(size_t)15) + sizeof(TqShared);
+    TqMaps maps;
+    memset(&maps, 0, sizeof maps);
+    for (int i = 0; i < n_tensors; i++) {
+        if (tensors[i].M == 0) continue;
+        const cuuint64_t dims[2] = { (cuuint64_t)rowbytes, (cuuint64_t)tensors[i].M };
+        const cuuint64_t strides[1] = { (cuuint64_t)rowbytes };
+        const cuuint32_t box[2] = { bits == 8 ? 128u : 64u, (cuuint32_t)R }, es[2] = { 1, 1 };
+        if (encode(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(tensors[i].w), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return IBCU_ERR_STATE;
+    }
+    GatherWait gw;
+    ibcu_take_gather_wait_x(ctx, &gw, x, (size_t)B * N * sizeof(float));
+    if (pro && pro->x2) ibcu_gather_wait_mark(ctx, &gw, pro->x2, (size_t)B * N * sizeof(float));
+    ibcu_gather_wait_settle(ctx, &gw);
+    {
+        float* outs[4];
+        for (int i = 0; i < n_tensors; i++) outs[i] = tensors[i].out;
+        if (ibcu_push_match(ctx, outs, n_tensors)) {
+            size_t bytes = 0;
+            for (int i = 0; i < n_tensors; i++) bytes += (size_t)tensors[i].M * B * sizeof(float);
+            ibcu_push_fill(ctx, &p.gp, bytes);
+            for (int i = 0; i < n_tensors; i++) p.t[i].win_off = (long)((const char*)tensors[i].out - ctx->win_base);
+        }
+    }
+    // the digits: a block per activation, or several when the maximum is known
+    int parts = 1;
+    if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
+    const int part_kb = (p.nkb + parts - 1) / parts;
+    parts = (p.nkb + part_kb - 1) / part_kb;
+    p.xparts = parts;
+    const size_t tiles = (size_t)p.nkb * b_stage, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
+    int rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, tiles + scales + (size_t)B * parts * LIN_LIMBS * sizeof(int));
+    if (rc) return rc;
+    int8_t* xtiles = (int8_t*)ctx->xpack;
+    float* xscale = (float*)((char*)ctx->xpack + tiles);
+    int* xsum = (int*)((char*)ctx->xpack + tiles + scales);
+    p.xtiles = xtiles; p.xscale = xscale; p.xsum = xsum; p.err = ctx->kern_err;
+    const XSource xsrc = { x, pro ? pro->x2 : nullptr, pro ? (const __half*)pro->norm_w : nullptr, pro ? pro->eps : 0.0f, op,
+                           op == IBCU_PRO_KNOWN_MAX ? pro->amax : nullptr, op == IBCU_PRO_KNOWN_MAX ? pro->n_amax : 0 };
+    const dim3 xg(parts, B);
+    const int perm8 = bits == 4 ? 1 : 0, cols = part_kb * 128, all = p.nkb * 128;
+    rc = cols > 2048 ? ibcu_launch(ctx, xprep_tc_kernel<512>, xg, dim3(512), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw)
+                     : ibcu_launch(ctx, xprep_tc_kernel<256>, xg, dim3(256), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
+    if (rc) return rc;
+    const int grid = S * (nruns < slots ? nruns : slots);
+    if (bits == 8) return T == 1 ? launch_tc<8, 1>(ctx, maps, p, grid, smem) : launch_tc<8, 2>(ctx, maps, p, grid, smem);
+    return T == 1 ? launch_tc<4, 1>(ctx, maps, p, grid, smem) : launch_tc<4, 2>(ctx, maps, p, grid, smem);
+}

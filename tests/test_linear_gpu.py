@@ -70,6 +70,31 @@ def test_batched_tcgen05_path(backend, cpu_libs, bits, M, N, B):
 
 
 @pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("M,N,B", [
+    (1, 128, 5), (8, 96, 32),           # one row; a single block of columns, partly filled
+    (129, 160, 32), (257, 2080, 31),    # one row more than a tile; columns that end inside a block of 128
+    (37889, 256, 6), (40001, 128, 32),  # one row more than one pass of 256-row runs over all SMs: a block walks a second run
+    (4096, 4096, 1), (1024, 14336, 17), # one activation; a cluster of eight blocks per run
+])
+def test_tcgen05_linear_edges(backend, cpu_libs, bits, M, N, B):
+    """Edges of the tcgen05 kernel's tiles, runs and column parts against the product in double precision. Bound: an activation
+    is rounded to half a unit of 2^-29 of its largest magnitude or finer, all sums are exact, the result is rounded to FP32
+    twice (before and after the row scale). (The scalar FP32 restatement's own running sum is off by more at 14336 columns.)"""
+    rng = np.random.default_rng(bits + M + N + B)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    backend.lib.ibcu_linear_use_tcgen05(backend.ctx, 2)
+    try:
+        got = backend.linear(w, s16, x, bits)
+    finally:
+        backend.lib.ibcu_linear_use_tcgen05(backend.ctx, 0)
+    v = w.astype(np.float64) if bits == 8 else np.stack([w & 15, w >> 4], axis=-1).reshape(M, N).astype(np.float64) - 8
+    sc = s16.view(np.float16).astype(np.float64)
+    want = (x.astype(np.float64) @ v.T) * sc
+    bound = 2.0 ** -22 * np.abs(want) + 2.0 ** -30 * np.abs(x).max(axis=1, keepdims=True).astype(np.float64) * (np.abs(v).sum(axis=1) * sc)
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("M,N,B", [(40, 66, 2), (9, 30, 1), (257, 1000, 3), (64, 4096, 4)])
 def test_portable_kernel(backend, cpu_libs, bits, M, N, B):
     """Shapes the tensor-core path does not take (row bytes not a multiple of 16) and the forced
