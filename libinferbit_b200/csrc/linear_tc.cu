@@ -13,6 +13,9 @@
 // All digit sums are exact int32, recombined to one int64 per (row, activation); the S parts of a run meet in the blocks'
 // shared memory (distributed shared memory, every block finishes the activations b = rank mod S), are added as integers and
 // converted once: the result does not depend on S or on how the rows are dealt.
+// No warp polls a barrier while it would have to poll until the kernel ahead has ended: everyone sleeps in the dependency wait.
+// (When the warps of weights and MMAs polled their barriers meanwhile, with suspended tries, the end of the kernel ahead was in
+// rare cases - once in tens of thousands of launches - not delivered until they gave up.)
 //   warps 0-7: INT4 widening, then epilogue    warp 8: weights (TMA)    warp 9: digits (bulk copies)    warp 10: MMA issue
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait. With at most 128 rows per run a
 // block takes no more than half of an SM's shared memory and tensor memory, so that the next launch's blocks move in beside it
@@ -28,7 +31,7 @@ void ibcu_push_fill(ibcu_ctx* ctx, GatherPush* gp, size_t bytes);
 namespace {
 
 constexpr int TQ_WORKERS = 8, TQ_A_WARP = 8, TQ_B_WARP = 9, TQ_MMA_WARP = 10, TQ_THREADS = 11 * 32;
-constexpr int TQ_MAX_STAGES = 8;
+constexpr int TQ_MAX_STAGES = 12;
 constexpr int TQ_MAX_B = 32;
 
 struct alignas(64) TqMaps { CUtensorMap m[4]; };
@@ -37,7 +40,9 @@ struct TqParams {
     LinTensor t[4];
     int n_tensors, run_start[5];               // runs of tensor i are [run_start[i], run_start[i + 1])
     int R, NC, B, nkb, S;                      // rows per run (a multiple of 8), MMA columns, activations, 128-column blocks per row, cluster size
-    int sa, sb, a_stage;                       // ring depths, bytes of a weight stage
+    int sa, sb, a_stage;                       // ring depths (weights; digits), bytes of a weight stage (one block of columns)
+    int gb;                                    // blocks of columns per digit stage
+    int recv_off;                              // where the parts of a run meet in shared memory; 0: in the rings, once they are free
     int tmem_cols, xparts;
     const int8_t* xtiles;                      // digit image [nkb][NC][128]
     const float* xscale;                       // [B][xparts], equal over the parts
@@ -47,9 +52,9 @@ struct TqParams {
 };
 
 struct TqShared {
-    unsigned long long full_a[TQ_MAX_STAGES], empty_a[TQ_MAX_STAGES];    // TMA -> MMA or widening warps, and back
-    unsigned long long full_b[TQ_MAX_STAGES], empty_b[TQ_MAX_STAGES];
-    unsigned long long full_t[4], empty_t[4];                            // INT4: widened blocks in tensor memory
+    unsigned long long full_a[TQ_MAX_STAGES], empty_a[TQ_MAX_STAGES];    // weights -> MMA (INT8) or widening warps (INT4), and back
+    unsigned long long full_b[TQ_MAX_STAGES], empty_b[TQ_MAX_STAGES];    // digits -> MMA, and back
+    unsigned long long full_t[4], empty_t[4];                            // INT4: widened blocks in tensor memory -> MMA, and back
     unsigned long long full_acc, empty_acc, drained;
     uint32_t tmem_base;
     int abort_flag;
@@ -73,13 +78,13 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
 }
 __device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                 :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
@@ -90,6 +95,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
                     "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
                     "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
                  "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
@@ -97,6 +108,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr) : "memory");
+}
+// One lane of a converged warp, chosen so that the compiler knows the branch is warp-uniform: tcgen05 and TMA instructions
+// take their operands from uniform registers, and behind a plain lane == 0 every one of them pays moves and a vote (measured:
+// four MMAs of 128 x 64 x 32 and a commit 378 cycles against 193).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -126,33 +145,38 @@ __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, i
 template <int BITS, int T>
 __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
     extern __shared__ __align__(1024) unsigned char tq_smem[];
-    constexpr int NT = T == 1 ? 4 : 2;                         // widened blocks in tensor memory
-    constexpr int TW = T == 1 ? 4 : 8;                         // worker warps that share a widened block
+    constexpr int NT = 4;                                      // INT4: widened blocks in tensor memory
+    constexpr int TW = TQ_WORKERS;                             // worker warps that share a widened block: one tile, half of every row's columns each; two tiles, one each
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = p.S, rank = (int)blockIdx.x % S, cl = (int)blockIdx.x / S, ncl = (int)gridDim.x / S;
     const int nruns = p.run_start[p.n_tensors];
     const int k0 = (int)((long)p.nkb * rank / S), k1 = (int)((long)p.nkb * (rank + 1) / S);
     unsigned char* ringA = tq_smem;
     unsigned char* ringB = tq_smem + (((size_t)p.sa * p.a_stage + 1023) & ~(size_t)1023);
-    const int b_stage = p.NC * 128;
+    const int b_block = p.NC * 128, b_stage = p.gb * b_block;
     size_t ring_bytes = (size_t)(ringB - tq_smem) + (size_t)p.sb * b_stage;
     if (BITS == 8 && ring_bytes < (size_t)p.sa * p.a_stage + T * 16384) ring_bytes = (size_t)p.sa * p.a_stage + T * 16384;   // an MMA reads 128 rows whatever the run has
+    if (p.recv_off) ring_bytes = p.recv_off + (size_t)S * ((p.B + S - 1) / S) * T * 1024;
     TqShared* sh = reinterpret_cast<TqShared*>(tq_smem + ((ring_bytes + 15) & ~(size_t)15));
     volatile int* abort_flag = &sh->abort_flag;
-    pdl_launch_dependents();
 
     if (tid == 0) {
         for (int s = 0; s < TQ_MAX_STAGES; s++) {
             mbar_init(smem_u32(&sh->full_a[s]), 1); mbar_init(smem_u32(&sh->empty_a[s]), BITS == 8 ? 1 : TW);
             mbar_init(smem_u32(&sh->full_b[s]), 1); mbar_init(smem_u32(&sh->empty_b[s]), 1);
         }
-        for (int s = 0; s < 4; s++) { mbar_init(smem_u32(&sh->full_t[s]), TW); mbar_init(smem_u32(&sh->empty_t[s]), 1); }
+        for (int s = 0; s < NT; s++) { mbar_init(smem_u32(&sh->full_t[s]), TW); mbar_init(smem_u32(&sh->empty_t[s]), 1); }
         mbar_init(smem_u32(&sh->full_acc), 1); mbar_init(smem_u32(&sh->empty_acc), TQ_WORKERS); mbar_init(smem_u32(&sh->drained), 1);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (S > 1) cluster_arrive();                               // waited for before the first store into a peer's shared memory: by then every block has started
 
+    // Blocks of a launch start at different blocks of columns: all of them read the same digits, fresh from the preparation
+    // kernel, and reading the same lines at the same moment they queue for them. (Integer sums: the order is free.)
+    const int nk = k1 - k0, rot = nk % p.gb == 0 ? (cl * p.gb) % nk : 0;
+    auto column_block = [&](int i) { const int k = i + rot; return k0 + (k < nk ? k : k - nk); };
     auto tensor_of = [&](int run, int& ti, int& row0) {
         ti = 0;
 #pragma unroll
@@ -162,19 +186,26 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
 
     // weights: the ring fills at once, before tensor memory is there and before the kernel ahead has ended
     if (warp == TQ_A_WARP) {
-        if (lane == 0) {
-            int s = 0; uint32_t ph = 1;                         // a fresh ring is free
-            bool ok = true;
-            for (int run = cl; run < nruns && ok; run += ncl) {
-                int ti, row0;
-                tensor_of(run, ti, row0);
-                for (int kb = k0; kb < k1; kb++) {
+        const bool one = elect_one();
+        int s = 0; uint32_t ph = 1;                             // a fresh ring is free
+        bool ok = true;
+        long n = 0;
+        for (int run = cl; run < nruns && ok; run += ncl) {
+            int ti, row0;
+            tensor_of(run, ti, row0);
+            for (int i = 0; i < nk; i++, n++) {
+                const int kb = column_block(i);
+                if (n == p.sa) pdl_wait();                      // see below: nobody polls a barrier while the kernel ahead runs
+                if (one) {
                     ok = mbar_wait(smem_u32(&sh->empty_a[s]), ph, abort_flag, 1);
-                    if (!ok) break;
-                    mbar_expect_tx(smem_u32(&sh->full_a[s]), (uint32_t)p.R * (BITS == 8 ? 128u : 64u));
-                    tma_load_2d(smem_u32(ringA + (size_t)s * p.a_stage), &maps.m[ti], kb * (BITS == 8 ? 128 : 64), row0, smem_u32(&sh->full_a[s]));
-                    if (++s == p.sa) { s = 0; ph ^= 1; }
+                    if (ok) {
+                        mbar_expect_tx(smem_u32(&sh->full_a[s]), (uint32_t)p.R * (BITS == 8 ? 128u : 64u));
+                        tma_load_2d(smem_u32(ringA + (size_t)s * p.a_stage), &maps.m[ti], kb * (BITS == 8 ? 128 : 64), row0, smem_u32(&sh->full_a[s]));
+                    }
                 }
+                ok = __any_sync(0xffffffffu, one && ok);
+                if (!ok) break;
+                if (++s == p.sa) { s = 0; ph ^= 1; }
             }
         }
         __syncwarp();
@@ -182,6 +213,9 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
     if (warp == TQ_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)p.tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        // Only now may the launches behind this one start: their blocks allocate tensor memory too and keep it until this launch
+        // has ended, so every block of this launch must hold its own first.
+        pdl_launch_dependents();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     // everyone but the weight warp, which is still filling its ring, needs the tensor-memory address
@@ -192,49 +226,58 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
 
     if (warp == TQ_B_WARP) {
         pdl_wait();
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0; uint32_t ph = 1;
             bool ok = true;
             for (int run = cl; run < nruns && ok; run += ncl)
-                for (int kb = k0; kb < k1; kb++) {
+                for (int i = 0; i < nk; i += p.gb) {
+                    const int kb = column_block(i);
                     ok = mbar_wait(smem_u32(&sh->empty_b[s]), ph, abort_flag, 2);
                     if (!ok) break;
-                    mbar_expect_tx(smem_u32(&sh->full_b[s]), (uint32_t)b_stage);
-                    bulk_load(smem_u32(ringB + (size_t)s * b_stage), p.xtiles + (size_t)kb * b_stage, (uint32_t)b_stage, smem_u32(&sh->full_b[s]));
+                    const uint32_t bytes = (uint32_t)(min(p.gb, nk - i) * b_block);
+                    mbar_expect_tx(smem_u32(&sh->full_b[s]), bytes);
+                    bulk_load(smem_u32(ringB + (size_t)s * b_stage), p.xtiles + (size_t)kb * b_block, bytes, smem_u32(&sh->full_b[s]));
                     if (++s == p.sb) { s = 0; ph ^= 1; }
                 }
         }
         __syncwarp();
     } else if (warp == TQ_MMA_WARP) {
-        if (lane == 0) {
+        pdl_wait();
+        if (elect_one()) {
             // s32 accumulators; A unsigned bytes for widened nibbles, signed for INT8; B signed digits
             const uint32_t idesc = (2u << 4) | ((BITS == 8 ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(p.NC >> 3) << 17) | (8u << 24);
-            int sA = 0, sB = 0, sT = 0;
-            uint32_t phA = 0, phB = 0, phT = 0;
+            const uint32_t ra = smem_u32(ringA), rb = smem_u32(ringB);
+            const int na = BITS == 8 ? p.sa : NT;                                       // weight stages, or widened blocks
+            unsigned long long* full_a = BITS == 8 ? sh->full_a : sh->full_t;
+            unsigned long long* empty_a = BITS == 8 ? sh->empty_a : sh->empty_t;
+            int sa = 0, sb = 0, j = 0;
+            uint32_t pha = 0, phb = 0;
             bool ok = true;
-            int j = 0;
             for (int run = cl; run < nruns && ok; run += ncl, j++) {
                 ok = mbar_wait(smem_u32(&sh->empty_acc), (uint32_t)((j & 1) ^ 1), abort_flag, 3);
-                for (int kb = k0; kb < k1 && ok; kb++) {
-                    ok = mbar_wait(smem_u32(&sh->full_b[sB]), phB, abort_flag, 4) &&
-                         (BITS == 8 ? mbar_wait(smem_u32(&sh->full_a[sA]), phA, abort_flag, 5) : mbar_wait(smem_u32(&sh->full_t[sT]), phT, abort_flag, 6));
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t b0 = smem_u32(ringB + (size_t)sB * b_stage), a0 = smem_u32(ringA + (size_t)sA * p.a_stage);
+                for (int i = 0; i < nk && ok;) {
+                    ok = mbar_wait(smem_u32(&sh->full_b[sb]), phb, abort_flag, 4);
+                    const int ie = min(i + p.gb, nk);
+                    uint64_t bd = smem_desc_sw128(rb + (uint32_t)(sb * b_stage));
+                    for (; i < ie && ok; i++, bd += (uint64_t)(b_block >> 4)) {
+                        ok = mbar_wait(smem_u32(&full_a[sa]), pha, abort_flag, 5);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t ad = smem_desc_sw128(ra + (uint32_t)(sa * p.a_stage));
 #pragma unroll
-                    for (int m = 0; m < 4; m++) {
-                        const uint64_t bd = smem_desc_sw128(b0 + m * 32);
+                        for (int m = 0; m < 4; m++) {                                  // 32 columns each: descriptors count 16-byte units
 #pragma unroll
-                        for (int tt = 0; tt < T; tt++) {
-                            const uint32_t d = tmem_base + (uint32_t)(tt * p.NC);
-                            if (BITS == 8) mma_i8_ss(d, smem_desc_sw128(a0 + tt * 16384 + m * 32), bd, idesc, (kb > k0 || m) ? 1u : 0u);
-                            else mma_i8_ts(d, tmem_a + (uint32_t)((sT * T + tt) * 32 + m * 8), bd, idesc, (kb > k0 || m) ? 1u : 0u);
+                            for (int tt = 0; tt < T; tt++) {
+                                const uint32_t d = tmem_base + (uint32_t)(tt * p.NC);
+                                if (BITS == 8) mma_i8_ss(d, ad + tt * 1024 + m * 2, bd + m * 2, idesc, (i | m) ? 1u : 0u);
+                                else mma_i8_ts(d, tmem_a + (uint32_t)((sa * T + tt) * 32 + m * 8), bd + m * 2, idesc, (i | m) ? 1u : 0u);
+                            }
                         }
+                        mma_commit(smem_u32(&empty_a[sa]));
+                        if (++sa == na) { sa = 0; pha ^= 1; }
                     }
-                    mma_commit(smem_u32(&sh->empty_b[sB]));
-                    if (++sB == p.sb) { sB = 0; phB ^= 1; }
-                    if (BITS == 8) { mma_commit(smem_u32(&sh->empty_a[sA])); if (++sA == p.sa) { sA = 0; phA ^= 1; } }
-                    else { mma_commit(smem_u32(&sh->empty_t[sT])); if (++sT == NT) { sT = 0; phT ^= 1; } }
+                    if (ok) mma_commit(smem_u32(&sh->empty_b[sb]));
+                    if (++sb == p.sb) { sb = 0; phb ^= 1; }
                 }
                 if (ok) mma_commit(smem_u32(&sh->full_acc));
             }
@@ -243,7 +286,7 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
         }
         __syncwarp();
     } else if (warp < TQ_WORKERS) {
-        const int q = warp & 3, h = warp >> 2;                                         // tensor-memory quarter; T == 1: which blocks / activations, T == 2: which tile
+        const int q = warp & 3, h = warp >> 2;                                         // tensor-memory quarter; T == 1: which half of the columns / activations, T == 2: which tile
         int s = 0, sT = 0, j = 0;
         uint32_t phA = 0, phT = 1;
         bool alive = true, staged = false;
@@ -258,31 +301,32 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
                 const uint32_t rawrow = (uint32_t)rl * 64u, sw = (uint32_t)((rl >> 1) & 3);
                 const bool have = rt * 128 + q * 32 < p.R;                              // the box has rows for this warp
                 for (int kb = k0; kb < k1; kb++) {
-                    if (T == 2 || ((kb - k0) & 1) == h) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_a[s]), phA, abort_flag, 8))) { alive = false; break; }
-                        uint32_t o[32];
-                        if (have) {
-                            const unsigned char* raw = ringA + (size_t)s * p.a_stage + (rl < p.R ? rawrow : 0u);
+                    if (kb == k0 + NT && !staged) pdl_wait();                           // the first widened blocks do not need the digits; the next wait for them to be used
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_a[s]), phA, abort_flag, 8))) { alive = false; break; }
+                    constexpr int NP = T == 1 ? 2 : 4;                                  // 16-byte pieces of the row's 64 bytes that this warp widens
+                    uint32_t o[8 * NP];
+                    if (have) {
+                        const unsigned char* raw = ringA + (size_t)s * p.a_stage + (rl < p.R ? rawrow : 0u);
 #pragma unroll
-                            for (int c = 0; c < 4; c++) {                              // the 64-byte swizzle: piece c of row r at piece c ^ (r / 2 % 4)
-                                const uint4 v = *reinterpret_cast<const uint4*>(raw + (((uint32_t)c ^ sw) << 4));
-                                const uint32_t w[4] = { v.x, v.y, v.z, v.w };
+                        for (int c = 0; c < NP; c++) {                                 // the 64-byte swizzle: piece c of row r at piece c ^ (r / 2 % 4)
+                            const uint4 v = *reinterpret_cast<const uint4*>(raw + (((uint32_t)((T == 1 ? 2 * h : 0) + c) ^ sw) << 4));
+                            const uint32_t w[4] = { v.x, v.y, v.z, v.w };
 #pragma unroll
-                                for (int u = 0; u < 4; u++) { o[c * 8 + 2 * u] = w[u] & 0x0F0F0F0Fu; o[c * 8 + 2 * u + 1] = (w[u] >> 4) & 0x0F0F0F0Fu; }
-                            }
+                            for (int u = 0; u < 4; u++) { o[c * 8 + 2 * u] = w[u] & 0x0F0F0F0Fu; o[c * 8 + 2 * u + 1] = (w[u] >> 4) & 0x0F0F0F0Fu; }
                         }
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&sh->empty_a[s]));          // the nibbles are in registers
-                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_t[sT]), phT, abort_flag, 9))) { alive = false; break; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (have) {
-                            tmem_st32(tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)((sT * T + rt) * 32), o);
-                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                        }
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[sT]));
                     }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sh->empty_a[s]));              // the nibbles are in registers
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_t[sT]), phT, abort_flag, 9))) { alive = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (have) {
+                        const uint32_t at = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)((sT * T + rt) * 32);
+                        if constexpr (T == 1) tmem_st16(at + 16 * h, o); else tmem_st32(at, o);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[sT]));
                     if (++s == p.sa) { s = 0; phA ^= 1; }
                     if (++sT == NT) { sT = 0; phT ^= 1; }
                 }
@@ -339,17 +383,18 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
         }
     }
     if (S > 1) {
-        // one run per cluster: the parts of the columns meet. Rings are free once every block's MMAs are done; block b mod S takes activation b.
+        // One run per cluster: the parts of the columns meet; block b mod S takes activation b. A meeting place inside the rings
+        // is free once every block's MMAs are done; one of its own only needs the peers to have started.
         __syncwarp();
-        cluster_arrive();
         cluster_wait();
+        if (!p.recv_off) { cluster_arrive(); cluster_wait(); }
         const int BL = (p.B + S - 1) / S;                                               // activations per block
         constexpr int RP = T * 128;
         int ti, row0;
         tensor_of(cl, ti, row0);
         const LinTensor& W = p.t[ti];
         const int rows = min(p.R, W.M - row0);
-        const uint32_t recv = smem_u32(tq_smem);                                        // [source block][activation][row] int64
+        const uint32_t recv = smem_u32(tq_smem + p.recv_off);                           // [source block][activation][row] int64
         if (warp < TQ_WORKERS && !*abort_flag) {
             const int q = warp & 3, h = warp >> 2, rt = T == 1 ? 0 : h, rl = rt * 128 + q * 32 + lane;
             const int g0 = T == 1 ? h : 0, gstep = T == 1 ? 2 : 1;
@@ -371,24 +416,28 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
         }
         __syncwarp();
         cluster_arrive();
+        // a thread finishes one row; what it needs from memory is under way while the parts arrive
+        const int frl = tid % RP, row = row0 + frl;
+        const bool mine = warp < TQ_WORKERS && frl < rows;
+        const int nb = (p.B - rank + S - 1) / S, bl0 = tid / RP;
+        constexpr int BSTEP = TQ_WORKERS * 32 / RP;
+        const float sc = mine ? row_scale(W, row) : 0.0f;
+        float old = mine && bl0 < nb && W.epilogue == IBCU_EPI_ADD ? W.out[(size_t)(bl0 * S + rank) * W.out_stride + row] : 0.0f;
         cluster_wait();
-        if (warp < TQ_WORKERS && !*abort_flag) {
+        if (mine && !*abort_flag) {
             const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
-            const long long* rv = reinterpret_cast<const long long*>(tq_smem);
-            const int nb = (p.B - rank + S - 1) / S;
-            for (int e = tid; e < nb * RP; e += TQ_WORKERS * 32) {
-                const int rl = e % RP, bl = e / RP, b = bl * S + rank;
-                if (rl >= rows) continue;
-                const int row = row0 + rl;
-                const float sc = row_scale(W, row);
+            const long long* rv = reinterpret_cast<const long long*>(tq_smem + p.recv_off);
+            for (int bl = bl0; bl < nb; bl += BSTEP) {
+                const int b = bl * S + rank;
                 float* o = W.out + (size_t)b * W.out_stride + row;
-                const float old = W.epilogue == IBCU_EPI_ADD ? *o : 0.0f;
+                const float next = bl + BSTEP < nb && W.epilogue == IBCU_EPI_ADD ? W.out[(size_t)((bl + BSTEP) * S + rank) * W.out_stride + row] : 0.0f;
                 long long V = BITS == 4 ? -sh->bias[b] : 0ll;
-                for (int k = 0; k < S; k++) V += rv[(size_t)(k * BL + bl) * RP + rl];
+                for (int k = 0; k < S; k++) V += rv[(size_t)(k * BL + bl) * RP + frl];
                 const float y = (float)((double)V * (double)sh->back[b]);
                 const float v = W.epilogue == IBCU_EPI_ADD ? old + y * sc : y * sc;
                 *o = v;
                 if (p.gp.world) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
+                old = next;
             }
         }
     }
@@ -475,27 +524,45 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     for (int i = n_tensors; i <= 4; i++) p.run_start[i] = nruns;
     if (S > 1 && nruns > slots) return IBCU_ERR_STATE;
     // shared memory: half an SM's for runs of one tile, so that consecutive launches overlap; tensor memory likewise
-    const int tcols = T * p.NC + (bits == 4 ? 128 : 0);
+    const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;
     while (p.tmem_cols < tcols) p.tmem_cols *= 2;
     const size_t cap = (T == 1 ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
-    const size_t b_stage = (size_t)p.NC * 128;
+    const size_t b_block = (size_t)p.NC * 128;
     p.a_stage = R * (bits == 8 ? 128 : 64);
     const int nk = (p.nkb + S - 1) / S;
-    p.sb = T == 1 ? (p.NC > 96 ? 3 : 4) : 4;
-    if (p.sb > nk) p.sb = nk;
-    const int sa = (int)((cap - p.sb * b_stage - (bits == 8 ? 16384 : 0)) / p.a_stage);
-    p.sa = sa > TQ_MAX_STAGES ? TQ_MAX_STAGES : sa;
-    if (p.sa > nk && nruns <= slots) p.sa = nk;
-    auto ring_of = [&]() {
-        size_t r = (((size_t)p.sa * p.a_stage + 1023) & ~(size_t)1023) + (size_t)p.sb * b_stage;
-        if (bits == 8 && r < (size_t)p.sa * p.a_stage + T * 16384) r = (size_t)p.sa * p.a_stage + T * 16384;
-        return r;
-    };
     const size_t recv = S > 1 ? (size_t)S * ((B + S - 1) / S) * T * 128 * 8 : 0;
-    while (p.sa < TQ_MAX_STAGES && recv > ring_of()) p.sa++;                             // few digits and a short ring: the meeting place needs the room
-    if (recv > ring_of() || p.sa < 1) return IBCU_ERR_STATE;
-    const size_t smem = ((ring_of() + 15) & ~(size_t)15) + sizeof(TqShared);
+    const size_t spare = bits == 8 ? 16384 * T : 0;                                      // an MMA reads 128 rows whatever the run has
+    // digit stages of at least 8 KB; the rings share the room in the proportion of what a block of columns takes of each
+    p.gb = p.NC <= 16 ? 4 : (p.NC <= 32 ? 2 : 1);
+    const size_t b_stage = p.gb * b_block;
+    auto plan = [&](long room) {
+        long n = room / (long)(p.a_stage + b_block);                                     // blocks of columns in flight
+        if (n > nk && nruns <= slots) n = nk;
+        p.sb = (int)((n + p.gb - 1) / p.gb);
+        if (p.sb > TQ_MAX_STAGES) p.sb = TQ_MAX_STAGES;
+        if (p.sb < 1) p.sb = 1;
+        n = (room - (long)(p.sb * b_stage)) / p.a_stage;
+        if (n > nk && nruns <= slots) n = nk;
+        p.sa = n > TQ_MAX_STAGES ? TQ_MAX_STAGES : (int)n;
+    };
+    auto ring_of = [&]() {
+        const size_t a = ((size_t)p.sa * p.a_stage + 1023) & ~(size_t)1023, r = a + (size_t)p.sb * b_stage;
+        return spare && r < (size_t)p.sa * p.a_stage + spare ? (size_t)p.sa * p.a_stage + spare : r;
+    };
+    plan((long)cap - (long)recv - 1024);
+    size_t smem;
+    if (recv && p.sa >= (nk < 3 ? nk : 3) && ring_of() + recv + 1024 <= cap) {           // the meeting place beside the rings
+        p.recv_off = (int)((ring_of() + 1023) & ~(size_t)1023);
+        smem = p.recv_off + recv;
+    } else {
+        plan((long)cap);
+        while (p.sa > 1 && ring_of() > cap) p.sa--;
+        while (p.sa < TQ_MAX_STAGES && recv > ring_of()) p.sa++;
+        if (recv > ring_of() || p.sa < 1) return IBCU_ERR_STATE;
+        smem = ring_of();
+    }
+    smem = ((smem + 15) & ~(size_t)15) + sizeof(TqShared);
     TqMaps maps;
     memset(&maps, 0, sizeof maps);
     for (int i = 0; i < n_tensors; i++) {
@@ -527,7 +594,7 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     const int part_kb = (p.nkb + parts - 1) / parts;
     parts = (p.nkb + part_kb - 1) / part_kb;
     p.xparts = parts;
-    const size_t tiles = (size_t)p.nkb * b_stage, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
+    const size_t tiles = (size_t)p.nkb * b_block, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
     int rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, tiles + scales + (size_t)B * parts * LIN_LIMBS * sizeof(int));
     if (rc) return rc;
     int8_t* xtiles = (int8_t*)ctx->xpack;
