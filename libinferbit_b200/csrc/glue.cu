@@ -286,6 +286,173 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
     if (lane == 0) { dst[0] = m_run; dst[1] = l_run; }
 }
 
+// ── split attention for several positions ───────────────────────────────────────────────
+// With four or more positions per call the kernel above repeats too much: every block stages its K and V rows for one
+// position's queries, rotates all new K rows for itself (64 sines per row and head: at 32 positions most of its 45 us), and
+// its two tiles of up to 128 rows leave one block per SM. Here rope_stage_kernel rotates the queries (into scratch) and the
+// new K rows (into the cache, with their V rows) once, the angles of a position shared by all its heads; then
+// attn_batch_kernel walks the cache in double-buffered tiles of 32 rows that serve ATT_QPW positions per warp and
+// 8 / group warps per query head, so a tile row read from shared memory is used ATT_QPW times.
+constexpr int ATT_QPW = 4;           // positions per warp
+constexpr int ATT_TILE = 32;         // cache rows per tile
+
+// `cap` cache positions in at most `want` chunks of whole tiles
+__host__ __device__ __forceinline__ void att_plan_tiles(int cap, int want, int& chunk, int& nsplit) {
+    const int tiles = (cap + ATT_TILE - 1) / ATT_TILE, per = (tiles + want - 1) / want;
+    chunk = per * ATT_TILE;
+    nsplit = (tiles + per - 1) / per;
+}
+
+// grid (B, parts): position pos0 + b, its heads dealt out among the parts
+__global__ void __launch_bounds__(256) rope_stage_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                         float* __restrict__ q_rot, float* __restrict__ k_cache, float* __restrict__ v_cache,
+                                                         int n_heads, int n_kv, int hd, int pos0, const int* pos0_ptr, float theta, const GatherWait gw) {
+    __shared__ float2 cs[128];
+    pdl_launch_dependents();
+    pdl_wait();
+    gather_wait(gw);
+    if (pos0_ptr) pos0 = __ldcg(pos0_ptr);
+    const int b = blockIdx.x, pos = pos0 + b, half = hd / 2, kv_dim = n_kv * hd;
+    for (int m = threadIdx.x; m < half; m += blockDim.x) {
+        const float ang = (float)pos * (1.0f / powf(theta, (float)(2 * m) / (float)hd));
+        cs[m] = make_float2(cosf(ang), sinf(ang));
+    }
+    __syncthreads();
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < (n_heads + n_kv) * half; e += gridDim.y * blockDim.x) {
+        const int h = e / half, m = e - h * half;
+        const bool is_k = h >= n_heads;
+        const float* src = is_k ? k + (size_t)b * kv_dim + (size_t)(h - n_heads) * hd + 2 * m : q + ((size_t)b * n_heads + h) * hd + 2 * m;
+        const float2 a = make_float2(src[0], src[1]);                                       // k may start anywhere
+        const float2 r = make_float2(a.x * cs[m].x - a.y * cs[m].y, a.x * cs[m].y + a.y * cs[m].x);
+        *reinterpret_cast<float2*>(is_k ? k_cache + (size_t)pos * kv_dim + (size_t)(h - n_heads) * hd + 2 * m : q_rot + ((size_t)b * n_heads + h) * hd + 2 * m) = r;
+    }
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < kv_dim; e += gridDim.y * blockDim.x) v_cache[(size_t)pos * kv_dim + e] = v[(size_t)b * kv_dim + e];
+}
+
+// grid (kv heads, chunks, groups of positions), 32 * group * nb threads: warp w serves query head w % group of the KV head and
+// the ATT_QPW positions (blockIdx.z * nb + w / group) * ATT_QPW ..; the cache holds rows 0 .. pos0 + B - 1
+__global__ void __launch_bounds__(256) attn_batch_kernel(const float* q, const float* k_cache, const float* v_cache, float* __restrict__ part,
+                                                         int n_heads, int n_kv, int hd, int B, int nb, int pos0, const int* pos0_ptr, int want, const GatherWait gw) {
+    extern __shared__ __align__(16) float asm_[];
+    const int group = n_heads / n_kv, ld = hd + 4, nwarp = group * nb;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
+    float* qs = asm_;                                    // [warp][ATT_QPW][hd]
+    float* ps = qs + (size_t)nwarp * ATT_QPW * hd;       // [warp][ATT_QPW][32]
+    float* kt = ps + (size_t)nwarp * ATT_QPW * 32;       // [2][ATT_TILE][ld]
+    float* vt = kt + 2 * ATT_TILE * ld;                  // [2][ATT_TILE][ld]
+    pdl_launch_dependents();
+    pdl_wait();
+    gather_wait(gw);
+    if (pos0_ptr) pos0 = __ldcg(pos0_ptr);
+    int chunk, nsplit;
+    att_plan_tiles(pos0 + B, want, chunk, nsplit);
+    const int kvh = blockIdx.x, sp = blockIdx.y, bz = blockIdx.z * nb * ATT_QPW;
+    if (sp >= nsplit) return;
+    const int kv_dim = n_kv * hd, h = kvh * group + warp % group, b0 = bz + (warp / group) * ATT_QPW;
+    const int t0 = sp * chunk, t1 = min(pos0 + min(B, bz + nb * ATT_QPW), t0 + chunk);      // no row beyond this block's last position
+    const int ntile = t1 > t0 ? (t1 - t0 + ATT_TILE - 1) / ATT_TILE : 0;
+    const int per_row = hd / 4;
+    const uint32_t kd = (uint32_t)__cvta_generic_to_shared(kt), vd = (uint32_t)__cvta_generic_to_shared(vt);
+    auto fetch = [&](int i) {
+        if (i < ntile) {
+            const uint32_t off = (uint32_t)((i & 1) * ATT_TILE * ld);
+            for (int e = tid; e < ATT_TILE * per_row; e += nth) {
+                const int r = e / per_row, c = e - r * per_row, t = t0 + i * ATT_TILE + r;
+                const int nbytes = t < t1 ? 16 : 0;                                         // rows past the end read as zeros
+                const size_t go = (size_t)(t < t1 ? t : 0) * kv_dim + (size_t)kvh * hd + 4 * c;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(kd + (off + r * ld + 4 * c) * 4), "l"(k_cache + go), "r"(nbytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(vd + (off + r * ld + 4 * c) * 4), "l"(v_cache + go), "r"(nbytes) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    fetch(1);
+    float* myq = qs + (size_t)warp * ATT_QPW * hd;
+    for (int e = lane; e < ATT_QPW * per_row; e += 32) {
+        const int j = e / per_row, c = e - j * per_row;
+        reinterpret_cast<float4*>(myq)[e] = b0 + j < B ? __ldcg(reinterpret_cast<const float4*>(q + ((size_t)(b0 + j) * n_heads + h) * hd) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float scale = 1.0f / sqrtf((float)hd);
+    const float4* q4 = reinterpret_cast<const float4*>(myq);
+    float* pw = ps + (size_t)warp * ATT_QPW * 32;
+    float m_run[ATT_QPW], l_run[ATT_QPW];
+    float4 acc[ATT_QPW][2];
+#pragma unroll
+    for (int j = 0; j < ATT_QPW; j++) { m_run[j] = -INFINITY; l_run[j] = 0.0f; acc[j][0] = acc[j][1] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    const bool own0 = lane < per_row, own1 = lane + 32 < per_row;
+    for (int i = 0; i < ntile; i++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float4* kr = reinterpret_cast<const float4*>(kt + (size_t)((i & 1) * ATT_TILE + lane) * ld);
+        float4 s[ATT_QPW];
+#pragma unroll
+        for (int j = 0; j < ATT_QPW; j++) s[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int d = 0; d < per_row; d++) {
+            const float4 kk = kr[d];
+#pragma unroll
+            for (int j = 0; j < ATT_QPW; j++) {
+                const float4 qq = q4[j * per_row + d];
+                s[j].x = fmaf(qq.x, kk.x, s[j].x); s[j].y = fmaf(qq.y, kk.y, s[j].y); s[j].z = fmaf(qq.z, kk.z, s[j].z); s[j].w = fmaf(qq.w, kk.w, s[j].w);
+            }
+        }
+        const int t = t0 + i * ATT_TILE + lane;
+#pragma unroll
+        for (int j = 0; j < ATT_QPW; j++) {
+            const bool on = t < t1 && t <= pos0 + b0 + j && b0 + j < B;
+            const float sc = on ? ((s[j].x + s[j].y) + (s[j].z + s[j].w)) * scale : -INFINITY;
+            const float m_new = fmaxf(m_run[j], warp_max(sc));
+            const float e = on ? expf(sc - m_new) : 0.0f;
+            const float corr = m_run[j] == -INFINITY ? 0.0f : expf(m_run[j] - m_new);
+            l_run[j] = l_run[j] * corr + warp_sum(e);
+            m_run[j] = m_new;
+            pw[j * 32 + lane] = e;
+            acc[j][0].x *= corr; acc[j][0].y *= corr; acc[j][0].z *= corr; acc[j][0].w *= corr;
+            acc[j][1].x *= corr; acc[j][1].y *= corr; acc[j][1].z *= corr; acc[j][1].w *= corr;
+        }
+        __syncwarp();
+        const float4* vr = reinterpret_cast<const float4*>(vt + (size_t)(i & 1) * ATT_TILE * ld) + lane;
+        const int ld4 = ld / 4;
+#pragma unroll 2
+        for (int r = 0; r < ATT_TILE; r += 4) {
+            float4 p4[ATT_QPW];
+#pragma unroll
+            for (int j = 0; j < ATT_QPW; j++) p4[j] = *reinterpret_cast<const float4*>(pw + j * 32 + r);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (own0) {
+                    const float4 v = vr[(size_t)(r + u) * ld4];
+#pragma unroll
+                    for (int j = 0; j < ATT_QPW; j++) {
+                        const float pt = u == 0 ? p4[j].x : (u == 1 ? p4[j].y : (u == 2 ? p4[j].z : p4[j].w));
+                        acc[j][0].x = fmaf(pt, v.x, acc[j][0].x); acc[j][0].y = fmaf(pt, v.y, acc[j][0].y); acc[j][0].z = fmaf(pt, v.z, acc[j][0].z); acc[j][0].w = fmaf(pt, v.w, acc[j][0].w);
+                    }
+                }
+                if (own1) {
+                    const float4 v = vr[(size_t)(r + u) * ld4 + 32];
+#pragma unroll
+                    for (int j = 0; j < ATT_QPW; j++) {
+                        const float pt = u == 0 ? p4[j].x : (u == 1 ? p4[j].y : (u == 2 ? p4[j].z : p4[j].w));
+                        acc[j][1].x = fmaf(pt, v.x, acc[j][1].x); acc[j][1].y = fmaf(pt, v.y, acc[j][1].y); acc[j][1].z = fmaf(pt, v.z, acc[j][1].z); acc[j][1].w = fmaf(pt, v.w, acc[j][1].w);
+                    }
+                }
+            }
+        }
+        __syncthreads();                                                                    // the tile's buffer is free
+        fetch(i + 2);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < ATT_QPW; j++) {
+        if (b0 + j >= B) continue;
+        float* dst = part + (((size_t)(b0 + j) * n_heads + h) * gridDim.y + sp) * (size_t)(hd + 4);
+        if (own0) *reinterpret_cast<float4*>(dst + 4 + 4 * lane) = acc[j][0];
+        if (own1) *reinterpret_cast<float4*>(dst + 4 + 4 * (lane + 32)) = acc[j][1];
+        if (lane == 0) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
+    }
+}
+
 // grid (query heads, B): merges the chunk results of one head. All of them are loaded at once, as float4s.
 constexpr int ATT_CMB_V = 8;
 __global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restrict__ part, float* __restrict__ out,
@@ -294,7 +461,11 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restri
     extern __shared__ __align__(16) float cs[];      // the head's chunk results: [nsplit][hd + 4], then weights [nsplit]
     pdl_launch_dependents();
     pdl_wait();
-    if (pos0_ptr) { int chunk; att_plan(__ldcg(pos0_ptr) + (int)gridDim.y, want, chunk_cap, chunk, nsplit); }
+    if (pos0_ptr) {
+        int chunk;
+        if (chunk_cap) att_plan(__ldcg(pos0_ptr) + (int)gridDim.y, want, chunk_cap, chunk, nsplit);
+        else att_plan_tiles(__ldcg(pos0_ptr) + (int)gridDim.y, want, chunk, nsplit);      // chunks of attn_batch_kernel
+    }
     const int h = blockIdx.x, b = blockIdx.y;
     const int pstride = hd + 4, total = nsplit * pstride, total4 = total / 4;
     const float4* src = reinterpret_cast<const float4*>(part + ((size_t)b * n_heads + h) * (size_t)part_rows * pstride);
@@ -429,6 +600,45 @@ static bool attn_split_ok(const float* q, const float* k_cache, const float* v_c
            ((uintptr_t)k_cache & 15) == 0 && ((uintptr_t)v_cache & 15) == 0 && ((uintptr_t)q & 15) == 0;
 }
 
+static int combine_chunks(ibcu_ctx* ctx, float* out, int n_heads, int head_dim, int B, int nsplit, int grid_y, const int* pos0_dev, int want, int chunk_cap) {
+    const size_t csmem = ((size_t)grid_y * (head_dim + 4) + grid_y) * sizeof(float);
+    IBCU_REQUIRE(ctx, csmem <= 200 * 1024, "ibcu_attention: %d chunks of cache positions are more than the merge step holds", grid_y);
+    if (csmem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
+    return ibcu_launch(ctx, attn_combine_kernel, dim3(n_heads, B), dim3(128), csmem, 1, true,
+                       (const float*)ctx->scratch, out, n_heads, head_dim, nsplit, grid_y, pos0_dev, want, chunk_cap);
+}
+
+// The same for four or more positions (see attn_batch_kernel). k NULL: q is rotated and the cache complete.
+static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float* v_cache, float* out, int n_heads, int n_kv_heads, int head_dim,
+                           int pos0, int B, const float* k, const float* v, float theta, const int* pos0_dev, int max_ctx) {
+    const int group = n_heads / n_kv_heads, nb = ATT_GMAX / group, gz = (B + nb * ATT_QPW - 1) / (nb * ATT_QPW);
+    const int cap = pos0_dev ? max_ctx : pos0 + B, tiles = (cap + ATT_TILE - 1) / ATT_TILE;
+    int want = (2 * ctx->sm_count + n_kv_heads * gz - 1) / (n_kv_heads * gz);             // two blocks fit an SM
+    if (want > tiles) want = tiles;
+    int chunk, nsplit;
+    att_plan_tiles(cap, want, chunk, nsplit);
+    const size_t part = ((size_t)B * n_heads * want * (head_dim + 4) * sizeof(float) + 255) & ~(size_t)255;
+    const size_t rot = k ? (size_t)B * n_heads * head_dim * sizeof(float) : 0;
+    int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, part + rot);
+    if (rc) return rc;
+    const size_t smem = ((size_t)group * nb * ATT_QPW * (head_dim + 32) + 4 * (size_t)ATT_TILE * (head_dim + 4)) * sizeof(float);
+    if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GatherWait gw;
+    ibcu_take_gather_wait(ctx, &gw);
+    if (k) {
+        float* q_rot = (float*)((char*)ctx->scratch + part);
+        rc = ibcu_launch(ctx, rope_stage_kernel, dim3(B, 4), dim3(256), 0, 1, true, q, k, v, q_rot, k_cache, v_cache, n_heads, n_kv_heads, head_dim,
+                         pos0, pos0_dev, theta, gw);
+        if (rc) return rc;
+        q = q_rot;
+        memset(&gw, 0, sizeof gw);
+    }
+    rc = ibcu_launch(ctx, attn_batch_kernel, dim3(n_kv_heads, want, gz), dim3(32 * group * nb), smem, 1, true, q, (const float*)k_cache, (const float*)v_cache,
+                     (float*)ctx->scratch, n_heads, n_kv_heads, head_dim, B, nb, pos0, pos0_dev, want, gw);
+    if (rc) return rc;
+    return combine_chunks(ctx, out, n_heads, head_dim, B, nsplit, want, pos0_dev, want, 0);
+}
+
 // k_new / v_new NULL: q is rotated already and the cache holds rows 0..pos0+B-1. Otherwise the fused decode step.
 // pos0_dev NULL: the position is the argument pos0 and the grid is cut for it. Otherwise the position is read
 // on the device and the grid, shared memory and scratch are sized for max_ctx positions, so that one
@@ -436,6 +646,8 @@ static bool attn_split_ok(const float* q, const float* k_cache, const float* v_c
 static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float* v_cache, float* out,
                            int n_heads, int n_kv_heads, int head_dim, int pos0, int B, const float* k_new, const float* v_new, float theta,
                            const int* pos0_dev, int max_ctx) {
+    // four positions fill a warp of the batched kernel; with fewer the fused kernel's two launches are quicker than three
+    if (B >= ATT_QPW) return attention_batch(ctx, q, k_cache, v_cache, out, n_heads, n_kv_heads, head_dim, pos0, B, k_new, v_new, theta, pos0_dev, max_ctx);
     const int group = n_heads / n_kv_heads;
     // Enough blocks to cover the machine several times over: a block's shared memory grows with its chunk of positions (two
     // tiles of chunk x head_dim floats), so short chunks let several blocks share an SM; with B activations every chunk
@@ -468,11 +680,7 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
                      q, (const float*)k_cache, (const float*)v_cache, (float*)ctx->scratch, n_heads, n_kv_heads, head_dim, pos0, chunk, nsplit,
                      k_new, v_new, k_cache, v_cache, theta, pos0_dev, want, chunk_cap, gw);
     if (rc) return rc;
-    const size_t csmem = ((size_t)grid_y * (head_dim + 4) + grid_y) * sizeof(float);
-    IBCU_REQUIRE(ctx, csmem <= 200 * 1024, "ibcu_attention: %d chunks of cache positions are more than the merge step holds", grid_y);
-    if (csmem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
-    return ibcu_launch(ctx, attn_combine_kernel, dim3(n_heads, B), dim3(128), csmem, 1, true,
-                       (const float*)ctx->scratch, out, n_heads, head_dim, nsplit, grid_y, pos0_dev, want, chunk_cap);
+    return combine_chunks(ctx, out, n_heads, head_dim, B, nsplit, grid_y, pos0_dev, want, chunk_cap);
 }
 
 extern "C" int ibcu_attention(ibcu_ctx* ctx, const float* q, const float* k_cache, const float* v_cache, float* out,

@@ -100,6 +100,15 @@ def test_rope_kv_write_and_attention(backend, cpu_libs, n_heads, n_kv, hd, pos0,
     assert _cpu.close(be.download(dout, np.float32, B * H).reshape(B, H), want, RTOL, ATOL)
 
 
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B", [(32, 8, 128, 0, 32), (32, 8, 128, 1000, 31), (8, 8, 64, 31, 4), (6, 2, 40, 33, 5), (8, 1, 256, 100, 9),
+                                                     (10, 2, 64, 0, 7)])
+def test_attention_of_several_positions(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused):
+    """The kernel for four and more positions: groups that do and do not divide eight, positions that end inside a warp's four,
+    tiles that end on and off their 32 rows, heads wider than a warp's float4s."""
+    test_rope_kv_write_and_attention(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused)
+
+
 def test_peer_window_single_rank():
     """The peer-window calls on a one-rank context: create, bump allocation with equal alignment, window
     memory survives ibcu_free, the gather of one rank is a no-op, and a second window is refused. (The
