@@ -148,26 +148,86 @@ int ib_b200_pq_lm_head_topk(const ib_b200_pq_tensor* t, const float* x, int K_to
 }
 
 /* ── k-means ── */
-typedef struct { void *X, *C, *idx, *dist, *sums, *counts, *inertia; int owns_X; } km_bufs;
+/* Device arrays of a call, kept from call to call: a converter trains one codebook after another, and seven allocations
+ * and frees (each waits for the device) took several milliseconds of a call whose kernels take one. What is kept is
+ * bounded by KM_KEEP (larger calls give their arrays back at once), given back by ib_b200_shutdown, and used under the
+ * entries' lock. */
+enum { KM_X, KM_C, KM_IDX, KM_DIST, KM_SUMS, KM_COUNTS, KM_SCALARS, KM_SLOTS };
+#define KM_KEEP ((size_t)256 << 20)
+static struct { void* p; size_t bytes; } g_km[KM_SLOTS];
 
-static void km_free(km_bufs* b) {
-    if (b->owns_X && b->X) ibcu_free(g_ib.ctx, b->X);
-    void* v[] = { b->C, b->idx, b->dist, b->sums, b->counts, b->inertia };
-    for (int i = 0; i < 6; i++) if (v[i]) ibcu_free(g_ib.ctx, v[i]);
+void ib_b200_kmeans_release(void) {
+    for (int i = 0; i < KM_SLOTS; i++) {
+        if (g_km[i].p) ibcu_free(g_ib.ctx, g_km[i].p);
+        g_km[i].p = NULL; g_km[i].bytes = 0;
+    }
+}
+static void km_trim(void) {
+    size_t total = 0;
+    for (int i = 0; i < KM_SLOTS; i++) total += g_km[i].bytes;
+    if (total > KM_KEEP) ib_b200_kmeans_release();
+}
+static int km_get(int slot, size_t bytes, void** p) {
+    if (g_km[slot].bytes < bytes) {
+        if (g_km[slot].p) ibcu_free(g_ib.ctx, g_km[slot].p);
+        g_km[slot].p = NULL; g_km[slot].bytes = 0;
+        int rc = ibcu_malloc(g_ib.ctx, bytes, &g_km[slot].p);
+        if (rc) { g_km[slot].p = NULL; return rc; }
+        g_km[slot].bytes = bytes;
+    }
+    *p = g_km[slot].p;
+    return 0;
 }
 
-static int km_alloc(km_bufs* b, const float* X, int N, int D, int K) {
-    memset(b, 0, sizeof *b);
-    const size_t xb = (size_t)N * D * sizeof(float);
+typedef struct { void *X, *C, *idx, *dist, *sums, *counts, *inertia, *shift; } km_bufs;
+
+/* Pageable arrays go through the pinned staging area in pieces, so that a piece is on its way while the next is copied
+ * (the driver's own path for pageable memory copies and transfers one after the other). The result area is separate. */
+#define KM_PIECE ((size_t)512 << 10)
+#define KM_STAGE ((size_t)16 << 20)
+static int km_upload(void* dst, const void* src, size_t bytes) {
+    void *h, *d;
+    int rc = ib_b200_stage(0, bytes < KM_STAGE ? bytes : KM_STAGE, &h, &d);
+    size_t at = 0;
+    for (size_t off = 0; !rc && off < bytes; off += KM_PIECE) {
+        const size_t n = bytes - off < KM_PIECE ? bytes - off : KM_PIECE;
+        if (at + n > KM_STAGE) { rc = ibcu_sync_spin(g_ib.ctx); at = 0; }
+        memcpy((char*)h + at, (const char*)src + off, n);
+        if (!rc) rc = ibcu_memcpy_h2d(g_ib.ctx, (char*)dst + off, (char*)h + at, n);
+        at += n;
+    }
+    return rc;
+}
+static int km_download(void* dst, const void* src, size_t bytes) {
+    void *h, *d;
+    int rc = ib_b200_stage(2, bytes < KM_STAGE ? bytes : KM_STAGE, &h, &d);
+    for (size_t off = 0; !rc && off < bytes; off += KM_STAGE) {
+        const size_t n = bytes - off < KM_STAGE ? bytes - off : KM_STAGE;
+        rc = ibcu_memcpy_d2h(g_ib.ctx, h, (const char*)src + off, n);
+        if (!rc) rc = ibcu_sync_spin(g_ib.ctx);
+        if (!rc) memcpy((char*)dst + off, h, n);
+    }
+    return rc;
+}
+
+static int km_begin(km_bufs* b, const float* X, int N, int D, int K, const float* centers) {
+    const size_t xb = (size_t)N * D * sizeof(float), cb = (size_t)K * D * sizeof(float);
     b->X = ib_b200_translate(X, xb);
     int rc = 0;
-    if (!b->X) { b->owns_X = 1; rc = ibcu_malloc(g_ib.ctx, xb, &b->X); if (!rc) rc = ibcu_memcpy_h2d(g_ib.ctx, b->X, X, xb); }
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, (size_t)K * D * sizeof(float), &b->C);
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, (size_t)N * sizeof(int32_t), &b->idx);
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, (size_t)N * sizeof(float), &b->dist);
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, (size_t)K * D * sizeof(float), &b->sums);
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, (size_t)K * sizeof(int32_t), &b->counts);
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, 16, &b->inertia);
+    if (!b->X) {
+        rc = km_get(KM_X, xb, &b->X);
+        if (!rc) rc = km_upload(b->X, X, xb);
+    }
+    if (!rc) rc = km_get(KM_C, cb, &b->C);
+    if (!rc) rc = km_get(KM_IDX, (size_t)N * sizeof(int32_t), &b->idx);
+    if (!rc) rc = km_get(KM_DIST, (size_t)N * sizeof(float), &b->dist);
+    if (!rc) rc = km_get(KM_SUMS, cb, &b->sums);
+    if (!rc) rc = km_get(KM_COUNTS, (size_t)K * sizeof(int32_t), &b->counts);
+    if (!rc) rc = km_get(KM_SCALARS, 32, &b->inertia);
+    b->shift = (char*)b->inertia + 16;
+    void *h, *d;
+    if (!rc) rc = ib_b200_stage(3, cb, &h, &d);                   /* not the area the points are still leaving from */
+    if (!rc) { memcpy(h, centers, cb); rc = ibcu_memcpy_h2d(g_ib.ctx, b->C, h, cb); }
     return rc;
 }
 
@@ -176,13 +236,12 @@ static int ib_b200_kmeans_assign_unlocked(const float* X, int N, int D, const fl
     if (!X || !centers || !indices_out || N <= 0 || K <= 0 || D <= 0) return -1;      /* src/pq_kmeans.c:403 */
     if (!g_ib.ctx) { ib_b200_set_error(IBCU_ERR_STATE, "ib_b200_kmeans_assign before ib_b200_init"); return -1; }
     km_bufs b;
-    int rc = km_alloc(&b, X, N, D, K);
-    if (!rc) rc = ibcu_memcpy_h2d(g_ib.ctx, b.C, centers, (size_t)K * D * sizeof(float));
+    int rc = km_begin(&b, X, N, D, K, centers);
     if (!rc) rc = ibcu_kmeans_assign(g_ib.ctx, (const float*)b.X, N, D, (const float*)b.C, K, (int32_t*)b.idx, NULL);
-    if (!rc) rc = ibcu_memcpy_d2h(g_ib.ctx, indices_out, b.idx, (size_t)N * sizeof(int32_t));
-    if (!rc) rc = ibcu_sync(g_ib.ctx);
+    if (!rc) rc = km_download(indices_out, b.idx, (size_t)N * sizeof(int32_t));
+    if (rc) ibcu_sync(g_ib.ctx);                                   /* nothing is left on its way out of the staging areas */
     ib_b200_check(rc, "ib_b200_kmeans_assign");
-    km_free(&b);
+    km_trim();
     return rc ? -1 : 0;
 }
 
@@ -191,36 +250,43 @@ static int ib_b200_kmeans_lloyd_unlocked(const float* X, int N, int D, int K, in
     if (!X || !centers || N <= 0 || K <= 0 || D <= 0 || iters <= 0) return -1;
     if (!g_ib.ctx) { ib_b200_set_error(IBCU_ERR_STATE, "ib_b200_kmeans_lloyd before ib_b200_init"); return -1; }
     km_bufs b;
-    int rc = km_alloc(&b, X, N, D, K), done = 0;
-    void* shift_d = NULL;
-    if (!rc) rc = ibcu_malloc(g_ib.ctx, 16, &shift_d);
-    if (!rc) rc = ibcu_memcpy_h2d(g_ib.ctx, b.C, centers, (size_t)K * D * sizeof(float));
-    double prev = 0.0, inertia = 0.0;
+    int rc = km_begin(&b, X, N, D, K, centers), done = 0;
+    double prev = 0.0;
+    /* a fixed number of iterations needs no scalars on the host between them: whole iterations of the backend (with a
+     * communicator on the context those would add up other ranks' tables, which this call never does) */
+    int rank = 0, world = 1;
+    ibcu_comm_rank(g_ib.ctx, &rank, &world);
+    const int whole = tol < 0.0f && world == 1;
     for (int it = 0; !rc && it < iters; it++) {
+        if (whole) {
+            rc = ibcu_kmeans_lloyd_iter(g_ib.ctx, (const float*)b.X, N, D, (float*)b.C, K, (int32_t*)b.idx, (float*)b.dist,
+                                        (float*)b.sums, (int32_t*)b.counts, (double*)b.inertia);
+            done = it + 1;
+            continue;
+        }
         rc = ibcu_kmeans_assign(g_ib.ctx, (const float*)b.X, N, D, (const float*)b.C, K, (int32_t*)b.idx, (float*)b.dist);
         if (!rc) rc = ibcu_kmeans_accumulate(g_ib.ctx, (const float*)b.X, N, D, K, (const int32_t*)b.idx, (const float*)b.dist,
                                              (float*)b.sums, (int32_t*)b.counts, (double*)b.inertia);
-        if (!rc) rc = ibcu_kmeans_update(g_ib.ctx, (float*)b.C, K, D, (const float*)b.sums, (const int32_t*)b.counts, (float*)shift_d);
+        if (!rc) rc = ibcu_kmeans_update(g_ib.ctx, (float*)b.C, K, D, (const float*)b.sums, (const int32_t*)b.counts, (float*)b.shift);
         done = it + 1;
         if (rc || tol < 0.0f) continue;
         /* the reference's two stopping rules (src/pq_kmeans.c:285-288) need the scalars on the host */
-        float shift = 0.0f;
-        rc = ibcu_memcpy_d2h(g_ib.ctx, &shift, shift_d, sizeof shift);
-        if (!rc) rc = ibcu_memcpy_d2h(g_ib.ctx, &inertia, b.inertia, sizeof inertia);
-        if (!rc) rc = ibcu_sync(g_ib.ctx);
+        char two[32];
+        rc = km_download(two, b.inertia, sizeof two);
         if (rc) break;
+        double inertia; float shift;
+        memcpy(&inertia, two, sizeof inertia); memcpy(&shift, two + 16, sizeof shift);
         if (shift < tol) break;
         double diff = prev - inertia; if (diff < 0) diff = -diff;
         if (it > 0 && diff < (double)tol * (prev + 1e-12)) break;
         prev = inertia;
     }
-    if (!rc) rc = ibcu_memcpy_d2h(g_ib.ctx, centers, b.C, (size_t)K * D * sizeof(float));
-    if (!rc && indices_out) rc = ibcu_memcpy_d2h(g_ib.ctx, indices_out, b.idx, (size_t)N * sizeof(int32_t));
-    if (!rc && inertia_out) rc = ibcu_memcpy_d2h(g_ib.ctx, inertia_out, b.inertia, sizeof(double));
-    if (!rc) rc = ibcu_sync(g_ib.ctx);
+    if (!rc) rc = km_download(centers, b.C, (size_t)K * D * sizeof(float));
+    if (!rc && indices_out) rc = km_download(indices_out, b.idx, (size_t)N * sizeof(int32_t));
+    if (!rc && inertia_out) rc = km_download(inertia_out, b.inertia, sizeof(double));
+    if (rc) ibcu_sync(g_ib.ctx);
     ib_b200_check(rc, "ib_b200_kmeans_lloyd");
-    if (shift_d) ibcu_free(g_ib.ctx, shift_d);
-    km_free(&b);
+    km_trim();
     return rc ? -1 : done;
 }
 

@@ -55,6 +55,7 @@ static void scale_entry_drop(ib_b200_scale_entry* e) {
 void ib_b200_shutdown(void) {
     if (!g_ib.ctx) return;
     ib_b200_pq_release_all();
+    ib_b200_kmeans_release();
     for (int i = 0; i < IB_B200_SCALE_SLOTS; i++) if (g_ib.scales[i].weights) scale_entry_drop(&g_ib.scales[i]);
     for (int i = 0; i < g_ib.n_ranges; i++) ibcu_free(g_ib.ctx, g_ib.ranges[i].dev);
     for (int i = 0; i < IB_B200_NSTAGE; i++) {
