@@ -485,7 +485,15 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
         return IBCU_OK;
     }
 
-    if (ctx->linear_tc > 0 ? (bits == 4 || ctx->linear_tc > 1) : (ctx->linear_tc == 0 && B >= 5)) {
+    // Which kernel, as measured in a chain of launches: the tcgen05 kernel pays a preparation launch (about 2.5 us) and then hardly
+    // notices the activations; this file's kernel costs a second group of columns from the third activation on and is bound
+    // by its own instructions. 4096 x 10240 INT8 (42 MB): 16.4 against 13.2 us at two, 28.3 against 13.8 at four; gate and up
+    // of 14336 x 4096 INT4 (59 MB): 18.9 / 16.5 and 23.4 / 15.9; 6144 x 4096 INT8 (25 MB): 9.5 / 9.7 and 11.3 / 10.0; 4096 x 4096
+    // INT8 (17 MB): 6.5 / 8.4 and 7.6 / 8.7. From five on the tcgen05 kernel wins at any size.
+    size_t weight_bytes = 0;
+    for (int i = 0; i < n_tensors; i++) weight_bytes += (size_t)tensors[i].M * rowbytes;
+    const bool many = B >= 5 || (B >= 3 && weight_bytes >= (20u << 20)) || (B == 2 && weight_bytes >= (32u << 20));
+    if (ctx->linear_tc > 0 ? (bits == 4 || ctx->linear_tc > 1) : (ctx->linear_tc == 0 && many)) {
         const int rc_tc = ibcu_linear_tc(ctx, tensors, n_tensors, x, N, B, bits, pro, op);
         if (rc_tc != IBCU_ERR_STATE) return rc_tc;
     }

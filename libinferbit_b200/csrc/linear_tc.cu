@@ -16,7 +16,11 @@
 // No warp polls a barrier while it would have to poll until the kernel ahead has ended: everyone sleeps in the dependency wait.
 // (When the warps of weights and MMAs polled their barriers meanwhile, with suspended tries, the end of the kernel ahead was in
 // rare cases - once in tens of thousands of launches - not delivered until they gave up.)
-//   warps 0-7: INT4 widening, then epilogue    warp 8: weights (TMA)    warp 9: digits (bulk copies)    warp 10: MMA issue
+// Workers (INT4 widening, then epilogue): eight warps per tile of 128 rows, in two teams that take the blocks of columns in turn;
+// then one warp each for the weights (TMA), the digits (bulk copies) and the MMAs. What a block of columns costs a warp is waits
+// and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
+// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4; at 32 the digits, which every SM reads from L2,
+// bound the kernel (26 us, 75 MB of them).
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait. With at most 128 rows per run a
 // block takes no more than half of an SM's shared memory and tensor memory, so that the next launch's blocks move in beside it
 // and have their weights under way while this launch ends.
@@ -30,7 +34,8 @@ void ibcu_push_fill(ibcu_ctx* ctx, GatherPush* gp, size_t bytes);
 
 namespace {
 
-constexpr int TQ_WORKERS = 8, TQ_A_WARP = 8, TQ_B_WARP = 9, TQ_MMA_WARP = 10, TQ_THREADS = 11 * 32;
+// Warps of a block whose runs have T tiles: 8 T workers, then one each for the weights, the digits and the MMAs.
+template <int T> struct Tq { static constexpr int WORKERS = 8 * T, A_WARP = WORKERS, B_WARP = WORKERS + 1, MMA_WARP = WORKERS + 2, THREADS = (WORKERS + 3) * 32; };
 constexpr int TQ_MAX_STAGES = 12;
 constexpr int TQ_MAX_B = 32;
 
@@ -62,19 +67,9 @@ struct TqShared {
     long long bias[TQ_MAX_B];
 };
 
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory"); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// shared-memory matrix descriptor, K-major with the 128-byte swizzle: 8-row atoms of 1024 bytes follow one another; the K
-// offset inside the 128-byte rows is part of the start address
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 __device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -85,37 +80,6 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
                  :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
-                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                    "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-// One lane of a converged warp, chosen so that the compiler knows the branch is warp-uniform: tcgen05 and TMA instructions
-// take their operands from uniform registers, and behind a plain lane == 0 every one of them pays moves and a vote (measured:
-// four MMAs of 128 x 64 x 32 and a commit 378 cycles against 193).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}" : "=r"(p));
-    return p != 0;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -143,10 +107,13 @@ __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, i
 
 // BITS 4 or 8; T: 128-row tiles per run
 template <int BITS, int T>
-__global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
+__global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
     extern __shared__ __align__(1024) unsigned char tq_smem[];
     constexpr int NT = 4;                                      // INT4: widened blocks in tensor memory
-    constexpr int TW = TQ_WORKERS;                             // worker warps that share a widened block: one tile, half of every row's columns each; two tiles, one each
+    constexpr int TQ_WORKERS = Tq<T>::WORKERS, TQ_A_WARP = Tq<T>::A_WARP, TQ_B_WARP = Tq<T>::B_WARP, TQ_MMA_WARP = Tq<T>::MMA_WARP, TQ_THREADS = Tq<T>::THREADS;
+    // INT4: two teams of workers, a warp per 32 rows, widen alternate blocks of columns. A warp's way from the nibbles to the MMA is
+    // a chain of waits and latencies (about 1300 cycles measured, a few hundred of them work), and two chains run side by side.
+    constexpr int TW = TQ_WORKERS / 2;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = p.S, rank = (int)blockIdx.x % S, cl = (int)blockIdx.x / S, ncl = (int)gridDim.x / S;
     const int nruns = p.run_start[p.n_tensors];
@@ -286,30 +253,28 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
         }
         __syncwarp();
     } else if (warp < TQ_WORKERS) {
-        const int q = warp & 3, h = warp >> 2;                                         // tensor-memory quarter; T == 1: which half of the columns / activations, T == 2: which tile
-        int s = 0, sT = 0, j = 0;
+        const int q = warp & 3, rt = (warp >> 2) % T, team = warp / (4 * T);           // tensor-memory quarter, tile, and which blocks (INT4) / groups of activations
+        int s = team, sT = team, j = 0, next = team;                                   // next: this team's next block of columns, counted from the run's first
         uint32_t phA = 0, phT = 1;
-        bool alive = true, staged = false;
+        bool alive = true, staged = false, waited = false;
         for (int run = cl; run < nruns && alive; run += ncl, j++) {
             int ti, row0;
             tensor_of(run, ti, row0);
             const LinTensor& W = p.t[ti];
             const int rows = min(p.R, W.M - row0);
-            const int rt = T == 1 ? 0 : h;                                              // tile of this warp
             const int rl = rt * 128 + q * 32 + lane;                                    // this thread's row of the run
             if (BITS == 4) {
                 const uint32_t rawrow = (uint32_t)rl * 64u, sw = (uint32_t)((rl >> 1) & 3);
                 const bool have = rt * 128 + q * 32 < p.R;                              // the box has rows for this warp
-                for (int kb = k0; kb < k1; kb++) {
-                    if (kb == k0 + NT && !staged) pdl_wait();                           // the first widened blocks do not need the digits; the next wait for them to be used
+                for (; next < nk; next += 2) {
+                    if (!waited && next >= NT) { pdl_wait(); waited = true; }           // the first widened blocks do not need the digits; the next wait for them to be used
                     if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_a[s]), phA, abort_flag, 8))) { alive = false; break; }
-                    constexpr int NP = T == 1 ? 2 : 4;                                  // 16-byte pieces of the row's 64 bytes that this warp widens
-                    uint32_t o[8 * NP];
+                    uint32_t o[32];
                     if (have) {
                         const unsigned char* raw = ringA + (size_t)s * p.a_stage + (rl < p.R ? rawrow : 0u);
 #pragma unroll
-                        for (int c = 0; c < NP; c++) {                                 // the 64-byte swizzle: piece c of row r at piece c ^ (r / 2 % 4)
-                            const uint4 v = *reinterpret_cast<const uint4*>(raw + (((uint32_t)((T == 1 ? 2 * h : 0) + c) ^ sw) << 4));
+                        for (int c = 0; c < 4; c++) {                                  // the 64-byte swizzle: piece c of row r at piece c ^ (r / 2 % 4)
+                            const uint4 v = *reinterpret_cast<const uint4*>(raw + (((uint32_t)c ^ sw) << 4));
                             const uint32_t w[4] = { v.x, v.y, v.z, v.w };
 #pragma unroll
                             for (int u = 0; u < 4; u++) { o[c * 8 + 2 * u] = w[u] & 0x0F0F0F0Fu; o[c * 8 + 2 * u + 1] = (w[u] >> 4) & 0x0F0F0F0Fu; }
@@ -320,16 +285,18 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
                     if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_t[sT]), phT, abort_flag, 9))) { alive = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (have) {
-                        const uint32_t at = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)((sT * T + rt) * 32);
-                        if constexpr (T == 1) tmem_st16(at + 16 * h, o); else tmem_st32(at, o);
+                        tmem_st32(tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)((sT * T + rt) * 32), o);
                         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[sT]));
-                    if (++s == p.sa) { s = 0; phA ^= 1; }
-                    if (++sT == NT) { sT = 0; phT ^= 1; }
+                    s += 2;
+                    if (s >= p.sa) { s -= p.sa; phA ^= 1; }
+                    sT += 2;
+                    if (sT >= NT) { sT -= NT; phT ^= 1; }
                 }
+                next -= nk;
                 if (!alive) break;
             }
             if (!staged) {
@@ -352,8 +319,7 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
                 const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc), (uint32_t)(j & 1), abort_flag, 10))) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int g0 = T == 1 ? h : 0, gstep = T == 1 ? 2 : 1;
-                for (int g = g0; g * 4 < p.B; g += gstep) {
+                for (int g = team; g * 4 < p.B; g += 2) {
                     uint32_t acc[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
                     float* o = W.out + (size_t)(g * 4) * W.out_stride + row;
@@ -381,6 +347,7 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
         }
+        if (!staged) asm volatile("bar.sync 2, %0;" :: "n"(TQ_WORKERS * 32) : "memory");    // a warp that gave up: the others may be waiting there
     }
     if (S > 1) {
         // One run per cluster: the parts of the columns meet; block b mod S takes activation b. A meeting place inside the rings
@@ -396,10 +363,9 @@ __global__ void __launch_bounds__(TQ_THREADS, T == 1 ? 2 : 1) linear_tc_kernel(c
         const int rows = min(p.R, W.M - row0);
         const uint32_t recv = smem_u32(tq_smem + p.recv_off);                           // [source block][activation][row] int64
         if (warp < TQ_WORKERS && !*abort_flag) {
-            const int q = warp & 3, h = warp >> 2, rt = T == 1 ? 0 : h, rl = rt * 128 + q * 32 + lane;
-            const int g0 = T == 1 ? h : 0, gstep = T == 1 ? 2 : 1;
+            const int q = warp & 3, rt = (warp >> 2) % T, team = warp / (4 * T), rl = rt * 128 + q * 32 + lane;
             if (rt * 128 + q * 32 < rows) {
-                for (int g = g0; g * 4 < p.B; g += gstep) {
+                for (int g = team; g * 4 < p.B; g += 2) {
                     uint32_t acc[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
 #pragma unroll
@@ -476,7 +442,7 @@ int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, si
         if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(linear_tc_kernel, smem=%zu): %s", smem, cudaGetErrorString(e));
         have = smem;
     }
-    return ibcu_launch(ctx, kern, dim3(grid), dim3(TQ_THREADS), smem, p.S, true, maps, p);
+    return ibcu_launch(ctx, kern, dim3(grid), dim3(Tq<T>::THREADS), smem, p.S, true, maps, p);
 }
 
 }  // namespace
@@ -561,6 +527,14 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
         while (p.sa < TQ_MAX_STAGES && recv > ring_of()) p.sa++;
         if (recv > ring_of() || p.sa < 1) return IBCU_ERR_STATE;
         smem = ring_of();
+    }
+    if (bits == 4 && p.sa < nk) {
+        // a ring that is used again: an even one, so that a stage always belongs to the same team of widening warps (a warp that
+        // misses every other phase of a barrier cannot tell a phase from the next but one)
+        if (p.sa < 2) return IBCU_ERR_STATE;
+        p.sa &= ~1;
+        if (!p.recv_off && recv > ring_of()) return IBCU_ERR_STATE;
+        smem = p.recv_off ? smem : ring_of();
     }
     smem = ((smem + 15) & ~(size_t)15) + sizeof(TqShared);
     TqMaps maps;

@@ -94,6 +94,23 @@ def test_tcgen05_linear_edges(backend, cpu_libs, bits, M, N, B):
     assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
 
 
+@pytest.mark.parametrize("M,N,B", [(38000, 1664, 6), (25000, 1920, 32), (3000, 4224, 24)])
+def test_tcgen05_int4_teams(backend, M, N, B):
+    """Odd numbers of 128-column blocks through rings that are used again, over one and two runs of rows: the two teams of
+    widening warps change places from run to run. Bound as above."""
+    rng = np.random.default_rng(M + N + B)
+    w, s16, x = _cpu.make_int4_case(rng, M, N, B)
+    got = backend.linear(w, s16, x, 4)
+    sc = s16.view(np.float16).astype(np.float64)
+    want, mag = np.empty((B, M)), np.empty(M)
+    for r in range(0, M, 4096):
+        v = np.stack([w[r:r + 4096] & 15, w[r:r + 4096] >> 4], axis=-1).reshape(-1, N).astype(np.float64) - 8
+        want[:, r:r + 4096], mag[r:r + 4096] = x.astype(np.float64) @ v.T, np.abs(v).sum(axis=1)
+    want *= sc
+    bound = 2.0 ** -22 * np.abs(want) + 2.0 ** -30 * np.abs(x).max(axis=1, keepdims=True).astype(np.float64) * (mag * sc)
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("M,N,B", [(40, 66, 2), (9, 30, 1), (257, 1000, 3), (64, 4096, 4)])
 def test_portable_kernel(backend, cpu_libs, bits, M, N, B):
