@@ -1,5 +1,6 @@
 // Context, memory, timing, graph capture and the counter-based fill kernels of the CUDA backend.
 #include "common.cuh"
+#include "pq_tc.cuh"
 #include <stdarg.h>
 #include <stdlib.h>
 
@@ -160,6 +161,7 @@ static int ibcu_collect_kernel_errors(ibcu_ctx* ctx) {
     if (ctx->kern_err && *(volatile int*)ctx->kern_err) {
         const int e = *(volatile int*)ctx->kern_err;
         *(volatile int*)ctx->kern_err = 0;
+        if (e >= IBCU_PQ_TC_ERR && e < IBCU_PQ_TC_ERR + 100 && ctx->pq_acc) IBCU_CUDA(ctx, cudaMemsetAsync(ctx->pq_acc, 0, ctx->pq_acc_bytes, ctx->stream));
         return ibcu_fail(ctx, IBCU_ERR_CUDA, "a kernel gave up a bounded wait (code %d): its results are not valid", e);
     }
     return ctx->status;

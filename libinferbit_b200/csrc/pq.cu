@@ -1,5 +1,6 @@
 // Product-quantised matvec: out[r] = row_scale[r] * sum over subspaces s of LUT_s[code[r][s]],
-// LUT_s[k] = codebook_s[k] . x_s (FP32), for 1..32 activations. One launch per call.
+// LUT_s[k] = codebook_s[k] . x_s (FP32), for 1..32 activations: the kernels with tables, one launch per call. Calls with several
+// activations and entries of 4 or 16 values go to the tensor cores instead (pq_tc.cu, pq_takes_tc).
 //
 // Data in HBM: codebooks, row scales and the two row-major code planes exactly as the reference
 // holds them, plus one derived array made once per tensor by ibcu_pq_prepare: the codes regrouped into
@@ -21,6 +22,7 @@
 // largest codebook magnitude and N. The block that arrives last for its rows (an arrival counter) reads the
 // accumulators back, leaves them zero for the next call, applies the row scale and stores.
 #include "common.cuh"
+#include "pq_tc.cuh"
 #include <cooperative_groups.h>
 #include <mutex>
 
@@ -100,19 +102,7 @@ __global__ void __launch_bounds__(512) pq_amax_kernel(const float* __restrict__ 
     pdl_launch_dependents();
     pdl_wait();
     const float* xb = x + (size_t)blockIdx.x * N;
-    unsigned m = 0u;
-    if (inner) {
-        for (int j = threadIdx.x; j < n_inner; j += 512) m = max(m, __float_as_uint(xb[inner[j]]) & 0x7fffffffu);
-    } else if ((N & 3) == 0 && ((uintptr_t)x & 15) == 0) {
-        const uint4* x4 = reinterpret_cast<const uint4*>(xb);
-#pragma unroll 8
-        for (int j = threadIdx.x; j < (N >> 2); j += 512) {
-            const uint4 v = x4[j];
-            m = max(max(m, v.x & 0x7fffffffu), max(max(v.y & 0x7fffffffu, v.z & 0x7fffffffu), v.w & 0x7fffffffu));
-        }
-    } else {
-        for (int j = threadIdx.x; j < N; j += 512) m = max(m, __float_as_uint(xb[j]) & 0x7fffffffu);
-    }
+    unsigned m = pq_absmax_bits<512>(xb, inner, n_inner, !inner && (N & 3) == 0 && ((uintptr_t)x & 15) == 0, threadIdx.x);
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
@@ -221,20 +211,7 @@ __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p
         if (t >= nb) continue;
         if (p.amax_bits) { ab[t] = p.amax_bits[b0 + t]; continue; }            // made by pq_amax_kernel ahead of this launch
         const float* xb = p.x + (size_t)(b0 + t) * p.N;
-        if (EX && p.inner) {                                 // outlier columns do not count (src/pq_decode.c:1582-1588)
-            for (int j = tid; j < p.n_inner; j += PQ_THREADS) ab[t] = max(ab[t], __float_as_uint(xb[p.inner[j]]) & 0x7fffffffu);
-        } else if (vec_x) {
-            const uint4* x4 = reinterpret_cast<const uint4*>(xb);
-            const int n4 = p.N >> 2;
-#pragma unroll 8
-            for (int j = tid; j < n4; j += PQ_THREADS) {
-                const uint4 v = x4[j];
-                ab[t] = max(max(ab[t], v.x & 0x7fffffffu), max(max(v.y & 0x7fffffffu, v.z & 0x7fffffffu), v.w & 0x7fffffffu));
-            }
-        } else {
-#pragma unroll 8
-            for (int j = tid; j < p.N; j += PQ_THREADS) ab[t] = max(ab[t], __float_as_uint(xb[j]) & 0x7fffffffu);
-        }
+        ab[t] = pq_absmax_bits<PQ_THREADS>(xb, EX ? p.inner : nullptr, p.n_inner, vec_x && !(EX && p.inner), tid);        // outlier columns do not count (src/pq_decode.c:1582-1588)
     }
     float amax[BT], inv_q[BT];
     int anybad = 0;
@@ -456,235 +433,6 @@ __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p
     }
 }
 
-// ── Several activations, plain tensor with shared codebooks of 8-wide entries: pq_wide_kernel ──
-// The gather is bound by the shared-memory pipe: a table read and a lane-to-lane shuffle each move 32 values per cycle, and
-// the reduction over the lanes costs one shuffle per 32 values looked up. Here a lane owns four subspaces (a unit of work is
-// one activation x 128 subspaces, table of 128 KB) and adds their entries in registers before the lanes meet: a quarter of
-// the shuffles. Units x groups of 16 rows form one list that the blocks (one per SM) cut into equal contiguous pieces, so
-// every SM has the same share whatever the shape; a piece that crosses a unit builds a second table. Sums meet in the same
-// fixed-point accumulators; the block whose arrival completes an activation's count of pieces converts that activation.
-constexpr int PW_THREADS = 1024;
-constexpr int PW_WARPS = PW_THREADS / 32;
-constexpr int PW_Q = 4;                                      // subspaces per lane: slabs 4 u .. 4 u + 3 of the code plane
-constexpr int PW_MAXSEG = 8;
-// Table layout: quarters 2 h and 2 h + 1 share a region of 64 KB that starts at shared-memory address 64 KB * (h + 1); entry k of
-// quarter q, lane l sits at byte k * 256 + (q & 1) * 128 + 4 l of its region: bank l as before, and the code is byte 1 of the
-// address, so one byte-permute of the code word and the lane's base address yields the address of a table read. The codebooks
-// and the slices of x live below the first region.
-constexpr size_t PW_SMEM = 3 * 65536;
-constexpr size_t PW_LOW_BYTES = 256 * 2 * 2 * sizeof(float4) + PW_Q * 32 * 9 * sizeof(float);
-
-__global__ void __launch_bounds__(PW_THREADS, 1) pq_wide_kernel(const PqParams p, int nunit, int per_block, int* err) {
-    extern __shared__ __align__(16) unsigned char pw_smem[];
-    const uint32_t dyn = (uint32_t)__cvta_generic_to_shared(pw_smem);                                                           // shared-memory address of the dynamic part
-    float4 (*cbf)[2][2] = reinterpret_cast<float4 (*)[2][2]>(pw_smem);                                // [k][side][half of the entry], FP32
-    float (*xs)[9] = reinterpret_cast<float (*)[9]>(pw_smem + 256 * 2 * 2 * sizeof(float4));          // [4 * 32 subspaces][8 (+1)]
-    unsigned char* lut_b = pw_smem + (65536u - dyn);                                                  // the byte at shared-memory address 64 KB
-    if (dyn + PW_LOW_BYTES > 65536u) { if (threadIdx.x == 0) *err = 7001; return; }               // the host reports it at the next sync; cannot happen with this kernel's static data
-    __shared__ int seg_tok[PW_MAXSEG], seg_n[PW_MAXSEG], seg_last[PW_MAXSEG];
-    __shared__ unsigned char sub_dead[PW_Q * 32];             // per subspace of the unit: its chunk falls under the 1 % rule
-    __shared__ unsigned amax_s[32], red_s[2][PW_WARPS];       // bit pattern of max |x| of the activations this block meets
-    pdl_launch_dependents();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int G16 = p.M_pad >> 4, nsub = 2 * p.C;
-    // positions in the list of (unit, activation, group) fit 32 bits (the host checks): 64-bit divisions would cost more
-    // instructions per segment than the table build
-    const unsigned total = (unsigned)nunit * (unsigned)p.B * (unsigned)G16;
-    const unsigned lo = min(total, blockIdx.x * (unsigned)per_block);
-    const unsigned hi = min(total, lo + (unsigned)per_block);
-    // weights first, they do not depend on the previous kernel
-    if (tid < 512) {
-        const int side = tid >> 8, k = tid & 255;
-        const uint4 raw = k < p.K ? reinterpret_cast<const uint4*>(side ? p.cb_r : p.cb_l)[k] : make_uint4(0, 0, 0, 0);
-        const __half2* h = reinterpret_cast<const __half2*>(&raw);
-        const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]), f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
-        cbf[k][side][0] = make_float4(f0.x, f0.y, f1.x, f1.y);
-        cbf[k][side][1] = make_float4(f2.x, f2.y, f3.x, f3.y);
-    }
-    const float cbmax = __int_as_float(*reinterpret_cast<const int*>(p.idx_t + (size_t)p.tail_slabs * G16 * 512));
-    const uint4* plane = reinterpret_cast<const uint4*>(p.idx_t) + lane;
-    // this thread's activation of a segment: subspace s of a unit covers x[8 s, 8 s + 8)
-    auto load_x = [&](unsigned at_) -> float {
-        if (at_ >= hi) return 0.0f;
-        const unsigned ut_ = at_ / (unsigned)G16;
-        const int u_ = (int)(ut_ / (unsigned)p.B), t_ = (int)(ut_ - (unsigned)u_ * (unsigned)p.B);
-        const int sb = u_ * (PW_Q * 32) + (tid >> 3);
-        return sb < nsub ? p.x[(size_t)t_ * p.N + (size_t)sb * 8 + (tid & 7)] : 0.0f;
-    };
-    pdl_wait();
-    float xnext = load_x(lo);                                // in flight while the maxima are taken
-    // max |x| of the activations in this block's piece of the list (consecutive ones, two at a time so that their loads
-    // travel together): the 1 % rule and the fixed-point scale need it. As bit patterns: those of non-negative floats
-    // order like the floats, and NaN / Inf sort last.
-    if (lo < hi) {
-        const unsigned ut_lo = lo / (unsigned)G16, ut_hi = (hi - 1) / (unsigned)G16;
-        const int ntok = (int)min((unsigned)p.B, ut_hi - ut_lo + 1);
-        const bool vec_x = (p.N & 3) == 0 && ((uintptr_t)p.x & 15) == 0;
-        for (int j0 = 0; j0 < ntok; j0 += 2) {
-            unsigned m[2] = { 0u, 0u };
-            int tk[2];
-            tk[0] = (int)((ut_lo + (unsigned)j0) % (unsigned)p.B);
-            tk[1] = j0 + 1 < ntok ? (int)((ut_lo + (unsigned)j0 + 1u) % (unsigned)p.B) : tk[0];       // alone: the same activation twice
-            const float* xb0 = p.x + (size_t)tk[0] * p.N;
-            const float* xb1 = p.x + (size_t)tk[1] * p.N;
-            if (vec_x) {
-                const uint4* xa = reinterpret_cast<const uint4*>(xb0);
-                const uint4* xc = reinterpret_cast<const uint4*>(xb1);
-#pragma unroll 4
-                for (int i = tid; i < (p.N >> 2); i += PW_THREADS) {
-                    const uint4 v = xa[i], w = xc[i];
-                    m[0] = max(max(m[0], v.x & 0x7fffffffu), max(max(v.y & 0x7fffffffu, v.z & 0x7fffffffu), v.w & 0x7fffffffu));
-                    m[1] = max(max(m[1], w.x & 0x7fffffffu), max(max(w.y & 0x7fffffffu, w.z & 0x7fffffffu), w.w & 0x7fffffffu));
-                }
-            } else {
-                for (int i = tid; i < p.N; i += PW_THREADS) {
-                    m[0] = max(m[0], __float_as_uint(xb0[i]) & 0x7fffffffu);
-                    m[1] = max(m[1], __float_as_uint(xb1[i]) & 0x7fffffffu);
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                m[h] = __reduce_max_sync(0xffffffffu, m[h]);
-                if (lane == 0) red_s[h][warp] = m[h];
-            }
-            __syncthreads();
-            if (warp < 2 && j0 + warp < ntok) {
-                const unsigned r = __reduce_max_sync(0xffffffffu, red_s[warp][lane]);
-                if (lane == 0) amax_s[tk[warp]] = r;
-            }
-            __syncthreads();
-        }
-    }
-
-    // what the block owes the arrival counters: (activation, pieces) of every segment since the last flush
-    int nseg = 0;
-    auto flush = [&]() {
-        __threadfence();
-        __syncthreads();
-        if (tid < nseg) {
-            const unsigned want = (unsigned)nunit * (unsigned)G16;
-            const unsigned old = atomicAdd(p.arrive + seg_tok[tid], (unsigned)seg_n[tid]);
-            seg_last[tid] = old + (unsigned)seg_n[tid] == want;
-            if (seg_last[tid]) p.arrive[seg_tok[tid]] = 0;
-        }
-        __syncthreads();
-        for (int sgi = 0; sgi < nseg; sgi++) {
-            if (!seg_last[sgi]) continue;
-            // every piece of this activation has arrived, each behind its block's fence: plain loads past L1 read the sums
-            __threadfence();
-            const int t = seg_tok[sgi];
-            const unsigned ab = amax_s[t];
-            const float bound = (float)p.N * cbmax * __uint_as_float(ab);
-            int ex = (int)((__float_as_uint(bound) >> 23) & 0xFF) - 126;
-            ex = max(-60, min(120, ex));
-            const double q = __longlong_as_double((long long)(1023 + ex - 62) << 52);                  // 2^(ex - 62)
-            const bool bad = ab > 0x7f7fffffu;                                                            // a NaN or an Inf among the activations
-            unsigned long long* acc = p.acc + (size_t)t * p.M_pad;
-            for (int r0 = 0; r0 < p.M_pad; r0 += 4 * PW_THREADS) {
-                long long sum[4];
-                float sc[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int r = r0 + tid + i * PW_THREADS;
-                    sum[i] = r < p.M_pad ? (long long)__ldcg(acc + r) : 0;
-                    sc[i] = r < p.M ? __half2float(p.row_scale[r]) : 0.0f;
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int r = r0 + tid + i * PW_THREADS;
-                    if (r < p.M_pad) acc[r] = 0ull;                                                      // zero for the next call, padded rows too
-                    if (r < p.M) p.out[(size_t)t * p.out_stride + r] = bad ? __int_as_float(0x7fc00000) : (float)((double)sum[i] * q) * sc[i];
-                }
-            }
-        }
-        __syncthreads();
-        nseg = 0;
-    };
-
-    for (unsigned at = lo; at < hi;) {
-        const unsigned ut = at / (unsigned)G16;               // unit * B + activation
-        const int g0 = (int)(at - ut * (unsigned)G16);
-        const int g1 = (int)min((unsigned)G16, (unsigned)g0 + (hi - at));
-        const int u = (int)(ut / (unsigned)p.B), t = (int)(ut - (unsigned)u * (unsigned)p.B);
-        at += (unsigned)(g1 - g0);
-        // codes of this warp's first group: in flight during the table build
-        uint4 cd[PW_Q];
-        auto load_codes = [&](int g, int q) {
-            return (4 * u + q < p.nslab && g < g1) ? ld_stream_u4(plane + ((size_t)(4 * u + q) * G16 + g) * 32) : make_uint4(0, 0, 0, 0);
-        };
-#pragma unroll
-        for (int q = 0; q < PW_Q; q++) cd[q] = load_codes(g0 + warp, q);
-        __syncthreads();                                      // the previous segment's gather is done with the table and the slices (first: cbf is staged)
-        if (nseg == PW_MAXSEG) flush();
-        if (tid == 0) { seg_tok[nseg] = t; seg_n[nseg] = g1 - g0; }
-        nseg++;
-        xs[tid >> 3][tid & 7] = xnext;                        // this unit's 1024 activations
-        xnext = load_x(at);                                   // the next segment's, in flight during this one
-        const float amax = __uint_as_float(amax_s[t]);         // written before the barriers above
-        const float bound = (float)p.N * cbmax * amax;
-        int e = (int)((__float_as_uint(bound) >> 23) & 0xFF) - 126;                                     // bound < 2^e
-        e = max(-60, min(120, e));
-        const float inv_q = __uint_as_float((uint32_t)(127 + 62 - e) << 23);                              // 2^(62 - e)
-        __syncthreads();
-        // the reference drops a chunk (both of its subspaces) whose largest |x| is under 1 % of the largest overall
-        if (tid < PW_Q * 16) {                                // one thread per chunk of the unit
-            float cm = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) cm = fmaxf(cm, fmaxf(fabsf(xs[2 * tid][i]), fabsf(xs[2 * tid + 1][i])));
-            const unsigned char d = amax > 0.0f && !p.no_skip && u * (PW_Q * 32) + 2 * tid < nsub && !(cm >= amax * 0.01f);
-            sub_dead[2 * tid] = d; sub_dead[2 * tid + 1] = d;
-        }
-        __syncthreads();
-        // table: warp w builds entries k = w + 32 i, two quarters at a time (a codebook entry is read once for the two);
-        // each entry is summed in the same order as in the slab kernel
-        const int side = lane & 1;
-#pragma unroll 1
-        for (int qp = 0; qp < PW_Q; qp += 2) {
-            float xr[2][8];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const bool dead = sub_dead[(qp + q) * 32 + lane];            // a dropped subspace gets a table of zeros: the gather need not know
-#pragma unroll
-                for (int i = 0; i < 8; i++) xr[q][i] = dead ? 0.0f : xs[(qp + q) * 32 + lane][i];
-            }
-#pragma unroll 2
-            for (int k = warp; k < 256; k += PW_WARPS) {
-                const float4 ca = cbf[k][side][0], cc = cbf[k][side][1];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    float a = 0.0f;
-                    a = fmaf(ca.x, xr[q][0], a); a = fmaf(ca.y, xr[q][1], a); a = fmaf(ca.z, xr[q][2], a); a = fmaf(ca.w, xr[q][3], a);
-                    a = fmaf(cc.x, xr[q][4], a); a = fmaf(cc.y, xr[q][5], a); a = fmaf(cc.z, xr[q][6], a); a = fmaf(cc.w, xr[q][7], a);
-                    *reinterpret_cast<float*>(lut_b + (size_t)(qp >> 1) * 65536 + (size_t)k * 256 + q * 128 + lane * 4) = a;
-                }
-            }
-        }
-        __syncthreads();                                      // the table is complete
-        for (int g = g0 + warp; g < g1; g += PW_WARPS) {
-            float v[16];
-#pragma unroll
-            for (int q = 0; q < PW_Q; q++) {
-                const uint4 cw = cd[q];
-                cd[q] = load_codes(g + PW_WARPS, q);          // the next group's codes travel while this one is looked up
-                const uint32_t tb = 65536u * (1u + (q >> 1)) + (q & 1) * 128u + lane * 4u;     // entry 0 of this lane's subspace; byte 1 of the address is zero
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const uint32_t w = i < 4 ? cw.x : (i < 8 ? cw.y : (i < 12 ? cw.z : cw.w));
-                    const uint32_t addr = __byte_perm(w, tb, 0x7604u | ((i & 3) << 4));          // bytes (tb3, tb2, code, tb0)
-                    float val;
-                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(val) : "r"(addr) : "memory");
-                    v[i] = q == 0 ? val : v[i] + val;
-                }
-            }
-            fold<16>(v, 16); fold<8>(v, 8); fold<4>(v, 4); fold<2>(v, 2);
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-            if ((lane & 1) == 0)                              // value 0 of lane l: row l >> 1 of the group
-                atomicAdd(p.acc + (size_t)t * p.M_pad + 16 * g + (lane >> 1), (unsigned long long)__float2ll_rn(v[0] * inv_q));
-        }
-    }
-    if (nseg) flush();
-}
-
 // Outlier sidecar (src/pq_decode.c:1394-1409): out[r] += sum over j of (sidecar[r][j] * scale[j]) * x[col[j]], added to the finished
 // rows. grid (blocks of 8 rows, activations), a warp per row, lanes over the outlier columns.
 __global__ void __launch_bounds__(256) pq_outlier_kernel(const int8_t* __restrict__ side, const int32_t* __restrict__ cols, const __half* __restrict__ scale,
@@ -706,7 +454,7 @@ __global__ void __launch_bounds__(256) pq_outlier_kernel(const int8_t* __restric
     if (lane == 0) out[(size_t)b * out_stride + r] += acc;
 }
 
-struct PqPlan { int C, nslab1, nslab, bt, passes, row_blocks, rows_per_block, slab_blocks; size_t acc_words; int wide, nunit, per_block, nblocks; };
+struct PqPlan { int C, nslab1, nslab, bt, passes, row_blocks, rows_per_block, slab_blocks; size_t acc_words; };
 
 PqPlan pq_plan(const ibcu_ctx* ctx, const ibcu_pq_t* t, int B, bool l1_only = false) {
     PqPlan pl;
@@ -733,17 +481,13 @@ PqPlan pq_plan(const ibcu_ctx* ctx, const ibcu_pq_t* t, int B, bool l1_only = fa
     pl.rows_per_block = gpb * 16;
     pl.row_blocks = (groups + gpb - 1) / gpb;
     pl.acc_words = (size_t)B * t->M_pad;
-    // three or more activations of a plain tensor with shared 8-wide codebooks: the kernel with four subspaces per lane
-    // (4096 x 14336: 21.8 against 26.5 us at three activations; at two the slab kernel's single pass wins, 17.6 against 20.2 us)
-    pl.wide = B >= 3 && !l1_only && t->K_l2 == 0 && t->n_outlier == 0 && t->G == 16 && t->cb_chunk_stride == 0 &&
-              (((uintptr_t)t->codebook_l | (uintptr_t)t->codebook_r) & 15) == 0;
-    pl.nunit = (pl.nslab + PW_Q - 1) / PW_Q;
-    const long total = (long)pl.nunit * B * groups;
-    if (total >= (1l << 30)) pl.wide = 0;                    // the kernel counts its pieces in 32 bits
-    const long nb = total < ctx->sm_count ? total : ctx->sm_count;
-    pl.per_block = (int)((total + nb - 1) / nb);
-    pl.nblocks = (int)((total + pl.per_block - 1) / pl.per_block);
     return pl;
+}
+
+// the sidecar's share is added to the finished rows (src/pq_decode.c:1676)
+int pq_outliers(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B) {
+    return ibcu_launch(ctx, pq_outlier_kernel, dim3((t->M + 7) / 8, B), dim3(256), (size_t)t->n_outlier * sizeof(float), 1, true,
+                       t->outlier_sidecar, t->outlier_cols, (const __half*)t->outlier_scale, t->n_outlier, x, t->N, out, t->M, out_stride);
 }
 
 int pq_launch(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B, const PqPlan& pl,
@@ -767,11 +511,8 @@ int pq_launch(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int
         if (e == cudaSuccess) e = cudaFuncSetAttribute(pq_slab_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 32 * (int)sizeof(float));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(pq_slab_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 32 * 2 * (int)sizeof(float));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(pq_slab_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 32 * (int)sizeof(float));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(pq_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
     });
     if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(pq_slab_kernel): %s", cudaGetErrorString(e));
-    if (pl.wide)                               // takes the maxima of the activations it meets itself
-        return ibcu_launch(ctx, pq_wide_kernel, dim3(pl.nblocks), dim3(PW_THREADS), PW_SMEM, 1, true, p, pl.nunit, pl.per_block, ctx->kern_err);
     if (pl.bt == 2) {
         // with several activations every block would scan all of them for their maxima: one small launch does it once;
         // its results sit in the last 64 counter slots, which no pass uses
@@ -787,10 +528,7 @@ int pq_launch(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int
                           : ibcu_launch(ctx, pq_slab_kernel<1, false>, grid, block, (size_t)256 * 32 * sizeof(float), 1, true, p);
         if (rc) return rc;
     }
-    if (t->n_outlier > 0)                                    // the sidecar's share is added to the finished rows (src/pq_decode.c:1676)
-        return ibcu_launch(ctx, pq_outlier_kernel, dim3((t->M + 7) / 8, B), dim3(256), (size_t)t->n_outlier * sizeof(float), 1, true,
-                           t->outlier_sidecar, t->outlier_cols, (const __half*)t->outlier_scale, t->n_outlier, x, t->N, out, t->M, out_stride);
-    return IBCU_OK;
+    return t->n_outlier > 0 ? pq_outliers(ctx, t, x, out, out_stride, B) : IBCU_OK;
 }
 
 int pq_check(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int B, const char* who) {
@@ -809,6 +547,31 @@ int pq_check(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int 
 }  // namespace
 
 static size_t pq_scratch_bytes(const PqPlan& pl) { return PQ_COUNTER_BYTES + pl.acc_words * sizeof(unsigned long long); }
+
+constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;         // scratch of the allocation-free entry point (see there)
+
+// Whether a call takes the tensor-core kernel (pq_tc.cu), the same for both entry points, so that they agree to the bit. Measured in a
+// chain of calls, us, table kernels / tensor cores. Entries of 4 and 16 values: always ahead (2048 x 2048, one activation 13.8 / 7.9 and
+// 19.6 / 7.9; 4096 x 8192, eight 49 / 17.6 and 37 / 23). Entries of 8: one activation 11.2 / 18.0 at 4096 x 14336; two 16.4 / 18.2
+// there, 11.2 / 11.2 at 4096 x 4096, 10.0 / 7.2 at 1500 x 2000; three 21.9 / 19.0, eight 28.1 / 21.2, sixteen 46 / 27. Outlier columns
+// make its preparation gather: 17.6 / 18.6 at four activations, 24.7 / 22.1 at eight.
+static bool pq_takes_tc(const ibcu_pq_t* t, int B) {
+    if (t->G != 16) return true;
+    if (t->n_outlier > 0) return B >= 5;
+    return B >= 3 || (B == 2 && (long)t->M * t->N <= 20000000l);
+}
+// counters and accumulators at base (counter area: arrival counters, the top-K head's own 128 slots from the end, max |x| in the last 64)
+static int pq_run(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B, const PqPlan& pl, void* base, void* image) {
+    unsigned long long* acc = (unsigned long long*)((char*)base + PQ_COUNTER_BYTES);
+    unsigned* slots = (unsigned*)base;
+    constexpr int N_SLOTS = PQ_COUNTER_BYTES / sizeof(unsigned);
+    if (image) {
+        int rc = ibcu_pq_tc(ctx, t, x, out, out_stride, B, false, acc, slots, N_SLOTS - 128, slots + N_SLOTS - 64, image);
+        if (rc == IBCU_OK && t->n_outlier > 0) rc = pq_outliers(ctx, t, x, out, out_stride, B);
+        if (rc != IBCU_ERR_STATE) return rc;
+    }
+    return pq_launch(ctx, t, x, out, out_stride, B, pl, acc, slots);
+}
 
 extern "C" size_t ibcu_pq_idx_t_bytes(int M, int N, int G) {
     if (M <= 0 || N <= 0 || G <= 0 || N % G) return 0;
@@ -908,7 +671,13 @@ extern "C" int ibcu_pq_matmul_fp32_strided(ibcu_ctx* ctx, const ibcu_pq_t* t, co
         if (rc) return rc;
         IBCU_CUDA(ctx, cudaMemsetAsync(ctx->pq_acc, 0, ctx->pq_acc_bytes, ctx->stream));
     }
-    return pq_launch(ctx, t, x, out, out_stride, B, pl, (unsigned long long*)((char*)ctx->pq_acc + PQ_COUNTER_BYTES), (unsigned int*)ctx->pq_acc);
+    void* image = nullptr;
+    if (pq_takes_tc(t, B)) {
+        rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, ibcu_pq_tc_image_bytes(t, B));
+        if (rc) return rc;
+        image = ctx->xpack;
+    }
+    return pq_run(ctx, t, x, out, out_stride, B, pl, ctx->pq_acc, image);
 }
 
 // ── top-K LM head (src/pq_decode.c:2259-2341) ───────────────────────────────────────────
@@ -1280,7 +1049,6 @@ extern "C" int ibcu_pq_lm_head_topk(ibcu_ctx* ctx, const ibcu_pq_t* t, const flo
 // counters live in a fixed array that is part of the library image: every GPU that loads the library
 // holds PQ_STATIC_FLOATS four-byte words (4 MiB) from load until exit, whether or not this entry point is
 // used.
-constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;
 static __device__ __align__(256) float pq_static_scratch[PQ_STATIC_FLOATS];
 
 // In host code `pq_static_scratch` is only a handle for the runtime, not a device address; the
@@ -1320,5 +1088,17 @@ extern "C" int ibcu_pq_matmul_fp32_noalloc(ibcu_ctx* ctx, const ibcu_pq_t* t, co
     // array is shared by every caller on the device and one that was cut short may not have: clear the part
     // this call uses (an asynchronous fill on the stream, no allocation).
     IBCU_CUDA(ctx, cudaMemsetAsync(base, 0, need, ctx->stream));
-    return pq_launch(ctx, t, x, out, t->M, B, pl, (unsigned long long*)((char*)base + PQ_COUNTER_BYTES), (unsigned int*)base);
+    if (!pq_takes_tc(t, B)) return pq_run(ctx, t, x, out, t->M, B, pl, base, nullptr);
+    // the operand image stands behind the accumulators; where there is no room for all activations at once they go in turns (an
+    // activation's result does not depend on the others), and where there is none for one by the table kernels
+    int turn = B;
+    auto bytes = [&](int b) { return (pq_scratch_bytes(pq_plan(ctx, t, b)) + 255) / 256 * 256 + ibcu_pq_tc_image_bytes(t, b); };
+    while (turn > 1 && bytes(turn) > PQ_STATIC_FLOATS * sizeof(float)) turn--;
+    if (bytes(turn) > PQ_STATIC_FLOATS * sizeof(float)) return pq_run(ctx, t, x, out, t->M, B, pl, base, nullptr);
+    for (int b = 0; b < B && !rc; b += turn) {
+        const int n = B - b < turn ? B - b : turn;
+        if (b) IBCU_CUDA(ctx, cudaMemsetAsync(base, 0, pq_scratch_bytes(pq_plan(ctx, t, n)), ctx->stream));
+        rc = pq_run(ctx, t, x + (size_t)b * t->N, out + (size_t)b * t->M, t->M, n, pq_plan(ctx, t, n), base, (char*)base + (bytes(n) - ibcu_pq_tc_image_bytes(t, n)));
+    }
+    return rc;
 }

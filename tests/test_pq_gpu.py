@@ -58,6 +58,51 @@ def test_pq_second_level_and_outliers(backend, cpu_libs, M, N, G, K, K_l2, n_out
     assert np.array_equal(got, got2)
 
 
+@pytest.mark.parametrize("M,N,G,K,K_l2,n_out,B", [
+    (1, 16, 16, 256, 0, 0, 3), (129, 528, 16, 100, 0, 0, 16),         # one row, one chunk; one row past a tile, one chunk past a slab
+    (127, 4096, 16, 256, 16, 0, 9), (300, 2000, 16, 256, 256, 0, 17), # second level; one activation past an instance, past a launch
+    (20000, 256, 16, 256, 0, 0, 8), (40, 16384, 16, 256, 0, 0, 32),   # a block meets several tiles; many blocks share one tile
+    (257, 1000, 8, 256, 0, 0, 1), (64, 8 * 37, 8, 77, 16, 0, 5),      # entries of four values
+    (257, 2080, 32, 256, 0, 0, 1), (513, 32 * 33, 32, 200, 16, 0, 7), # entries of sixteen: two units per slab
+    (200, 1024 + 32, 16, 256, 0, 32, 6),                              # outlier columns
+])
+def test_pq_on_the_tensor_cores(backend, M, N, G, K, K_l2, n_out, B):
+    """Edges of the tensor-core kernel against the product in double precision. Bound: the pieces hold every activation to FP32
+    precision and the products are exact; the additions lose at most one part in 2^23 each of the terms' magnitudes: four per chain of
+    MMAs of first pieces, two joining chains, two joining pieces, one row scale, which is below 2^-19 of the sum of magnitudes."""
+    rng = np.random.default_rng(M + N + G + B)
+    d = _cpu.make_pq_case_ex(rng, M, N, G, K, K_l2, n_out, B)
+    d["x"][B - 1, :min(N, 3 * G)] *= 1e-4                    # some chunks fall under the 1 % rule
+    t = backend.make_pq_ex(d)
+    got = backend.pq_matmul(t, d["x"])
+    half, C_ = G // 2, (N - n_out) // G
+    f = lambda a: np.asarray(a).view(np.float16).astype(np.float64)
+    w = np.empty((M, C_, 2, half))
+    for side, s in enumerate("lr"):
+        w[:, :, side] = f(d["cb1_" + s]).reshape(-1, half)[d["idx1_" + s].reshape(M, C_)]
+        if K_l2:
+            i2 = d["idx2_" + s].reshape(M, -1)
+            if K_l2 == 16:
+                i2 = np.stack([i2 & 15, i2 >> 4], axis=-1).reshape(M, -1)[:, :C_]
+            w[:, :, side] += f(d["cb2_" + s]).reshape(-1, half)[i2]
+    w = w.reshape(M, -1)
+    inner = np.setdiff1d(np.arange(N), d["ocols"]) if n_out else np.arange(N)
+    x = d["x"].astype(np.float64)[:, inner].reshape(B, C_, G)
+    top = np.abs(x).max(axis=2)
+    x = (x * ~((top.max(axis=1, keepdims=True) > 0) & (top < top.max(axis=1, keepdims=True) * np.float32(0.01)))[:, :, None]).reshape(B, -1)
+    rs = f(d["rs"])
+    want, mag = (x @ w.T) * rs, (np.abs(x) @ np.abs(w).T) * np.abs(rs)
+    if n_out:
+        wo = d["oside"].reshape(M, n_out).astype(np.float64) * f(d["oscale"])
+        xo = d["x"].astype(np.float64)[:, d["ocols"]]
+        want, mag = want + xo @ wo.T, mag + np.abs(xo) @ np.abs(wo).T
+    assert np.all(np.abs(got - want) <= 2.0 ** -19 * mag), float(np.max(np.abs(got - want) / mag))
+    assert np.array_equal(got, backend.pq_matmul(t, d["x"]))  # accumulators and counters were left clean
+    d["x"][0, inner[0]] = np.inf
+    bad = backend.pq_matmul(t, d["x"])
+    assert np.all(np.isnan(bad[0])) and np.array_equal(bad[1:], got[1:])
+
+
 @pytest.mark.parametrize("M,N,G,K,K_l2,n_out,k_top", [
     (32000, 4096, 16, 256, 16, 0, 64),     # LM head of the 7B shape, 16-entry second level
     (32000, 4096 + 32, 16, 256, 256, 32, 256),
