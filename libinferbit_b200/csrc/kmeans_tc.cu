@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
             issue(i + TC_STAGES - 1);
             asm volatile("cp.async.wait_group %0;" :: "n"(TC_STAGES - 1) : "memory");
             __syncwarp();
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_a[s]), (uint32_t)(((i / TC_STAGES) & 1) ^ 1), abort_flag, 1))) break;   // the whole warp leaves or stays
+            if (!__all_sync(0xffffffffu, mbar_wait<false>(smem_u32(&sh->empty_a[s]), (uint32_t)(((i / TC_STAGES) & 1) ^ 1), abort_flag, 1))) break;   // the whole warp leaves or stays
             const unsigned char* raw = sRaw + s * TC_RAW_STAGE;
             unsigned char* dstA = sA + s * TC_A_STAGE;
             {
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
             bool ok = true;
             for (long i = 0; i < n_my && ok; i++) {
                 const int s = (int)(i % TC_STAGES), b = (int)(i & 1);
-                ok = mbar_wait(smem_u32(&sh->full_a[s]), (uint32_t)((i / TC_STAGES) & 1), abort_flag, 2) &&
-                     mbar_wait(smem_u32(&sh->empty_acc[b]), (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag, 3);
+                ok = mbar_wait<false>(smem_u32(&sh->full_a[s]), (uint32_t)((i / TC_STAGES) & 1), abort_flag, 2) &&
+                     mbar_wait<false>(smem_u32(&sh->empty_acc[b]), (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag, 3);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem_base + (uint32_t)b * 256u;
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
                 mma_commit(smem_u32(&sh->full_acc[b]));              // and the accumulator tile is complete
             }
             mma_commit(smem_u32(&sh->drained));
-            mbar_wait(smem_u32(&sh->drained), 0u, abort_flag, 4);    // nothing of this block is left in the tensor pipe
+            mbar_wait<false>(smem_u32(&sh->drained), 0u, abort_flag, 4);    // nothing of this block is left in the tensor pipe
         }
     } else {
         // ── epilogue: warp w drains accumulator tile w / 4, rows 32 (w % 4) .. + 31 ──
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
                 const float4 v = have ? *reinterpret_cast<const float4*>(X + row * 8 + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
                 xr[0] = u.x; xr[1] = u.y; xr[2] = u.z; xr[3] = u.w; xr[4] = v.x; xr[5] = v.y; xr[6] = v.z; xr[7] = v.w;
             }
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc[b]), (uint32_t)((i >> 1) & 1), abort_flag, 5))) break;            // the whole warp leaves or stays
+            if (!__all_sync(0xffffffffu, mbar_wait<false>(smem_u32(&sh->full_acc[b]), (uint32_t)((i >> 1) & 1), abort_flag, 5))) break;            // the whole warp leaves or stays
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             Top2 tr[4];
 #pragma unroll

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p
         if (t >= nb) continue;
         if (p.amax_bits) { ab[t] = p.amax_bits[b0 + t]; continue; }            // made by pq_amax_kernel ahead of this launch
         const float* xb = p.x + (size_t)(b0 + t) * p.N;
-        ab[t] = pq_absmax_bits<PQ_THREADS>(xb, EX ? p.inner : nullptr, p.n_inner, vec_x && !(EX && p.inner), tid);        // outlier columns do not count (src/pq_decode.c:1582-1588)
+        ab[t] = pq_absmax_bits<PQ_THREADS, 4>(xb, EX ? p.inner : nullptr, p.n_inner, vec_x && !(EX && p.inner), tid);        // outlier columns do not count (src/pq_decode.c:1582-1588)
     }
     float amax[BT], inv_q[BT];
     int anybad = 0;

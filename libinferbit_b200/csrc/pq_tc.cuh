@@ -12,28 +12,28 @@ int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, in
 size_t ibcu_pq_tc_image_bytes(const ibcu_pq_t* t, int B);
 
 // Largest bit pattern of |x| that thread `tid` of T meets among n values (patterns of non-negative floats order like the floats,
-// NaN and Inf sort last). Eight loads travel together whatever n is: a loop left to the compiler's unrolling takes what is over
+// NaN and Inf sort last). U loads travel together whatever n is: a loop left to the compiler's unrolling takes what is over
 // its multiple of eight one by one, and 14336 values are seven rounds of 512 threads.
-template <int T>
+template <int T, int U = 8>
 __device__ __forceinline__ unsigned pq_absmax_bits(const float* xb, const int* inner, int n, bool vec, int tid) {
     unsigned m = 0u;
     if (vec) {
         const uint4* x4 = reinterpret_cast<const uint4*>(xb);
-        for (int j0 = tid; j0 < (n >> 2); j0 += 8 * T) {
-            uint4 v[8];
+        for (int j0 = tid; j0 < (n >> 2); j0 += U * T) {
+            uint4 v[U];
 #pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = j0 + u * T < (n >> 2) ? x4[j0 + u * T] : make_uint4(0, 0, 0, 0);
+            for (int u = 0; u < U; u++) v[u] = j0 + u * T < (n >> 2) ? x4[j0 + u * T] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int u = 0; u < 8; u++) m = max(max(m, v[u].x & 0x7fffffffu), max(max(v[u].y & 0x7fffffffu, v[u].z & 0x7fffffffu), v[u].w & 0x7fffffffu));
+            for (int u = 0; u < U; u++) m = max(max(m, v[u].x & 0x7fffffffu), max(max(v[u].y & 0x7fffffffu, v[u].z & 0x7fffffffu), v[u].w & 0x7fffffffu));
         }
         return m;
     }
-    for (int j0 = tid; j0 < n; j0 += 8 * T) {
-        unsigned v[8];
+    for (int j0 = tid; j0 < n; j0 += U * T) {
+        unsigned v[U];
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = j0 + u * T < n ? __float_as_uint(xb[inner ? inner[j0 + u * T] : j0 + u * T]) & 0x7fffffffu : 0u;
+        for (int u = 0; u < U; u++) v[u] = j0 + u * T < n ? __float_as_uint(xb[inner ? inner[j0 + u * T] : j0 + u * T]) & 0x7fffffffu : 0u;
 #pragma unroll
-        for (int u = 0; u < 8; u++) m = max(m, v[u]);
+        for (int u = 0; u < U; u++) m = max(m, v[u]);
     }
     return m;
 }

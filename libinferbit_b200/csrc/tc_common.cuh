@@ -22,9 +22,11 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait. Returns false when the block is giving up (this wait ran out, or another role's did). A phase that is complete
-// already is seen by the plain test in 65 cycles; the try with a hint takes 112 to say so.
+// already is seen by the plain test in 65 cycles; the try with a hint takes 112 to say so. (Where phases are rarely complete the
+// test only delays the try: k-means takes the wait without it, 2864 against 2850 us.)
+template <bool TEST = true>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
-    if (mbar_test(bar, parity)) return true;
+    if (TEST && mbar_test(bar, parity)) return true;
     for (int it = 0; it < TC_SPIN_LIMIT; it++) {
         if (mbar_try(bar, parity)) return true;
         if (*abort_flag) return false;
