@@ -115,7 +115,8 @@ struct WtParams {
     int dld;                                                  // words per row of the parked dot products: B made odd, so that rows fall on different banks
 };
 
-template <int STAGES, int RT>
+// XF: FP32 activations, quantised by every block for itself
+template <int STAGES, int RT, bool XF>
 __global__ void __launch_bounds__(WT_W * 32) w4a8_mma_kernel(const WtParams p) {
     constexpr int R = WT_R * RT;                              // rows per tile
     constexpr int STAGE_BYTES = R * WT_LD;
@@ -157,45 +158,69 @@ __global__ void __launch_bounds__(WT_W * 32) w4a8_mma_kernel(const WtParams p) {
     pdl_wait();
 
     // activations: bytes of every 8 columns reordered to evens then odds; per group 8 x the sum of its bytes and its scale
-    if (p.xf) {
+    if constexpr (XF) {
         // the reference's quantiser (src/threading.c:401-432) on the fly: a warp per (activation, group of 128 columns),
         // scale = max|x| / 127 (1e-10 and all zeros for a dead group), round half away from zero, clamp to +-127
-        for (int e = warp; e < p.B * nk; e += WT_W) {
-            const int b = e / nk, k = e % nk;
-            const float4 v = *reinterpret_cast<const float4*>(p.xf + (size_t)b * p.N + (size_t)k * 128 + 4 * lane);
-            const float amax = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-            const bool dead = amax < 1e-10f;
-            const float scale = dead ? 1e-10f : __fdiv_rn(amax, 127.0f);
-            const float inv = dead ? 0.0f : __fdiv_rn(1.0f, scale);
-            const float f[4] = { v.x, v.y, v.z, v.w };
-            int q[4];
+        // Four groups of a warp are read together: one after another, every group costs a round trip to L2.
+        for (int e0 = warp; e0 < p.B * nk; e0 += 4 * WT_W) {
+            float4 vv[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                int qi = 0;
-                if (!dead) {
-                    qi = __float2int_rz(__fadd_rn(__fmul_rn(f[i], inv), f[i] >= 0.0f ? 0.5f : -0.5f));
-                    qi = max(-127, min(127, qi));
-                }
-                q[i] = qi;
+            for (int u = 0; u < 4; u++) {
+                const int e = min(e0 + u * WT_W, p.B * nk - 1);
+                vv[u] = *reinterpret_cast<const float4*>(p.xf + (size_t)(e / nk) * p.N + (size_t)(e % nk) * 128 + 4 * lane);
             }
-            // lane holds columns 4 lane .. 4 lane + 3: the even lane of a pair has c0..c3 of its 8 columns, the odd lane c4..c7
-            const uint32_t mine = (uint32_t)(q[0] & 255) | ((uint32_t)(q[1] & 255) << 8) | ((uint32_t)(q[2] & 255) << 16) | ((uint32_t)(q[3] & 255) << 24);
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const uint32_t lo = (lane & 1) ? other : mine, hi = (lane & 1) ? mine : other;
-            if ((lane & 1) == 0)
-                *reinterpret_cast<uint2*>(xs + (size_t)b * p.xs_ld + (size_t)k * 128 + 4 * lane) =
-                    make_uint2(__byte_perm(lo, hi, 0x6420), __byte_perm(lo, hi, 0x7531));
-            int ssum = q[0] + q[1] + q[2] + q[3];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
-            if (lane == 0) { qsum[e] = 8 * ssum; s_sa[e] = scale; }
+            for (int u = 0; u < 4; u++) {
+                const int e = e0 + u * WT_W;
+                if (e >= p.B * nk) break;
+                const int b = e / nk, k = e % nk;
+                const float4 v = vv[u];
+                const float amax = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+                const bool dead = amax < 1e-10f;
+                const float scale = dead ? 1e-10f : __fdiv_rn(amax, 127.0f);
+                const float inv = dead ? 0.0f : __fdiv_rn(1.0f, scale);
+                const float f[4] = { v.x, v.y, v.z, v.w };
+                int q[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    int qi = 0;
+                    if (!dead) {
+                        qi = __float2int_rz(__fadd_rn(__fmul_rn(f[i], inv), f[i] >= 0.0f ? 0.5f : -0.5f));
+                        qi = max(-127, min(127, qi));
+                    }
+                    q[i] = qi;
+                }
+                // lane holds columns 4 lane .. 4 lane + 3: the even lane of a pair has c0..c3 of its 8 columns, the odd lane c4..c7
+                const uint32_t mine = (uint32_t)(q[0] & 255) | ((uint32_t)(q[1] & 255) << 8) | ((uint32_t)(q[2] & 255) << 16) | ((uint32_t)(q[3] & 255) << 24);
+                const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
+                const uint32_t lo = (lane & 1) ? other : mine, hi = (lane & 1) ? mine : other;
+                if ((lane & 1) == 0)
+                    *reinterpret_cast<uint2*>(xs + (size_t)b * p.xs_ld + (size_t)k * 128 + 4 * lane) =
+                        make_uint2(__byte_perm(lo, hi, 0x6420), __byte_perm(lo, hi, 0x7531));
+                const int ssum = __reduce_add_sync(0xffffffffu, q[0] + q[1] + q[2] + q[3]);
+                if (lane == 0) { qsum[e] = 8 * ssum; s_sa[e] = scale; }
+            }
         }
     } else {
-        for (int e = threadIdx.x; e < p.B * (p.N / 8); e += WT_W * 32) {
+        const int n8 = p.B * (p.N / 8);
+        auto put8 = [&](int e, uint2 v) {
             const int b = e / (p.N / 8), c8 = e % (p.N / 8);
-            const uint2 v = *reinterpret_cast<const uint2*>(p.xq + (size_t)b * p.N + (size_t)c8 * 8);
-            const uint2 o = make_uint2(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.x, v.y, 0x7531));
-            *reinterpret_cast<uint2*>(xs + (size_t)b * p.xs_ld + (size_t)c8 * 8) = o;
+            *reinterpret_cast<uint2*>(xs + (size_t)b * p.xs_ld + (size_t)c8 * 8) = make_uint2(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.x, v.y, 0x7531));
+        };
+        if (n8 <= 8 * WT_W * 32) {                            // up to one row of 16384 columns: all reads of a thread in flight at once
+            uint2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int e = threadIdx.x + u * WT_W * 32;
+                if (e < n8) v[u] = *reinterpret_cast<const uint2*>(p.xq + (size_t)e * 8);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int e = threadIdx.x + u * WT_W * 32;
+                if (e < n8) put8(e, v[u]);
+            }
+        } else {
+            for (int e = threadIdx.x; e < n8; e += WT_W * 32) put8(e, *reinterpret_cast<const uint2*>(p.xq + (size_t)e * 8));
         }
         for (int e = threadIdx.x; e < p.B * nk; e += WT_W * 32) {
             const int b = e / nk, k = e % nk;
@@ -277,9 +302,9 @@ __global__ void __launch_bounds__(WT_W * 32) w4a8_mma_kernel(const WtParams p) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int STAGES, int RT>
-int w4a8_mma_launch(ibcu_ctx* ctx, const WtParams& p, int grid, size_t smem) {
-    auto kern = w4a8_mma_kernel<STAGES, RT>;
+template <int STAGES, int RT, bool XF>
+int w4a8_mma_launch_x(ibcu_ctx* ctx, const WtParams& p, int grid, size_t smem) {
+    auto kern = w4a8_mma_kernel<STAGES, RT, XF>;
     if (smem > 48 * 1024) {
         static size_t allowed[64];
         size_t& have = allowed[ctx->device & 63];
@@ -290,6 +315,11 @@ int w4a8_mma_launch(ibcu_ctx* ctx, const WtParams& p, int grid, size_t smem) {
         }
     }
     return ibcu_launch(ctx, kern, dim3(grid), dim3(WT_W * 32), smem, 1, true, p);
+}
+
+template <int STAGES, int RT>
+int w4a8_mma_launch(ibcu_ctx* ctx, const WtParams& p, int grid, size_t smem) {
+    return p.xf ? w4a8_mma_launch_x<STAGES, RT, true>(ctx, p, grid, smem) : w4a8_mma_launch_x<STAGES, RT, false>(ctx, p, grid, smem);
 }
 
 }  // namespace
