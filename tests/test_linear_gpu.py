@@ -422,3 +422,15 @@ def test_group_scaled_int4_rows(backend, cpu_libs, M, N, G, K_out, eps):
     assert np.array_equal(got, backend.int4g_matmul(q, s, G, x, oi, ov, eps))       # same bits again
     # linearity at full size: f(2x) = 2 f(x) exactly (every product and sum scales by a power of two)
     assert np.array_equal(backend.int4g_matmul(q, s, G, 2.0 * x, oi, ov, eps), 2.0 * got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [32, 2048, 2080, 8192, 8224, 16384, 16416])
+def test_group_scaled_int4_row_lengths(backend, cpu_libs, N):
+    """Where the fast kernel changes how it holds the activation: one and several groups of eight columns per thread, the last length of
+    each register instance and the first one of the next, the first that is read twice."""
+    rng = np.random.default_rng(N)
+    q, s, x, oi, ov = _cpu.make_int4g_case(rng, 50, N, 32, 0)
+    got = backend.int4g_matmul(q, s, 32, x, oi, ov, 0.0)
+    want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, 32, x, oi, ov, 0.0)
+    assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
