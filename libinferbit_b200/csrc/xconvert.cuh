@@ -295,31 +295,40 @@ __device__ __forceinline__ void xconvert_regs(const XSource& src, int N, int b, 
     }
 }
 
+// Groups of 8 columns in flight per thread. One: every block of a launch converts the same row while its weights are on their way, and
+// more requests for the same lines at once only queue in front of them (step of a 7B shape: one 1929, two 1972, four 1975, eight 2040 us).
+constexpr int XKNOWN_U = 1;
 // The conversion when the caller knows max|x[b]| (IBCU_PRO_KNOWN_MAX): no reduction before the digits, so
-// rows of any length stream through in one pass, four groups of 8 columns in flight per thread.
+// rows of any length stream through in one pass.
 template <class D>
 __device__ __forceinline__ void xconvert_known(const XSource& src, int N, int b, int c0, int slice_cols, const D& dst,
                                                int perm8, XScratch& sc, float* back_out, int* sum_out) {
     const int nth = blockDim.x, nwarp = nth >> 5;
     const int valid = max(0, min(slice_cols, N - c0));
     const float* xb = src.x + (size_t)b * N + c0;
+    // the pieces of the maximum, a lane each, and the first columns are on their way together
     float vmax = 0.0f;
-    for (int q = 0; q < src.n_amax; q++) vmax = fmaxf(vmax, src.amax[(size_t)b * src.n_amax + q]);
-    const int e = (int)((__float_as_uint(vmax) >> 23) & 0xFF);
-    int sh = (vmax > 0.0f && e != 255) ? 156 - e : 0;
-    sh = max(-126, min(126, sh));
-    const float mul = __uint_as_float((uint32_t)(127 + sh) << 23);
-    if (threadIdx.x == 0) *back_out = __uint_as_float((uint32_t)(127 - sh) << 23);
+    for (int q = threadIdx.x & 31; q < src.n_amax; q += 32) vmax = fmaxf(vmax, src.amax[(size_t)b * src.n_amax + q]);
     int lsum[LIN_LIMBS] = {0, 0, 0, 0};
-    constexpr int U = 4;
-    for (int j0 = threadIdx.x * 8; j0 < slice_cols; j0 += nth * 8 * U) {
-        float4 va[U], vc[U];
+    constexpr int U = XKNOWN_U;
+    float4 va[U], vc[U];
+    auto load = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int j = j0 + u * nth * 8;
             va[u] = vc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (j < valid) { va[u] = *reinterpret_cast<const float4*>(xb + j); vc[u] = *reinterpret_cast<const float4*>(xb + j + 4); }
         }
+    };
+    load(threadIdx.x * 8);
+    vmax = warp_max(vmax);
+    const int e = (int)((__float_as_uint(vmax) >> 23) & 0xFF);
+    int sh = (vmax > 0.0f && e != 255) ? 156 - e : 0;
+    sh = max(-126, min(126, sh));
+    const float mul = __uint_as_float((uint32_t)(127 + sh) << 23);
+    if (threadIdx.x == 0) *back_out = __uint_as_float((uint32_t)(127 - sh) << 23);
+    for (int j0 = threadIdx.x * 8; j0 < slice_cols; j0 += nth * 8 * U) {
+        if (j0 != threadIdx.x * 8) load(j0);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int j = j0 + u * nth * 8;
