@@ -119,7 +119,10 @@ __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc, 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
-template <int BITS, int NCG, int RT, int W, int STAGES>
+// XV: 4 XV columns of an activation per thread are held in registers while the block converts it. The instance with 4 takes 76
+// registers against 120: a block of the next launch then finds room beside this launch's two and has its weights under way earlier
+// (hidden size 4096, one token, 8-bit projections of 12 layers: 171.8 -> 161.1 us; 2048: 128.1 -> 115.6).
+template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
 __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p) {
     constexpr int R = RT * 16;                                // most rows per tile
     constexpr int RLD = lin_rld(NCG);                         // words per row of the reduction buffer
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p
     if (p.fused_x) {
         __shared__ XScratch xsc;
         for (int b = 0; b < p.B; b++)
-            xconvert_any(p.xsrc, p.N, b, kb_begin * XB, p.slice_kb * XB, XRows{xs + (size_t)b * LIN_LIMBS * p.xs_ld, p.xs_ld}, BITS == 4 ? 1 : 0,
+            xconvert_any<XV>(p.xsrc, p.N, b, kb_begin * XB, p.slice_kb * XB, XRows{xs + (size_t)b * LIN_LIMBS * p.xs_ld, p.xs_ld}, BITS == 4 ? 1 : 0,
                          xsc, s_back + b, s_xsum + b * LIN_LIMBS);
     } else {
         const uint4* gsrc = reinterpret_cast<const uint4*>(p.xpack + (size_t)ks * p.ncols * p.xs_ld);
@@ -404,9 +407,9 @@ __global__ void __launch_bounds__(256) linear_generic_kernel(LinTensor T, const 
     }
 }
 
-template <int BITS, int NCG, int RT, int W, int STAGES>
-int launch_mma(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
-    auto kern = linear_mma_kernel<BITS, NCG, RT, W, STAGES>;
+template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
+int launch_mma_x(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
+    auto kern = linear_mma_kernel<BITS, NCG, RT, W, STAGES, XV>;
     const size_t smem = (size_t)STAGES * RT * 16 * lin_ld(W) + (size_t)(BITS == 4 ? 2 : 1) * W * RT * 16 * lin_rld(NCG) * 4 + smem_tail;   // ring + reduction buffer + limbs
     if (smem > 48 * 1024) {
         static size_t allowed[64];                                 // per device, per kernel instance: raised only when a call needs more
@@ -418,6 +421,14 @@ int launch_mma(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail)
         }
     }
     return ibcu_launch(ctx, kern, dim3(grid), dim3(W * 32), smem, 1, true, p);
+}
+
+// a block that converts more than 4096 columns itself, and has to find their maximum first, holds up to 8192
+template <int BITS, int NCG, int RT, int W, int STAGES>
+int launch_mma(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
+    const bool longer = p.fused_x && p.xsrc.op != IBCU_PRO_KNOWN_MAX && p.slice_kb * (BITS == 8 ? 64 : 128) > 4 * 4 * W * 32;
+    if (NCG <= 2 && longer) return launch_mma_x<BITS, NCG, RT, W, STAGES, 8>(ctx, p, grid, smem_tail);
+    return launch_mma_x<BITS, NCG, RT, W, STAGES, 4>(ctx, p, grid, smem_tail);
 }
 
 // Eight warps and 512-byte stages; the ring is as deep as two resident blocks per SM allow.

@@ -359,10 +359,10 @@ __device__ __forceinline__ void xconvert_known(const XSource& src, int N, int b,
 }
 
 constexpr int XREG_V = 8;                                     // 32 columns per thread in registers
-template <class D>
+template <int V = XREG_V, class D>
 __device__ __forceinline__ void xconvert_any(const XSource& src, int N, int b, int c0, int slice_cols, const D& dst,
                                              int perm8, XScratch& sc, float* back_out, int* sum_out, int xregs = 1) {
     if (src.op == IBCU_PRO_KNOWN_MAX) { xconvert_known(src, N, b, c0, slice_cols, dst, perm8, sc, back_out, sum_out); return; }
-    if (xregs && slice_cols <= XREG_V * 4 * (int)blockDim.x) xconvert_regs<XREG_V>(src, N, b, c0, slice_cols, dst, perm8, sc, back_out, sum_out);
+    if (xregs && slice_cols <= V * 4 * (int)blockDim.x) xconvert_regs<V>(src, N, b, c0, slice_cols, dst, perm8, sc, back_out, sum_out);
     else xconvert(src, N, b, c0, slice_cols, dst, perm8, sc, back_out, sum_out);
 }

@@ -94,6 +94,15 @@ def test_tcgen05_linear_edges(backend, cpu_libs, bits, M, N, B):
     assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N", [4096, 4224, 8192, 8320])
+def test_row_lengths_converted_in_the_block(backend, cpu_libs, bits, N):
+    """The last and first row lengths of the two instances that convert one activation in the block, and of the conversion kernel."""
+    rng = np.random.default_rng(N + bits)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, 70, N, 1)
+    assert _cpu.close(backend.linear(w, s16, x, bits), oracle_linear(cpu_libs, w, s16, x, bits), RTOL, ATOL)
+
+
 @pytest.mark.parametrize("M,N,B", [(38000, 1664, 6), (25000, 1920, 32), (3000, 4224, 24)])
 def test_tcgen05_int4_teams(backend, M, N, B):
     """Odd numbers of 128-column blocks through rings that are used again, over one and two runs of rows: the two teams of
