@@ -112,7 +112,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
     int* wcnt = reinterpret_cast<int*>(wtab + (ACC ? (size_t)TC_EPI_WARPS * K * 8 : 0));
     TcShared* sh = reinterpret_cast<TcShared*>(wcnt + (ACC ? (size_t)TC_EPI_WARPS * K : 0));
     volatile int* abort_flag = &sh->abort_flag;
-    pdl_launch_dependents();
 
     if (tid == 0) {
         for (int s = 0; s < TC_STAGES; s++) { mbar_init(smem_u32(&sh->full_a[s]), TC_LOAD_WARPS); mbar_init(smem_u32(&sh->empty_a[s]), 1); }
@@ -125,6 +124,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
     if (warp == TC_MMA_WARP) {               // all 512 columns of tensor memory: two accumulator tiles of up to 256 columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        // Not before: a block of a later launch that moves in beside this one may allocate tensor memory too and keeps it until
+        // this launch has ended, so every block of this launch must hold its own first.
+        pdl_launch_dependents();
     }
     pdl_wait();
 

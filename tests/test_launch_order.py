@@ -1,0 +1,26 @@
+"""Order inside the kernels that hold tensor memory, read from their source (no GPU).
+
+A launch lets its successors start once every block of it has said so, and a successor's block keeps its tensor memory until
+this launch has ended. A kernel that allocates must therefore hold its columns before it says so: otherwise a successor's block on the
+same SM can take them first, and the two wait for one another in tcgen05.alloc and the dependency wait, which no bounded wait covers."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "libinferbit_b200", "csrc")
+SOURCES = [p for p in sorted(glob.glob(os.path.join(CSRC, "*.cu"))) if "tcgen05.alloc" in open(p).read()]
+
+
+def _code(path):
+    return re.sub(r"//[^\n]*", "", open(path).read())
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=[os.path.basename(p) for p in SOURCES])
+def test_successors_start_after_the_allocation(path):
+    kernels = [k for k in _code(path).split("__global__")[1:] if "tcgen05.alloc" in k]
+    assert kernels
+    for k in kernels:
+        starts = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", k)]
+        assert starts and k.index("tcgen05.alloc") < starts[0], "successors may start before this kernel's blocks hold their tensor memory"
