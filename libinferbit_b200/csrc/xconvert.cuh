@@ -343,6 +343,7 @@ __device__ __forceinline__ void xconvert_known(const XSource& src, int N, int b,
         }
     }
     if (!perm8) return;                                       // the limb sums only remove the nibble bias of INT4 weights
+    if (b > 0) __syncthreads();                               // a block that converts several in turn: threads 0..3 may still be adding up the sums of the one before
 #pragma unroll
     for (int l = 0; l < LIN_LIMBS; l++) {
         int v = lsum[l];

@@ -1,6 +1,6 @@
-"""Order inside the kernels that hold tensor memory, read from their source (no GPU).
+"""Order of steps inside kernels that no run on a GPU would show reliably, read from their source (no GPU).
 
-A launch lets its successors start once every block of it has said so, and a successor's block keeps its tensor memory until
+Tensor memory: a launch lets its successors start once every block of it has said so, and a successor's block keeps its tensor memory until
 this launch has ended. A kernel that allocates must therefore hold its columns before it says so: otherwise a successor's block on the
 same SM can take them first, and the two wait for one another in tcgen05.alloc and the dependency wait, which no bounded wait covers."""
 import glob
@@ -24,3 +24,14 @@ def test_successors_start_after_the_allocation(path):
     for k in kernels:
         starts = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", k)]
         assert starts and k.index("tcgen05.alloc") < starts[0], "successors may start before this kernel's blocks hold their tensor memory"
+
+
+def test_digit_sums_of_two_activations_are_kept_apart():
+    """A block may convert several activations one after the other through the same shared scratch. Each warp leaves its digit sums there
+    and threads 0 to 3 add them up: a barrier has to stand between that adding and the next activation's writes, so every
+    conversion needs one before it writes."""
+    code = _code(os.path.join(CSRC, "xconvert.cuh"))
+    bodies = [b for b in re.split(r"\n(?:template|__device__)", code) if "sc.sred[threadIdx.x >> 5][l] = v" in b]
+    assert len(bodies) == 3                                  # in registers, in a loop, with a known maximum
+    for b in bodies:
+        assert "__syncthreads()" in b[:b.index("sc.sred[threadIdx.x >> 5][l] = v")], b.strip().splitlines()[1]

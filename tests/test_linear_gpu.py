@@ -363,6 +363,27 @@ def test_silu_mul_amax_then_known_max_prologue(backend, cpu_libs, bits, M, N, B,
     assert _cpu.close(got2, oracle_linear(cpu_libs, w, s16, want_h, bits), 2e-3, 2e-4)
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,N,parts", [(64, 128, 3), (300, 2048, 5), (96, 14336, 28)])
+def test_known_max_of_two_activations(backend, bits, M, N, parts):
+    """A block that converts two activations with a known maximum one after the other gives bit for bit what two calls with one
+    give: the digit sums of the first are added up before the second overwrites their scratch."""
+    from libinferbit_b200 import _ffi
+    rng = np.random.default_rng(bits + M + N)
+    be, B = backend, 2
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    am = np.stack([[np.abs(p).max() for p in np.array_split(row, parts)] for row in x]).astype(np.float32)
+    dw, ds, dx, da = be.upload(w), be.upload(s16), be.upload(x), be.upload(am)
+    both, one = be.alloc(B * M * 4), be.alloc(B * M * 4)
+    for out, b0, n in ((both, 0, 2), (one, 0, 1), (one, 1, 1)):
+        t = LinearT(dw.ptr, ds.ptr, out.at(4 * b0 * M), M, M, 0, 0)
+        pro = _ffi.PrologueT(3, None, None, 0.0, da.at(4 * b0 * parts), parts)
+        for _ in range(20 if n == 2 else 1):
+            be._check(be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.at(4 * b0 * N), N, n, bits, C.byref(pro)))
+    be.sync()
+    assert np.array_equal(be.download(both, np.float32, B * M), be.download(one, np.float32, B * M))
+
+
 @pytest.mark.parametrize("bits,Ms,N,B", [
     (8, [7, 250, 3], 512, 1),            # ragged tensors: runs of rows never cross a tensor, tiles shorter than 16 rows
     (4, [1, 2, 5000, 33], 1024, 2),      # four tensors, one of them larger than the whole grid's worth of 4-row runs
