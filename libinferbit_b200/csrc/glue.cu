@@ -600,9 +600,11 @@ static bool attn_split_ok(const float* q, const float* k_cache, const float* v_c
            ((uintptr_t)k_cache & 15) == 0 && ((uintptr_t)v_cache & 15) == 0 && ((uintptr_t)q & 15) == 0;
 }
 
+constexpr size_t ATT_CMB_SMEM = 200 * 1024;      // what the merge step may hold of a head's chunk results
+static size_t combine_smem(int head_dim, int nsplit) { return (size_t)nsplit * (head_dim + 5) * sizeof(float); }
+
 static int combine_chunks(ibcu_ctx* ctx, float* out, int n_heads, int head_dim, int B, int nsplit, int grid_y, const int* pos0_dev, int want, int chunk_cap) {
-    const size_t csmem = ((size_t)grid_y * (head_dim + 4) + grid_y) * sizeof(float);
-    IBCU_REQUIRE(ctx, csmem <= 200 * 1024, "ibcu_attention: %d chunks of cache positions are more than the merge step holds", grid_y);
+    const size_t csmem = combine_smem(head_dim, grid_y);
     if (csmem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
     return ibcu_launch(ctx, attn_combine_kernel, dim3(n_heads, B), dim3(128), csmem, 1, true,
                        (const float*)ctx->scratch, out, n_heads, head_dim, nsplit, grid_y, pos0_dev, want, chunk_cap);
@@ -615,6 +617,8 @@ static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     const int cap = pos0_dev ? max_ctx : pos0 + B, tiles = (cap + ATT_TILE - 1) / ATT_TILE;
     int want = (2 * ctx->sm_count + n_kv_heads * gz - 1) / (n_kv_heads * gz);             // two blocks fit an SM
     if (want > tiles) want = tiles;
+    const int most = (int)(ATT_CMB_SMEM / combine_smem(head_dim, 1));                      // longer chunks where the merge step would not hold as many
+    if (want > most) want = most;
     int chunk, nsplit;
     att_plan_tiles(cap, want, chunk, nsplit);
     const size_t part = ((size_t)B * n_heads * want * (head_dim + 4) * sizeof(float) + 255) & ~(size_t)255;
@@ -669,6 +673,7 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
         grid_y = nsplit;
         chunk_cap = chunk;
     }
+    IBCU_REQUIRE(ctx, combine_smem(head_dim, grid_y) <= ATT_CMB_SMEM, "ibcu_attention: %d chunks of cache positions are more than the merge step holds", grid_y);
     const size_t pbytes = (size_t)B * n_heads * grid_y * (head_dim + 4) * sizeof(float);
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, pbytes);
     if (rc) return rc;

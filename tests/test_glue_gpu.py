@@ -109,6 +109,45 @@ def test_attention_of_several_positions(backend, cpu_libs, n_heads, n_kv, hd, po
     test_rope_kv_write_and_attention(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused)
 
 
+@pytest.mark.parametrize("entry", ["attention", "decode", "decode_at"])
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B", [(4, 1, 256, 8184, 8), (2, 1, 256, 9000, 4), (4, 2, 64, 9500, 5)])
+def test_attention_of_a_long_context(backend, n_heads, n_kv, hd, pos0, B, entry):
+    """One KV head of 256 values over thousands of positions: more blocks than the merge step could hold chunks of. Bound: a score
+    is a sum of hd products of size 1, off by at most hd 2^-23 times their magnitudes' mean (below 1e-4 of a unit here), and the result
+    is a mean of values of size 1 with those weights."""
+    rng = np.random.default_rng(n_heads + hd + pos0)
+    be, H, kv_dim, ctx, group = backend, n_heads * hd, n_kv * hd, pos0 + B, n_heads // n_kv
+    draw = lambda *shape: rng.standard_normal(shape, dtype=np.float32)
+    q, k, v, kc, vc = draw(B, H), draw(B, kv_dim), draw(B, kv_dim), draw(ctx, kv_dim), draw(ctx, kv_dim)
+    dq, dk, dv, dkc, dvc, dout, dpos = be.upload(q), be.upload(k), be.upload(v), be.upload(kc), be.upload(vc), be.alloc(B * H * 4), be.upload(np.array([pos0], np.int32))
+    lib, shape = be.lib, (n_heads, n_kv, hd)
+    if entry == "attention":
+        be._check(lib.ibcu_rope_kv_write(be.ctx, dq.ptr, dk.ptr, dv.ptr, dkc.ptr, dvc.ptr, *shape, pos0, B, 10000.0))
+        be._check(lib.ibcu_attention(be.ctx, dq.ptr, dkc.ptr, dvc.ptr, dout.ptr, *shape, pos0, B))
+    elif entry == "decode":
+        be._check(lib.ibcu_attention_decode(be.ctx, dq.ptr, dk.ptr, dv.ptr, dkc.ptr, dvc.ptr, dout.ptr, *shape, pos0, B, 10000.0))
+    else:
+        be._check(lib.ibcu_attention_decode_at(be.ctx, dq.ptr, dk.ptr, dv.ptr, dkc.ptr, dvc.ptr, dout.ptr, *shape, dpos.ptr, ctx, B, 10000.0))
+    be.sync()
+
+    def rope(rows, heads):
+        z = rows.astype(np.float64).reshape(B, heads, hd // 2, 2)
+        # angles as the kernels and the reference form them, in FP32: pos / theta^(2m / hd)
+        a = np.arange(pos0, pos0 + B, dtype=np.float32)[:, None] * (np.float32(1) / np.float32(10000.0) ** (np.arange(0, hd, 2, dtype=np.float32) / np.float32(hd)))
+        c, s_ = np.cos(a.astype(np.float64))[:, None], np.sin(a.astype(np.float64))[:, None]
+        return np.stack([z[..., 0] * c - z[..., 1] * s_, z[..., 0] * s_ + z[..., 1] * c], -1).reshape(B, heads * hd)
+
+    keys, vals, qr = kc.astype(np.float64), vc.astype(np.float64), rope(q, n_heads).reshape(B, n_heads, hd)
+    keys[pos0:], vals[pos0:] = rope(k, n_kv), v
+    got = be.download(dout, np.float32, B * H).reshape(B, n_heads, hd)
+    for h in range(n_heads):
+        kv = slice(h // group * hd, (h // group + 1) * hd)
+        sc = qr[:, h] @ keys[:, kv].T / np.sqrt(hd)
+        sc[np.arange(ctx)[None, :] > pos0 + np.arange(B)[:, None]] = -np.inf
+        p = np.exp(sc - sc.max(axis=1, keepdims=True))
+        assert np.allclose(got[:, h], (p / p.sum(axis=1, keepdims=True)) @ vals[:, kv], rtol=RTOL, atol=ATOL)
+
+
 def test_peer_window_single_rank():
     """The peer-window calls on a one-rank context: create, bump allocation with equal alignment, window
     memory survives ibcu_free, the gather of one rank is a no-op, and a second window is refused. (The
