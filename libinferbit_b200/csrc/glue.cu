@@ -3,6 +3,7 @@
 // residual add, softmax. They move O(hidden) or O(context) bytes per token; the design goal is few
 // launches and programmatic-dependent-launch friendliness, not bandwidth.
 #include "common.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -413,32 +414,36 @@ __global__ void __launch_bounds__(256) attn_batch_kernel(const float* q, const f
         }
         __syncwarp();
         const float4* vr = reinterpret_cast<const float4*>(vt + (size_t)(i & 1) * ATT_TILE * ld) + lane;
-        const int ld4 = ld / 4;
-#pragma unroll 2
-        for (int r = 0; r < ATT_TILE; r += 4) {
-            float4 p4[ATT_QPW];
+        const int ld4 = ld / 4, seen = pos0 + b0 - t0 - i * ATT_TILE;                       // position j of this warp sees the tile's rows 0 .. seen + j
+        // MASK: rows that some position of this warp does not see. Their weight is zero, but a value may be Inf or NaN, and zero
+        // times that must not reach an earlier position: such rows are left out, those that none of them sees with the loop's end.
+        auto weigh = [&](int r_begin, int r_end, auto mask) {
+            constexpr bool MASK = decltype(mask)::value;
+#pragma unroll (MASK ? 1 : 2)
+            for (int r = r_begin; r < r_end; r += 4) {
+                float4 p4[ATT_QPW];
 #pragma unroll
-            for (int j = 0; j < ATT_QPW; j++) p4[j] = *reinterpret_cast<const float4*>(pw + j * 32 + r);
+                for (int j = 0; j < ATT_QPW; j++) p4[j] = *reinterpret_cast<const float4*>(pw + j * 32 + r);
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (own0) {
-                    const float4 v = vr[(size_t)(r + u) * ld4];
+                for (int u = 0; u < 4; u++) {
 #pragma unroll
-                    for (int j = 0; j < ATT_QPW; j++) {
-                        const float pt = u == 0 ? p4[j].x : (u == 1 ? p4[j].y : (u == 2 ? p4[j].z : p4[j].w));
-                        acc[j][0].x = fmaf(pt, v.x, acc[j][0].x); acc[j][0].y = fmaf(pt, v.y, acc[j][0].y); acc[j][0].z = fmaf(pt, v.z, acc[j][0].z); acc[j][0].w = fmaf(pt, v.w, acc[j][0].w);
-                    }
-                }
-                if (own1) {
-                    const float4 v = vr[(size_t)(r + u) * ld4 + 32];
+                    for (int half = 0; half < 2; half++) {
+                        if (!(half ? own1 : own0)) continue;
+                        const float4 v = vr[(size_t)(r + u) * ld4 + 32 * half];
 #pragma unroll
-                    for (int j = 0; j < ATT_QPW; j++) {
-                        const float pt = u == 0 ? p4[j].x : (u == 1 ? p4[j].y : (u == 2 ? p4[j].z : p4[j].w));
-                        acc[j][1].x = fmaf(pt, v.x, acc[j][1].x); acc[j][1].y = fmaf(pt, v.y, acc[j][1].y); acc[j][1].z = fmaf(pt, v.z, acc[j][1].z); acc[j][1].w = fmaf(pt, v.w, acc[j][1].w);
+                        for (int j = 0; j < ATT_QPW; j++) {
+                            if (MASK && r + u > seen + j) continue;
+                            const float pt = u == 0 ? p4[j].x : (u == 1 ? p4[j].y : (u == 2 ? p4[j].z : p4[j].w));
+                            float4& a = acc[j][half];
+                            a.x = fmaf(pt, v.x, a.x); a.y = fmaf(pt, v.y, a.y); a.z = fmaf(pt, v.z, a.z); a.w = fmaf(pt, v.w, a.w);
+                        }
                     }
                 }
             }
-        }
+        };
+        const int all = max(0, min(ATT_TILE, (seen + 1) & ~3));
+        weigh(0, all, std::false_type());
+        weigh(all, min(ATT_TILE, seen + ATT_QPW), std::true_type());
         __syncthreads();                                                                    // the tile's buffer is free
         fetch(i + 2);
     }

@@ -148,6 +148,32 @@ def test_attention_of_a_long_context(backend, n_heads, n_kv, hd, pos0, B, entry)
         assert np.allclose(got[:, h], (p / p.sum(axis=1, keepdims=True)) @ vals[:, kv], rtol=RTOL, atol=ATOL)
 
 
+@pytest.mark.parametrize("entry", ["attention", "decode"])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B,at", [(8, 2, 64, 0, 6, 3), (4, 4, 128, 29, 9, 1), (4, 1, 256, 60, 8, 7), (8, 8, 64, 0, 40, 33)])
+def test_a_later_position_does_not_reach_an_earlier_one(backend, n_heads, n_kv, hd, pos0, B, at, bad, entry):
+    """Key and value of position `at` hold Inf or NaN: the positions before it do not see them and keep their bits, in every tile
+    and group of positions."""
+    rng = np.random.default_rng(hd + pos0 + B)
+    be, H, kv_dim, ctx = backend, n_heads * hd, n_kv * hd, pos0 + B
+    draw = lambda *shape: rng.standard_normal(shape, dtype=np.float32)
+    q, k, v, kc, vc = draw(B, H), draw(B, kv_dim), draw(B, kv_dim), draw(ctx, kv_dim), draw(ctx, kv_dim)
+    outs = []
+    for poison in (False, True):
+        if poison:
+            k[at], v[at] = bad, bad
+        kc[pos0:], vc[pos0:] = k, v
+        dq, dk, dv, dkc, dvc, dout = be.upload(q), be.upload(k), be.upload(v), be.upload(kc), be.upload(vc), be.alloc(B * H * 4)
+        if entry == "attention":
+            be._check(be.lib.ibcu_attention(be.ctx, dq.ptr, dkc.ptr, dvc.ptr, dout.ptr, n_heads, n_kv, hd, pos0, B))
+        else:
+            be._check(be.lib.ibcu_attention_decode(be.ctx, dq.ptr, dk.ptr, dv.ptr, dkc.ptr, dvc.ptr, dout.ptr, n_heads, n_kv, hd, pos0, B, 10000.0))
+        be.sync()
+        outs.append(be.download(dout, np.float32, B * H).reshape(B, H))
+    assert np.all(np.isfinite(outs[0])) and np.array_equal(outs[0][:at], outs[1][:at])
+    assert not np.any(np.isfinite(outs[1][at]))
+
+
 def test_peer_window_single_rank():
     """The peer-window calls on a one-rank context: create, bump allocation with equal alignment, window
     memory survives ibcu_free, the gather of one rank is a no-op, and a second window is refused. (The
