@@ -489,6 +489,10 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     }
     for (int i = n_tensors; i <= 4; i++) p.run_start[i] = nruns;
     if (S > 1 && nruns > slots) return IBCU_ERR_STATE;
+    // a block adds up its part of the columns in s32: weights of up to 128 (INT4, before the bias is taken off: 15) times digits of
+    // up to 128 stay exact for 131071 (1118481) columns; rows with longer parts go to the kernel that cuts them into slices
+    const long part_cols = (long)((p.nkb + S - 1) / S) * 128;
+    if ((part_cols < N ? part_cols : N) * (bits == 8 ? 128L : 15L) * 128L > 0x7fffffffL) return IBCU_ERR_STATE;
     // shared memory: half an SM's for runs of one tile, so that consecutive launches overlap; tensor memory likewise
     const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;

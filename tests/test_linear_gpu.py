@@ -94,6 +94,20 @@ def test_tcgen05_linear_edges(backend, cpu_libs, bits, M, N, B):
     assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
 
 
+@pytest.mark.parametrize("bits,N", [(8, 1048576 - 128), (8, 1048576), (8, 1048704), (4, 1048576)])
+def test_rows_longer_than_s32_sums_hold(backend, bits, N):
+    """Weights of -128 times digits of -128 reach 2^31 at 131072 columns of one s32 sum, which eight blocks of a row meet at 1048576 columns.
+    Every product is the same number, so the sum is N times it: exact up to the two roundings of the result."""
+    M, B = 3, 5
+    w = np.full((M, N), -128, np.int8) if bits == 8 else np.zeros((M, N // 2), np.uint8)
+    digit = np.float32(64 * 2 ** 24 - 128 * 2 ** 16 - 128 * 2 ** 8)                  # digits 64, -128, -128, 0
+    x = np.full((B, N), digit) * np.array([1, -1, 0.5, -0.5, 2], np.float32)[:, None]
+    s16 = _cpu.fp16_bits(np.array([2.0 ** -10, 2.0 ** -11, 2.0 ** -12]))
+    got = backend.linear(w, s16, x, bits)
+    want = x[:, :1].astype(np.float64) * N * (-128 if bits == 8 else -8) * s16.view(np.float16).astype(np.float64)
+    assert np.all(np.abs(got - want) <= 2.0 ** -23 * np.abs(want))
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("N", [4096, 4224, 8192, 8320])
 def test_row_lengths_converted_in_the_block(backend, cpu_libs, bits, N):
