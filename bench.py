@@ -114,6 +114,8 @@ class CpuBaseline:
             if not os.path.exists(port):
                 subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle"), "oracle"], check=True)
             self.kind, self.lib, self.threads = "port", C.CDLL(port), 1
+            for fn in (self.lib.ibo_matmul_int8, self.lib.ibo_matmul_int4):     # addresses come as plain integers: without types they would be cut to 32 bits
+                fn.restype, fn.argtypes = None, [C.c_void_p] * 4 + [C.c_int] * 2
 
     def _base(self, value, unit, sample, cores=None):
         return {"value": value, "unit": unit, "cores": self.threads if cores is None else cores, "kind": self.kind, "sample": sample}
