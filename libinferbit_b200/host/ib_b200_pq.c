@@ -212,6 +212,7 @@ static int km_download(void* dst, const void* src, size_t bytes) {
 
 static int km_begin(km_bufs* b, const float* X, int N, int D, int K, const float* centers) {
     const size_t xb = (size_t)N * D * sizeof(float), cb = (size_t)K * D * sizeof(float);
+    memset(b, 0, sizeof *b);                                       /* a step that fails leaves the rest empty */
     b->X = ib_b200_translate(X, xb);
     int rc = 0;
     if (!b->X) {
@@ -224,7 +225,7 @@ static int km_begin(km_bufs* b, const float* X, int N, int D, int K, const float
     if (!rc) rc = km_get(KM_SUMS, cb, &b->sums);
     if (!rc) rc = km_get(KM_COUNTS, (size_t)K * sizeof(int32_t), &b->counts);
     if (!rc) rc = km_get(KM_SCALARS, 32, &b->inertia);
-    b->shift = (char*)b->inertia + 16;
+    if (!rc) b->shift = (char*)b->inertia + 16;
     void *h, *d;
     if (!rc) rc = ib_b200_stage(3, cb, &h, &d);                   /* not the area the points are still leaving from */
     if (!rc) { memcpy(h, centers, cb); rc = ibcu_memcpy_h2d(g_ib.ctx, b->C, h, cb); }
