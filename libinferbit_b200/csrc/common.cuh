@@ -99,6 +99,10 @@ int ibcu_flush_gather_wait(ibcu_ctx* ctx);
 
 int ibcu_fail(ibcu_ctx* ctx, int code, const char* fmt, ...);
 
+// What a kernel's host part returns when the call is not one for it: nothing was launched, reserved or taken and the context's error
+// is untouched, so the caller takes another kernel. Positive, unlike every error, so that no failure can be taken for it.
+constexpr int IBCU_DECLINED = 1;
+
 #define IBCU_CHECK_CTX(ctx) do { if (!(ctx)) return IBCU_ERR_PARAM; } while (0)
 #define IBCU_CUDA(ctx, expr) do { cudaError_t e_ = (expr); if (e_ != cudaSuccess) \
     return ibcu_fail((ctx), IBCU_ERR_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e_), __FILE__, __LINE__); } while (0)

@@ -519,7 +519,7 @@ extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, 
     if (D == 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
         if (ctx->kmeans_path != IBCU_KMEANS_MMA_SYNC) {
             const int rc = ibcu_kmeans_assign_tc(ctx, X, N, C, K, idx, dist);
-            if (rc != IBCU_ERR_STATE) return rc;
+            if (rc != IBCU_DECLINED) return rc;
         }
     }
     if (D == 8 && K % 8 == 0 && K >= 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
@@ -616,7 +616,7 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
                              (const float*)part_sums, (const int32_t*)part_counts, (const double*)part_inertia, nblocks, (int)KD, K,
                              sums, counts, inertia, ex);
             if (rc) return rc;
-        } else if (rc != IBCU_ERR_STATE) return rc;
+        } else if (rc != IBCU_DECLINED) return rc;
     }
     if (!fused) {
         rc = ibcu_kmeans_assign(ctx, X, N, D, C, K, idx, dist);

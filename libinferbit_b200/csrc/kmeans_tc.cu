@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) assign_tc_kernel(const float* _
 
 }  // namespace
 
-// D == 8, K a multiple of 64 up to 256, 16-byte aligned X: the tensor-memory kernel. Returns IBCU_ERR_STATE without
+// D == 8, K a multiple of 64 up to 256, 16-byte aligned X: the tensor-memory kernel. Returns IBCU_DECLINED without
 // touching the context's error when the shape is not its own (the caller takes another kernel).
 static size_t tc_smem_bytes(int K, bool acc) {
     return 1024 + (size_t)3 * 2 * K * 16 + 2 * TC_A_CHUNK + (size_t)TC_STAGES * (TC_A_STAGE + TC_RAW_STAGE) + (size_t)K * 8 * sizeof(float) +
@@ -422,7 +422,7 @@ static size_t tc_smem_bytes(int K, bool acc) {
 }
 
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, const float* C, int K, int32_t* idx, float* dist) {
-    if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_ERR_STATE;
+    if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_DECLINED;
     const size_t smem = tc_smem_bytes(K, false);
     IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long ntile = (N + TC_TILE - 1) / TC_TILE;
@@ -437,9 +437,9 @@ int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, const float* C,
 // return convention as above.
 int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, const float* C, int K, int32_t* idx, float* dist,
                                      float* part_sums, int32_t* part_counts, double* part_inertia, int nblocks) {
-    if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_ERR_STATE;
+    if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_DECLINED;
     const size_t smem = tc_smem_bytes(K, true);
-    if (smem > 227 * 1024) return IBCU_ERR_STATE;
+    if (smem > 227 * 1024) return IBCU_DECLINED;
     IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return ibcu_launch(ctx, assign_tc_kernel<true>, dim3((unsigned)nblocks), dim3(TC_THREADS), smem, 1, true, X, N, C, K, idx, dist, ctx->kern_err,
                        part_sums, part_counts, part_inertia);

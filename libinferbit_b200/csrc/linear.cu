@@ -506,7 +506,7 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
     const bool many = B >= 5 || (B >= 3 && weight_bytes >= (20u << 20)) || (B == 2 && weight_bytes >= (32u << 20));
     if (ctx->linear_tc > 0 ? (bits == 4 || ctx->linear_tc > 1) : (ctx->linear_tc == 0 && many)) {
         const int rc_tc = ibcu_linear_tc(ctx, tensors, n_tensors, x, N, B, bits, pro, op);
-        if (rc_tc != IBCU_ERR_STATE) return rc_tc;
+        if (rc_tc != IBCU_DECLINED) return rc_tc;
     }
     if (B > 16) {
         // sixteen activations fill the eight column groups of one pass; more go in a second pass

@@ -447,12 +447,12 @@ int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, si
 
 }  // namespace
 
-// The call as the preparation kernel and the tcgen05 kernel. Returns IBCU_ERR_STATE without touching the context's error when
+// The call as the preparation kernel and the tcgen05 kernel. Returns IBCU_DECLINED without touching the context's error when
 // the call is not its own (the caller takes the other kernels).
 int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, const float* x, int N, int B, int bits, const ibcu_prologue_t* pro, int op) {
     EncodeFn encode = encode_fn();
     const int rowbytes = bits == 8 ? N : N / 2;
-    if (!encode || rowbytes % 16 || B > TQ_MAX_B) return IBCU_ERR_STATE;
+    if (!encode || rowbytes % 16 || B > TQ_MAX_B) return IBCU_DECLINED;
     long total_rows = 0;
     for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
     if (total_rows == 0) return IBCU_OK;
@@ -488,11 +488,11 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
         row += tensors[i].M;
     }
     for (int i = n_tensors; i <= 4; i++) p.run_start[i] = nruns;
-    if (S > 1 && nruns > slots) return IBCU_ERR_STATE;
+    if (S > 1 && nruns > slots) return IBCU_DECLINED;
     // a block adds up its part of the columns in s32: weights of up to 128 (INT4, before the bias is taken off: 15) times digits of
     // up to 128 stay exact for 131071 (1118481) columns; rows with longer parts go to the kernel that cuts them into slices
     const long part_cols = (long)((p.nkb + S - 1) / S) * 128;
-    if ((part_cols < N ? part_cols : N) * (bits == 8 ? 128L : 15L) * 128L > 0x7fffffffL) return IBCU_ERR_STATE;
+    if ((part_cols < N ? part_cols : N) * (bits == 8 ? 128L : 15L) * 128L > 0x7fffffffL) return IBCU_DECLINED;
     // shared memory: half an SM's for runs of one tile, so that consecutive launches overlap; tensor memory likewise
     const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;
@@ -529,15 +529,15 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
         plan((long)cap);
         while (p.sa > 1 && ring_of() > cap) p.sa--;
         while (p.sa < TQ_MAX_STAGES && recv > ring_of()) p.sa++;
-        if (recv > ring_of() || p.sa < 1) return IBCU_ERR_STATE;
+        if (recv > ring_of() || p.sa < 1) return IBCU_DECLINED;
         smem = ring_of();
     }
     if (bits == 4 && p.sa < nk) {
         // a ring that is used again: an even one, so that a stage always belongs to the same team of widening warps (a warp that
         // misses every other phase of a barrier cannot tell a phase from the next but one)
-        if (p.sa < 2) return IBCU_ERR_STATE;
+        if (p.sa < 2) return IBCU_DECLINED;
         p.sa &= ~1;
-        if (!p.recv_off && recv > ring_of()) return IBCU_ERR_STATE;
+        if (!p.recv_off && recv > ring_of()) return IBCU_DECLINED;
         smem = p.recv_off ? smem : ring_of();
     }
     smem = ((smem + 15) & ~(size_t)15) + sizeof(TqShared);
@@ -550,8 +550,18 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
         const cuuint32_t box[2] = { bits == 8 ? 128u : 64u, (cuuint32_t)R }, es[2] = { 1, 1 };
         if (encode(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(tensors[i].w), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return IBCU_ERR_STATE;
+            return IBCU_DECLINED;
     }
+    // The digits: a block per activation, or several when the maximum is known. Their room is there before a pending gather is taken:
+    // growing it may fail (under capture), and the call must then leave the gather to the next one.
+    int parts = 1;
+    if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
+    const int part_kb = (p.nkb + parts - 1) / parts;
+    parts = (p.nkb + part_kb - 1) / part_kb;
+    p.xparts = parts;
+    const size_t tiles = (size_t)p.nkb * b_block, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
+    int rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, tiles + scales + (size_t)B * parts * LIN_LIMBS * sizeof(int));
+    if (rc) return rc;
     GatherWait gw;
     ibcu_take_gather_wait_x(ctx, &gw, x, (size_t)B * N * sizeof(float));
     if (pro && pro->x2) ibcu_gather_wait_mark(ctx, &gw, pro->x2, (size_t)B * N * sizeof(float));
@@ -566,15 +576,6 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
             for (int i = 0; i < n_tensors; i++) p.t[i].win_off = (long)((const char*)tensors[i].out - ctx->win_base);
         }
     }
-    // the digits: a block per activation, or several when the maximum is known
-    int parts = 1;
-    if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
-    const int part_kb = (p.nkb + parts - 1) / parts;
-    parts = (p.nkb + part_kb - 1) / part_kb;
-    p.xparts = parts;
-    const size_t tiles = (size_t)p.nkb * b_block, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
-    int rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, tiles + scales + (size_t)B * parts * LIN_LIMBS * sizeof(int));
-    if (rc) return rc;
     int8_t* xtiles = (int8_t*)ctx->xpack;
     float* xscale = (float*)((char*)ctx->xpack + tiles);
     int* xsum = (int*)((char*)ctx->xpack + tiles + scales);

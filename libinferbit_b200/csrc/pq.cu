@@ -568,7 +568,7 @@ static int pq_run(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out,
     if (image) {
         int rc = ibcu_pq_tc(ctx, t, x, out, out_stride, B, false, acc, slots, N_SLOTS - 128, slots + N_SLOTS - 64, image);
         if (rc == IBCU_OK && t->n_outlier > 0) rc = pq_outliers(ctx, t, x, out, out_stride, B);
-        if (rc != IBCU_ERR_STATE) return rc;
+        if (rc != IBCU_DECLINED) return rc;
     }
     return pq_launch(ctx, t, x, out, out_stride, B, pl, acc, slots);
 }

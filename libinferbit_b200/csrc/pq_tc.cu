@@ -466,14 +466,14 @@ size_t ibcu_pq_tc_image_bytes(const ibcu_pq_t* t, int B) {
     return slabs * 32 * (t->G / 2) * 2 * pt_rows(B > PT_MAXB ? (B + 1) / 2 : B);
 }
 
-// Returns IBCU_ERR_STATE without touching the context's error when the tensor is not one for this kernel.
+// Returns IBCU_DECLINED without touching the context's error when the tensor is not one for this kernel.
 int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B, bool l1_only, unsigned long long* acc, unsigned* arrive, int max_counters,
                unsigned* amax_bits, void* image) {
     const int half = t->G >> 1;
     const bool two = t->K_l2 > 0 && !l1_only;
     const uintptr_t align = half == 4 ? 7 : 15;
-    if ((half != 4 && half != 8 && half != 16) || t->cb_chunk_stride || B > 32 || (((uintptr_t)t->codebook_l | (uintptr_t)t->codebook_r) & align)) return IBCU_ERR_STATE;
-    if (two && (((uintptr_t)t->codebook2_l | (uintptr_t)t->codebook2_r) & align)) return IBCU_ERR_STATE;
+    if ((half != 4 && half != 8 && half != 16) || t->cb_chunk_stride || B > 32 || (((uintptr_t)t->codebook_l | (uintptr_t)t->codebook_r) & align)) return IBCU_DECLINED;
+    if (two && (((uintptr_t)t->codebook2_l | (uintptr_t)t->codebook2_r) & align)) return IBCU_DECLINED;
     if (B > PT_MAXB) {
         const int b0 = (B + 1) / 2;
         const int rc = ibcu_pq_tc(ctx, t, x, out, out_stride, b0, l1_only, acc, arrive, max_counters, amax_bits, image);
@@ -486,7 +486,7 @@ int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, in
     p.nslab1 = (2 * C + 31) / 32;
     p.nslab = two ? 2 * p.nslab1 : p.nslab1;
     p.tiles = (t->M + 127) / 128;
-    if (4 * p.tiles > max_counters || (long)p.tiles * p.nslab > (1l << 28)) return IBCU_ERR_STATE;
+    if (4 * p.tiles > max_counters || (long)p.tiles * p.nslab > (1l << 28)) return IBCU_DECLINED;
     p.rows2 = two ? (t->K_l2 == 16 ? 16 : 256) : 0;          // one-byte codes may be any, 4-bit ones not above 15
     p.NC = pt_rows(B);
     // Tensor memory: two units of 128 columns of entries and two times up to 96 of sums. Shared memory: the codebook
@@ -497,7 +497,7 @@ int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, in
     auto fits = [&]() { return fixed + p.sc * PT_SLAB + 2 * x_stage <= cap; };
     p.sc = PT_MAX_C;
     if (!fits()) p.sc = 4;
-    if (!fits()) return IBCU_ERR_STATE;
+    if (!fits()) return IBCU_DECLINED;
     p.sx = (int)((cap - fixed - p.sc * PT_SLAB) / x_stage);
     if (p.sx > PT_MAX_X) p.sx = PT_MAX_X;
     p.tab_off = (int)(p.sx * x_stage);

@@ -5,7 +5,7 @@
 constexpr int IBCU_PQ_TC_ERR = 200;            // error codes of a launch that gave up a bounded wait: this + the wait; its accumulators are not zero then
 
 // acc, arrive: as the kernels of pq.cu leave them (zero between calls); max_counters: how many counters arrive has; amax_bits: room
-// for 32 words; image: ibcu_pq_tc_image_bytes(t, B) bytes for the activations' operand image, 16-byte aligned. IBCU_ERR_STATE:
+// for 32 words; image: ibcu_pq_tc_image_bytes(t, B) bytes for the activations' operand image, 16-byte aligned. IBCU_DECLINED:
 // not a tensor for this kernel, nothing has been launched.
 int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B, bool l1_only, unsigned long long* acc, unsigned* arrive, int max_counters,
                unsigned* amax_bits, void* image);

@@ -109,6 +109,38 @@ def test_rows_longer_than_s32_sums_hold(backend, bits, N):
 
 
 @pytest.mark.parametrize("bits", [8, 4])
+def test_capture_without_room_for_the_digits(bits):
+    """Under capture the digits of the tcgen05 kernel cannot be given more room: the call says so and launches nothing, it does not
+    go on with another kernel under a context that holds an error. Afterwards the same call, run once outside, can be captured."""
+    from libinferbit_b200 import Backend
+    rng = np.random.default_rng(bits)
+    M, N, B = 64, 2048, 5
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    with Backend(0) as be:
+        lib = be.lib
+        lib.ibcu_linear_use_tcgen05(be.ctx, -1)
+        other = be.linear(w, s16, x, bits)                   # the other kernel has its room now, which is less
+        lib.ibcu_linear_use_tcgen05(be.ctx, 2)
+        dw, ds, dx, do = be.upload(w), be.upload(s16), be.upload(x), be.alloc(B * M * 4)
+        t = LinearT(dw.ptr, ds.ptr, do.ptr, M, M, 0, 0)
+        call = lambda: lib.ibcu_linear(be.ctx, C.byref(t), 1, dx.ptr, N, B, bits)
+        g = C.c_int(-1)
+        be._check(lib.ibcu_graph_begin(be.ctx))
+        before = be.launches()
+        rc, launched, message = call(), be.launches() - before, lib.ibcu_last_error(be.ctx)
+        lib.ibcu_clear_error(be.ctx)
+        be._check(lib.ibcu_graph_end(be.ctx, C.byref(g)))
+        assert rc == -5 and launched == 0 and b"during graph capture" in message
+        be._check(call()); be.sync()
+        be._check(lib.ibcu_graph_begin(be.ctx))
+        be._check(call())
+        be._check(lib.ibcu_graph_end(be.ctx, C.byref(g)))
+        be._check(lib.ibcu_memset(be.ctx, do.ptr, 0xFF, B * M * 4))
+        be._check(lib.ibcu_graph_launch(be.ctx, g.value)); be.sync()
+        assert np.allclose(be.download(do, np.float32, B * M).reshape(B, M), other, rtol=2e-6, atol=1e-6 * float(np.abs(other).max()))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("N", [4096, 4224, 8192, 8320])
 def test_row_lengths_converted_in_the_block(backend, cpu_libs, bits, N):
     """The last and first row lengths of the two instances that convert one activation in the block, and of the conversion kernel."""
