@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <string.h>
 #include "../../include/ibcu.h"
+#include "smem_optin.h"
 
 #define IBCU_MAX_GRAPHS 16
 #define IBCU_MAX_EVENTS 16
@@ -112,6 +113,14 @@ constexpr int IBCU_DECLINED = 1;
 // holds instantiated graphs the outgrown buffer is kept (their kernels carry its address) until the
 // last graph is destroyed.
 int ibcu_reserve(ibcu_ctx* ctx, void** buf, size_t* have, size_t want);
+
+// Opt `kernel` in to `smem` bytes of dynamic shared memory; `opt` is that kernel's own, static at the place of the launch.
+template <typename K>
+static inline int ibcu_allow_smem(ibcu_ctx* ctx, SmemOptIn& opt, K* kernel, size_t smem) {
+    if (smem <= 48 * 1024) return IBCU_OK;
+    const int e = opt.raise(ctx->device, smem, [&](size_t n) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n); });
+    return e ? ibcu_fail(ctx, IBCU_ERR_CUDA, "%zu bytes of shared memory refused: %s", smem, cudaGetErrorString((cudaError_t)e)) : IBCU_OK;
+}
 
 // Launch `kernel` on the context's stream. With pdl_ok and ctx->pdl the launch carries the
 // programmatic-stream-serialization attribute: the kernel may start while its predecessor drains,

@@ -610,7 +610,8 @@ static size_t combine_smem(int head_dim, int nsplit) { return (size_t)nsplit * (
 
 static int combine_chunks(ibcu_ctx* ctx, float* out, int n_heads, int head_dim, int B, int nsplit, int grid_y, const int* pos0_dev, int want, int chunk_cap) {
     const size_t csmem = combine_smem(head_dim, grid_y);
-    if (csmem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, attn_combine_kernel, csmem)) return rc;
     return ibcu_launch(ctx, attn_combine_kernel, dim3(n_heads, B), dim3(128), csmem, 1, true,
                        (const float*)ctx->scratch, out, n_heads, head_dim, nsplit, grid_y, pos0_dev, want, chunk_cap);
 }
@@ -631,7 +632,8 @@ static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, part + rot);
     if (rc) return rc;
     const size_t smem = ((size_t)group * nb * ATT_QPW * (head_dim + 32) + 4 * (size_t)ATT_TILE * (head_dim + 4)) * sizeof(float);
-    if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if ((rc = ibcu_allow_smem(ctx, opt, attn_batch_kernel, smem))) return rc;
     GatherWait gw;
     ibcu_take_gather_wait(ctx, &gw);
     if (k) {
@@ -683,7 +685,8 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, pbytes);
     if (rc) return rc;
     const size_t smem = ((size_t)group * head_dim + group * 32 + 2 * (size_t)chunk_cap * (head_dim + 4)) * sizeof(float);
-    if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attn_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if ((rc = ibcu_allow_smem(ctx, opt, attn_partial_kernel, smem))) return rc;
     GatherWait gw;
     ibcu_take_gather_wait(ctx, &gw);
     rc = ibcu_launch(ctx, attn_partial_kernel, dim3(n_kv_heads, grid_y, B), dim3(32 * group), smem, 1, true,
@@ -704,7 +707,8 @@ extern "C" int ibcu_attention(ibcu_ctx* ctx, const float* q, const float* k_cach
     int cap = pos0 + B;
     size_t smem = ((size_t)cap + 8 * (size_t)head_dim) * sizeof(float);
     IBCU_REQUIRE(ctx, smem <= 200 * 1024, "ibcu_attention: context %d too long for one block's shared memory", cap);
-    if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, attention_kernel, smem)) return rc;
     return ibcu_launch(ctx, attention_kernel, dim3(n_heads, B), dim3(256), smem, 1, true, q, k_cache, v_cache, out,
                        n_heads, n_kv_heads, head_dim, pos0, cap);
 }

@@ -487,7 +487,8 @@ int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const floa
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
 #define KM_LAUNCH(DT) do { \
-        if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_exact_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        static SmemOptIn opt; \
+        if (int rc = ibcu_allow_smem(ctx, opt, assign_exact_kernel<DT>, smem)) return rc; \
         return ibcu_launch(ctx, assign_exact_kernel<DT>, dim3((unsigned)blocks), dim3(256), smem, 1, true, X, N, D, C, K, idx, dist, todo, n_todo); \
     } while (0)
     switch (D) {
@@ -524,7 +525,8 @@ extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, 
     }
     if (D == 8 && K % 8 == 0 && K >= 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
         const size_t smem = ((size_t)K * 16 + K + (size_t)K * 8 + 4) * sizeof(float);
-        if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        static SmemOptIn opt;
+        if (int rc = ibcu_allow_smem(ctx, opt, assign_filter_kernel, smem)) return rc;
         long tiles = (N + 15) / 16;
         long blocks = (tiles + 7) / 8;
         const long cap = (long)ctx->sm_count * 6;
@@ -556,7 +558,8 @@ static int kmeans_accumulate(ibcu_ctx* ctx, const float* X, long N, int D, int K
     double* part_inertia = (double*)ctx->scratch;
     float* part_sums = (float*)(part_inertia + ((nblocks + 1) & ~1L));
     int32_t* part_counts = (int32_t*)(part_sums + (size_t)nblocks * KD);
-    if (smem > 48 * 1024) IBCU_CUDA(ctx, cudaFuncSetAttribute(accumulate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if ((rc = ibcu_allow_smem(ctx, opt, accumulate_kernel, smem))) return rc;
     rc = ibcu_launch(ctx, accumulate_kernel, dim3((unsigned)nblocks), dim3(nwarp * 32), smem, 1, true,
                      X, N, D, K, idx, dist, chunk, part_sums, part_counts, part_inertia);
     if (rc) return rc;

@@ -424,7 +424,8 @@ static size_t tc_smem_bytes(int K, bool acc) {
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, const float* C, int K, int32_t* idx, float* dist) {
     if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_DECLINED;
     const size_t smem = tc_smem_bytes(K, false);
-    IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, assign_tc_kernel<false>, smem)) return rc;
     const long ntile = (N + TC_TILE - 1) / TC_TILE;
     long blocks = ntile < ctx->sm_count ? ntile : ctx->sm_count;
     if (blocks < 1) blocks = 1;
@@ -440,7 +441,8 @@ int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, cons
     if (K < 64 || K > 256 || (K & 63) || ((uintptr_t)X & 15)) return IBCU_DECLINED;
     const size_t smem = tc_smem_bytes(K, true);
     if (smem > 227 * 1024) return IBCU_DECLINED;
-    IBCU_CUDA(ctx, cudaFuncSetAttribute(assign_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, assign_tc_kernel<true>, smem)) return rc;
     return ibcu_launch(ctx, assign_tc_kernel<true>, dim3((unsigned)nblocks), dim3(TC_THREADS), smem, 1, true, X, N, C, K, idx, dist, ctx->kern_err,
                        part_sums, part_counts, part_inertia);
 }

@@ -411,15 +411,8 @@ template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
 int launch_mma_x(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
     auto kern = linear_mma_kernel<BITS, NCG, RT, W, STAGES, XV>;
     const size_t smem = (size_t)STAGES * RT * 16 * lin_ld(W) + (size_t)(BITS == 4 ? 2 : 1) * W * RT * 16 * lin_rld(NCG) * 4 + smem_tail;   // ring + reduction buffer + limbs
-    if (smem > 48 * 1024) {
-        static size_t allowed[64];                                 // per device, per kernel instance: raised only when a call needs more
-        size_t& have = allowed[ctx->device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-            have = smem;
-        }
-    }
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(W * 32), smem, 1, true, p);
 }
 

@@ -435,13 +435,8 @@ EncodeFn encode_fn() {
 template <int BITS, int T>
 int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
     auto kern = linear_tc_kernel<BITS, T>;
-    static size_t allowed[64];
-    size_t& have = allowed[ctx->device & 63];
-    if (smem > have) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(linear_tc_kernel, smem=%zu): %s", smem, cudaGetErrorString(e));
-        have = smem;
-    }
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(Tq<T>::THREADS), smem, p.S, true, maps, p);
 }
 

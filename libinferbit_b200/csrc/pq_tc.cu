@@ -444,13 +444,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
 template <int HALF, int NG>
 int launch_pt(ibcu_ctx* ctx, const PtParams& p, int grid, size_t smem) {
     auto kern = pq_tc_kernel<HALF, NG>;
-    static size_t allowed[64];
-    size_t& have = allowed[ctx->device & 63];
-    if (smem > have) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(pq_tc_kernel, smem=%zu): %s", smem, cudaGetErrorString(e));
-        have = smem;
-    }
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(PT_THREADS), smem, 1, true, p);
 }
 template <int HALF>

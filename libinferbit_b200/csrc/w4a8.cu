@@ -305,15 +305,8 @@ __global__ void __launch_bounds__(WT_W * 32) w4a8_mma_kernel(const WtParams p) {
 template <int STAGES, int RT, bool XF>
 int w4a8_mma_launch_x(ibcu_ctx* ctx, const WtParams& p, int grid, size_t smem) {
     auto kern = w4a8_mma_kernel<STAGES, RT, XF>;
-    if (smem > 48 * 1024) {
-        static size_t allowed[64];
-        size_t& have = allowed[ctx->device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return ibcu_fail(ctx, IBCU_ERR_CUDA, "cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-            have = smem;
-        }
-    }
+    static SmemOptIn opt;
+    if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(WT_W * 32), smem, 1, true, p);
 }
 

@@ -1,4 +1,5 @@
 """Error paths of the host layer that need no GPU: its sources compiled into a small program without a context."""
+import glob
 import os
 import subprocess
 
@@ -27,3 +28,49 @@ def test_kmeans_buffers_are_empty_when_a_step_fails(tmp_path):
                     f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}", "-lm", "-lpthread"], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stdout)
+
+
+OPTIN = r"""
+#include "smem_optin.h"
+#include <chrono>
+#include <stdio.h>
+#include <thread>
+int main() {
+    // two threads with a context each on one device: one of them asks first and takes its time in the driver
+    for (int first = 0; first < 2; first++) {
+        SmemOptIn opt;
+        std::atomic<size_t> set{0};
+        size_t seen[2];
+        const size_t want[2] = { 100, 150 };
+        auto ask = [&](int i) {
+            opt.raise(0, want[i], [&](size_t n) { std::this_thread::sleep_for(std::chrono::milliseconds(i == first ? 200 : 1)); set = n; return 0; });
+            seen[i] = set;                            // what a launch of this thread would meet
+        };
+        std::thread a(ask, first);
+        std::this_thread::sleep_for(std::chrono::milliseconds(50));
+        std::thread b(ask, 1 - first);
+        a.join(); b.join();
+        if (seen[0] < 100 || seen[1] < 150 || set != 150) { printf("%zu %zu %zu\n", seen[0], seen[1], set.load()); return 1; }
+        if (opt.raise(0, 160, [](size_t) { return 7; }) != 7) return 2;               // a refusal is passed on and not remembered
+        if (opt.raise(0, 155, [&](size_t n) { set = n; return 0; }) != 0 || set != 155) return 3;
+        if (opt.raise(1, 10, [&](size_t n) { set = n; return 0; }) != 0 || set != 10) return 4;     // another device has its own
+    }
+    return 0;
+}
+"""
+
+
+def test_shared_memory_opt_in_only_grows(tmp_path):
+    src, exe = tmp_path / "optin.cpp", tmp_path / "optin"
+    src.write_text(OPTIN)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-Werror", f"-I{LIB}/csrc", "-o", str(exe), str(src), "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout)
+
+
+def test_every_opt_in_goes_through_it():
+    """A kernel is opted in to the size of a call only through the growing opt-in; two others ask once for a fixed size."""
+    for path in glob.glob(os.path.join(LIB, "csrc", "*.cu")):
+        code = open(path).read()
+        if "cudaFuncAttributeMaxDynamicSharedMemorySize" in code:
+            assert "std::call_once" in code and "(int)smem)" not in code and "(int)csmem)" not in code, path
