@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
 }
 
 // ── split attention for several positions ───────────────────────────────────────────────
-// With four or more positions per call the kernel above repeats too much: every block stages its K and V rows for one
+// With many positions per call the kernel above repeats too much: every block stages its K and V rows for one
 // position's queries, rotates all new K rows for itself (64 sines per row and head: at 32 positions most of its 45 us), and
 // its two tiles of up to 128 rows leave one block per SM. Here rope_stage_kernel rotates the queries (into scratch) and the
 // new K rows (into the cache, with their V rows) once, the angles of a position shared by all its heads; then
@@ -616,7 +616,7 @@ static int combine_chunks(ibcu_ctx* ctx, float* out, int n_heads, int head_dim, 
                        (const float*)ctx->scratch, out, n_heads, head_dim, nsplit, grid_y, pos0_dev, want, chunk_cap);
 }
 
-// The same for four or more positions (see attn_batch_kernel). k NULL: q is rotated and the cache complete.
+// The same for four and more positions (see attn_batch_kernel, attn_batched_pays). k NULL: q is rotated and the cache complete.
 static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float* v_cache, float* out, int n_heads, int n_kv_heads, int head_dim,
                            int pos0, int B, const float* k, const float* v, float theta, const int* pos0_dev, int max_ctx) {
     const int group = n_heads / n_kv_heads, nb = ATT_GMAX / group, gz = (B + nb * ATT_QPW - 1) / (nb * ATT_QPW);
@@ -650,6 +650,18 @@ static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     return combine_chunks(ctx, out, n_heads, head_dim, B, nsplit, want, pos0_dev, want, 0);
 }
 
+// Whether four and more positions go to the three launches of attention_batch. Those cost a launch more than the two of the fused
+// kernel, which does everything once per position instead: every block stages its chunk of the cache and rotates all new keys for
+// itself. So the batched kernels pay where that is much: from 24000 staged values per SM on (a cache whose length only the device
+// knows is taken as half full), or where the new keys are many for the warps of a block. Measured over 4 to 32 positions, 10 shapes
+// and contexts up to 8192, fused / batched, us per call in a graph: 32 heads of 128 over 8, four positions after 16 7.7 / 13.4,
+// after 1000 22.8 / 18.6; 16 positions after 60 13.1 / 16.3, after 500 37.4 / 20.2; 32 heads over 32, 32 positions 187 / 17.6. The
+// line is the one that loses least (1 % on the mean against the better of the two; always the batched one 16 %, always the fused 97 %).
+static bool attn_batched_pays(const ibcu_ctx* ctx, int n_kv, int group, int hd, int B, int pos0, bool at, int max_ctx) {
+    const double staged = (double)n_kv * hd * B * (at ? max_ctx / 2 : pos0 + B);
+    return staged >= 24000.0 * ctx->sm_count || (long)B * hd >= 800L * group;
+}
+
 // k_new / v_new NULL: q is rotated already and the cache holds rows 0..pos0+B-1. Otherwise the fused decode step.
 // pos0_dev NULL: the position is the argument pos0 and the grid is cut for it. Otherwise the position is read
 // on the device and the grid, shared memory and scratch are sized for max_ctx positions, so that one
@@ -657,8 +669,6 @@ static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float*
 static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float* v_cache, float* out,
                            int n_heads, int n_kv_heads, int head_dim, int pos0, int B, const float* k_new, const float* v_new, float theta,
                            const int* pos0_dev, int max_ctx) {
-    // four positions fill a warp of the batched kernel; with fewer the fused kernel's two launches are quicker than three
-    if (B >= ATT_QPW) return attention_batch(ctx, q, k_cache, v_cache, out, n_heads, n_kv_heads, head_dim, pos0, B, k_new, v_new, theta, pos0_dev, max_ctx);
     const int group = n_heads / n_kv_heads;
     // Enough blocks to cover the machine several times over: a block's shared memory grows with its chunk of positions (two
     // tiles of chunk x head_dim floats), so short chunks let several blocks share an SM; with B activations every chunk
@@ -680,11 +690,14 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
         grid_y = nsplit;
         chunk_cap = chunk;
     }
+    const size_t smem = ((size_t)group * head_dim + group * 32 + 2 * (size_t)chunk_cap * (head_dim + 4)) * sizeof(float);
+    // four positions fill a warp of the batched kernel; it also takes what the fused kernel's tiles or the merge step would not hold
+    if (B >= ATT_QPW && (attn_batched_pays(ctx, n_kv_heads, group, head_dim, B, pos0, pos0_dev != nullptr, max_ctx) || smem > 227 * 1024 || combine_smem(head_dim, grid_y) > ATT_CMB_SMEM))
+        return attention_batch(ctx, q, k_cache, v_cache, out, n_heads, n_kv_heads, head_dim, pos0, B, k_new, v_new, theta, pos0_dev, max_ctx);
     IBCU_REQUIRE(ctx, combine_smem(head_dim, grid_y) <= ATT_CMB_SMEM, "ibcu_attention: %d chunks of cache positions are more than the merge step holds", grid_y);
     const size_t pbytes = (size_t)B * n_heads * grid_y * (head_dim + 4) * sizeof(float);
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, pbytes);
     if (rc) return rc;
-    const size_t smem = ((size_t)group * head_dim + group * 32 + 2 * (size_t)chunk_cap * (head_dim + 4)) * sizeof(float);
     static SmemOptIn opt;
     if ((rc = ibcu_allow_smem(ctx, opt, attn_partial_kernel, smem))) return rc;
     GatherWait gw;

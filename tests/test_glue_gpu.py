@@ -109,6 +109,31 @@ def test_attention_of_several_positions(backend, cpu_libs, n_heads, n_kv, hd, po
     test_rope_kv_write_and_attention(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused)
 
 
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B", [(32, 32, 128, 300, 4), (8, 8, 64, 33, 13), (30, 10, 40, 900, 11), (8, 1, 256, 960, 16), (20, 4, 64, 980, 15)])
+def test_attention_of_several_positions_with_much_to_stage(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused):
+    """As above where the three launches are taken: the contexts are long enough, or the new keys many enough, for them to pay. (Positions
+    stay below 1000: two libraries' angles differ by a unit in the last place, 6e-5 there, which is what the bar leaves room for.)"""
+    before = backend.launches()
+    test_rope_kv_write_and_attention(backend, cpu_libs, n_heads, n_kv, hd, pos0, B, fused)
+    assert backend.launches() - before == 3
+
+
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B,launches", [
+    (32, 8, 128, 0, 4, 2), (32, 8, 128, 60, 16, 2), (32, 8, 128, 1000, 4, 3), (32, 32, 128, 0, 6, 2), (32, 32, 128, 0, 7, 3),   # values to stage; new keys
+    (2, 1, 256, 9000, 4, 3),             # more than the fused kernel holds
+    (32, 8, 128, 5000, 3, 2),            # three positions stay with it
+])
+def test_attention_launches(backend, n_heads, n_kv, hd, pos0, B, launches):
+    """Few positions over a short context take the two launches of the fused kernel, much work the three of the batched one."""
+    be, H, kv = backend, n_heads * hd, n_kv * hd
+    q, k, v, kc, vc, o = (be.upload(np.zeros(n, np.float32)) for n in (B * H, B * kv, B * kv, (pos0 + B) * kv, (pos0 + B) * kv, B * H))
+    before = be.launches()
+    be._check(be.lib.ibcu_attention_decode(be.ctx, q.ptr, k.ptr, v.ptr, kc.ptr, vc.ptr, o.ptr, n_heads, n_kv, hd, pos0, B, 10000.0))
+    assert be.launches() - before == launches
+    be.sync()
+
+
 @pytest.mark.parametrize("entry", ["attention", "decode", "decode_at"])
 @pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B", [(4, 1, 256, 8184, 8), (2, 1, 256, 9000, 4), (4, 2, 64, 9500, 5)])
 def test_attention_of_a_long_context(backend, n_heads, n_kv, hd, pos0, B, entry):
@@ -150,7 +175,8 @@ def test_attention_of_a_long_context(backend, n_heads, n_kv, hd, pos0, B, entry)
 
 @pytest.mark.parametrize("entry", ["attention", "decode"])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
-@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B,at", [(8, 2, 64, 0, 6, 3), (4, 4, 128, 29, 9, 1), (4, 1, 256, 60, 8, 7), (8, 8, 64, 0, 40, 33)])
+@pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B,at", [(8, 2, 64, 0, 6, 3), (4, 4, 128, 29, 9, 1), (4, 1, 256, 60, 8, 7), (8, 8, 64, 0, 40, 33),
+                                                        (8, 2, 64, 4700, 6, 3), (4, 1, 256, 2000, 8, 7)])
 def test_a_later_position_does_not_reach_an_earlier_one(backend, n_heads, n_kv, hd, pos0, B, at, bad, entry):
     """Key and value of position `at` hold Inf or NaN: the positions before it do not see them and keep their bits, in every tile
     and group of positions."""
