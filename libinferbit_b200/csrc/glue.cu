@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(256) attn_batch_kernel(const float* q, const f
         // times that must not reach an earlier position: such rows are left out, those that none of them sees with the loop's end.
         auto weigh = [&](int r_begin, int r_end, auto mask) {
             constexpr bool MASK = decltype(mask)::value;
-#pragma unroll (MASK ? 1 : 2)
+#pragma unroll 2
             for (int r = r_begin; r < r_end; r += 4) {
                 float4 p4[ATT_QPW];
 #pragma unroll
