@@ -550,15 +550,24 @@ static size_t pq_scratch_bytes(const PqPlan& pl) { return PQ_COUNTER_BYTES + pl.
 
 constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;         // scratch of the allocation-free entry point (see there)
 
-// Whether a call takes the tensor-core kernel (pq_tc.cu), the same for both entry points, so that they agree to the bit. Measured in a
-// chain of calls, us, table kernels / tensor cores. Entries of 4 and 16 values: always ahead (2048 x 2048, one activation 13.8 / 7.9 and
-// 19.6 / 7.9; 4096 x 8192, eight 49 / 17.6 and 37 / 23). Entries of 8: one activation 11.2 / 18.0 at 4096 x 14336; two 16.4 / 18.2
-// there, 11.2 / 11.2 at 4096 x 4096, 10.0 / 7.2 at 1500 x 2000; three 21.9 / 19.0, eight 28.1 / 21.2, sixteen 46 / 27. Outlier columns
-// make its preparation gather: 17.6 / 18.6 at four activations, 24.7 / 22.1 at eight.
+// Whether a call takes the tensor-core kernel (pq_tc.cu), the same for both entry points, so that they agree to the bit.
+// The table kernels pay per pair of activations: a table per slab, then a table read per code. The tensor cores pay per code whatever the
+// activations, G / 2 weights each, and a preparation launch. So what is looked up (`work`: weights, over both levels) decides.
+// Both measured over M 1024 to 32000, N 1024 to 14336, one to eight activations, with second levels and outlier columns, direct and in
+// graphs; us, tables / tensor cores:
+//   entries of 4: from two activations on always ahead (8192 x 8192 31 / 23); one: 4096 x 8192 16.8 / 15.5, 14336 x 8192 29.5 / 32.7
+//   entries of 16: up to 62 M weights per activation; one: 4096 x 8192 22.0 / 17.5, 14336 x 8192 24.2 / 33.9, 14336 x 14336 27.3 / 50.7;
+//     eight: 32000 x 8192 103 / 70
+//   entries of 8: one never (4096 x 14336 10.8 / 17.9), three and more always (26.3 / 18.8); two where the rows are
+//     short or few: 14336 x 2048 17.0 / 13.5, 4096 x 4096 11.8 / 11.5, 4096 x 8192 13.4 / 14.9
+// The loss against the better of the two is 0.1 % on the mean and at most 30 %.
 static bool pq_takes_tc(const ibcu_pq_t* t, int B) {
-    if (t->G != 16) return true;
-    if (t->n_outlier > 0) return B >= 5;
-    return B >= 3 || (B == 2 && (long)t->M * t->N <= 20000000l);
+    const double cols = (double)(t->N - t->n_outlier) * (t->K_l2 > 0 ? 2 : 1), work = cols * t->M;
+    if (t->G == 32) return work <= 62e6 * B;
+    if (t->G == 8) return B >= 2 || work <= 50e6;
+    if (B != 2) return B > 2;
+    if (t->n_outlier > 0) return cols <= 1024 || work <= 10e6;          // its preparation gathers then
+    return cols <= 2048 || work <= (t->K_l2 > 16 ? 9e6 : 17.5e6);
 }
 // counters and accumulators at base (counter area: arrival counters, the top-K head's own 128 slots from the end, max |x| in the last 64)
 static int pq_run(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, int out_stride, int B, const PqPlan& pl, void* base, void* image) {

@@ -363,3 +363,22 @@ def test_linearity_at_full_size(backend):
     assert np.array_equal(backend.pq_matmul(t, 2.0 * x[:1]), 2.0 * f1) and _cpu.close(f1[0], fx[0], 1e-5, 1e-5)
     fs = backend.pq_matmul(t, (x[0] + x[1])[None, :])
     assert _cpu.close(fs[0], fx[0] + fx[1], 1e-3, 1e-4)
+
+
+@pytest.mark.parametrize("M,N,G,B,launches", [
+    (8192, 8192, 32, 1, 1), (4096, 8192, 32, 1, 2),          # entries of 16, one activation: 67 and 34 million weights
+    (8192, 7168, 8, 1, 1), (4096, 8192, 8, 1, 2), (8192, 7168, 8, 2, 2),
+    (4096, 8192, 16, 2, 2), (4096, 4096, 16, 2, 2), (8192, 2048, 16, 2, 2), (4096, 4096, 16, 1, 1),
+])
+def test_pq_kernel_by_work(backend, M, N, G, B, launches):
+    """Which kernel takes a call: one launch of the table kernel (two with two activations: their maxima), or the tensor cores' two. Either
+    way an activation's result is that of a call of six, which the tensor cores take: both are off by about 1e-7 of the result's root
+    mean square per element, at most ten times that."""
+    rng = np.random.default_rng(M + N + G + B)
+    d = _cpu.make_pq_case_ex(rng, M, N, G, 256, 0, 0, B)
+    t = backend.make_pq_ex(d)
+    before = backend.launches()
+    got = backend.pq_matmul(t, d["x"])
+    assert backend.launches() - before == launches
+    want = backend.pq_matmul(t, np.concatenate([d["x"]] * 6)[:6])[:B]
+    assert np.max(np.abs(got - want)) <= 2e-6 * np.sqrt(np.mean(want.astype(np.float64) ** 2))
