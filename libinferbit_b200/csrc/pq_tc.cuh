@@ -31,7 +31,10 @@ __device__ __forceinline__ unsigned pq_absmax_bits(const float* xb, const int* i
     for (int j0 = tid; j0 < n; j0 += U * T) {
         unsigned v[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) v[u] = j0 + u * T < n ? __float_as_uint(xb[inner ? inner[j0 + u * T] : j0 + u * T]) & 0x7fffffffu : 0u;
+        for (int u = 0; u < U; u++) {                         // past the end: the last value again, so that no load waits for a test
+            const int j = min(j0 + u * T, n - 1);
+            v[u] = __float_as_uint(xb[inner ? inner[j] : j]) & 0x7fffffffu;
+        }
 #pragma unroll
         for (int u = 0; u < U; u++) m = max(m, v[u]);
     }
