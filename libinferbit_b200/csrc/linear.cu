@@ -435,6 +435,97 @@ int dispatch_shape(ibcu_ctx* ctx, const LinearParams& p, int grid, int rt, int s
     return launch_mma<BITS, NCG, 1, 8, 4>(ctx, p, grid, smem_tail);
 }
 
+// How linear_mma_kernel takes a call of up to 16 activations.
+struct LinPlan {
+    int ncols, ncg, nkb, rt, stages;           // limb columns and groups of eight of them, 64-byte k-blocks per row, 16-row MMA tiles per tile of rows, ring depth
+    int slice_kb, nks, xs_ld;                  // k-blocks per column slice, slices, bytes per limb row
+    size_t piece_smem;                         // bytes of a slice's limbs
+    int fit, rows_per_block, nblk;             // blocks per SM, longest run of rows, blocks per slice
+    int blk_start[4], rows_per[4];             // of every tensor
+    bool fused;                                // every block converts the activations for itself
+};
+
+LinPlan lin_plan(const ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, long total_rows, int N, int B, int bits, int op) {
+    LinPlan pl;
+    const int rowbytes = bits == 8 ? N : N / 2;
+    pl.ncols = B * LIN_LIMBS;
+    const int groups = (pl.ncols + 7) / 8;
+    pl.ncg = groups <= 1 ? 1 : (groups <= 2 ? 2 : (groups <= 4 ? 4 : 8));
+    pl.nkb = (rowbytes + 63) / 64;
+    const int xk = bits == 8 ? 64 : 128;
+    const int xpad = bits == 8 ? 64 : 16;                     // keeps limb rows of neighbouring columns on different banks
+    // Rows are dealt out evenly: every block of the persistent grid owns one contiguous run of rows and
+    // walks it in tiles of up to R = 16 or 32 rows. 32-row tiles once a block's run is longer than 16.
+    const int w = 8;                                          // warps per block; two blocks share an SM
+    pl.rt = (pl.ncg >= 4 || total_rows <= 16L * 2 * ctx->sm_count) ? 1 : 2;
+    const int R = 16 * pl.rt;
+    // Shared memory per block: stage ring + reduction buffer + the slice's limbs. Columns are
+    // split over several blocks only when the limbs of a whole row do not fit.
+    const int kbs = w;
+    const int LIN_LD = lin_ld(w);
+    // ring depth: the deeper ring when two blocks per SM still fit with it, else the shallower one
+    const size_t red_bytes = (size_t)(bits == 4 ? 2 : 1) * w * R * lin_rld(pl.ncg) * 4;
+    const size_t whole_row_pieces = (size_t)pl.ncols * ((size_t)pl.nkb * xk + xpad);
+    pl.stages = pl.rt == 2 ? 6 : 8;
+    if (2 * ((size_t)pl.stages * R * LIN_LD + red_bytes + whole_row_pieces + 2048) > 227 * 1024) pl.stages = 4;
+    const size_t fixed_smem = (size_t)pl.stages * R * LIN_LD + red_bytes + 1024;
+    const size_t smem_cap = 200 * 1024;
+    long piece_budget = (long)smem_cap - (long)fixed_smem;
+    int max_slice_kb = (int)((piece_budget / pl.ncols - xpad) / xk) / kbs * kbs;
+    if (max_slice_kb < kbs) max_slice_kb = kbs;
+    pl.slice_kb = (pl.nkb + kbs - 1) / kbs * kbs;             // whole stages per slice
+    if (pl.slice_kb > max_slice_kb) pl.slice_kb = max_slice_kb;
+    pl.nks = (pl.nkb + pl.slice_kb - 1) / pl.slice_kb;
+    pl.xs_ld = pl.slice_kb * xk + xpad;
+    pl.piece_smem = (((size_t)pl.ncols * pl.xs_ld) + 15) & ~(size_t)15;
+    // persistent grid: as many blocks as fit on the machine at once, a multiple of nks, at most one per item
+    pl.fit = (int)((227 * 1024) / (fixed_smem + pl.piece_smem + 1024));
+    if (pl.fit < 1) pl.fit = 1;
+    if (pl.fit > 4) pl.fit = 4;
+    const int slots = pl.fit * ctx->sm_count;
+    int per_slice = slots / pl.nks;
+    if (per_slice < 1) per_slice = 1;
+    // every tensor gets blocks in proportion to its rows, and its rows are dealt out evenly among them;
+    // the run length grows until all blocks are resident at once
+    pl.rows_per_block = (int)((total_rows + per_slice - 1) / per_slice);
+    if (pl.rows_per_block < 4) pl.rows_per_block = 4;
+    for (;; pl.rows_per_block++) {
+        pl.nblk = 0;
+        for (int i = 0; i < n_tensors; i++) pl.nblk += (tensors[i].M + pl.rows_per_block - 1) / pl.rows_per_block;
+        if (pl.nblk <= per_slice || pl.rows_per_block >= total_rows) break;
+    }
+    pl.nblk = 0;
+    for (int i = 0; i < n_tensors; i++) {
+        const int n = (tensors[i].M + pl.rows_per_block - 1) / pl.rows_per_block;
+        pl.blk_start[i] = pl.nblk;
+        pl.rows_per[i] = n ? (tensors[i].M + n - 1) / n : 0;
+        pl.nblk += n;
+    }
+    // Cheap conversions are done by every block of the main kernel for itself (no extra launch, no
+    // dependency chain); expensive ones (SiLU, several activations, long rows) once, by xprep_kernel.
+    pl.fused = op != IBCU_PRO_SILU_MUL && (long)B * pl.slice_kb * xk <= 8192 && pl.nks == 1;
+    if (op == IBCU_PRO_KNOWN_MAX && pl.nks == 1 && B <= 2) pl.fused = true;          // no reduction: cheap at any row length
+    return pl;
+}
+
+// Which kernel takes a call of 2 to 16 activations: the time of either, in us, from what it does. The coefficients are least squares
+// (relative error 6 %) over 2296 calls on a B200, direct and in graphs: 2, 3, 4, 5, 6, 8, 12 and 16 activations, 512 to 14336 columns, 512
+// to 32000 rows in one to three tensors, 4 and 8 bits. The choice is 0.2 % behind the better kernel on the mean and more than 5 % behind
+// it in one call of 60; choosing by the number of activations and the bytes of the weights was 2.2 % behind, up to 95 %.
+// mma.sync kernel: per block the MMAs of its tiles, the weights, and a reduction per tile; the conversion in the block, or a launch ahead.
+double lin_mma_us(const LinPlan& pl, int N, int B, int bits) {
+    const int R = 16 * pl.rt, tiles = (pl.rows_per_block + R - 1) / R, stages = ((pl.slice_kb < pl.nkb ? pl.slice_kb : pl.nkb) + 7) / 8;
+    const double i4 = bits == 4 ? 1.0 : 0.0;
+    double us = 1.73 + (pl.fused ? 0.69 * B + 0.171e-3 * N * B : 2.03 + 0.345e-3 * N);
+    us += pl.fit * (tiles * stages * pl.ncg * pl.rt * (0.045 + 0.037 * i4) + 0.168e-4 * pl.rows_per_block * stages * 512 + 0.043 * tiles * B * pl.rt * (1.0 + i4));
+    return us + (pl.nks > 1 ? 1.1 : 0.0) + (pl.fit == 1 ? 0.6 : 0.0);
+}
+// tcgen05 kernel: a preparation launch, and per block of 128 columns the weights and the digits, which hardly grow with the activations.
+double lin_tc_us(const TqCut& c, int N, int bits) {
+    const int per_block = (c.nruns + c.slots - 1) / c.slots * ((c.nkb + c.S - 1) / c.S);
+    return 6.3 + 0.16e-3 * N + per_block * ((bits == 4 ? 0.084 : 0.0) + 0.151e-4 * c.R * bits * 16 + 0.317e-4 * c.NC * 128);
+}
+
 }  // namespace
 
 extern "C" void ibcu_linear_force_generic(ibcu_ctx* ctx, int on) { if (ctx) ctx->force_generic = on; }
@@ -489,15 +580,14 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
         return IBCU_OK;
     }
 
-    // Which kernel, as measured in a chain of launches: the tcgen05 kernel pays a preparation launch (about 2.5 us) and then hardly
-    // notices the activations; this file's kernel costs a second group of columns from the third activation on and is bound
-    // by its own instructions. 4096 x 10240 INT8 (42 MB): 16.4 against 13.2 us at two, 28.3 against 13.8 at four; gate and up
-    // of 14336 x 4096 INT4 (59 MB): 18.9 / 16.5 and 23.4 / 15.9; 6144 x 4096 INT8 (25 MB): 9.5 / 9.7 and 11.3 / 10.0; 4096 x 4096
-    // INT8 (17 MB): 6.5 / 8.4 and 7.6 / 8.7. From five on the tcgen05 kernel wins at any size.
-    size_t weight_bytes = 0;
-    for (int i = 0; i < n_tensors; i++) weight_bytes += (size_t)tensors[i].M * rowbytes;
-    const bool many = B >= 5 || (B >= 3 && weight_bytes >= (20u << 20)) || (B == 2 && weight_bytes >= (32u << 20));
-    if (ctx->linear_tc > 0 ? (bits == 4 || ctx->linear_tc > 1) : (ctx->linear_tc == 0 && many)) {
+    long total_rows = 0;
+    for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
+    if (total_rows == 0) return IBCU_OK;
+    const LinPlan pl = lin_plan(ctx, tensors, n_tensors, total_rows, N, B < 16 ? B : 16, bits, op);
+    bool tc = ctx->linear_tc > 0 && (bits == 4 || ctx->linear_tc > 1);
+    if (ctx->linear_tc == 0)                                  // see lin_mma_us; beyond 16 activations the mma.sync kernel goes over the weights twice
+        tc = B > 16 || (B > 1 && lin_tc_us(ibcu_linear_tc_cut(ctx->sm_count, tensors, n_tensors, N, B), N, bits) < lin_mma_us(pl, N, B, bits));
+    if (tc) {
         const int rc_tc = ibcu_linear_tc(ctx, tensors, n_tensors, x, N, B, bits, pro, op);
         if (rc_tc != IBCU_DECLINED) return rc_tc;
     }
@@ -512,26 +602,15 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
         }
         return IBCU_OK;
     }
-    const int ncols = B * LIN_LIMBS;
-    const int ncg = (ncols + 7) / 8 <= 1 ? 1 : ((ncols + 7) / 8 <= 2 ? 2 : ((ncols + 7) / 8 <= 4 ? 4 : 8));
-    const int nkb = (rowbytes + 63) / 64;
+    const int ncols = pl.ncols, ncg = pl.ncg, nks = pl.nks, slice_kb = pl.slice_kb, xs_ld = pl.xs_ld, rt = pl.rt, stages = pl.stages;
     const int xk = bits == 8 ? 64 : 128;
-    const int xpad = bits == 8 ? 64 : 16;                     // keeps limb rows of neighbouring columns on different banks
-    long total_rows = 0;
-    for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
-    if (total_rows == 0) return IBCU_OK;
-    // Rows are dealt out evenly: every block of the persistent grid owns one contiguous run of rows and
-    // walks it in tiles of up to R = 16 or 32 rows. 32-row tiles once a block's run is longer than 16.
-    const int w = 8;                                          // warps per block; two blocks share an SM
-    const int rt = (ncg >= 4 || total_rows <= 16L * 2 * ctx->sm_count) ? 1 : 2;
-    const int R = 16 * rt;
     LinearParams p;
     memset(&p, 0, sizeof p);
     {
         int row_start = 0;
         for (int i = 0; i < n_tensors; i++) {
             p.t[i] = { (const uint8_t*)tensors[i].w, tensors[i].scales, tensors[i].out, tensors[i].M,
-                       tensors[i].out_stride, tensors[i].scales_fp32, tensors[i].epilogue, row_start, 0, 0, -1 };
+                       tensors[i].out_stride, tensors[i].scales_fp32, tensors[i].epilogue, row_start, pl.blk_start[i], pl.rows_per[i], -1 };
             row_start += tensors[i].M;
         }
     }
@@ -551,50 +630,7 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
             for (int i = 0; i < n_tensors; i++) p.t[i].win_off = (long)((const char*)tensors[i].out - ctx->win_base);
         }
     }
-    // Shared memory per block: stage ring + reduction buffer + the slice's limbs. Columns are
-    // split over several blocks only when the limbs of a whole row do not fit.
-    const int kbs = w;
-    const int LIN_LD = lin_ld(w);
-    // ring depth: the deeper ring when two blocks per SM still fit with it, else the shallower one
-    const size_t red_bytes = (size_t)(bits == 4 ? 2 : 1) * w * R * lin_rld(ncg) * 4;
-    const size_t whole_row_pieces = (size_t)ncols * ((size_t)nkb * xk + xpad);
-    int stages = rt == 2 ? 6 : 8;
-    if (2 * ((size_t)stages * R * LIN_LD + red_bytes + whole_row_pieces + 2048) > 227 * 1024) stages = 4;
-    const size_t fixed_smem = (size_t)stages * R * LIN_LD + red_bytes + 1024;
-    const size_t smem_cap = 200 * 1024;
-    long piece_budget = (long)smem_cap - (long)fixed_smem;
-    int max_slice_kb = (int)((piece_budget / ncols - xpad) / xk) / kbs * kbs;
-    if (max_slice_kb < kbs) max_slice_kb = kbs;
-    int slice_kb = (nkb + kbs - 1) / kbs * kbs;               // whole stages per slice
-    if (slice_kb > max_slice_kb) slice_kb = max_slice_kb;
-    const int nks = (nkb + slice_kb - 1) / slice_kb;
-    const int xs_ld = slice_kb * xk + xpad;
-    const size_t piece_smem = (((size_t)ncols * xs_ld) + 15) & ~(size_t)15;
-    // persistent grid: as many blocks as fit on the machine at once, a multiple of nks, at most one per item
-    int fit = (int)((227 * 1024) / (fixed_smem + piece_smem + 1024));
-    if (fit < 1) fit = 1;
-    if (fit > 4) fit = 4;
-    const int slots = fit * ctx->sm_count;
-    int per_slice = slots / nks;
-    if (per_slice < 1) per_slice = 1;
-    // every tensor gets blocks in proportion to its rows, and its rows are dealt out evenly among them;
-    // the run length grows until all blocks are resident at once
-    int rows_per_block = (int)((total_rows + per_slice - 1) / per_slice);
-    if (rows_per_block < 4) rows_per_block = 4;
-    int nblk;
-    for (;; rows_per_block++) {
-        nblk = 0;
-        for (int i = 0; i < n_tensors; i++) nblk += (tensors[i].M + rows_per_block - 1) / rows_per_block;
-        if (nblk <= per_slice || rows_per_block >= total_rows) break;
-    }
-    nblk = 0;
-    for (int i = 0; i < n_tensors; i++) {
-        const int n = (tensors[i].M + rows_per_block - 1) / rows_per_block;
-        p.t[i].blk_start = nblk;
-        p.t[i].rows_per = n ? (tensors[i].M + n - 1) / n : 0;
-        nblk += n;
-    }
-    const int grid = nblk * nks;
+    const int grid = pl.nblk * nks;
 
     const size_t xpack_bytes = (((size_t)nks * ncols * xs_ld) + 255) & ~(size_t)255;
     const size_t xscale_bytes = (((size_t)B * nks * sizeof(float)) + 255) & ~(size_t)255;
@@ -603,7 +639,7 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
     int8_t* xpack = (int8_t*)ctx->xpack;
     float* xscale = (float*)((char*)ctx->xpack + xpack_bytes);
     int* xsum = (int*)((char*)ctx->xpack + xpack_bytes + xscale_bytes);
-    p.n_tensors = n_tensors; p.total_rows = (int)total_rows; p.rowbytes = rowbytes; p.nkb = nkb; p.N = N; p.B = B; p.ncols = ncols;
+    p.n_tensors = n_tensors; p.total_rows = (int)total_rows; p.rowbytes = rowbytes; p.nkb = pl.nkb; p.N = N; p.B = B; p.ncols = ncols;
     p.slice_kb = slice_kb; p.nks = nks; p.xs_ld = xs_ld;
     p.xpack = xpack; p.xscale = xscale; p.xsum = xsum;
     if (nks > 1) {
@@ -614,11 +650,8 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
     }
     XSource xsrc = { x, pro ? pro->x2 : nullptr, pro ? (const __half*)pro->norm_w : nullptr, pro ? pro->eps : 0.0f, op,
                      op == IBCU_PRO_KNOWN_MAX ? pro->amax : nullptr, op == IBCU_PRO_KNOWN_MAX ? pro->n_amax : 0 };
-    // Cheap conversions are done by every block of the main kernel for itself (no extra launch, no
-    // dependency chain); expensive ones (SiLU, several activations, long rows) once, by xprep_kernel.
-    int fused = (op != IBCU_PRO_SILU_MUL && (long)B * slice_kb * xk <= 8192 && nks == 1) ? 1 : 0;
-    if (op == IBCU_PRO_KNOWN_MAX && nks == 1 && B <= 2) fused = 1;          // no reduction: cheap at any row length
-    p.xsrc = xsrc; p.fused_x = fused;
+    const bool fused = pl.fused;
+    p.xsrc = xsrc; p.fused_x = fused ? 1 : 0;
     // 512 threads hold up to 16384 columns in registers; longer slices take 1024 threads and the looping conversion
     const int xthreads = slice_kb * xk > XREG_V * 4 * 512 ? 1024 : (slice_kb * xk >= 2048 ? 512 : 256);
     if (!fused) {
@@ -631,7 +664,7 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
     }
     p.gw = gw;
     if (rc) return rc;
-    const size_t smem = piece_smem + 32 * sizeof(float) + 32 * LIN_LIMBS * sizeof(int);
+    const size_t smem = pl.piece_smem + 32 * sizeof(float) + 32 * LIN_LIMBS * sizeof(int);
 #define IBCU_DISPATCH(BITS) \
     switch (ncg) { \
         case 1: rc = dispatch_shape<BITS, 1>(ctx, p, grid, rt, stages, smem); break; \

@@ -442,6 +442,31 @@ int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, si
 
 }  // namespace
 
+TqCut ibcu_linear_tc_cut(int sm_count, const ibcu_linear_t* tensors, int n_tensors, int N, int B) {
+    TqCut c;
+    long total_rows = 0;
+    for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
+    c.nkb = (N + 127) / 128;
+    c.NC = (B * LIN_LIMBS + 15) / 16 * 16;
+    // Columns over S blocks of a cluster: enough rows per block that the digits every block fetches stay few against the
+    // weights, and no more than 256 of them.
+    const int slots_of[4] = { sm_count, sm_count / 2, sm_count * 9 / 40, sm_count / 9 };
+    int lg = 0;
+    while (lg < 3 && total_rows / slots_of[lg] < 80 && c.nkb >= (4 << lg)) lg++;
+    while (lg > 0 && (c.nkb < (1 << lg) || total_rows > 256L * slots_of[lg])) lg--;
+    c.S = 1 << lg;
+    c.slots = slots_of[lg];
+    const long per = (total_rows + c.slots - 1) / c.slots;
+    c.R = per > 256 ? 256 : (int)(per + 7) & ~7;
+    for (;; c.R += 8) {
+        c.nruns = 0;
+        for (int i = 0; i < n_tensors; i++) c.nruns += (tensors[i].M + c.R - 1) / c.R;
+        if (c.R >= 256 || c.nruns <= c.slots) break;
+    }
+    c.T = c.R > 128 ? 2 : 1;
+    return c;
+}
+
 // The call as the preparation kernel and the tcgen05 kernel. Returns IBCU_DECLINED without touching the context's error when
 // the call is not its own (the caller takes the other kernels).
 int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, const float* x, int N, int B, int bits, const ibcu_prologue_t* pro, int op) {
@@ -451,28 +476,11 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     long total_rows = 0;
     for (int i = 0; i < n_tensors; i++) total_rows += tensors[i].M;
     if (total_rows == 0) return IBCU_OK;
+    const TqCut cut = ibcu_linear_tc_cut(ctx->sm_count, tensors, n_tensors, N, B);
+    const int S = cut.S, R = cut.R, T = cut.T, slots = cut.slots;
     TqParams p;
     memset(&p, 0, sizeof p);
-    p.n_tensors = n_tensors; p.B = B; p.nkb = (N + 127) / 128;
-    p.NC = (B * LIN_LIMBS + 15) / 16 * 16;
-    // Columns over S blocks of a cluster: enough rows per block that the digits every block fetches stay few against the
-    // weights, and no more than 256 of them.
-    int S = 1;
-    const int slots_of[4] = { ctx->sm_count, ctx->sm_count / 2, ctx->sm_count * 9 / 40, ctx->sm_count / 9 };
-    int lg = 0;
-    while (lg < 3 && total_rows / slots_of[lg] < 80 && p.nkb >= (4 << lg)) lg++;
-    while (lg > 0 && (p.nkb < (1 << lg) || total_rows > 256L * slots_of[lg])) lg--;
-    S = 1 << lg;
-    const int slots = slots_of[lg];
-    int R = (int)((total_rows + slots - 1) / slots);
-    if (R > 256) R = 256;
-    R = (R + 7) & ~7;
-    for (; R < 256; R += 8) {
-        int n = 0;
-        for (int i = 0; i < n_tensors; i++) n += (tensors[i].M + R - 1) / R;
-        if (n <= slots) break;
-    }
-    const int T = R > 128 ? 2 : 1;
+    p.n_tensors = n_tensors; p.B = B; p.nkb = cut.nkb; p.NC = cut.NC;
     p.R = R; p.S = S;
     int nruns = 0;
     for (int i = 0, row = 0; i < n_tensors; i++) {

@@ -26,6 +26,11 @@ struct XSource {                   // where an activation value comes from
 
 constexpr int LIN_LIMBS = 4;
 
+// How the tcgen05 kernel cuts a call: runs of R rows in T tiles of 128, each by a cluster of S blocks that share its nkb blocks of 128
+// columns; slots clusters are resident at once.
+struct TqCut { int S, R, T, nkb, slots, nruns, NC; };
+TqCut ibcu_linear_tc_cut(int sm_count, const ibcu_linear_t* tensors, int n_tensors, int N, int B);      // linear_tc.cu
+
 // rows of digits, one per limb, ld bytes apart (mma.sync kernels)
 struct XRows {
     int8_t* p; int ld;

@@ -510,3 +510,39 @@ def test_group_scaled_int4_row_lengths(backend, cpu_libs, N):
     got = backend.int4g_matmul(q, s, 32, x, oi, ov, 0.0)
     want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, 32, x, oi, ov, 0.0)
     assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
+
+
+@pytest.mark.parametrize("bits,Ms,N,B,tc", [
+    (8, [1408] * 3, 1408, 7, False), (4, [1152, 128, 128], 1152, 6, False),      # few short rows: the preparation launch does not pay
+    (8, [4096] * 3, 4096, 2, False), (8, [2048, 512, 512], 2048, 3, False),
+    (8, [14336], 4096, 4, True), (4, [14336, 14336], 4096, 3, True), (8, [4096], 14336, 3, True), (8, [4096, 1024, 1024], 4096, 8, True),
+    (8, [64], 512, 17, True), (8, [32000], 4096, 1, False),
+])
+def test_linear_kernel_by_cost(backend, bits, Ms, N, B, tc):
+    """Which kernel a call takes by itself: the launches and the bits are those of the call that is told to."""
+    rng = np.random.default_rng(bits + sum(Ms) + N + B)
+    be = backend
+    w = rng.integers(0, 256, sum(Ms) * N * bits // 8, dtype=np.uint8)
+    s16, x = _cpu.fp16_bits(rng.uniform(0.001, 0.01, sum(Ms))), rng.standard_normal((B, N)).astype(np.float32)
+    dw, ds, dx = be.upload(w), be.upload(s16), be.upload(x)
+
+    def run(mode):
+        out, ts, row = be.alloc(B * sum(Ms) * 4), [], 0
+        for M in Ms:
+            ts.append(LinearT(dw.at(row * N * bits // 8), ds.at(2 * row), out.at(4 * B * row), M, M, 0, 0)); row += M
+        be.lib.ibcu_linear_use_tcgen05(be.ctx, mode)
+        try:
+            before = be.launches()
+            be._check(be.lib.ibcu_linear(be.ctx, (LinearT * len(ts))(*ts), len(ts), dx.ptr, N, B, bits))
+            n = be.launches() - before
+        finally:
+            be.lib.ibcu_linear_use_tcgen05(be.ctx, 0)
+        be.sync()
+        got = be.download(out, np.float32, B * sum(Ms)); out.free(); be._bufs.remove(out)
+        return n, got
+
+    n, got = run(0)
+    want_n, want = run(2 if tc else -1)
+    assert n == want_n and np.array_equal(got, want)
+    if tc:
+        assert n == 2
