@@ -454,14 +454,19 @@ TqCut ibcu_linear_tc_cut(int sm_count, const ibcu_linear_t* tensors, int n_tenso
     int lg = 0;
     while (lg < 3 && total_rows / slots_of[lg] < 80 && c.nkb >= (4 << lg)) lg++;
     while (lg > 0 && (c.nkb < (1 << lg) || total_rows > 256L * slots_of[lg])) lg--;
-    c.S = 1 << lg;
-    c.slots = slots_of[lg];
-    const long per = (total_rows + c.slots - 1) / c.slots;
-    c.R = per > 256 ? 256 : (int)(per + 7) & ~7;
-    for (;; c.R += 8) {
-        c.nruns = 0;
-        for (int i = 0; i < n_tensors; i++) c.nruns += (tensors[i].M + c.R - 1) / c.R;
-        if (c.R >= 256 || c.nruns <= c.slots) break;
+    // A cluster of eight blocks of two tiles, an SM each, does not find room for all sixteen clusters at once: 2280 rows of 2048 columns at
+    // four activations took 11.8 us, rows of 3840 at sixteen 16.4; four blocks of one tile take over there.
+    for (;; lg--) {
+        c.S = 1 << lg;
+        c.slots = slots_of[lg];
+        const long per = (total_rows + c.slots - 1) / c.slots;
+        c.R = per > 256 ? 256 : (int)(per + 7) & ~7;
+        for (;; c.R += 8) {
+            c.nruns = 0;
+            for (int i = 0; i < n_tensors; i++) c.nruns += (tensors[i].M + c.R - 1) / c.R;
+            if (c.R >= 256 || c.nruns <= c.slots) break;
+        }
+        if (lg < 3 || c.R <= 128) break;
     }
     c.T = c.R > 128 ? 2 : 1;
     return c;

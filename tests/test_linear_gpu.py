@@ -149,6 +149,30 @@ def test_row_lengths_converted_in_the_block(backend, cpu_libs, bits, N):
     assert _cpu.close(backend.linear(w, s16, x, bits), oracle_linear(cpu_libs, w, s16, x, bits), RTOL, ATOL)
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("Ms,N,B", [([2048], 1024, 5), ([2049], 1024, 16), ([1520, 380, 380], 2048, 6), ([2639], 4224, 9)])
+def test_tcgen05_rows_around_clusters_of_eight(backend, bits, Ms, N, B):
+    """The last row count that clusters of eight blocks take with one tile each, and those that go to clusters of four: the sums of
+    the mma.sync kernel, to the last place where that cuts a row into slices."""
+    rng = np.random.default_rng(bits + sum(Ms) + N + B)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, sum(Ms), N, B)
+    be = backend
+    dw, ds, dx = be.upload(w), be.upload(s16), be.upload(x)
+    outs = []
+    for mode in (2, -1):
+        out, ts, row = be.alloc(B * sum(Ms) * 4), [], 0
+        for M in Ms:
+            ts.append(LinearT(dw.at(row * N * bits // 8), ds.at(2 * row), out.at(4 * B * row), M, M, 0, 0)); row += M
+        be.lib.ibcu_linear_use_tcgen05(be.ctx, mode)
+        try:
+            be._check(be.lib.ibcu_linear(be.ctx, (LinearT * len(ts))(*ts), len(ts), dx.ptr, N, B, bits))
+        finally:
+            be.lib.ibcu_linear_use_tcgen05(be.ctx, 0)
+        be.sync()
+        outs.append(be.download(out, np.float32, B * sum(Ms)))
+    assert np.allclose(outs[0], outs[1], rtol=2e-6, atol=1e-6 * float(np.abs(outs[1]).max()))
+
+
 @pytest.mark.parametrize("M,N,B", [(38000, 1664, 6), (25000, 1920, 32), (3000, 4224, 24)])
 def test_tcgen05_int4_teams(backend, M, N, B):
     """Odd numbers of 128-column blocks through rings that are used again, over one and two runs of rows: the two teams of
