@@ -119,9 +119,9 @@ __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc, 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
-// XV: 4 XV columns of an activation per thread are held in registers while the block converts it. The instance with 4 takes 76
-// registers against 120: a block of the next launch then finds room beside this launch's two and has its weights under way earlier
-// (hidden size 4096, one token, 8-bit projections of 12 layers: 171.8 -> 161.1 us; 2048: 128.1 -> 115.6).
+// XV: 4 XV columns of an activation per thread are held in registers while the block converts it. Up to 4096 columns the instance with 4
+// is enough (76 registers; the one with 8 takes 120): hidden size 4096, one token, 8-bit projections of 12 layers 171.8 -> 161.1 us; 2048:
+// 128.1 -> 115.6. Two blocks fill an SM's shared memory with either, so it is not room for a third; what else it is was not measured apart.
 template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
 __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p) {
     constexpr int R = RT * 16;                                // most rows per tile
@@ -416,20 +416,21 @@ int launch_mma_x(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tai
     return ibcu_launch(ctx, kern, dim3(grid), dim3(W * 32), smem, 1, true, p);
 }
 
-// a block that converts more than 4096 columns itself, and has to find their maximum first, holds up to 8192
+// a block that converts more than 4096 columns itself, and has to find their maximum first, holds up to 8192 (one activation: see lin_plan)
 template <int BITS, int NCG, int RT, int W, int STAGES>
 int launch_mma(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
-    const bool longer = p.fused_x && p.xsrc.op != IBCU_PRO_KNOWN_MAX && p.slice_kb * (BITS == 8 ? 64 : 128) > 4 * 4 * W * 32;
-    if (NCG <= 2 && longer) return launch_mma_x<BITS, NCG, RT, W, STAGES, 8>(ctx, p, grid, smem_tail);
+    if constexpr (NCG == 1) {
+        const bool longer = p.fused_x && p.xsrc.op != IBCU_PRO_KNOWN_MAX && p.slice_kb * (BITS == 8 ? 64 : 128) > 4 * 4 * W * 32;
+        if (longer) return launch_mma_x<BITS, NCG, RT, W, STAGES, 8>(ctx, p, grid, smem_tail);
+    }
     return launch_mma_x<BITS, NCG, RT, W, STAGES, 4>(ctx, p, grid, smem_tail);
 }
 
 // Eight warps and 512-byte stages; the ring is as deep as two resident blocks per SM allow.
 template <int BITS, int NCG>
 int dispatch_shape(ibcu_ctx* ctx, const LinearParams& p, int grid, int rt, int stages, size_t smem_tail) {
-    if (rt == 2) {
-        if (stages >= 6) return launch_mma<BITS, NCG, 2, 8, 6>(ctx, p, grid, smem_tail);
-        return launch_mma<BITS, NCG, 2, 8, 4>(ctx, p, grid, smem_tail);
+    if constexpr (NCG <= 2) {                                  // more groups of columns take tiles of 16 rows
+        if (rt == 2) return stages >= 6 ? launch_mma<BITS, NCG, 2, 8, 6>(ctx, p, grid, smem_tail) : launch_mma<BITS, NCG, 2, 8, 4>(ctx, p, grid, smem_tail);
     }
     if (stages >= 8) return launch_mma<BITS, NCG, 1, 8, 8>(ctx, p, grid, smem_tail);
     return launch_mma<BITS, NCG, 1, 8, 4>(ctx, p, grid, smem_tail);

@@ -19,7 +19,7 @@
 // Workers (INT4 widening, then epilogue): eight warps per tile of 128 rows, in two teams that take the blocks of columns in turn;
 // then one warp each for the weights (TMA), the digits (bulk copies) and the MMAs. What a block of columns costs a warp is waits
 // and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
-// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4; at 32 the digits, which every SM reads from L2,
+// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4 (the INT4 instance of one tile spills 32 bytes a thread); at 32 the digits, which every SM reads from L2,
 // bound the kernel (26 us, 75 MB of them).
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait. With at most 128 rows per run a
 // block takes no more than half of an SM's shared memory and tensor memory, so that the next launch's blocks move in beside it

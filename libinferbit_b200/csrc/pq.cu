@@ -1,6 +1,6 @@
 // Product-quantised matvec: out[r] = row_scale[r] * sum over subspaces s of LUT_s[code[r][s]],
-// LUT_s[k] = codebook_s[k] . x_s (FP32), for 1..32 activations: the kernels with tables, one launch per call. Calls with several
-// activations and entries of 4 or 16 values go to the tensor cores instead (pq_tc.cu, pq_takes_tc).
+// LUT_s[k] = codebook_s[k] . x_s (FP32), for 1..32 activations: the kernels with tables, one launch per call of one activation. Most calls
+// with several activations, and smaller tensors with entries of 4 or 16 values, go to the tensor cores instead (pq_tc.cu, pq_takes_tc).
 //
 // Data in HBM: codebooks, row scales and the two row-major code planes exactly as the reference
 // holds them, plus one derived array made once per tensor by ibcu_pq_prepare: the codes regrouped into
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const uint32_t w = i < 4 ? cw.x : (i < 8 ? cw.y : (i < 12 ? cw.z : cw.w));
-                    const uint32_t code = __byte_perm(w, 0u, 0x4440u | (i & 3));     // one byte-permute; shift-and-mask became a byte-to-word conversion on the quarter-rate conversion pipe, which then bounded the gather
+                    const uint32_t code = __byte_perm(w, 0u, 0x4440u | (i & 3));     // one byte-permute: with shift-and-mask the conversion pipe stood at 75 % of its peak, with this at 4 %
                     if constexpr (BT == 2) {
                         const float2 q = *reinterpret_cast<const float2*>(lut + ((size_t)code * 32 + lane) * 2);
                         v[2 * i] = q.x; v[2 * i + 1] = q.y;                                 // value 2 i + u: row i ^ (lane >> 1), activation u ^ (lane & 1)

@@ -18,8 +18,8 @@
 //                root mean square, over 128 1.9e-7, now 1.25e-7; the tables' 1.0e-7.)
 //   warps 24-26  codes (cp.async), operand image (bulk copies), MMA issue
 // What bounds it: the latency of every role's chain of waits, not a pipe (a unit takes about 1300 cycles of which the entries
-// keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500), and about 7 us around the units: the
-// preparation, staging the codebooks, and the meeting of the parts. 4096 x 14336, entries of eight, 24 tensors in turn: eight
+// keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500; 864 threads leave 72 registers each, so every
+// instance spills, 36 to 364 bytes of stores: part of those waits), and about 7 us around the units: the preparation, staging the codebooks, and the meeting of the parts. 4096 x 14336, entries of eight, 24 tensors in turn: eight
 // activations 28.1 -> 21.2 us, sixteen 46 -> 27; 4096 x 8192 with entries of four at eight 49 -> 17.6, of sixteen 37 -> 23, with a
 // second level 45 -> 22.
 #include "tc_common.cuh"
