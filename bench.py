@@ -298,6 +298,9 @@ def run_reference(args, rank):
     if rank != 0:
         return
     cpu = CpuBaseline()
+    if cpu.kind != "reference":                              # the scalar port is not the reference
+        print(json.dumps({"impl": "reference", "unavailable": "the compiled reference (oracle/_ref/libinferbit_ref.so) is not here and there is no checkout to build it from"}), flush=True)
+        return
     steps = max(1, min(args.steps, 200))
     dt, gbs = cpu.time_steps(steps, max(3, min(args.warmup, 10)))
     line = {"impl": "reference", "metric": "int8_matvec_weight_GBps", "value": gbs, "unit": "GB/s", "n_gpus": args.gpus,

@@ -1,4 +1,5 @@
 """bench.py's CPU legs on a machine without the compiled reference: the scalar port is called with whole addresses."""
+import json
 import os
 import subprocess
 import sys
@@ -29,3 +30,12 @@ print("ok")
 def test_port_legs_run():
     r = subprocess.run([sys.executable, "-c", CHILD], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.returncode, r.stderr[-1000:])
+
+
+def test_reference_arm_without_the_reference(tmp_path):
+    """Without the compiled reference its arm says so; it does not time the port under the reference's name."""
+    code = "import os, sys, bench; real = os.path.exists; os.path.exists = lambda p: real(p) and not str(p).endswith('libinferbit_ref.so'); " \
+           "sys.argv = ['bench.py', '--impl', 'reference', '--steps', '2', '--warmup', '1']; bench.main()"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    line = json.loads(r.stdout.strip().splitlines()[-1])
+    assert r.returncode == 0 and line["impl"] == "reference" and "unavailable" in line and "value" not in line
