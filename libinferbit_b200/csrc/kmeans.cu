@@ -503,9 +503,12 @@ int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const floa
 
 }  // namespace
 
-int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, const float* C, int K, int32_t* idx, float* dist);   // kmeans_tc.cu
-int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, const float* C, int K, int32_t* idx, float* dist,
-                                     float* part_sums, int32_t* part_counts, double* part_inertia, int nblocks);
+// kmeans_tc.cu
+bool ibcu_kmeans_tc_takes(const float* X, long N, int D, const float* C, int K);
+long ibcu_kmeans_tc_blocks(const ibcu_ctx* ctx, long N);
+int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist);
+int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
+                                     float* part_sums, int32_t* part_counts, double* part_inertia);
 
 extern "C" void ibcu_kmeans_set_path(ibcu_ctx* ctx, int path) { if (ctx) ctx->kmeans_path = path; }
 
@@ -515,13 +518,11 @@ extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, 
     IBCU_REQUIRE(ctx, X && C && idx, "ibcu_kmeans_assign: null pointer");
     IBCU_REQUIRE(ctx, N > 0 && D >= 1 && D <= KM_MAX_D && K >= 1 && K <= 1024, "ibcu_kmeans_assign: N=%ld D=%d K=%d out of range", N, D, K);
     IBCU_REQUIRE(ctx, (size_t)K * D * sizeof(float) <= 128 * 1024, "ibcu_kmeans_assign: K*D=%d too large", K * D);
-    // D == 8: scores on the tensor cores as a filter, exact re-evaluation of the candidates. The tcgen05 kernel takes
-    // K a multiple of 64 up to 256; other multiples of 8 take the register-operand (mma.sync) filter.
-    if (D == 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
-        if (ctx->kmeans_path != IBCU_KMEANS_MMA_SYNC) {
-            const int rc = ibcu_kmeans_assign_tc(ctx, X, N, C, K, idx, dist);
-            if (rc != IBCU_DECLINED) return rc;
-        }
+    // Scores on the tensor cores as a filter, exact re-evaluation of the candidates: the tcgen05 kernel for 4, 8 and 16 dimensions and
+    // up to 256 centroids; for D == 8 and more centroids, in multiples of 8, the register-operand (mma.sync) filter.
+    if (ctx->kmeans_path == IBCU_KMEANS_AUTO) {
+        const int rc = ibcu_kmeans_assign_tc(ctx, X, N, D, C, K, idx, dist);
+        if (rc != IBCU_DECLINED) return rc;
     }
     if (D == 8 && K % 8 == 0 && K >= 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
         const size_t smem = ((size_t)K * 16 + K + (size_t)K * 8 + 4) * sizeof(float);
@@ -598,12 +599,11 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
     const size_t slot_bytes = (size_t)K * D * sizeof(float) + (size_t)K * sizeof(int32_t) + 16;
     const int windowed = ctx->world > 1 && !ctx->capturing ? ibcu_exchange_begin(ctx, slot_bytes, &ex) : 0;
     if (!windowed) memset(&ex, 0, sizeof ex);
-    // D == 8 on the tensor-memory kernel: the assignment kernel's epilogue adds the points into per-block tables as it
-    // goes, so the accumulate pass costs no second read of X and no launch; only the per-block tables are left to add up
+    // On the tensor-memory kernel the points go into per-block tables as they are assigned, so the accumulate pass costs no
+    // second read of X and no launch; only the per-block tables are left to add up
     bool fused = false;
-    if (D == 8 && ctx->kmeans_path == IBCU_KMEANS_AUTO && ((uintptr_t)X & 15) == 0 && K >= 64 && K <= 256 && (K & 63) == 0) {
-        const long ntile = (N + 127) / 128;
-        const int nblocks = (int)(ntile < ctx->sm_count ? ntile : ctx->sm_count);
+    if (ctx->kmeans_path == IBCU_KMEANS_AUTO && ibcu_kmeans_tc_takes(X, N, D, C, K)) {
+        const int nblocks = (int)ibcu_kmeans_tc_blocks(ctx, N);
         const size_t KD = (size_t)K * D;
         const size_t need = (size_t)nblocks * (KD * sizeof(float) + K * sizeof(int32_t) + sizeof(double)) + 64;
         rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, need);
@@ -611,7 +611,7 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
         double* part_inertia = (double*)ctx->scratch;
         float* part_sums = (float*)(part_inertia + ((nblocks + 1) & ~1));
         int32_t* part_counts = (int32_t*)(part_sums + (size_t)nblocks * KD);
-        rc = ibcu_kmeans_assign_accumulate_tc(ctx, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia, nblocks);
+        rc = ibcu_kmeans_assign_accumulate_tc(ctx, X, N, D, C, K, idx, dist, part_sums, part_counts, part_inertia);
         if (rc == IBCU_OK) {
             fused = true;
             const int fin_blocks = (int)((KD + 31) / 32) + (K + 31) / 32 + 1;

@@ -179,3 +179,63 @@ def test_full_size_codes_against_the_reference(backend, cpu_libs):
             Cn[:, d] = np.where(cnt > 0, s / np.maximum(cnt, 1), Cn[:, d]).astype(np.float32)
     if pool:
         cpu_libs.ref.ib_pool_destroy(pool)
+
+
+@pytest.mark.parametrize("D", [4, 8, 16])
+@pytest.mark.parametrize("N,K", [(1, 1), (127, 7), (128, 32), (129, 33), (148 * 128 + 1, 200), (40001, 256), (6000, 130), (300, 16)])
+def test_tensor_core_assign_and_sums_at_the_edges(backend, cpu_libs, D, N, K):
+    """Tiles of 128 points and groups of 8 centroids, padded: last rows, first and last group, one centroid; codes and distances are the
+    checker's bits, and the sums a Lloyd iteration leaves are those of the codes (FP32 sums of at most N terms)."""
+    rng = np.random.default_rng(N * 31 + K + D)
+    X = (rng.standard_normal((N, D)) * 0.02).astype(np.float32)
+    Cn = (rng.standard_normal((K, D)) * 0.02).astype(np.float32)
+    m = min(N, K) // 2
+    Cn[K - m:] = X[:m]
+    if K > 20:
+        Cn[K - 1] = Cn[K - 9]                                    # exact ties between two groups
+    got, gd = backend.kmeans_assign(X, Cn, want_dist=True)
+    want, wd = oracle_assign(cpu_libs, X, Cn)
+    assert np.array_equal(got, want) and np.array_equal(gd, wd)
+    h = _lloyd_gpu(backend, X, Cn, 1)[0]
+    assert np.array_equal(h["idx"], want)
+    assert np.array_equal(h["counts"], np.bincount(want, minlength=K))
+    for d in range(D):
+        ref = np.bincount(want, weights=X[:, d].astype(np.float64), minlength=K)
+        mag = np.bincount(want, weights=np.abs(X[:, d]).astype(np.float64), minlength=K)
+        assert np.all(np.abs(h["sums"][:, d] - ref) <= 2.0 ** -24 * (N + 16) * mag)
+    assert abs(h["inertia"] - wd.astype(np.float64).sum()) <= 1e-12 * wd.astype(np.float64).sum()
+
+
+@pytest.mark.parametrize("D", [4, 8, 16])
+def test_tensor_core_filter_hands_over_what_it_cannot_decide(backend, cpu_libs, D):
+    """Near ties across groups, NaN and Inf in points and centroids (centroid 0 among them: the reference's scan starts from it and a NaN
+    there is never replaced), squares that overflow or vanish."""
+    rng = np.random.default_rng(90 + D)
+    K, N = 72, 20000
+    Cn = (rng.standard_normal((K, D)) * 0.02).astype(np.float32)
+    mid = (Cn[3].astype(np.float64) + Cn[60]) / 2
+    d = Cn[60].astype(np.float64) - Cn[3]; d /= np.linalg.norm(d)
+    noise = rng.standard_normal((N, D)) * 0.002
+    noise -= (noise @ d)[:, None] * d
+    X = (mid + noise).astype(np.float32)
+    X[5, 1] = np.nan; X[6, 0] = np.inf; X[7, 2] = -np.inf
+    X[8] *= np.float32(1e20); X[9] *= np.float32(1e-22); X[10] = 0
+    for scale, bad in ((1.0, None), (1.0, (0, np.nan)), (1.0, (70, np.nan)), (1.0, (9, np.inf)), (1e-20, None), (3e18, None), (2e19, None)):
+        Cs, Xs = Cn * np.float32(scale), X * np.float32(scale)
+        if bad:
+            Cs[bad[0], 1] = bad[1]
+        got, gd = backend.kmeans_assign(Xs, Cs, want_dist=True)
+        want, wd = oracle_assign(cpu_libs, Xs, Cs)
+        assert np.array_equal(got, want), (scale, bad)
+        assert np.array_equal(gd, wd, equal_nan=True), (scale, bad)
+
+
+def test_tensor_core_assign_points_far_from_small_centroids(backend, cpu_libs):
+    """Points up to 2^20 times longer than every centroid, on all sides, with padded centroids in the last group."""
+    rng = np.random.default_rng(17)
+    for D in (4, 8, 16):
+        Cn = (rng.standard_normal((41, D)) * 0.02).astype(np.float32)
+        X = rng.standard_normal((6000, D)).astype(np.float32) * np.exp2(rng.integers(-8, 14, (6000, 1))).astype(np.float32)
+        got, gd = backend.kmeans_assign(X, Cn, want_dist=True)
+        want, wd = oracle_assign(cpu_libs, X, Cn)
+        assert np.array_equal(got, want) and np.array_equal(gd, wd)
