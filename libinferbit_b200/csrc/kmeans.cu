@@ -353,6 +353,8 @@ __global__ void __launch_bounds__(256) accumulate_kernel(const float* __restrict
 // (g, c) adds partials g, g + 8, ... of column c with its loads in flight eight at a time, then the
 // eight group sums are combined in a fixed order. Blocks [0, nS) do the sums (in double), [nS, nS + nC)
 // the counts, the last one the inertia.
+// UPDATE: the block that finishes an entry of the sums adds up the counts of its cluster too and moves the centroid, as
+// update_kernel does (same roundings), so that an iteration of one GPU is two launches; no blocks for the counts then.
 // With ex.gp.world > 0 the totals also go into this rank's slot of the exchange area (sums, then counts, then the
 // inertia); the last block copies the slot into every peer's window and publishes: every rank then adds the slots up.
 __device__ __forceinline__ size_t exch_counts_off(int KD) { return (size_t)KD * sizeof(float); }
@@ -362,28 +364,43 @@ __device__ __forceinline__ void exch_store(const ExchSlots& ex, size_t byte_off,
     *reinterpret_cast<T*>(ex.gp.peer[ex.gp.rank] + ex.off + (size_t)ex.gp.rank * ex.slot + byte_off) = v;
 }
 
+// c = sum * (1/count) with the reference's two roundings
+__device__ __forceinline__ float centroid_of(float sum, int n) { return __fmul_rn(sum, __fdiv_rn(1.0f, (float)n)); }
+
+template <bool UPDATE>
 __global__ void __launch_bounds__(256) accumulate_finish_kernel(const float* __restrict__ part_sums, const int32_t* __restrict__ part_counts,
                                                                 const double* __restrict__ part_inertia, int nblocks, int KD, int K,
                                                                 float* __restrict__ sums, int32_t* __restrict__ counts, double* __restrict__ inertia,
-                                                                const ExchSlots ex) {
+                                                                float* __restrict__ C, const ExchSlots ex) {
     __shared__ double dsh[8][32];
     __shared__ int ish[8][32];
     pdl_launch_dependents();
     pdl_wait();
     const int c = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int nS = (KD + 31) / 32, nC = (K + 31) / 32;
+    const int nS = (KD + 31) / 32, nC = UPDATE ? 0 : (K + 31) / 32;
     if ((int)blockIdx.x < nS) {
         const int e = blockIdx.x * 32 + c;
+        const int D = KD / K, k = e / D;
         double s = 0.0;
+        int n = 0;
         if (e < KD) {
 #pragma unroll 8
-            for (int b = g; b < nblocks; b += 8) s += (double)part_sums[(size_t)b * KD + e];
+            for (int b = g; b < nblocks; b += 8) {
+                s += (double)part_sums[(size_t)b * KD + e];
+                if (UPDATE) n += part_counts[(size_t)b * K + k];
+            }
         }
         dsh[g][c] = s;
+        if (UPDATE) ish[g][c] = n;
         __syncthreads();
         if (g == 0 && e < KD) {
             const float v = (float)(((dsh[0][c] + dsh[1][c]) + (dsh[2][c] + dsh[3][c])) + ((dsh[4][c] + dsh[5][c]) + (dsh[6][c] + dsh[7][c])));
             sums[e] = v;
+            if (UPDATE) {
+                n = ish[0][c] + ish[1][c] + ish[2][c] + ish[3][c] + ish[4][c] + ish[5][c] + ish[6][c] + ish[7][c];
+                if (e == k * D) counts[k] = n;
+                if (n > 0) C[e] = centroid_of(v, n);          // empty clusters keep their centroid
+            }
             if (ex.gp.world) exch_store(ex, (size_t)e * sizeof(float), v);
         }
     } else if ((int)blockIdx.x < nS + nC) {
@@ -451,7 +468,7 @@ __global__ void __launch_bounds__(1024) exchange_sum_kernel(const ExchSlots ex, 
     }
 }
 
-// c = sum * (1/count) with the reference's two roundings; empty clusters stay; shift = sum dv^2.
+// The centroid move of every non-empty cluster; shift = sum dv^2.
 __global__ void __launch_bounds__(1024) update_kernel(float* __restrict__ C, int K, int D, const float* __restrict__ sums,
                                                       const int32_t* __restrict__ counts, float* __restrict__ shift) {
     __shared__ float red[32];
@@ -462,8 +479,7 @@ __global__ void __launch_bounds__(1024) update_kernel(float* __restrict__ C, int
         const int k = e / D;
         const int n = counts[k];
         if (n > 0) {
-            const float inv = __fdiv_rn(1.0f, (float)n);
-            const float nv = __fmul_rn(sums[e], inv);
+            const float nv = centroid_of(sums[e], n);
             const float dv = nv - C[e];
             local = fmaf(dv, dv, local);
             C[e] = nv;
@@ -477,6 +493,14 @@ __global__ void __launch_bounds__(1024) update_kernel(float* __restrict__ C, int
         t = warp_sum(t);
         if (threadIdx.x == 0 && shift) *shift = t;
     }
+}
+
+// Adds up the per-block tables; with C given, moves the centroids too (one GPU only: ex says nothing then).
+int finish_launch(ibcu_ctx* ctx, const float* part_sums, const int32_t* part_counts, const double* part_inertia, int nblocks, int D, int K,
+                  float* sums, int32_t* counts, double* inertia, float* C, const ExchSlots& ex) {
+    const int KD = K * D, nS = (KD + 31) / 32;
+    if (C) return ibcu_launch(ctx, accumulate_finish_kernel<true>, dim3(nS + 1), dim3(256), 0, 1, true, part_sums, part_counts, part_inertia, nblocks, KD, K, sums, counts, inertia, C, ex);
+    return ibcu_launch(ctx, accumulate_finish_kernel<false>, dim3(nS + (K + 31) / 32 + 1), dim3(256), 0, 1, true, part_sums, part_counts, part_inertia, nblocks, KD, K, sums, counts, inertia, C, ex);
 }
 
 int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
@@ -538,7 +562,7 @@ extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, 
 }
 
 static int kmeans_accumulate(ibcu_ctx* ctx, const float* X, long N, int D, int K, const int32_t* idx, const float* dist,
-                             float* sums, int32_t* counts, double* inertia, const ExchSlots& ex) {
+                             float* sums, int32_t* counts, double* inertia, float* C, const ExchSlots& ex) {
     IBCU_CHECK_CTX(ctx);
     IBCU_REQUIRE(ctx, X && idx && sums && counts, "ibcu_kmeans_accumulate: null pointer");
     IBCU_REQUIRE(ctx, N > 0 && D >= 1 && D <= KM_MAX_D && K >= 1 && K <= 1024, "ibcu_kmeans_accumulate: N=%ld D=%d K=%d out of range", N, D, K);
@@ -564,10 +588,7 @@ static int kmeans_accumulate(ibcu_ctx* ctx, const float* X, long N, int D, int K
     rc = ibcu_launch(ctx, accumulate_kernel, dim3((unsigned)nblocks), dim3(nwarp * 32), smem, 1, true,
                      X, N, D, K, idx, dist, chunk, part_sums, part_counts, part_inertia);
     if (rc) return rc;
-    int fin_blocks = (int)((KD + 31) / 32) + (K + 31) / 32 + 1;
-    return ibcu_launch(ctx, accumulate_finish_kernel, dim3(fin_blocks), dim3(256), 0, 1, true,
-                       (const float*)part_sums, (const int32_t*)part_counts, (const double*)part_inertia, (int)nblocks, (int)KD, K,
-                       sums, counts, inertia, ex);
+    return finish_launch(ctx, part_sums, part_counts, part_inertia, (int)nblocks, D, K, sums, counts, inertia, C, ex);
 }
 
 extern "C" int ibcu_kmeans_accumulate(ibcu_ctx* ctx, const float* X, long N, int D, int K,
@@ -575,7 +596,7 @@ extern "C" int ibcu_kmeans_accumulate(ibcu_ctx* ctx, const float* X, long N, int
                                       float* sums, int32_t* counts, double* inertia) {
     ExchSlots none;
     memset(&none, 0, sizeof none);
-    return kmeans_accumulate(ctx, X, N, D, K, idx, dist, sums, counts, inertia, none);
+    return kmeans_accumulate(ctx, X, N, D, K, idx, dist, sums, counts, inertia, nullptr, none);
 }
 
 extern "C" int ibcu_kmeans_update(ibcu_ctx* ctx, float* C, int K, int D, const float* sums,
@@ -602,6 +623,7 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
     // On the tensor-memory kernel the points go into per-block tables as they are assigned, so the accumulate pass costs no
     // second read of X and no launch; only the per-block tables are left to add up
     bool fused = false;
+    float* const move = ctx->world > 1 ? nullptr : C;       // one GPU: the kernel that adds up the tables moves the centroids
     if (ctx->kmeans_path == IBCU_KMEANS_AUTO && ibcu_kmeans_tc_takes(X, N, D, C, K)) {
         const int nblocks = (int)ibcu_kmeans_tc_blocks(ctx, N);
         const size_t KD = (size_t)K * D;
@@ -614,19 +636,17 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
         rc = ibcu_kmeans_assign_accumulate_tc(ctx, X, N, D, C, K, idx, dist, part_sums, part_counts, part_inertia);
         if (rc == IBCU_OK) {
             fused = true;
-            const int fin_blocks = (int)((KD + 31) / 32) + (K + 31) / 32 + 1;
-            rc = ibcu_launch(ctx, accumulate_finish_kernel, dim3(fin_blocks), dim3(256), 0, 1, true,
-                             (const float*)part_sums, (const int32_t*)part_counts, (const double*)part_inertia, nblocks, (int)KD, K,
-                             sums, counts, inertia, ex);
+            rc = finish_launch(ctx, part_sums, part_counts, part_inertia, nblocks, D, K, sums, counts, inertia, move, ex);
             if (rc) return rc;
         } else if (rc != IBCU_DECLINED) return rc;
     }
     if (!fused) {
         rc = ibcu_kmeans_assign(ctx, X, N, D, C, K, idx, dist);
         if (rc) return rc;
-        rc = kmeans_accumulate(ctx, X, N, D, K, idx, dist, sums, counts, inertia, ex);
+        rc = kmeans_accumulate(ctx, X, N, D, K, idx, dist, sums, counts, inertia, move, ex);
         if (rc) return rc;
     }
+    if (move) return IBCU_OK;
     if (windowed) {
         ctx->gather_pending = 1;
         GatherWait gw;

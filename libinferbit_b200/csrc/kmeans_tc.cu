@@ -435,16 +435,14 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
                         dk[2 * k + 1] = __fadd_rn(dk[2 * k + 1], p1);
                     }
                 }
-                float be[2] = { dk[0], dk[4] };                      // the first half read, the second
-                int at[2] = { 0, 0 };
+                const float m0 = fminf(fminf(dk[0], dk[1]), fminf(dk[2], dk[3])), m4 = fminf(fminf(dk[4], dk[5]), fminf(dk[6], dk[7]));
+                best = fminf(m0, m4);
+                int at0 = 3, at4 = 3;                                // lowest index of the minimum in the half read first, in the second
 #pragma unroll
-                for (int s = 0; s < 2; s++)
-#pragma unroll
-                    for (int k = 1; k < 4; k++) if (dk[4 * s + k] < be[s]) { be[s] = dk[4 * s + k]; at[s] = k; }
-                const float lo = swap ? be[1] : be[0], hi = swap ? be[0] : be[1];
-                const bool upper = hi < lo;
-                best = upper ? hi : lo;
-                win = g1 * 8 + (upper ? 4 : 0) + ((upper != (swap != 0)) ? at[1] : at[0]);
+                for (int k = 2; k >= 0; k--) { if (dk[k] == best) at0 = k; if (dk[4 + k] == best) at4 = k; }
+                // the lower half wins a tie between the two (with the halves exchanged it is the second one read)
+                const bool second = swap ? m4 == best : m0 != best;
+                win = g1 * 8 + (second ? at4 : at0) + (second != (swap != 0) ? 4 : 0);
             }
             // rows the filter could not decide: the whole warp evaluates all centroids exactly
             unsigned todo = __ballot_sync(0xffffffffu, have && !sure);
@@ -473,14 +471,9 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
             if (have) { idx[row] = win; if (dist) dist[row] = best; }
             if (ACC) {
                 // Points of the warp that share a cluster: the first of them fetches the others' rows and adds them behind its own, in
-                // index order; different clusters go together. Equal clusters are found bit by bit with votes: match.any took 60 cycles,
-                // 285 with eight warps at it.
-                unsigned grp = __ballot_sync(0xffffffffu, have);
-#pragma unroll
-                for (int bit = 0; bit < 8; bit++) {
-                    const unsigned ones = __ballot_sync(0xffffffffu, (win >> bit) & 1);
-                    grp &= (win >> bit) & 1 ? ones : ~ones;
-                }
+                // index order; different clusters go together. (Equal clusters bit by bit with votes: eight votes and thirty-odd more
+                // instructions for the pipe that bounds the kernel.)
+                const unsigned grp = __match_any_sync(0xffffffffu, have ? win : -1 - lane);
                 const bool first = have && (grp & ((1u << lane) - 1u)) == 0;
                 const int turns = __reduce_max_sync(0xffffffffu, (unsigned)__popc(grp));
                 float4* t = reinterpret_cast<float4*>(mytab + (size_t)win * S::row_stride);
