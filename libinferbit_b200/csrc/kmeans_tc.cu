@@ -13,7 +13,7 @@
 //                          steps of a unit as soon as the accumulator has been scanned
 //   scan (16 warps)        tcgen05.ld (32x32b: a thread owns one point) and the best and second-best maxima over groups of 8 centroids
 //                          (three-input max; the group's number rides in the four low bits of its maximum), handed on per tile
-//   finish (8 or 4 warps)  the best group in the exact form, results, and the point into its cluster's sums
+//   finish (12 warps)      the best group in the exact form, results, and the point into its cluster's sums
 // A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 209 us (285 with scan and finish in the same eight warps, whose chains of
 // TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide); 4 Mi of 4: 172 (652 on the CUDA cores,
 // with a second pass to accumulate); 1 Mi of 16: 114 (582).
@@ -40,7 +40,7 @@ constexpr int TC_TILE = 128;                 // points per accumulator tile
 constexpr int TC_PIPES = 4;                  // pipelines: tile i goes through pipeline i % 4
 constexpr int TC_ACC_COLS = 128;             // columns of a pipeline's accumulator: the centroids of a unit
 constexpr int TC_SCAN_WARPS = 4 * TC_PIPES;  // warp w scans for pipeline w / 4, rows 32 (w % 4) .. + 31
-constexpr int TC_SLOTS = 2;                  // tiles a scan warp may be ahead of the warp that finishes its rows
+constexpr int TC_SLOTS = 3;                  // tiles a scan warp may be ahead of the warp that finishes its rows
 constexpr int TC_CHUNK = 16 * 128;           // one 16-byte K chunk of 128 rows: 16 core matrices of 128 bytes
 
 // What the number of dimensions decides. Chunks are 16 bytes (8 FP16 values) of every row.
@@ -57,7 +57,7 @@ template <int D> struct Shape {
     static constexpr int copies = D == 16 ? 1 : 4;
     static constexpr int dim_stride = 8 * copies;                 // floats
     static constexpr int group_stride = dim_stride * D + (copies == 1 ? 4 : 0);
-    static constexpr int row_stride = D == 4 ? 4 : D + 4;         // floats per cluster in a table of sums: 16-byte pieces of all clusters on all banks
+    static constexpr int row_stride = D == 16 ? 20 : D;           // floats per cluster in a table of sums (16: skewed, or all clusters' pieces would share two places in the banks)
 };
 
 __device__ __forceinline__ uint32_t f16x2_of(float lo, float hi) { uint32_t r; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo)); return r; }
@@ -95,7 +95,7 @@ struct TcShared {
     uint32_t tmem_base;
     int abort_flag;
     unsigned cmax2_bits;
-    double inert[8];
+    double inert[12];
 };
 
 // Best and second-best of the maxima over groups of 8 scores, two groups (16 scores) at a time. The group's number within the unit
@@ -116,10 +116,11 @@ __device__ __forceinline__ void top2_groups(const uint32_t* r, int gid0, Top2& t
     t.m1 = fmaxf(t.m1, hi);
 }
 
+// Read past L1 and not as a read-only load: the kernel just ahead may have written the row (centroids of the last iteration).
 template <int D> __device__ __forceinline__ void load_row(const float* X, long row, bool have, float* x) {
 #pragma unroll
     for (int d = 0; d < D; d += 4) {
-        const float4 v = have ? *reinterpret_cast<const float4*>(X + row * D + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 v = have ? __ldcg(reinterpret_cast<const float4*>(X + row * D + d)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         x[d] = v.x; x[d + 1] = v.y; x[d + 2] = v.z; x[d + 3] = v.w;
     }
 }
@@ -142,10 +143,10 @@ template <int D> __device__ __forceinline__ float group_sqdist(const float* x, c
 // [Kp / 8][D dims][copies][8] | ACC: a table of K sums per finishing warp, then [warp][K] counts | TcShared
 // ACC: the finishing warps also add every point into the table of its cluster (points of a warp in index order), and the block leaves
 // the sum of its tables, its counts and its share of the inertia in part_*[blockIdx.x]: the accumulate pass over X of a Lloyd iteration
-// then needs no kernel and no second read of X. The order of the adds is fixed by the grid. FIN = 4 where eight tables do not fit.
+// then needs no kernel and no second read of X. The order of the adds is fixed by the grid. FIN = 8 or 4 where twelve tables do not fit.
 template <int D, bool ACC, int FIN>
 __global__ void __launch_bounds__((TC_SCAN_WARPS + FIN + TC_PIPES) * 32, 1)
-assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ C, int K, int32_t* __restrict__ idx, float* __restrict__ dist,
+assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restrict__ idx, float* __restrict__ dist,
                  int* __restrict__ err, float* __restrict__ part_sums, int32_t* __restrict__ part_counts, double* __restrict__ part_inertia) {
     using S = Shape<D>;
     constexpr int THREADS = (TC_SCAN_WARPS + FIN + TC_PIPES) * 32;
@@ -191,12 +192,38 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
     __syncthreads();
     pdl_wait();
 
+    const long ntile = (N + TC_TILE - 1) / TC_TILE;
+    const int n_my = (long)blockIdx.x < ntile ? (int)((ntile - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;      // tiles blockIdx.x + i gridDim.x
+    auto tile_row = [&](int i) { return ((long)blockIdx.x + (long)i * gridDim.x) * TC_TILE; };
+
+    // raw rows of a tile into a loader's own buffers (pieces of a row permuted so that eight rows read at once lie on all banks); the
+    // first ones travel while the centroids are prepared
+    unsigned char* const raws = sRaw + max(warp - LOAD0, 0) * (S::raws * S::raw_stage);
+    auto piece_at = [](int r, int p) { return r * PP + (p ^ ((r / (8 / PP)) & (PP - 1))); };
+    auto issue = [&](int i) {
+        if (i < n_my) {
+            const long p0 = tile_row(i);
+            const uint32_t dst = smem_u32(raws + (i / TC_PIPES) % S::raws * S::raw_stage);
+#pragma unroll
+            for (int j = 0; j < 4 * PP; j++) {
+                const int e = lane + 32 * j, r = e / PP, p = e % PP;
+                const long pt = p0 + r;
+                const int nbytes = pt < N ? 16 : 0;              // points past the end read as zeros
+                const float* src = X + (pt < N ? pt : 0) * D + p * 4;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst + piece_at(r, p) * 16), "l"(src), "r"(nbytes) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (warp >= LOAD0) for (int t = 0; t < S::raws; t++) issue(warp - LOAD0 + t * TC_PIPES);
+
     // ── centroids: exact copies by group (padding is NaN: never nearer than anything), max |c|^2 ──
+    static_assert(THREADS >= 256, "a thread per centroid");
     unsigned cm_bits = 0u;
-    for (int n = tid; n < Kp; n += THREADS) {
-        float c[D];
+    const int n = tid;
+    float c[D], nn = 0.0f;
+    if (n < Kp) {
         load_row<D>(C, n, n < K, c);
-        float nn = 0.0f;
 #pragma unroll
         for (int d = 0; d < D; d++) {
 #pragma unroll
@@ -204,7 +231,7 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
                 cgrp[(n >> 3) * S::group_stride + d * S::dim_stride + j * 8 + (n & 7)] = n < K ? c[d] : __uint_as_float(0x7FFFFFFFu);
             nn = fmaf(c[d], c[d], nn);
         }
-        cm_bits = max(cm_bits, __float_as_uint(nn));         // nn >= 0 or NaN: NaN and Inf sort above everything finite
+        cm_bits = __float_as_uint(nn);                       // nn >= 0 or NaN: NaN and Inf sort above everything finite
     }
     cm_bits = __reduce_max_sync(0xffffffffu, cm_bits);
     if (lane == 0) atomicMax(&sh->cmax2_bits, cm_bits);
@@ -213,10 +240,8 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
     const float cm2 = __uint_as_float(sh->cmax2_bits);
     const int cexp = ((int)(sh->cmax2_bits >> 23) - 127) >> 1;                 // -64 for zero, 64 for Inf and NaN (where everything goes the exact way)
     const float scale = __uint_as_float((uint32_t)(min(max(3 - cexp, -60), 60) + 127) << 23);
-    for (int n = tid; n < Kp; n += THREADS) {
-        float c[D];
-        load_row<D>(C, n, n < K, c);
-        float nn = 0.0f;
+    if (n < Kp) {
+        nn = 0.0f;
 #pragma unroll
         for (int d = 0; d < D; d++) nn = fmaf(c[d] * scale, c[d] * scale, nn);
         uint32_t h[D / 2], l[D / 2], t[2];
@@ -252,34 +277,11 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = sh->tmem_base;
 
-    const long ntile = (N + TC_TILE - 1) / TC_TILE;
-    const int n_my = (long)blockIdx.x < ntile ? (int)((ntile - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;      // tiles blockIdx.x + i gridDim.x
-    auto tile_row = [&](int i) { return ((long)blockIdx.x + (long)i * gridDim.x) * TC_TILE; };
-
     if (warp >= LOAD0) {
-        // ── loaders: warp lw owns pipeline lw: raw rows by cp.async (one or two of its tiles ahead; pieces of a row permuted so that
-        //    eight rows read at once lie on all banks), the two FP16 terms into the operand stage, and the MMAs. (One warp issuing for
+        // ── loaders: warp lw owns pipeline lw: raw rows by cp.async (one or two of its tiles ahead), the two FP16 terms into the operand stage, and the MMAs. (One warp issuing for
         //    all accumulators was a chain of 1000 cycles per tile: two waits, two issues and three commits one after the other.) ──
         const int lw = warp - LOAD0;
         const uint32_t a0 = smem_u32(sA + lw * S::a_stage), b0 = smem_u32(sB), aug = smem_u32(sAug), acc = tmem_base + (uint32_t)(lw * TC_ACC_COLS);
-        unsigned char* const raws = sRaw + lw * (S::raws * S::raw_stage);
-        auto piece_at = [](int r, int p) { return r * PP + (p ^ ((r / (8 / PP)) & (PP - 1))); };
-        auto issue = [&](int i) {
-            if (i < n_my) {
-                const long p0 = tile_row(i);
-                const uint32_t dst = smem_u32(raws + (i / TC_PIPES) % S::raws * S::raw_stage);
-#pragma unroll
-                for (int j = 0; j < 4 * PP; j++) {
-                    const int e = lane + 32 * j, r = e / PP, p = e % PP;
-                    const long pt = p0 + r;
-                    const int nbytes = pt < N ? 16 : 0;              // points past the end read as zeros
-                    const float* src = X + (pt < N ? pt : 0) * D + p * 4;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst + piece_at(r, p) * 16), "l"(src), "r"(nbytes) : "memory");
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        for (int t = 0; t < S::raws; t++) issue(lw + t * TC_PIPES);
         bool ok = true;
         for (int i = lw, use = 0; i < n_my && ok; i += TC_PIPES) {
             asm volatile("cp.async.wait_group %0;" :: "n"(S::raws - 1) : "memory");
@@ -377,6 +379,9 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
     } else {
         // ── finish ──
         constexpr int STEP = FIN / 4;                                // warp f of the role takes tiles f / 4, f / 4 + STEP, ...
+        // A slot's tiles are TC_PIPES * TC_SLOTS apart and must all be one warp's: were they several warps', one could wait for a phase of
+        // full_h while another has yet to take the one two before it, which has the same parity.
+        static_assert(TC_PIPES * TC_SLOTS % STEP == 0, "the tiles of a slot go to one finishing warp");
         const int f = warp - FIN0, q = f & 3;
         float* mytab = wtab + (size_t)f * K * S::row_stride;
         int* mycnt = wcnt + (size_t)f * K;
@@ -508,21 +513,21 @@ assign_tc_kernel(const float* __restrict__ X, long N, const float* __restrict__ 
         }
         if (ACC) {
             // the tables of the block, added in warp order; every finishing warp gets here, also after a wait ran out
-            const int ft = tid - FIN0 * 32;
+            const int ft = tid - FIN0 * 32, used = min(FIN, 4 * n_my);       // warps that had a tile
             for (int o = 16; o > 0; o >>= 1) inert += __shfl_xor_sync(0xffffffffu, inert, o);
             if (lane == 0) sh->inert[f] = inert;
             asm volatile("bar.sync 1, %0;" :: "n"(FIN * 32) : "memory");
             for (int e = ft; e < K * D; e += FIN * 32) {
                 const float* t = wtab + (e / D) * S::row_stride + e % D;
                 double v = (double)t[0];
-#pragma unroll
-                for (int w = 1; w < FIN; w++) v += (double)t[(size_t)w * K * S::row_stride];
+#pragma unroll 4
+                for (int w = 1; w < used; w++) v += (double)t[(size_t)w * K * S::row_stride];
                 part_sums[(size_t)blockIdx.x * K * D + e] = (float)v;
             }
             for (int e = ft; e < K; e += FIN * 32) {
                 int v = wcnt[e];
-#pragma unroll
-                for (int w = 1; w < FIN; w++) v += wcnt[(size_t)w * K + e];
+#pragma unroll 4
+                for (int w = 1; w < used; w++) v += wcnt[(size_t)w * K + e];
                 part_counts[(size_t)blockIdx.x * K + e] = v;
             }
             if (ft == 0) {
@@ -579,9 +584,9 @@ int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const fl
     if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
     const long blocks = ibcu_kmeans_tc_blocks(ctx, N);
     switch (D) {
-        case 4: return tc_launch<4, false, 8>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
-        case 8: return tc_launch<8, false, 8>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
-        default: return tc_launch<16, false, 8>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
+        case 4: return tc_launch<4, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
+        case 8: return tc_launch<8, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
+        default: return tc_launch<16, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
     }
 }
 
@@ -593,9 +598,10 @@ int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int 
     if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
     const long blocks = ibcu_kmeans_tc_blocks(ctx, N);
     switch (D) {
-        case 4: return tc_launch<4, true, 8>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
-        case 8: return tc_launch<8, true, 8>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
-        default:                             // eight tables of 256 clusters do not fit, four do
+        case 4: return tc_launch<4, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
+        case 8: return tc_launch<8, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
+        default:                             // of 256 clusters only four tables fit
+            if (tc_smem_bytes<16>(K, true, 12) <= TC_SMEM_MAX) return tc_launch<16, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
             if (tc_smem_bytes<16>(K, true, 8) <= TC_SMEM_MAX) return tc_launch<16, true, 8>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
             return tc_launch<16, true, 4>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
     }
