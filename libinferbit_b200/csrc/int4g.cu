@@ -250,6 +250,237 @@ __global__ void __launch_bounds__(I4G_THREADS) int4g_kernel(const I4gParams p) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// ── tensor-core kernel ──────────────────────────────────────────────────────────────────
+// The same integer arithmetic on mma.sync.m16n8k32 (u8 x s8 -> s32), for groups of 32, 64 or a multiple of 128 columns and no outliers or
+// skipped groups. Weights stream through a cp.async ring of (16 RT rows x 512 bytes, and the scales of those rows and columns) stages,
+// a warp instruction per 512 contiguous bytes; warp w takes 64-byte k-block w (128 columns) of every stage: raw & 0x0F0F0F0F against the
+// limbs of the even columns, raw & 0xF0F0F0F0 (sixteen times the nibble; shifted back exactly) against those of the odd ones. The limbs
+// are the MMA's columns: four of the eight, so a k-block of two groups (G = 64) has the limbs of the first in columns 0 .. 3, zero where
+// the other group's columns are, and those of the second in 4 .. 7; four groups (G = 32) take two sets of MMAs. A thread then holds limbs
+// 0 and 1 or 2 and 3 of a row and group: their exact sum (limb a + 256 limb b, less 8 times the activations' own) goes to FP32, times the
+// group's scale into the row's sum. Sums of a row meet over lanes and warps once per tile of rows.
+// Against 32 dp4a per row and 32 columns (int4g_kernel), us per call: 14336 x 4096, G = 128: 13.7 -> 9.3, G = 64: 13.6 -> 9.8, G = 32: 13.6 ->
+// 12.4; 4096 x 14336: 17.0 -> 12.0; 4096 x 4096: 6.3 -> 4.8. What is left is the chain of a launch: the dependency, the activation, which
+// every block converts for itself, and the first weights.
+constexpr int IM_LD = I4G_WARPS * 64 + 64;                   // bytes per row of a stage, padded: conflict-free fragment reads
+struct I4gMma {
+    const uint8_t* q; const __half* s; const float* x; float* out;
+    int M, N, ng, gsh, rows_per, xs_ld;                      // groups per row; group of a k-block: k >> gsh (G >= 128); rows per block; bytes per limb row
+};
+// words of a row's scales in a stage (1024 columns): its halves may start in the middle of a word
+__host__ __device__ constexpr int im_sw(int G) { return 1024 / G / 2 + 1; }
+__host__ __device__ constexpr size_t im_stage(int RT, int G) { return (size_t)RT * 16 * (IM_LD + im_sw(G) * 4); }
+
+__device__ __forceinline__ void im_mma(int* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t im_word(const uint4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
+
+// Shared memory: stage ring | limbs [4][xs_ld] | 32 zero bytes | per group (limb 0 + 256 limb 1, limb 2 + 256 limb 3 sums, times 8) | row sums [2][8][16 RT]
+template <int G, int RT, int STAGES, int HELD>
+__global__ void __launch_bounds__(I4G_THREADS) int4g_mma_kernel(const I4gMma p) {
+    constexpr int R = 16 * RT, SW = im_sw(G), SETS = G == 32 ? 2 : 1, SUB = 128 / G;     // column sets, groups per k-block
+    constexpr size_t STAGE = im_stage(RT, G);
+    extern __shared__ __align__(128) unsigned char im_smem[];
+    __shared__ float s_amax[I4G_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    pdl_launch_dependents();
+    const int row_begin = blockIdx.x * p.rows_per, row_end = min(p.M, row_begin + p.rows_per);
+    const int rowbytes = p.N >> 1, nkb = (p.N + 127) >> 7, nst = (nkb + I4G_WARPS - 1) / I4G_WARPS;
+    unsigned char* xs = im_smem + STAGES * STAGE;
+    unsigned char* zero = xs + 4 * (size_t)p.xs_ld;
+    int* bias = reinterpret_cast<int*>(zero + 32);
+    float* red = reinterpret_cast<float*>(bias + 2 * SUB * nkb);
+
+    // producer: this thread owns 16-byte piece lane of rows warp + 8 i of every stage, and its share of the scales
+    int pf_row = row_begin, pf_it = 0, pf_slot = 0;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(im_smem);
+    auto issue = [&]() {
+        if (pf_row < row_end) {
+            const int rows = min(R, row_end - pf_row), col = pf_it * 512 + lane * 16;
+            const uint32_t d = ring + (uint32_t)(pf_slot * STAGE);
+#pragma unroll
+            for (int i = 0; i < 2 * RT; i++) {
+                const int r = warp + 8 * i;
+                const bool on = r < rows && col < rowbytes;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d + r * IM_LD + lane * 16),
+                             "l"(p.q + (size_t)(pf_row + (on ? r : 0)) * rowbytes + (on ? col : 0)), "r"(on ? 16 : 0) : "memory");
+            }
+            // the scales of group j of G columns; of a group longer than a k-block only once, at its place among the k-blocks
+            for (int e = tid; e < R * SW; e += I4G_THREADS) {
+                const int r = e / SW, w = e - r * SW;
+                const size_t first = (size_t)(pf_row + r) * p.ng + ((size_t)(pf_it * I4G_WARPS * SUB) >> p.gsh);
+                const size_t at = (first & ~(size_t)1) + 2 * w;
+                const bool on = r < rows && at < (size_t)p.M * p.ng;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(d + R * IM_LD + e * 4), "l"(p.s + (on ? at : 0)), "r"(on ? 4 : 0) : "memory");
+            }
+            pf_slot = pf_slot + 1 == STAGES ? 0 : pf_slot + 1;
+            if (++pf_it == nst) { pf_it = 0; pf_row += rows; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int q = 0; q < STAGES - 1; q++) issue();             // weights and scales do not depend on the kernel ahead
+    if (tid < 8) reinterpret_cast<int*>(zero)[tid] = 0;
+    pdl_wait();
+
+    // ── activation: max |x|, fixed point, limbs, and the limb sums of every group ──
+    const int n8 = p.N >> 3, n8p = nkb << 4;                  // groups of eight columns; with the padding of the last k-block
+    float4 xa[HELD], xb[HELD];
+    float amax = 0.0f;
+#pragma unroll
+    for (int u = 0; u < HELD; u++) {
+        const int i8 = tid + u * I4G_THREADS;
+        xa[u] = xb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i8 < n8) { xa[u] = __ldcg(reinterpret_cast<const float4*>(p.x) + 2 * i8); xb[u] = __ldcg(reinterpret_cast<const float4*>(p.x) + 2 * i8 + 1); }
+    }
+#pragma unroll
+    for (int u = 0; u < HELD; u++)
+        amax = fmaxf(amax, fmaxf(fmaxf(fmaxf(fabsf(xa[u].x), fabsf(xa[u].y)), fmaxf(fabsf(xa[u].z), fabsf(xa[u].w))),
+                                 fmaxf(fmaxf(fabsf(xb[u].x), fabsf(xb[u].y)), fmaxf(fabsf(xb[u].z), fabsf(xb[u].w)))));
+    amax = warp_max(amax);
+    if (lane == 0) s_amax[warp] = amax;
+    __syncthreads();
+    amax = s_amax[0];
+#pragma unroll
+    for (int w = 1; w < I4G_WARPS; w++) amax = fmaxf(amax, s_amax[w]);
+    const int ex = (int)((__float_as_uint(amax) >> 23) & 0xFF);      // amax in [2^(ex-127), 2^(ex-126))
+    const int sh = max(-126, min(126, (amax > 0.0f && ex != 255) ? 156 - ex : 0));
+    const float mul = __uint_as_float((uint32_t)(127 + sh) << 23), back = __uint_as_float((uint32_t)(127 - sh) << 23);
+#pragma unroll
+    for (int u = 0; u < HELD; u++) {
+        const int i8 = tid + u * I4G_THREADS;
+        if (i8 - lane >= n8p) break;                          // whole warps: the shuffles take all lanes
+        const int X[8] = { __float2int_rn(xa[u].x * mul), __float2int_rn(xa[u].y * mul), __float2int_rn(xa[u].z * mul), __float2int_rn(xa[u].w * mul),
+                           __float2int_rn(xb[u].x * mul), __float2int_rn(xb[u].y * mul), __float2int_rn(xb[u].z * mul), __float2int_rn(xb[u].w * mul) };
+        uint32_t D[8], ev[4], od[4];
+#pragma unroll
+        for (int i = 0; i < 8; i++) D[i] = ((uint32_t)X[i] + 0x00808080u) ^ 0x00808080u;     // the four balanced digits of X as bytes
+        transpose4x4_bytes(D[0], D[2], D[4], D[6], ev);       // ev[k]: limb k of columns 0, 2, 4, 6
+        transpose4x4_bytes(D[1], D[3], D[5], D[7], od);
+        int l[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (i8 < n8p) *reinterpret_cast<uint2*>(xs + (size_t)k * p.xs_ld + (size_t)i8 * 8) = make_uint2(ev[k], od[k]);
+            l[k] = __dp4a((int)ev[k], 0x01010101, __dp4a((int)od[k], 0x01010101, 0));
+        }
+        int s01 = l[0] + 256 * l[1], s23 = l[2] + 256 * l[3];
+#pragma unroll
+        for (int o = 1; o < G / 8; o <<= 1) { s01 += __shfl_xor_sync(0xffffffffu, s01, o); s23 += __shfl_xor_sync(0xffffffffu, s23, o); }
+        if (i8 < n8p && (i8 & (G / 8 - 1)) == 0) *reinterpret_cast<int2*>(bias + 2 * (i8 / (G / 8))) = make_int2(8 * s01, 8 * s23);
+    }
+    __syncthreads();
+
+    // B operand: limb g % 4 of the columns this lane's k positions stand for; zeros where they belong to another group's set
+    const unsigned char* xcol[SETS];
+    int kstep[SETS], xoff[SETS];
+#pragma unroll
+    for (int c = 0; c < SETS; c++) {
+        const bool mine = G == 128 || (G == 64 ? (t >> 1) == (g >> 2) : t == 2 * c + (g >> 2));
+        xcol[c] = mine ? xs + (size_t)(g & 3) * p.xs_ld + 32 * t : zero;
+        kstep[c] = mine ? 128 : 0;
+        xoff[c] = mine ? 16 : 0;
+    }
+    int slot = 0, buf = 0, tile_rows = 0;
+    for (int row0 = row_begin; row0 < row_end; row0 += tile_rows) {
+        tile_rows = min(R, row_end - row0);
+        float acc[RT][2];
+        int odd[RT][2];                                       // the row's first scale is the upper half of its word
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) { acc[i][h] = 0.0f; odd[i][h] = (row0 + i * 16 + 8 * h + g) & p.ng & 1; }
+        for (int it = 0; it < nst; it++) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2) : "memory");
+            __syncthreads();                                  // this stage has landed for everyone; the previous one is free
+            issue();
+            const int k = it * I4G_WARPS + warp;
+            if (k < nkb) {
+                const unsigned char* st = im_smem + slot * STAGE;
+                const unsigned char* sw = st + warp * 64 + 16 * t;
+                const __half* sc = reinterpret_cast<const __half*>(st + R * IM_LD);
+                const int g0 = (it * I4G_WARPS * SUB) >> p.gsh;                         // first group of the stage
+                uint4 cur[RT * 2];
+#pragma unroll
+                for (int j = 0; j < RT * 2; j++) cur[j] = *reinterpret_cast<const uint4*>(sw + ((j >> 1) * 16 + (j & 1) * 8 + g) * IM_LD);
+#pragma unroll
+                for (int c = 0; c < SETS; c++) {
+                    uint4 xf[2];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) xf[h] = *reinterpret_cast<const uint4*>(xcol[c] + (size_t)k * kstep[c] + h * xoff[c]);
+                    const int grp = G == 128 ? k >> p.gsh : k * SUB + 2 * c + (t >> 1);
+                    const int b8 = bias[2 * (G == 128 ? k : grp) + (t & 1)], gl = grp - g0;
+                    const bool on = grp < p.ng;               // the padding of the last k-block has no scale
+#pragma unroll
+                    for (int i = 0; i < RT; i++) {
+                        int lo[4] = { 0, 0, 0, 0 }, hi[4] = { 0, 0, 0, 0 };
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const uint32_t r0a = im_word(cur[2 * i], 2 * h), r0b = im_word(cur[2 * i], 2 * h + 1);
+                            const uint32_t r1a = im_word(cur[2 * i + 1], 2 * h), r1b = im_word(cur[2 * i + 1], 2 * h + 1);
+                            im_mma(lo, r0a & 0x0F0F0F0Fu, r1a & 0x0F0F0F0Fu, r0b & 0x0F0F0F0Fu, r1b & 0x0F0F0F0Fu, xf[h].x, xf[h].z);
+                            im_mma(hi, r0a & 0xF0F0F0F0u, r1a & 0xF0F0F0F0u, r0b & 0xF0F0F0F0u, r1b & 0xF0F0F0F0u, xf[h].y, xf[h].w);
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int v = lo[2 * h] + (hi[2 * h] >> 4) + 256 * (lo[2 * h + 1] + (hi[2 * h + 1] >> 4)) - b8;
+                            const __half w = sc[(i * 16 + 8 * h + g) * (2 * SW) + (odd[i][h] ^ (g0 & 1)) + gl];
+                            acc[i][h] = fmaf(on ? __half2float(w) : 0.0f, (float)v, acc[i][h]);
+                        }
+                    }
+                }
+            }
+            slot = slot + 1 == STAGES ? 0 : slot + 1;
+        }
+        float* rw = red + (size_t)buf * I4G_WARPS * R;
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float v = G == 128 && t >= 2 ? 0.0f : (t & 1 ? 65536.0f * acc[i][h] : acc[i][h]);       // G >= 128: columns 4 .. 7 repeat 0 .. 3
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (t == 0) rw[warp * R + i * 16 + 8 * h + g] = v;
+            }
+        __syncthreads();
+        if (tid < tile_rows) {
+            float v = rw[tid];
+#pragma unroll
+            for (int w = 1; w < I4G_WARPS; w++) v += rw[w * R + tid];
+            p.out[row0 + tid] = v * back;
+        }
+        buf ^= 1;                                             // the next tile's sums do not wait for these reads
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <int G, int RT, int STAGES>
+int im_launch(ibcu_ctx* ctx, const I4gMma& p, size_t smem) {
+    static SmemOptIn opt4, opt8;
+    const dim3 grid((p.M + p.rows_per - 1) / p.rows_per), block(I4G_THREADS);
+    if (p.N <= 4 * 8 * I4G_THREADS) {
+        if (int rc = ibcu_allow_smem(ctx, opt4, int4g_mma_kernel<G, RT, STAGES, 4>, smem)) return rc;
+        return ibcu_launch(ctx, int4g_mma_kernel<G, RT, STAGES, 4>, grid, block, smem, 1, true, p);
+    }
+    if (int rc = ibcu_allow_smem(ctx, opt8, int4g_mma_kernel<G, RT, STAGES, 8>, smem)) return rc;
+    return ibcu_launch(ctx, int4g_mma_kernel<G, RT, STAGES, 8>, grid, block, smem, 1, true, p);
+}
+
+// Rows in equal runs over two blocks per SM; tiles of 32 rows where a run is longer than 16 and three stages still fit beside the limbs.
+template <int G>
+int im_dispatch(ibcu_ctx* ctx, I4gMma& p) {
+    const int nkb = (p.N + 127) / 128;
+    const size_t tail = 4 * (size_t)p.xs_ld + 32 + (size_t)nkb * (128 / G) * 8, room = 112 * 1024;
+    p.rows_per = (p.M + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count);
+    auto total = [&](int rt, int stages) { return stages * im_stage(rt, G) + tail + 2 * (size_t)I4G_WARPS * 16 * rt * sizeof(float); };
+    if (p.rows_per > 16 && total(2, 5) <= room) return im_launch<G, 2, 5>(ctx, p, total(2, 5));
+    if (p.rows_per > 16 && total(2, 3) <= room) return im_launch<G, 2, 3>(ctx, p, total(2, 3));
+    if (total(1, 8) <= room) return im_launch<G, 1, 8>(ctx, p, total(1, 8));
+    return im_launch<G, 1, 4>(ctx, p, total(1, 4));
+}
+
 // Any N, G (even): a warp per row, lanes over the groups, columns in order inside a group; activations from global memory.
 __global__ void __launch_bounds__(I4G_THREADS) int4g_generic_kernel(const I4gParams p, const unsigned char* skip) {
     pdl_launch_dependents();
@@ -309,6 +540,15 @@ extern "C" int ibcu_int4g_matmul_fp32(ibcu_ctx* ctx, const ibcu_int4g_t* t, cons
     p.M = t->M; p.N = t->N; p.G = t->G; p.K_out = t->K_out;
     p.q = t->q; p.s = (const __half*)t->s; p.outl_idx = t->outl_idx; p.outl_val = (const __half*)t->outl_val;
     p.x = x; p.out = out; p.eps = eps_act_rel;
+    // groups of 32, 64 or a power-of-two multiple of 128 columns, nothing left out and nothing beside the groups: the tensor cores. Up to
+    // 16384 columns are held in registers while they are converted.
+    const int per128 = t->G / 128;
+    if (p.eps == 0.0f && t->K_out == 0 && (t->N & 31) == 0 && t->N <= 8 * 8 * I4G_THREADS && (t->G == 32 || t->G == 64 || (t->G % 128 == 0 && (per128 & (per128 - 1)) == 0)) &&
+        (((uintptr_t)t->q | (uintptr_t)x) & 15) == 0 && ((uintptr_t)t->s & 3) == 0) {
+        I4gMma m = { t->q, (const __half*)t->s, x, out, t->M, t->N, t->N / t->G, 0, 0, (t->N + 127) / 128 * 128 + 16 };
+        while ((128 << m.gsh) < t->G) m.gsh++;
+        return t->G == 32 ? im_dispatch<32>(ctx, m) : (t->G == 64 ? im_dispatch<64>(ctx, m) : im_dispatch<128>(ctx, m));
+    }
     const size_t xbytes = (size_t)t->N * sizeof(float) + (((size_t)(t->N / 32) + 3) & ~(size_t)3) * sizeof(float) + (((size_t)(t->N / t->G) + 15) & ~(size_t)15);
     const size_t smem = xbytes + (size_t)I4G_WARPS * I4G_STAGES * I4G_ROWS * 32 * 5 * sizeof(uint32_t);
     const bool fast = (t->N & 31) == 0 && (t->G & 31) == 0 && smem <= 200 * 1024 &&

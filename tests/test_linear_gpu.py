@@ -525,6 +525,21 @@ def test_group_scaled_int4_rows(backend, cpu_libs, M, N, G, K_out, eps):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,G", [(17, 128, 128), (1, 14336, 128), (300, 160, 32), (4737, 1088, 64), (2000, 2112, 64), (9473, 1024, 32),
+                                   (700, 4096, 512), (513, 3072, 1024), (65, 6144, 2048), (5000, 11008, 128), (641, 16384, 32), (33, 3232, 32)])
+def test_group_scaled_int4_on_the_tensor_cores(backend, cpu_libs, M, N, G):
+    """Tiles of 16 and 32 rows with a remainder, k-blocks that end inside a group or hold several, row scales that start in the middle of
+    a word (an odd number of groups), groups of several k-blocks."""
+    rng = np.random.default_rng(M * 7 + N + G)
+    q, s, x, oi, ov = _cpu.make_int4g_case(rng, M, N, G, 0)
+    got = backend.int4g_matmul(q, s, G, x, oi, ov, 0.0)
+    want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, G, x, oi, ov, 0.0)
+    assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
+    assert np.array_equal(got, backend.int4g_matmul(q, s, G, x, oi, ov, 0.0))
+    assert np.array_equal(backend.int4g_matmul(q, s, G, 2.0 * x, oi, ov, 0.0), 2.0 * got)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N", [32, 2048, 2080, 8192, 8224, 16384, 16416])
 def test_group_scaled_int4_row_lengths(backend, cpu_libs, N):
     """Where the fast kernel changes how it holds the activation: one and several groups of eight columns per thread, the last length of
