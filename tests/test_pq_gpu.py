@@ -171,6 +171,27 @@ def test_pq_lm_head_topk_equal_logits(backend, cpu_libs):
         assert gi.tolist() == list(range(14))
 
 
+@pytest.mark.parametrize("M,k_top,step", [(65536, 256, 4096), (32768, 200, 4096), (32771, 64, 1), (4097, 256, 4), (1023, 255, 1), (70000, 100, 4096)])
+def test_pq_lm_head_topk_order_of_scaled_rows(backend, cpu_libs, M, k_top, step):
+    """Rows that differ by their scale alone, many of them equal: the largest sit `step` apart (one thread of the selection holds several of
+    them), the boundary falls among equal rows, of which the lowest are taken."""
+    rng = np.random.default_rng(M + k_top)
+    d = _cpu.make_pq_case_ex(rng, M, 32, 16, 256, 0, 0, 1)
+    for key in ("idx1_l", "idx1_r"):
+        d[key][:] = d[key][0]
+    level = np.ones(M, np.float32)
+    level[::step][: k_top // 2] = 3.0
+    level[5::7][: k_top] += 0.5 * (1 + np.arange(len(level[5::7][: k_top])) % 3)
+    d["rs"][:] = _cpu.fp16_bits(level)
+    x = d["x"][0].copy()
+    if _cpu.oracle_pq_topk(cpu_libs.oracle, d, x, 1)[0][0] < 0:
+        x = -x                                                # larger scales then have larger logits
+    t = backend.make_pq_ex(d)
+    gl, gi = backend.pq_lm_head_topk(t, x, k_top)
+    assert gi.tolist() == np.argsort(-level, kind="stable")[:k_top].tolist()
+    assert np.all(np.diff(gl) <= 0)
+
+
 def test_pq_lm_head_topk_through_the_host_layer(cpu_libs):
     """ib_b200_pq_lm_head_topk takes the reference's own struct and host pointers."""
     from libinferbit_b200 import _ffi
