@@ -3,7 +3,7 @@
 #pragma once
 #include <cstdint>
 
-constexpr int TC_SPIN_LIMIT = 1 << 22;      // tries of a wait before the block gives up (each try can itself block for a while)
+constexpr unsigned long long TC_WAIT_NS = 2000000000ull;      // a wait gives up after two seconds
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -16,20 +16,28 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    // the hint lets the thread sleep up to about two microseconds per try instead of spinning on the issue slots
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
+    // (without a time of its own: with a hint of two microseconds k-means took 1903 us instead of 1872, eight activations through
+    // a product-quantised tensor 524 instead of 520, sixteen through INT8 projections 444 instead of 441)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
 // Bounded wait. Returns false when the block is giving up (this wait ran out, or another role's did). A phase that is complete
-// already is seen by the plain test in 65 cycles; the try with a hint takes 112 to say so. (Where phases are rarely complete the
+// already is seen by the plain test in 65 cycles; the try takes 112 to say so. (Where phases are rarely complete the
 // test only delays the try: k-means takes the wait without it, 2864 against 2850 us.)
 template <bool TEST = true>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
     if (TEST && mbar_test(bar, parity)) return true;
-    for (int it = 0; it < TC_SPIN_LIMIT; it++) {
+    unsigned long long since = 0;
+    for (int it = 1;; it++) {
         if (mbar_try(bar, parity)) return true;
         if (*abort_flag) return false;
+        if ((it & 63) == 0) {                                  // the clock is looked at now and then only
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (!since) since = now;
+            else if (now - since > TC_WAIT_NS) break;
+        }
     }
     *abort_flag = code;
     return false;
