@@ -74,3 +74,53 @@ def test_every_opt_in_goes_through_it():
         code = open(path).read()
         if "cudaFuncAttributeMaxDynamicSharedMemorySize" in code:
             assert "std::call_once" in code and "(int)smem)" not in code and "(int)csmem)" not in code, path
+
+
+UPLOAD = r"""
+#include "ib_b200_internal.h"
+#include <stdlib.h>
+#include <string.h>
+static char* area; static int copies, fail_at = -1, in_flight;
+static struct { void* dst; const void* src; size_t n; } queued[4096];
+static int fake_stage(int slot, size_t bytes, void** h, void** d) { (void)slot; area = realloc(area, bytes ? bytes : 1); *h = area; *d = NULL; return 0; }
+static int fake_sync(ibcu_ctx* c) { (void)c; for (int i = 0; i < in_flight; i++) memcpy(queued[i].dst, queued[i].src, queued[i].n); in_flight = 0; return 0; }
+static int fake_h2d(ibcu_ctx* c, void* dst, const void* src, size_t n) {       /* leaves the staging area as late as the device may */
+    (void)c;
+    if (copies++ == fail_at) return -2;
+    queued[in_flight].dst = dst; queued[in_flight].src = src; queued[in_flight++].n = n;
+    return 0;
+}
+#define ib_b200_stage fake_stage
+#define ibcu_sync_spin fake_sync
+#define ibcu_memcpy_h2d fake_h2d
+#include "ib_b200_pq.c"
+#include <stdio.h>
+int main(void) {
+    const size_t sizes[] = { 1, KM_PIECE - 1, KM_PIECE, 5 * KM_PIECE + 7, KM_STAGE, KM_STAGE + 3, 40u << 20 };
+    for (int s = 0; s < 7; s++)
+        for (int rep = 0; rep < 5; rep++) {
+            const size_t n = sizes[s];
+            char *src = malloc(n), *dst = calloc(n, 1);
+            for (size_t i = 0; i < n; i++) src[i] = (char)(i * 2654435761u >> 13) + rep;
+            if (km_upload(dst, src, n)) return 1;
+            fake_sync(NULL);
+            if (memcmp(src, dst, n)) { printf("size %zu differs\n", n); return 2; }
+            copies = 0; fail_at = (int)(n / KM_PIECE / 2);                     /* a transfer that fails ends the call, helpers and all */
+            if (km_upload(dst, src, n) != -2) return 3;
+            in_flight = 0; fail_at = -1;
+            free(src); free(dst);
+        }
+    return 0;
+}
+"""
+
+
+def test_kmeans_upload_in_pieces(tmp_path):
+    """Pieces copied by several threads into a staging area that is used more than once: every byte arrives, and a transfer that fails
+    leaves no thread behind."""
+    src, exe = tmp_path / "up.c", tmp_path / "up"
+    src.write_text(UPLOAD)
+    subprocess.run(["gcc", "-std=gnu11", "-O2", "-w", f"-I{ROOT}/include", f"-I{LIB}/host", "-o", str(exe), str(src), f"{LIB}/host/ib_b200_table.c",
+                    f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}", "-lm", "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout)
