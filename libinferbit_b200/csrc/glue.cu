@@ -179,6 +179,7 @@ __host__ __device__ __forceinline__ void att_plan(int cap, int want, int chunk_c
     }
 }
 
+template <bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                              const float* __restrict__ v_cache, float* __restrict__ part,
                                                              int n_heads, int n_kv, int hd, int pos0, int chunk, int nsplit,
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
     float* vt = kt + (size_t)chunk_cap * ld;        // [chunk_cap][ld]
     pdl_launch_dependents();
     pdl_wait();
-    gather_wait(gw);                                // q, k, v may be rows that peers pushed
+    if (MG) gather_wait(gw);                        // q, k, v may be rows that peers pushed
     if (pos0_ptr) {                                 // position read on the device: the same launch serves every position
         pos0 = __ldcg(pos0_ptr);
         att_plan(pos0 + (int)gridDim.z, want, chunk_cap, chunk, nsplit);
@@ -509,12 +510,13 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(float* __restrict__ out, 
 }
 
 // grid (parts, B): silu(gate) * up over one column range of one row, and the largest magnitude written
+template <bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(256) silu_mul_amax_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up,
                                                             int N, int chunk, float* __restrict__ amax, const GatherWait gw) {
     __shared__ float red[32];
     pdl_launch_dependents();
     pdl_wait();
-    gather_wait(gw);                                // gate and up may be rows that peers pushed
+    if (MG) gather_wait(gw);                        // gate and up may be rows that peers pushed
     const int p = blockIdx.x, b = blockIdx.y;
     const size_t base = (size_t)b * N;
     const int c1 = min(N, (p + 1) * chunk);
@@ -698,11 +700,13 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     const size_t pbytes = (size_t)B * n_heads * grid_y * (head_dim + 4) * sizeof(float);
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, pbytes);
     if (rc) return rc;
-    static SmemOptIn opt;
-    if ((rc = ibcu_allow_smem(ctx, opt, attn_partial_kernel, smem))) return rc;
+    static SmemOptIn opt, opt_mg;
+    if ((rc = ibcu_allow_smem(ctx, opt, attn_partial_kernel<false>, smem))) return rc;
+    if ((rc = ibcu_allow_smem(ctx, opt_mg, attn_partial_kernel<true>, smem))) return rc;
     GatherWait gw;
     ibcu_take_gather_wait(ctx, &gw);
-    rc = ibcu_launch(ctx, attn_partial_kernel, dim3(n_kv_heads, grid_y, B), dim3(32 * group), smem, 1, true,
+    auto kern = gw.flags || gw.tag.n ? attn_partial_kernel<true> : attn_partial_kernel<false>;
+    rc = ibcu_launch(ctx, kern, dim3(n_kv_heads, grid_y, B), dim3(32 * group), smem, 1, true,
                      q, (const float*)k_cache, (const float*)v_cache, (float*)ctx->scratch, n_heads, n_kv_heads, head_dim, pos0, chunk, nsplit,
                      k_new, v_new, k_cache, v_cache, theta, pos0_dev, want, chunk_cap, gw);
     if (rc) return rc;
@@ -757,7 +761,7 @@ extern "C" int ibcu_silu_mul_amax(ibcu_ctx* ctx, float* out, const float* gate, 
     const int chunk = (N + parts - 1) / parts;
     GatherWait gw;
     ibcu_take_gather_wait(ctx, &gw);
-    return ibcu_launch(ctx, silu_mul_amax_kernel, dim3(parts, B), dim3(256), 0, 1, true, out, gate, up, N, chunk, amax, gw);
+    return ibcu_launch(ctx, gw.flags || gw.tag.n ? silu_mul_amax_kernel<true> : silu_mul_amax_kernel<false>, dim3(parts, B), dim3(256), 0, 1, true, out, gate, up, N, chunk, amax, gw);
 }
 
 extern "C" int ibcu_silu_mul(ibcu_ctx* ctx, float* out, const float* gate, const float* up, size_t n) {

@@ -122,7 +122,9 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // XV: 4 XV columns of an activation per thread are held in registers while the block converts it. Up to 4096 columns the instance with 4
 // is enough (76 registers; the one with 8 takes 120): hidden size 4096, one token, 8-bit projections of 12 layers 171.8 -> 161.1 us; 2048:
 // 128.1 -> 115.6. Two blocks fill an SM's shared memory with either, so it is not room for a third; what else it is was not measured apart.
-template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
+// MG: the launch waits for rows of peers or pushes its own to them. Without that code, which a single GPU never runs, projections of a
+// 7B shape took 206 us instead of 216 (INT8, one activation, sixteen layers), a decode step 1812 instead of 1857.
+template <int BITS, int NCG, int RT, int W, int STAGES, int XV, bool MG>
 __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p) {
     constexpr int R = RT * 16;                                // most rows per tile
     constexpr int RLD = lin_rld(NCG);                         // words per row of the reduction buffer
@@ -192,7 +194,7 @@ __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p
 #pragma unroll
     for (int s = 0; s < STAGES - 1; s++) pf_issue();          // weights first: they do not depend on x
     pdl_wait();
-    const unsigned recv_tag = gather_wait(p.gw);             // not 0: this launch received a tagged gather; its own pushes then carry the next tag
+    const unsigned recv_tag = MG ? gather_wait(p.gw) : 0u;   // not 0: this launch received a tagged gather; its own pushes then carry the next tag
 
     // ── this slice's limbs, scale-back factors and limb sums ──
     if (p.fused_x) {
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p
         }
         __syncthreads();
         const int B = p.B;
-        const unsigned tag = p.gp.world ? (recv_tag ? recv_tag + 1u : tag_current(p.gp)) : 0u;
+        const unsigned tag = MG && p.gp.world ? (recv_tag ? recv_tag + 1u : tag_current(p.gp)) : 0u;
         // one thread per (row, activation): limb sums over the warps, bias, recombination
         for (int e = threadIdx.x; e < R * B; e += W * 32) {
             const int r = e % R, b = e / R;
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p
                     float* o = T.out + (size_t)b * T.out_stride + row;
                     const float v = T.epilogue == IBCU_EPI_ADD ? *o + y * sc : y * sc;
                     *o = v;
-                    if (p.gp.world) tag_push(p.gp, (size_t)T.win_off + ((size_t)b * T.out_stride + row) * sizeof(float), v, tag);
+                    if (MG && p.gp.world) tag_push(p.gp, (size_t)T.win_off + ((size_t)b * T.out_stride + row) * sizeof(float), v, tag);
                 }
             } else {
 #pragma unroll
@@ -407,13 +409,19 @@ __global__ void __launch_bounds__(256) linear_generic_kernel(LinTensor T, const 
     }
 }
 
-template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
-int launch_mma_x(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
-    auto kern = linear_mma_kernel<BITS, NCG, RT, W, STAGES, XV>;
+template <int BITS, int NCG, int RT, int W, int STAGES, int XV, bool MG>
+int launch_mma_mg(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
+    auto kern = linear_mma_kernel<BITS, NCG, RT, W, STAGES, XV, MG>;
     const size_t smem = (size_t)STAGES * RT * 16 * lin_ld(W) + (size_t)(BITS == 4 ? 2 : 1) * W * RT * 16 * lin_rld(NCG) * 4 + smem_tail;   // ring + reduction buffer + limbs
     static SmemOptIn opt;
     if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(W * 32), smem, 1, true, p);
+}
+
+template <int BITS, int NCG, int RT, int W, int STAGES, int XV>
+int launch_mma_x(ibcu_ctx* ctx, const LinearParams& p, int grid, size_t smem_tail) {
+    if (p.gp.world || p.gw.flags || p.gw.tag.n) return launch_mma_mg<BITS, NCG, RT, W, STAGES, XV, true>(ctx, p, grid, smem_tail);
+    return launch_mma_mg<BITS, NCG, RT, W, STAGES, XV, false>(ctx, p, grid, smem_tail);
 }
 
 // a block that converts more than 4096 columns itself, and has to find their maximum first, holds up to 8192 (one activation: see lin_plan)

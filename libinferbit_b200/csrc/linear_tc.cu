@@ -93,13 +93,13 @@ __device__ __forceinline__ float row_scale(const LinTensor& W, int row) {
 }
 
 // grid (parts, B): digits of one activation (or of one part of its columns when the caller knows the maximum)
-template <int T>
+template <int T, bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, int part_cols, int all_cols, int nc, int perm8, int8_t* __restrict__ xtiles,
                                                      float* __restrict__ xscale, int* __restrict__ xsum, const GatherWait gw) {
     __shared__ XScratch sc;
     pdl_launch_dependents();
     pdl_wait();
-    gather_wait(gw);
+    if (MG) gather_wait(gw);
     const int part = blockIdx.x, b = blockIdx.y, c0 = part * part_cols;
     const XTiles dst = { xtiles, nc, b * LIN_LIMBS, c0 };
     xconvert_any(src, N, b, c0, min(part_cols, all_cols - c0), dst, perm8, sc, xscale + b * gridDim.x + part, xsum + ((size_t)b * gridDim.x + part) * LIN_LIMBS);
@@ -592,8 +592,9 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
                            op == IBCU_PRO_KNOWN_MAX ? pro->amax : nullptr, op == IBCU_PRO_KNOWN_MAX ? pro->n_amax : 0 };
     const dim3 xg(parts, B);
     const int perm8 = bits == 4 ? 1 : 0, cols = part_kb * 128, all = p.nkb * 128;
-    rc = cols > 2048 ? ibcu_launch(ctx, xprep_tc_kernel<512>, xg, dim3(512), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw)
-                     : ibcu_launch(ctx, xprep_tc_kernel<256>, xg, dim3(256), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
+    const bool mg = gw.flags || gw.tag.n;
+    auto prep = cols > 2048 ? (mg ? xprep_tc_kernel<512, true> : xprep_tc_kernel<512, false>) : (mg ? xprep_tc_kernel<256, true> : xprep_tc_kernel<256, false>);
+    rc = ibcu_launch(ctx, prep, xg, dim3(cols > 2048 ? 512 : 256), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
     if (rc) return rc;
     const int grid = S * (nruns < slots ? nruns : slots);
     if (bits == 8) return T == 1 ? launch_tc<8, 1>(ctx, maps, p, grid, smem) : launch_tc<8, 2>(ctx, maps, p, grid, smem);
