@@ -193,7 +193,6 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
     float* ps = qs + group * hd;                    // [group][32]
     float* kt = ps + group * 32;                    // [chunk_cap][ld]
     float* vt = kt + (size_t)chunk_cap * ld;        // [chunk_cap][ld]
-    pdl_launch_dependents();
     pdl_wait();
     if (MG) gather_wait(gw);                        // q, k, v may be rows that peers pushed
     if (pos0_ptr) {                                 // position read on the device: the same launch serves every position
@@ -241,6 +240,7 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    pdl_launch_dependents();                         // not earlier: the weights that the launches behind ask for would be ahead of this tile (decode step 1785 -> 1766 us)
     const float scale = 1.0f / sqrtf((float)hd);
     const float4* q4 = reinterpret_cast<const float4*>(qs + g * hd);
     const int hd4 = hd / 4, ld4 = ld / 4;
@@ -306,13 +306,14 @@ __host__ __device__ __forceinline__ void att_plan_tiles(int cap, int want, int& 
 }
 
 // grid (B, parts): position pos0 + b, its heads dealt out among the parts
+template <bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(256) rope_stage_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                                          float* __restrict__ q_rot, float* __restrict__ k_cache, float* __restrict__ v_cache,
                                                          int n_heads, int n_kv, int hd, int pos0, const int* pos0_ptr, float theta, const GatherWait gw) {
     __shared__ float2 cs[128];
     pdl_launch_dependents();
     pdl_wait();
-    gather_wait(gw);
+    if (MG) gather_wait(gw);
     if (pos0_ptr) pos0 = __ldcg(pos0_ptr);
     const int b = blockIdx.x, pos = pos0 + b, half = hd / 2, kv_dim = n_kv * hd;
     for (int m = threadIdx.x; m < half; m += blockDim.x) {
@@ -333,6 +334,7 @@ __global__ void __launch_bounds__(256) rope_stage_kernel(const float* __restrict
 
 // grid (kv heads, chunks, groups of positions), 32 * group * nb threads: warp w serves query head w % group of the KV head and
 // the ATT_QPW positions (blockIdx.z * nb + w / group) * ATT_QPW ..; the cache holds rows 0 .. pos0 + B - 1
+template <bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(256) attn_batch_kernel(const float* q, const float* k_cache, const float* v_cache, float* __restrict__ part,
                                                          int n_heads, int n_kv, int hd, int B, int nb, int pos0, const int* pos0_ptr, int want, const GatherWait gw) {
     extern __shared__ __align__(16) float asm_[];
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(256) attn_batch_kernel(const float* q, const f
     float* vt = kt + 2 * ATT_TILE * ld;                  // [2][ATT_TILE][ld]
     pdl_launch_dependents();
     pdl_wait();
-    gather_wait(gw);
+    if (MG) gather_wait(gw);
     if (pos0_ptr) pos0 = __ldcg(pos0_ptr);
     int chunk, nsplit;
     att_plan_tiles(pos0 + B, want, chunk, nsplit);
@@ -634,19 +636,20 @@ static int attention_batch(ibcu_ctx* ctx, const float* q, float* k_cache, float*
     int rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, part + rot);
     if (rc) return rc;
     const size_t smem = ((size_t)group * nb * ATT_QPW * (head_dim + 32) + 4 * (size_t)ATT_TILE * (head_dim + 4)) * sizeof(float);
-    static SmemOptIn opt;
-    if ((rc = ibcu_allow_smem(ctx, opt, attn_batch_kernel, smem))) return rc;
+    static SmemOptIn opt, opt_mg;
+    if ((rc = ibcu_allow_smem(ctx, opt, attn_batch_kernel<false>, smem))) return rc;
+    if ((rc = ibcu_allow_smem(ctx, opt_mg, attn_batch_kernel<true>, smem))) return rc;
     GatherWait gw;
     ibcu_take_gather_wait(ctx, &gw);
     if (k) {
         float* q_rot = (float*)((char*)ctx->scratch + part);
-        rc = ibcu_launch(ctx, rope_stage_kernel, dim3(B, 4), dim3(256), 0, 1, true, q, k, v, q_rot, k_cache, v_cache, n_heads, n_kv_heads, head_dim,
+        rc = ibcu_launch(ctx, gw.flags || gw.tag.n ? rope_stage_kernel<true> : rope_stage_kernel<false>, dim3(B, 4), dim3(256), 0, 1, true, q, k, v, q_rot, k_cache, v_cache, n_heads, n_kv_heads, head_dim,
                          pos0, pos0_dev, theta, gw);
         if (rc) return rc;
         q = q_rot;
         memset(&gw, 0, sizeof gw);
     }
-    rc = ibcu_launch(ctx, attn_batch_kernel, dim3(n_kv_heads, want, gz), dim3(32 * group * nb), smem, 1, true, q, (const float*)k_cache, (const float*)v_cache,
+    rc = ibcu_launch(ctx, gw.flags || gw.tag.n ? attn_batch_kernel<true> : attn_batch_kernel<false>, dim3(n_kv_heads, want, gz), dim3(32 * group * nb), smem, 1, true, q, (const float*)k_cache, (const float*)v_cache,
                      (float*)ctx->scratch, n_heads, n_kv_heads, head_dim, B, nb, pos0, pos0_dev, want, gw);
     if (rc) return rc;
     return combine_chunks(ctx, out, n_heads, head_dim, B, nsplit, want, pos0_dev, want, 0);

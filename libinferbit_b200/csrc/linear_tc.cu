@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, i
     xconvert_any(src, N, b, c0, min(part_cols, all_cols - c0), dst, perm8, sc, xscale + b * gridDim.x + part, xsum + ((size_t)b * gridDim.x + part) * LIN_LIMBS);
 }
 
-// BITS 4 or 8; T: 128-row tiles per run
-template <int BITS, int T>
+// BITS 4 or 8; T: 128-row tiles per run; MG: see linear.cu
+template <int BITS, int T, bool MG>
 __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
     extern __shared__ __align__(1024) unsigned char tq_smem[];
     constexpr int NT = 4;                                      // INT4: widened blocks in tensor memory
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
                 const bool have = rl < rows;
                 const int row = row0 + rl;
                 const float sc = have ? row_scale(W, row) : 0.0f;
-                const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
+                const unsigned tag = MG ? tag_current(p.gp) : 0u;
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc), (uint32_t)(j & 1), abort_flag, 10))) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int g = team; g * 4 < p.B; g += 2) {
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
                         const float y = (float)((double)V * (double)sh->back[b]);
                         const float v = W.epilogue == IBCU_EPI_ADD ? old[u] + y * sc : y * sc;
                         o[(size_t)u * W.out_stride] = v;
-                        if (p.gp.world) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
+                        if (MG) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
         float old = mine && bl0 < nb && W.epilogue == IBCU_EPI_ADD ? W.out[(size_t)(bl0 * S + rank) * W.out_stride + row] : 0.0f;
         cluster_wait();
         if (mine && !*abort_flag) {
-            const unsigned tag = p.gp.world ? tag_current(p.gp) : 0u;
+            const unsigned tag = MG ? tag_current(p.gp) : 0u;
             const long long* rv = reinterpret_cast<const long long*>(tq_smem + p.recv_off);
             for (int bl = bl0; bl < nb; bl += BSTEP) {
                 const int b = bl * S + rank;
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
                 const float y = (float)((double)V * (double)sh->back[b]);
                 const float v = W.epilogue == IBCU_EPI_ADD ? old + y * sc : y * sc;
                 *o = v;
-                if (p.gp.world) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
+                if (MG) tag_push(p.gp, (size_t)W.win_off + ((size_t)b * W.out_stride + row) * sizeof(float), v, tag);
                 old = next;
             }
         }
@@ -432,12 +432,17 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-template <int BITS, int T>
-int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
-    auto kern = linear_tc_kernel<BITS, T>;
+template <int BITS, int T, bool MG>
+int launch_tc_mg(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
+    auto kern = linear_tc_kernel<BITS, T, MG>;
     static SmemOptIn opt;
     if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(Tq<T>::THREADS), smem, p.S, true, maps, p);
+}
+
+template <int BITS, int T>
+int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
+    return p.gp.world ? launch_tc_mg<BITS, T, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, false>(ctx, maps, p, grid, smem);
 }
 
 }  // namespace
