@@ -14,9 +14,10 @@
 //   scan (16 warps)        tcgen05.ld (32x32b: a thread owns one point) and the best and second-best maxima over groups of 8 centroids
 //                          (three-input max; the group's number rides in the four low bits of its maximum), handed on per tile
 //   finish (12 warps)      the best group in the exact form, results, and the point into its cluster's sums
-// A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 209 us (285 with scan and finish in the same eight warps, whose chains of
-// TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide); 4 Mi of 4: 172 (652 on the CUDA cores,
-// with a second pass to accumulate); 1 Mi of 16: 114 (582).
+// A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 186 us (285 with scan and finish in the same eight warps, whose chains of
+// TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide; 202 with eight finishing warps, 209 with votes
+// in place of match); 4 Mi of 4: 162 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 114 (582). What bounds it now
+// is the pipe for comparisons and logic, some 500 instructions per scheduler and tile, with issue slots close behind.
 //
 // The scores only FILTER. If the best group leads by more than 1.25 * 2^-16 (|x|^2 + max |c|^2), the reference's nearest centroid lies in
 // that group, and its 8 centroids are evaluated in the reference binary's exact order and rounding, lowest index winning ties. Otherwise

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(WT_W * 32) w4a8_mma_kernel(const WtParams p) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-#pragma unroll
+#pragma unroll 1                                              // code that runs once has to be fetched once: unrolled, an MLP of eight layers took 308 us, not 303
     for (int s = 0; s < STAGES - 1; s++) pf_issue();          // weights first: they do not depend on the activations
     pdl_wait();
 
