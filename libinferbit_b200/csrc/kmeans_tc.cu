@@ -14,7 +14,7 @@
 //   scan (16 warps)        tcgen05.ld (32x32b: a thread owns one point) and the best and second-best maxima over groups of 8 centroids
 //                          (three-input max; the group's number rides in the four low bits of its maximum), handed on per tile
 //   finish (12 warps)      the best group in the exact form, results, and the point into its cluster's sums
-// A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 186 us (285 with scan and finish in the same eight warps, whose chains of
+// A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 183 us (285 with scan and finish in the same eight warps, whose chains of
 // TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide; 202 with eight finishing warps, 209 with votes
 // in place of match); 4 Mi of 4: 162 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 114 (582). What bounds it now
 // is the pipe for comparisons and logic, some 500 instructions per scheduler and tile, with issue slots close behind.
@@ -290,7 +290,7 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
             ok = __all_sync(0xffffffffu, mbar_wait<false>(smem_u32(&sh->empty_a[lw]), (uint32_t)(((i / TC_PIPES) & 1) ^ 1), abort_flag, 1));   // the whole warp leaves or stays
             if (!ok) break;
             const unsigned char* raw = raws + (i / TC_PIPES) % S::raws * S::raw_stage;
-#pragma unroll
+#pragma unroll 1
             for (int t = 0; t < 4; t++) {
                 const int r = 32 * t + lane;
                 float v[D];
@@ -459,7 +459,7 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
 #pragma unroll
                 for (int d = 0; d < D; d++) xq[d] = __shfl_sync(0xffffffffu, xr[d], rl);
                 float bd = INFINITY; int bk = 0x7fffffff;
-#pragma unroll 4
+#pragma unroll 1                                              // rare: short code rather than short chains (ten iterations of 4 Mi x 8 1859 -> 1833 us)
                 for (int k = lane; k < K; k += 32) {
                     const float dk = group_sqdist<D>(xq, cgrp, k);
                     if (dk < bd || k == 0) { bd = dk; bk = k; }      // centroid 0 is the reference's seed whatever its distance
