@@ -16,7 +16,7 @@
 //   finish (12 warps)      the best group in the exact form, results, and the point into its cluster's sums
 // A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 183 us (285 with scan and finish in the same eight warps, whose chains of
 // TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide; 202 with eight finishing warps, 209 with votes
-// in place of match); 4 Mi of 4: 162 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 114 (582). What bounds it now
+// in place of match); 4 Mi of 4: 162 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 101 (582). What bounds it now
 // is the pipe for comparisons and logic, some 500 instructions per scheduler and tile, with issue slots close behind.
 //
 // The scores only FILTER. If the best group leads by more than 1.25 * 2^-16 (|x|^2 + max |c|^2), the reference's nearest centroid lies in
@@ -41,6 +41,7 @@ constexpr int TC_TILE = 128;                 // points per accumulator tile
 constexpr int TC_PIPES = 4;                  // pipelines: tile i goes through pipeline i % 4
 constexpr int TC_ACC_COLS = 128;             // columns of a pipeline's accumulator: the centroids of a unit
 constexpr int TC_SCAN_WARPS = 4 * TC_PIPES;  // warp w scans for pipeline w / 4, rows 32 (w % 4) .. + 31
+constexpr int TC_FIN_WARPS = 12;             // three per quarter of a tile's rows: warp f of the role takes tiles f / 4, f / 4 + 3, ...
 constexpr int TC_SLOTS = 3;                  // tiles a scan warp may be ahead of the warp that finishes its rows
 constexpr int TC_CHUNK = 16 * 128;           // one 16-byte K chunk of 128 rows: 16 core matrices of 128 bytes
 
@@ -91,12 +92,13 @@ struct TcShared {
     unsigned long long empty_a[TC_PIPES];                          // MMAs have read the operand stage
     unsigned long long full_acc[TC_PIPES], empty_acc[TC_PIPES];    // MMA -> scan, scan -> MMA
     unsigned long long full_h[TC_SCAN_WARPS][TC_SLOTS], empty_h[TC_SCAN_WARPS][TC_SLOTS];   // scan -> finish, finish -> scan
+    unsigned long long turn[4][TC_FIN_WARPS / 4];                  // warps that share a table -> the next of them
     unsigned long long drained;                                    // every MMA of the block has completed
     float2 found[TC_SCAN_WARPS][TC_SLOTS][32];                     // per point: gap between the best and the second-best group; the best group (an int)
     uint32_t tmem_base;
     int abort_flag;
     unsigned cmax2_bits;
-    double inert[12];
+    double inert[TC_FIN_WARPS];
 };
 
 // Best and second-best of the maxima over groups of 8 scores, two groups (16 scores) at a time. The group's number within the unit
@@ -144,13 +146,15 @@ template <int D> __device__ __forceinline__ float group_sqdist(const float* x, c
 // [Kp / 8][D dims][copies][8] | ACC: a table of K sums per finishing warp, then [warp][K] counts | TcShared
 // ACC: the finishing warps also add every point into the table of its cluster (points of a warp in index order), and the block leaves
 // the sum of its tables, its counts and its share of the inertia in part_*[blockIdx.x]: the accumulate pass over X of a Lloyd iteration
-// then needs no kernel and no second read of X. The order of the adds is fixed by the grid. FIN = 8 or 4 where twelve tables do not fit.
-template <int D, bool ACC, int FIN>
-__global__ void __launch_bounds__((TC_SCAN_WARPS + FIN + TC_PIPES) * 32, 1)
+// then needs no kernel and no second read of X. The order of the adds is fixed by the grid. TAB tables: one per
+// finishing warp, or, where twelve do not fit, one for the three warps of a quarter, which take turns tile by tile.
+template <int D, bool ACC, int TAB>
+__global__ void __launch_bounds__((TC_SCAN_WARPS + TC_FIN_WARPS + TC_PIPES) * 32, 1)
 assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restrict__ idx, float* __restrict__ dist,
                  int* __restrict__ err, float* __restrict__ part_sums, int32_t* __restrict__ part_counts, double* __restrict__ part_inertia) {
     using S = Shape<D>;
-    constexpr int THREADS = (TC_SCAN_WARPS + FIN + TC_PIPES) * 32;
+    constexpr int FIN = TC_FIN_WARPS, THREADS = (TC_SCAN_WARPS + FIN + TC_PIPES) * 32;
+    constexpr int STEP = FIN / 4, SHARE = FIN / TAB;             // tiles from one of a finishing warp to its next; warps that share a table
     constexpr int FIN0 = TC_SCAN_WARPS, LOAD0 = FIN0 + FIN, PP = D / 4;
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -162,14 +166,15 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
     unsigned char* sRaw = sAug + S::aug_chunks * TC_CHUNK;
     float* cgrp = reinterpret_cast<float*>(sRaw + TC_PIPES * S::raws * S::raw_stage);
     float* wtab = cgrp + (size_t)(Kp / 8) * S::group_stride;
-    int* wcnt = reinterpret_cast<int*>(wtab + (ACC ? (size_t)FIN * K * S::row_stride : 0));
-    TcShared* sh = reinterpret_cast<TcShared*>(((uintptr_t)(wcnt + (ACC ? (size_t)FIN * K : 0)) + 15) & ~(uintptr_t)15);
+    int* wcnt = reinterpret_cast<int*>(wtab + (ACC ? (size_t)TAB * K * S::row_stride : 0));
+    TcShared* sh = reinterpret_cast<TcShared*>(((uintptr_t)(wcnt + (ACC ? (size_t)TAB * K : 0)) + 15) & ~(uintptr_t)15);
     volatile int* abort_flag = &sh->abort_flag;
 
     if (tid == 0) {
         for (int b = 0; b < TC_PIPES; b++) { mbar_init(smem_u32(&sh->empty_a[b]), 1); mbar_init(smem_u32(&sh->full_acc[b]), 1); mbar_init(smem_u32(&sh->empty_acc[b]), 4); }
         for (int w = 0; w < TC_SCAN_WARPS; w++)
             for (int s = 0; s < TC_SLOTS; s++) { mbar_init(smem_u32(&sh->full_h[w][s]), 1); mbar_init(smem_u32(&sh->empty_h[w][s]), 1); }
+        for (int t = 0; t < FIN; t++) mbar_init(smem_u32(&sh->turn[t & 3][t >> 2]), 1);
         mbar_init(smem_u32(&sh->drained), TC_PIPES);
         sh->abort_flag = 0;
         sh->cmax2_bits = 0u;
@@ -183,8 +188,8 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
         pdl_launch_dependents();
     }
     if (ACC) {
-        for (int e = tid; e < FIN * K * S::row_stride; e += THREADS) wtab[e] = 0.0f;
-        for (int e = tid; e < FIN * K; e += THREADS) wcnt[e] = 0;
+        for (int e = tid; e < TAB * K * S::row_stride; e += THREADS) wtab[e] = 0.0f;
+        for (int e = tid; e < TAB * K; e += THREADS) wcnt[e] = 0;
     }
     if (D > 4) {                             // constant chunks of the point operand: row e = (1 1 1 0 0 0 0 0 | zeros)
         for (int e = tid; e < 128 * S::aug_chunks; e += THREADS)
@@ -379,13 +384,12 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
         }
     } else {
         // ── finish ──
-        constexpr int STEP = FIN / 4;                                // warp f of the role takes tiles f / 4, f / 4 + STEP, ...
         // A slot's tiles are TC_PIPES * TC_SLOTS apart and must all be one warp's: were they several warps', one could wait for a phase of
         // full_h while another has yet to take the one two before it, which has the same parity.
         static_assert(TC_PIPES * TC_SLOTS % STEP == 0, "the tiles of a slot go to one finishing warp");
         const int f = warp - FIN0, q = f & 3;
-        float* mytab = wtab + (size_t)f * K * S::row_stride;
-        int* mycnt = wcnt + (size_t)f * K;
+        float* mytab = wtab + (size_t)(f % TAB) * K * S::row_stride;
+        int* mycnt = wcnt + (size_t)(f % TAB) * K;
         double inert = 0.0;
         constexpr bool AHEAD = D <= 8;                               // the next row is fetched while this one is worked on (D = 16 lacks the registers)
         float xnext[AHEAD ? D : 4];
@@ -480,6 +484,9 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                 // index order; different clusters go together. (Equal clusters bit by bit with votes: eight votes and thirty-odd more
                 // instructions for the pipe that bounds the kernel.)
                 const unsigned grp = __match_any_sync(0xffffffffu, have ? win : -1 - lane);
+                if (SHARE > 1 && i > 0) {                    // the warp with the tile before has added its points
+                    if (!__all_sync(0xffffffffu, mbar_wait<false>(smem_u32(&sh->turn[q][f >> 2]), (uint32_t)(((i - 1) / SHARE) & 1), abort_flag, 8))) break;
+                }
                 const bool first = have && (grp & ((1u << lane) - 1u)) == 0;
                 const int turns = __reduce_max_sync(0xffffffffu, (unsigned)__popc(grp));
                 float4* t = reinterpret_cast<float4*>(mytab + (size_t)win * S::row_stride);
@@ -509,12 +516,13 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                     for (int p = 0; p < PP; p++) t[p] = sum[p];
                 }
                 __syncwarp();
+                if (SHARE > 1 && lane == 0) mbar_arrive(smem_u32(&sh->turn[q][((f >> 2) + 1) % SHARE]));
                 if (have) inert += (double)best;
             }
         }
         if (ACC) {
             // the tables of the block, added in warp order; every finishing warp gets here, also after a wait ran out
-            const int ft = tid - FIN0 * 32, used = min(FIN, 4 * n_my);       // warps that had a tile
+            const int ft = tid - FIN0 * 32, used = min(TAB, 4 * n_my);       // tables that had a tile
             for (int o = 16; o > 0; o >>= 1) inert += __shfl_xor_sync(0xffffffffu, inert, o);
             if (lane == 0) sh->inert[f] = inert;
             asm volatile("bar.sync 1, %0;" :: "n"(FIN * 32) : "memory");
@@ -549,20 +557,20 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
 }
 
 template <int D>
-size_t tc_smem_bytes(int K, bool acc, int fin) {
+size_t tc_smem_bytes(int K, bool acc, int tab) {
     using S = Shape<D>;
     const size_t Kp = (size_t)((K + 31) & ~31);
     return S::b_chunks * Kp * 16 + TC_PIPES * (size_t)(S::a_stage + S::raws * S::raw_stage) + S::aug_chunks * TC_CHUNK + Kp / 8 * S::group_stride * sizeof(float) +
-           (acc ? (size_t)fin * K * (S::row_stride + 1) * sizeof(float) : 0) + sizeof(TcShared) + 16;
+           (acc ? (size_t)tab * K * (S::row_stride + 1) * sizeof(float) : 0) + sizeof(TcShared) + 16;
 }
 
-template <int D, bool ACC, int FIN>
+template <int D, bool ACC, int TAB>
 int tc_launch(ibcu_ctx* ctx, long blocks, const float* X, long N, const float* C, int K, int32_t* idx, float* dist,
               float* part_sums, int32_t* part_counts, double* part_inertia) {
-    const size_t smem = tc_smem_bytes<D>(K, ACC, FIN);
+    const size_t smem = tc_smem_bytes<D>(K, ACC, TAB);
     static SmemOptIn opt;
-    if (int rc = ibcu_allow_smem(ctx, opt, assign_tc_kernel<D, ACC, FIN>, smem)) return rc;
-    return ibcu_launch(ctx, assign_tc_kernel<D, ACC, FIN>, dim3((unsigned)blocks), dim3((TC_SCAN_WARPS + FIN + TC_PIPES) * 32), smem, 1, true,
+    if (int rc = ibcu_allow_smem(ctx, opt, assign_tc_kernel<D, ACC, TAB>, smem)) return rc;
+    return ibcu_launch(ctx, assign_tc_kernel<D, ACC, TAB>, dim3((unsigned)blocks), dim3((TC_SCAN_WARPS + TC_FIN_WARPS + TC_PIPES) * 32), smem, 1, true,
                        X, N, C, K, idx, dist, ctx->kern_err, part_sums, part_counts, part_inertia);
 }
 
@@ -601,9 +609,10 @@ int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int 
     switch (D) {
         case 4: return tc_launch<4, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
         case 8: return tc_launch<8, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
-        default:                             // of 256 clusters only four tables fit
+        // Twelve tables fit up to 125 clusters or so. Beyond, the three warps of a quarter share one: 1 Mi points, ten iterations, 256
+        // clusters 1014 us (1152 with four finishing warps and a table each), 200 clusters 964 (1108), 128 clusters 820 (804 with eight).
+        default:
             if (tc_smem_bytes<16>(K, true, 12) <= TC_SMEM_MAX) return tc_launch<16, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
-            if (tc_smem_bytes<16>(K, true, 8) <= TC_SMEM_MAX) return tc_launch<16, true, 8>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
             return tc_launch<16, true, 4>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
     }
 }
