@@ -615,9 +615,9 @@ def with_roofline(entry, peaks, world=1):
     r = {"bound": entry.get("bound", "hbm"), "hbm_achieved_GBps": gbs, "hbm_peak_GBps": peaks["hbm_gbs"], "hbm_frac": gbs / peaks["hbm_gbs"], "peak_source": peaks["source"]}
     if "flops" in entry:
         tf = entry["flops"] / t / 1e12 / world
-        # TF32 is not among the measured peaks; half of the measured dense bf16 rate is the nominal ratio
-        r.update({"tensor_achieved_TFLOPs": tf, "tensor_peak_TFLOPs": peaks["bf16_tflops"] / 2, "tensor_frac": tf / (peaks["bf16_tflops"] / 2) if peaks["bf16_tflops"] else None,
-                  "tensor_peak_note": "half of the measured dense bf16 GEMM rate (TF32 nominal ratio)"})
+        # FP16 and BF16 run at the same rate
+        r.update({"tensor_achieved_TFLOPs": tf, "tensor_peak_TFLOPs": peaks["bf16_tflops"], "tensor_frac": tf / peaks["bf16_tflops"] if peaks["bf16_tflops"] else None,
+                  "tensor_peak_note": "the measured dense bf16 GEMM rate (FP16 runs at it too)"})
     entry["roofline"] = r
     return entry
 

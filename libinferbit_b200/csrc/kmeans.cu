@@ -5,7 +5,9 @@
 // separately for dimensions below 4*floor(D/4), fused for the remaining D%4), strict '<' so the
 // lowest index wins ties. Codes are therefore bit-identical to the reference, not "close".
 //   assign_exact_kernel   every distance in that exact form (CUDA cores).
-//   assign_filter_kernel  (D == 8, K % 8 == 0) TF32 tensor-core scores x.c - |c|^2/2 for all K
+//   assign_tc_kernel      (kmeans_tc.cu; D = 4, 8, 16, K <= 256) FP16 scores on tcgen05 as a filter, the
+//                         points added up as they are assigned.
+//   assign_filter_kernel  (D == 8, K % 8 == 0, larger K) TF32 tensor-core scores x.c - |c|^2/2 for all K
 //                         centroids per 16-point tile, best / second-best tracked in registers; a
 //                         point whose margin exceeds a rigorous error bound takes the tensor-core
 //                         winner, every other point is re-evaluated in the exact form. Same codes,
