@@ -36,10 +36,11 @@ __global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restri
     for (int i = threadIdx.x; i < K * d_all; i += blockDim.x) cs[i] = C[i];
     __syncthreads();
     const long total = todo ? (long)__ldcg(n_todo) : N;    // written by the kernel just ahead: read past L1, not as a read-only load
+    const bool wide = DT > 0 && DT % 4 == 0 && ((uintptr_t)X & 15) == 0;      // else rows lie at any float: the other kernels leave such arrays to this one
     for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long)gridDim.x * blockDim.x) {
         const long i = todo ? (long)todo[w] : w;
         float x[DT > 0 ? DT : KM_MAX_D];
-        if (DT > 0 && DT % 4 == 0) {
+        if (wide) {
 #pragma unroll
             for (int d = 0; d < DT; d += 4) {
                 float4 v = *reinterpret_cast<const float4*>(X + (size_t)i * DT + d);

@@ -239,3 +239,27 @@ def test_tensor_core_assign_points_far_from_small_centroids(backend, cpu_libs):
         got, gd = backend.kmeans_assign(X, Cn, want_dist=True)
         want, wd = oracle_assign(cpu_libs, X, Cn)
         assert np.array_equal(got, want) and np.array_equal(gd, wd)
+
+
+@pytest.mark.parametrize("D,K", [(4, 256), (4, 7), (8, 256), (8, 100), (8, 264), (16, 256), (16, 12), (3, 20)])
+@pytest.mark.parametrize("off_x,off_c", [(4, 0), (0, 4), (8, 12)])
+def test_arrays_at_any_float(backend, cpu_libs, D, K, off_x, off_c):
+    """Points or centroids that start at a float but not at 16 bytes (a caller's own offset into a registered range): same codes,
+    distances and counts, no 16-byte load of them anywhere."""
+    rng = np.random.default_rng(D * 1000 + K + off_x)
+    N, be = 3001, backend
+    X = (rng.standard_normal((N, D)) * 0.02).astype(np.float32)
+    Cn = (rng.standard_normal((K, D)) * 0.02).astype(np.float32)
+    dX, dC = be.alloc(X.nbytes + 16), be.alloc(Cn.nbytes + 16)
+    be.write(dX, X, off_x); be.write(dC, Cn, off_c)
+    di, dd, ds, dc, dn = be.alloc(N * 4), be.alloc(N * 4), be.alloc(K * D * 4), be.alloc(K * 4), be.alloc(8)
+    want, wd = oracle_assign(cpu_libs, X, Cn)
+    for call in ("assign", "lloyd"):
+        if call == "assign":
+            be._check(be.lib.ibcu_kmeans_assign(be.ctx, dX.ptr + off_x, N, D, dC.ptr + off_c, K, di.ptr, dd.ptr))
+        else:
+            be._check(be.lib.ibcu_kmeans_lloyd_iter(be.ctx, dX.ptr + off_x, N, D, dC.ptr + off_c, K, di.ptr, dd.ptr, ds.ptr, dc.ptr, dn.ptr))
+        be.sync()
+        assert np.array_equal(be.download(di, np.int32, N), want), call
+        assert np.array_equal(be.download(dd, np.float32, N), wd), call
+    assert np.array_equal(be.download(dc, np.int32, K), np.bincount(want, minlength=K))
