@@ -15,6 +15,8 @@
 // accumulate: per-cluster sums / counts / inertia with a fixed order of additions (no atomics):
 // each warp adds its points in index order into a private shared-memory table, warps and blocks are
 // then combined in index order.
+// These kernels start while the launch ahead of them still runs. What it writes (centroids, codes, distances, tables, sums) is read past
+// L1 (__ldcg) and not as read-only data, which may be fetched before the dependency wait.
 #include "common.cuh"
 #include "kmeans_ref.cuh"
 #include <stdlib.h>
@@ -33,7 +35,7 @@ __global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restri
     pdl_launch_dependents();
     pdl_wait();
     const int d_all = DT > 0 ? DT : D;
-    for (int i = threadIdx.x; i < K * d_all; i += blockDim.x) cs[i] = C[i];
+    for (int i = threadIdx.x; i < K * d_all; i += blockDim.x) cs[i] = __ldcg(C + i);
     __syncthreads();
     const long total = todo ? (long)__ldcg(n_todo) : N;    // written by the kernel just ahead: read past L1, not as a read-only load
     const bool wide = DT > 0 && DT % 4 == 0 && ((uintptr_t)X & 15) == 0;      // else rows lie at any float: the other kernels leave such arrays to this one
@@ -103,7 +105,7 @@ __global__ void __launch_bounds__(256) assign_filter_kernel(const float* __restr
     float* cex = nh + K;
     float* cmax2 = cex + (size_t)K * 8;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    for (int e = tid; e < K * 8; e += blockDim.x) cex[e] = C[e];
+    for (int e = tid; e < K * 8; e += blockDim.x) cex[e] = __ldcg(C + e);
     __syncthreads();
     for (int e = tid; e < (K / 8) * 32; e += blockDim.x) {
         const int j = e >> 5, l = e & 31, gg = l >> 2, tt = l & 3;
@@ -258,8 +260,8 @@ __global__ void __launch_bounds__(256) accumulate_kernel(const float* __restrict
         int code_n = 0; float dist_n = 0.0f; float4 xn[KM_MAX_D / 4];
         auto fetch = [&](long p) {
             const long mine = p + lane;
-            code_n = mine < p1 ? idx[mine] : 0;
-            dist_n = (dist && mine < p1) ? dist[mine] : 0.0f;
+            code_n = mine < p1 ? __ldcg(idx + mine) : 0;
+            dist_n = (dist && mine < p1) ? __ldcg(dist + mine) : 0.0f;
             const long lim = (p1 - p) * lpp;                      // float4s that exist
 #pragma unroll
             for (int u = 0; u < KM_MAX_D / 4; u++) {
@@ -301,8 +303,8 @@ __global__ void __launch_bounds__(256) accumulate_kernel(const float* __restrict
     for (long p = p0; p < p1; p += 32) {
         const long mine = p + lane;
         const int n = (int)((p1 - p) < 32 ? (p1 - p) : 32);
-        const int code = mine < p1 ? idx[mine] : 0;
-        if (dist && mine < p1) inert += (double)dist[mine];
+        const int code = mine < p1 ? __ldcg(idx + mine) : 0;
+        if (dist && mine < p1) inert += (double)__ldcg(dist + mine);
         for (int e = lane; e < n * D; e += 32) stage[e] = X[(size_t)p * D + e];
         __syncwarp();
         // 32/D points per step, one lane group per point. Points of a step that share a cluster are
@@ -389,8 +391,8 @@ __global__ void __launch_bounds__(256) accumulate_finish_kernel(const float* __r
         if (e < KD) {
 #pragma unroll 8
             for (int b = g; b < nblocks; b += 8) {
-                s += (double)part_sums[(size_t)b * KD + e];
-                if (UPDATE) n += part_counts[(size_t)b * K + k];
+                s += (double)__ldcg(part_sums + (size_t)b * KD + e);
+                if (UPDATE) n += __ldcg(part_counts + (size_t)b * K + k);
             }
         }
         dsh[g][c] = s;
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(256) accumulate_finish_kernel(const float* __r
         int s = 0;
         if (e < K) {
 #pragma unroll 8
-            for (int b = g; b < nblocks; b += 8) s += part_counts[(size_t)b * K + e];
+            for (int b = g; b < nblocks; b += 8) s += __ldcg(part_counts + (size_t)b * K + e);
         }
         ish[g][c] = s;
         __syncthreads();
@@ -423,7 +425,7 @@ __global__ void __launch_bounds__(256) accumulate_finish_kernel(const float* __r
     } else if (inertia || ex.gp.world) {
         double s = 0.0;
 #pragma unroll 4
-        for (int b = threadIdx.x; b < nblocks; b += 256) s += part_inertia[b];
+        for (int b = threadIdx.x; b < nblocks; b += 256) s += __ldcg(part_inertia + b);
         // fixed-order tree over the 256 threads
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -480,10 +482,10 @@ __global__ void __launch_bounds__(1024) update_kernel(float* __restrict__ C, int
     float local = 0.0f;
     for (int e = threadIdx.x; e < K * D; e += blockDim.x) {
         const int k = e / D;
-        const int n = counts[k];
+        const int n = __ldcg(counts + k);
         if (n > 0) {
-            const float nv = centroid_of(sums[e], n);
-            const float dv = nv - C[e];
+            const float nv = centroid_of(__ldcg(sums + e), n);
+            const float dv = nv - __ldcg(C + e);
             local = fmaf(dv, dv, local);
             C[e] = nv;
         }

@@ -35,3 +35,15 @@ def test_digit_sums_of_two_activations_are_kept_apart():
     assert len(bodies) == 3                                  # in registers, in a loop, with a known maximum
     for b in bodies:
         assert "__syncthreads()" in b[:b.index("sc.sred[threadIdx.x >> 5][l] = v")], b.strip().splitlines()[1]
+
+
+@pytest.mark.parametrize("kernel,arrays", [("assign_exact_kernel", ["C"]), ("assign_filter_kernel", ["C"]), ("accumulate_kernel", ["idx", "dist"]),
+                                           ("accumulate_finish_kernel", ["part_sums", "part_counts", "part_inertia"]), ("update_kernel", ["counts", "sums"])])
+def test_kmeans_kernels_read_the_launch_ahead_past_l1(kernel, arrays):
+    """Arrays that the launch just ahead may have written, in kernels that start before it has ended: no plain or read-only load."""
+    code = _code(os.path.join(CSRC, "kmeans.cu"))
+    body = next(k for k in code.split("__global__")[1:] if re.search(rf"\b{kernel}\(", k[:200]))
+    end = re.search(r"\n}\n", body).start()
+    for a in arrays:
+        assert not re.search(rf"\b{a}\[", body[:end]), a
+        assert re.search(rf"__ldcg\({a} \+", body[:end]), a
