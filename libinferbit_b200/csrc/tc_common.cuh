@@ -2,8 +2,7 @@
 // shared-memory matrix descriptors, bulk copies, tcgen05 commit / load / store / wait.
 #pragma once
 #include <cstdint>
-
-constexpr unsigned long long TC_WAIT_NS = 2000000000ull;      // a wait gives up after two seconds
+#include "wait_clock.h"
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -28,15 +27,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 template <bool TEST = true>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
     if (TEST && mbar_test(bar, parity)) return true;
-    unsigned long long since = 0;
+    WaitClock clock;
     for (int it = 1;; it++) {
         if (mbar_try(bar, parity)) return true;
         if (*abort_flag) return false;
         if ((it & 63) == 0) {                                  // the clock is looked at now and then only
             unsigned long long now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            if (!since) since = now;
-            else if (now - since > TC_WAIT_NS) break;
+            if (clock.spent(now)) break;
         }
     }
     *abort_flag = code;

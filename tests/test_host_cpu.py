@@ -124,3 +124,37 @@ def test_kmeans_upload_in_pieces(tmp_path):
                     f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}", "-lm", "-lpthread"], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stdout)
+
+
+WAIT = r"""
+#include "wait_clock.h"
+#include <stdio.h>
+static int looks(unsigned long long ns, unsigned long long at) { WaitClock c; int n = 1; while (!c.spent(at)) { at += ns; if (++n > 100000000) return -1; } return n; }
+int main() {
+    const unsigned long long start[] = { 1, 1ull << 40, (1ull << 52) - 3000000000ull, ~0ull - 1000000000ull };   // the short reading wraps, the long one too
+    for (unsigned long long at : start) {
+        const int n = looks(1000000, at);                    // a look every millisecond: some two seconds
+        if (n < 2000 || n > 2300) { printf("%d looks of a millisecond\n", n); return 1; }
+        if (looks(10000000000ull, at) != 10) return 2;       // looks ten seconds apart end too
+        WaitClock c;
+        for (int i = 0; i < 7; i++) {                        // stopped for a minute seven times, a few microseconds of waiting between
+            if (c.spent(at)) return 3;
+            at += 60000000000ull;
+            if (c.spent(at)) return 4;
+            at += 5000;
+        }
+    }
+    return 0;
+}
+"""
+
+
+def test_a_stopped_kernel_does_not_run_out_of_time(tmp_path):
+    """A wait that comes back after the GPU served somebody else goes on; every wait ends."""
+    src, exe = tmp_path / "wait.cpp", tmp_path / "wait"
+    src.write_text(WAIT)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-Werror", f"-I{LIB}/csrc", "-o", str(exe), str(src)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout)
+    code = open(os.path.join(LIB, "csrc", "tc_common.cuh")).read()
+    assert "clock.spent(now)" in code
