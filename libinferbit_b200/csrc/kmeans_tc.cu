@@ -480,8 +480,9 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
             }
             if (have) { idx[row] = win; if (dist) dist[row] = best; }
             if (ACC) {
-                // Points of the warp that share a cluster: the first of them fetches the others' rows and adds them behind its own, in
-                // index order; different clusters go together. (Equal clusters bit by bit with votes: eight votes and thirty-odd more
+                // Points of the warp that share a cluster: the first of them fetches the others' rows, adds them behind its own, in index
+                // order, and their sum to the table: an entry receives one value per tile, so that its error grows with the number of
+                // tiles of the table (74 at 4 Mi points) and not with that of points. Different clusters go together. (Equal clusters bit by bit with votes: eight votes and thirty-odd more
                 // instructions for the pipe that bounds the kernel.)
                 const unsigned grp = __match_any_sync(0xffffffffu, have ? win : -1 - lane);
                 if (SHARE > 1 && i > 0) {                    // the warp with the tile before has added its points
@@ -490,15 +491,9 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                 const bool first = have && (grp & ((1u << lane) - 1u)) == 0;
                 const int turns = __reduce_max_sync(0xffffffffu, (unsigned)__popc(grp));
                 float4* t = reinterpret_cast<float4*>(mytab + (size_t)win * S::row_stride);
-                float4 sum[PP] = {};
-                if (first) {
-                    mycnt[win] += __popc(grp);
+                float4 sum[PP];
 #pragma unroll
-                    for (int p = 0; p < PP; p++) {
-                        sum[p] = t[p];
-                        sum[p].x += xr[4 * p]; sum[p].y += xr[4 * p + 1]; sum[p].z += xr[4 * p + 2]; sum[p].w += xr[4 * p + 3];
-                    }
-                }
+                for (int p = 0; p < PP; p++) sum[p] = make_float4(xr[4 * p], xr[4 * p + 1], xr[4 * p + 2], xr[4 * p + 3]);
                 unsigned rest = grp & (grp - 1u);
                 for (int r = 1; r < turns; r++) {
                     const int src = rest ? __ffs(rest) - 1 : lane;
@@ -512,8 +507,12 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                     }
                 }
                 if (first) {
+                    mycnt[win] += __popc(grp);
 #pragma unroll
-                    for (int p = 0; p < PP; p++) t[p] = sum[p];
+                    for (int p = 0; p < PP; p++) {
+                        const float4 v = t[p];
+                        t[p] = make_float4(v.x + sum[p].x, v.y + sum[p].y, v.z + sum[p].z, v.w + sum[p].w);
+                    }
                 }
                 __syncwarp();
                 if (SHARE > 1 && lane == 0) mbar_arrive(smem_u32(&sh->turn[q][((f >> 2) + 1) % SHARE]));

@@ -263,3 +263,72 @@ def test_arrays_at_any_float(backend, cpu_libs, D, K, off_x, off_c):
         assert np.array_equal(be.download(di, np.int32, N), want), call
         assert np.array_equal(be.download(dd, np.float32, N), wd), call
     assert np.array_equal(be.download(dc, np.int32, K), np.bincount(want, minlength=K))
+
+
+def _iteration_sums(X, codes, K, tables):
+    """The sums of a fused iteration, bit for bit: tile t of 128 points goes to block t % 148 as its tile i. Rows of a quarter of a tile that share a
+    cluster are summed in index order in FP32, and the sums added, tile after tile, to that quarter's table for i % 3 (twelve tables) or its only
+    one (four). A block's tables are joined in double in order, blocks in double by eight interleaved groups."""
+    N, D = X.shape
+    nb = min((N + 127) // 128, 148)
+    p = np.arange(N)
+    group, inv = np.unique((p // 32) * K + codes, return_inverse=True)       # (tile, quarter, cluster), ascending
+    tile, q, k = group // K // 4, group // K % 4, group % K
+    i, b = tile // nb, tile % nb
+    key = (b * tables + (q + 4 * (i % 3) if tables == 12 else q)) * K + k
+    out = np.empty((K, D), np.float32)
+    for d in range(D):
+        s = np.zeros(len(group), np.float32)
+        np.add.at(s, inv, X[:, d])                           # one after the other, in index order
+        t = np.zeros(nb * tables * K, np.float32)
+        np.add.at(t, key, s)
+        t = t.reshape(nb, tables, K).astype(np.float64)
+        total = t[:, 0].copy()
+        for w in range(1, tables):
+            total += t[:, w]
+        part = total.astype(np.float32).astype(np.float64)
+        g = np.zeros((8, K))
+        for blk in range(nb):
+            g[blk % 8] += part[blk]
+        out[:, d] = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]))
+    return out
+
+
+@pytest.mark.parametrize("N,D,K,tables", [
+    (148 * 128 * 26 + 1, 4, 256, 12), (148 * 128 * 26 + 1, 4, 200, 12), (148 * 128 * 14 - 77, 8, 256, 12), (148 * 128 * 25 + 4000, 8, 40, 12),
+    (148 * 128 * 26 + 1, 16, 64, 12), (148 * 128 * 26 + 1, 16, 200, 4), (148 * 128 * 27 - 5, 16, 256, 4), (148 * 128 * 200 + 40, 4, 8, 12),
+])
+def test_fused_iteration_at_length(backend, cpu_libs, N, D, K, tables):
+    """Every ring of the kernel wrapped (more than twelve tiles a block; shared tables from tile 4 on): codes, distances and counts are the
+    checker's, the sums are the stated order's bits and within what a chain of one add per tile may err, and iterations launched without a
+    wait between them give what waited-for ones give."""
+    rng = np.random.default_rng(N + D + K)
+    X = (rng.standard_normal((N, D), dtype=np.float32) * np.float32(0.02))
+    X[rng.random(N) < 0.4] *= np.float32(0.1)                # a crowd around the origin: few clusters take many points
+    X[rng.random(N) < 0.2] = X[5]                             # and one point over and over
+    Cn = X[:K].copy()
+    Cn[0] = 0
+    h = _lloyd_gpu(backend, X, Cn, 3)
+    want, wd = oracle_assign(cpu_libs, X, Cn)
+    assert np.array_equal(h[0]["idx"], want)
+    assert np.array_equal(h[0]["counts"], np.bincount(want, minlength=K))
+    assert abs(h[0]["inertia"] - wd.astype(np.float64).sum()) <= 1e-11 * wd.astype(np.float64).sum()
+    assert np.array_equal(h[0]["sums"], _iteration_sums(X, want, K, tables))
+    assert np.array_equal(h[1]["sums"], _iteration_sums(X, h[1]["idx"], K, tables))
+    adds = 31 + -(-N // (128 * 148)) // (tables // 4) + 1 + 2           # within a quarter, tiles of a table, the block's sum and the total rounded
+    for d in range(D):
+        ref = np.bincount(want, weights=X[:, d].astype(np.float64), minlength=K)
+        mag = np.bincount(want, weights=np.abs(X[:, d]).astype(np.float64), minlength=K)
+        assert np.all(np.abs(h[0]["sums"][:, d] - ref) <= adds * 2.0 ** -24 * mag)
+    be = backend
+    dX, dC = be.upload(X), be.upload(Cn)
+    di, dd, ds, dc, dn = be.alloc(N * 4), be.alloc(N * 4), be.alloc(K * D * 4), be.alloc(K * 4), be.alloc(8)
+    for _ in range(3):
+        be._check(be.lib.ibcu_kmeans_lloyd_iter(be.ctx, dX.ptr, N, D, dC.ptr, K, di.ptr, dd.ptr, ds.ptr, dc.ptr, dn.ptr))
+    be.sync()
+    assert np.array_equal(be.download(di, np.int32, N), h[2]["idx"])
+    assert np.array_equal(be.download(dd, np.float32, N), oracle_assign(cpu_libs, X, h[1]["C"])[1])
+    assert np.array_equal(be.download(dC, np.float32, K * D).reshape(K, D), h[2]["C"])
+    assert np.array_equal(be.download(ds, np.float32, K * D).reshape(K, D), h[2]["sums"])
+    for b in (dX, dC, di, dd, ds, dc, dn):
+        b.free(); be._bufs.remove(b)
