@@ -534,7 +534,7 @@ int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const floa
 
 // kmeans_tc.cu
 bool ibcu_kmeans_tc_takes(const float* X, long N, int D, const float* C, int K);
-long ibcu_kmeans_tc_blocks(const ibcu_ctx* ctx, long N);
+long ibcu_kmeans_tc_blocks(long N);
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist);
 int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
                                      float* part_sums, int32_t* part_counts, double* part_inertia);
@@ -630,7 +630,7 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
     bool fused = false;
     float* const move = ctx->world > 1 ? nullptr : C;       // one GPU: the kernel that adds up the tables moves the centroids
     if (ctx->kmeans_path == IBCU_KMEANS_AUTO && ibcu_kmeans_tc_takes(X, N, D, C, K)) {
-        const int nblocks = (int)ibcu_kmeans_tc_blocks(ctx, N);
+        const int nblocks = (int)ibcu_kmeans_tc_blocks(N);
         const size_t KD = (size_t)K * D;
         const size_t need = (size_t)nblocks * (KD * sizeof(float) + K * sizeof(int32_t) + sizeof(double)) + 64;
         rc = ibcu_reserve(ctx, &ctx->scratch, &ctx->scratch_bytes, need);

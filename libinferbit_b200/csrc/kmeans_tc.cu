@@ -43,6 +43,7 @@ constexpr int TC_ACC_COLS = 128;             // columns of a pipeline's accumula
 constexpr int TC_SCAN_WARPS = 4 * TC_PIPES;  // warp w scans for pipeline w / 4, rows 32 (w % 4) .. + 31
 constexpr int TC_FIN_WARPS = 12;             // three per quarter of a tile's rows: warp f of the role takes tiles f / 4, f / 4 + 3, ...
 constexpr int TC_SLOTS = 3;                  // tiles a scan warp may be ahead of the warp that finishes its rows
+constexpr int TC_BLOCKS = 148;               // the most blocks of a launch: one per SM; a number of its own, so that sums depend on the points alone
 constexpr int TC_CHUNK = 16 * 128;           // one 16-byte K chunk of 128 rows: 16 core matrices of 128 bytes
 
 // What the number of dimensions decides. Chunks are 16 bytes (8 FP16 values) of every row.
@@ -582,15 +583,15 @@ constexpr size_t TC_SMEM_MAX = 227 * 1024;
 bool ibcu_kmeans_tc_takes(const float* X, long N, int D, const float* C, int K) {
     return (D == 4 || D == 8 || D == 16) && K >= 1 && K <= 256 && (((uintptr_t)X | (uintptr_t)C) & 15) == 0 && N <= (1L << 37);
 }
-long ibcu_kmeans_tc_blocks(const ibcu_ctx* ctx, long N) {
+long ibcu_kmeans_tc_blocks(long N) {
     const long ntile = (N + TC_TILE - 1) / TC_TILE;
-    return ntile < ctx->sm_count ? ntile : ctx->sm_count;
+    return ntile < TC_BLOCKS ? ntile : TC_BLOCKS;
 }
 
 // Returns IBCU_DECLINED without touching the context's error when the call is not its own (the caller takes another kernel).
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist) {
     if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
-    const long blocks = ibcu_kmeans_tc_blocks(ctx, N);
+    const long blocks = ibcu_kmeans_tc_blocks(N);
     switch (D) {
         case 4: return tc_launch<4, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
         case 8: return tc_launch<8, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
@@ -604,7 +605,7 @@ int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const fl
 int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
                                      float* part_sums, int32_t* part_counts, double* part_inertia) {
     if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
-    const long blocks = ibcu_kmeans_tc_blocks(ctx, N);
+    const long blocks = ibcu_kmeans_tc_blocks(N);
     switch (D) {
         case 4: return tc_launch<4, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
         case 8: return tc_launch<8, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
