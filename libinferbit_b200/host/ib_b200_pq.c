@@ -312,6 +312,17 @@ static int ib_b200_kmeans_assign_unlocked(const float* X, int N, int D, const fl
     return rc ? -1 : 0;
 }
 
+/* squared length of all centroids' moves; empty clusters stay where they are */
+static float km_shift(const float* now, const float* was, const int32_t* counts, int K, int D) {
+    float shift = 0.0f;
+    for (int k = 0; k < K; k++)
+        for (int d = 0; d < D && counts[k] > 0; d++) {
+            const float move = now[(size_t)k * D + d] - was[(size_t)k * D + d];
+            shift += move * move;
+        }
+    return shift;
+}
+
 static int ib_b200_kmeans_lloyd_unlocked(const float* X, int N, int D, int K, int iters, float tol,
                          float* centers, int32_t* indices_out, double* inertia_out) {
     if (!X || !centers || N <= 0 || K <= 0 || D <= 0 || iters <= 0) return -1;
@@ -319,36 +330,44 @@ static int ib_b200_kmeans_lloyd_unlocked(const float* X, int N, int D, int K, in
     km_bufs b;
     int rc = km_begin(&b, X, N, D, K, centers), done = 0;
     double prev = 0.0;
-    /* a fixed number of iterations needs no scalars on the host between them: whole iterations of the backend (with a
-     * communicator on the context those would add up other ranks' tables, which this call never does) */
+    /* Whole iterations of the backend, with a tolerance as without one: both give the same bits. (With a communicator on the context
+     * those would add up other ranks' tables, which this call never does.) */
     int rank = 0, world = 1;
     ibcu_comm_rank(g_ib.ctx, &rank, &world);
-    const int whole = tol < 0.0f && world == 1;
+    const size_t KD = (size_t)K * D;
+    float* was = NULL;                                             /* centroids and, behind them, those of the iteration before */
+    int32_t* counts = NULL;
+    const int by_tol = !(tol < 0.0f);
+    if (!rc && by_tol) {
+        was = (float*)malloc(2 * KD * sizeof(float) + (size_t)K * sizeof(int32_t));
+        if (!was) rc = IBCU_ERR_NOMEM;
+        else { counts = (int32_t*)(was + 2 * KD); memcpy(was + KD, centers, KD * sizeof(float)); }
+    }
     for (int it = 0; !rc && it < iters; it++) {
-        if (whole) {
+        if (world == 1) {
             rc = ibcu_kmeans_lloyd_iter(g_ib.ctx, (const float*)b.X, N, D, (float*)b.C, K, (int32_t*)b.idx, (float*)b.dist,
                                         (float*)b.sums, (int32_t*)b.counts, (double*)b.inertia);
-            done = it + 1;
-            continue;
+        } else {
+            rc = ibcu_kmeans_assign(g_ib.ctx, (const float*)b.X, N, D, (const float*)b.C, K, (int32_t*)b.idx, (float*)b.dist);
+            if (!rc) rc = ibcu_kmeans_accumulate(g_ib.ctx, (const float*)b.X, N, D, K, (const int32_t*)b.idx, (const float*)b.dist,
+                                                 (float*)b.sums, (int32_t*)b.counts, (double*)b.inertia);
+            if (!rc) rc = ibcu_kmeans_update(g_ib.ctx, (float*)b.C, K, D, (const float*)b.sums, (const int32_t*)b.counts, (float*)b.shift);
         }
-        rc = ibcu_kmeans_assign(g_ib.ctx, (const float*)b.X, N, D, (const float*)b.C, K, (int32_t*)b.idx, (float*)b.dist);
-        if (!rc) rc = ibcu_kmeans_accumulate(g_ib.ctx, (const float*)b.X, N, D, K, (const int32_t*)b.idx, (const float*)b.dist,
-                                             (float*)b.sums, (int32_t*)b.counts, (double*)b.inertia);
-        if (!rc) rc = ibcu_kmeans_update(g_ib.ctx, (float*)b.C, K, D, (const float*)b.sums, (const int32_t*)b.counts, (float*)b.shift);
         done = it + 1;
-        if (rc || tol < 0.0f) continue;
-        /* the reference's two stopping rules (src/pq_kmeans.c:285-288) need the scalars on the host */
-        char two[32];
-        const km_result scalars = { two, b.inertia, sizeof two };
-        rc = km_download(&scalars, 1);
+        if (rc || !by_tol) continue;
+        /* the reference's two stopping rules (src/pq_kmeans.c:285-288); the moves are added up as it adds them (:262-282) */
+        double inertia;
+        const km_result now[3] = { { was, b.C, KD * sizeof(float) }, { counts, b.counts, (size_t)K * sizeof(int32_t) }, { &inertia, b.inertia, sizeof inertia } };
+        rc = km_download(now, 3);
         if (rc) break;
-        double inertia; float shift;
-        memcpy(&inertia, two, sizeof inertia); memcpy(&shift, two + 16, sizeof shift);
+        const float shift = km_shift(was, was + KD, counts, K, D);
+        memcpy(was + KD, was, KD * sizeof(float));
         if (shift < tol) break;
         double diff = prev - inertia; if (diff < 0) diff = -diff;
         if (it > 0 && diff < (double)tol * (prev + 1e-12)) break;
         prev = inertia;
     }
+    free(was);
     km_result out[3] = { { centers, b.C, (size_t)K * D * sizeof(float) } };
     int n_out = 1;
     if (indices_out) out[n_out++] = (km_result){ indices_out, b.idx, (size_t)N * sizeof(int32_t) };

@@ -156,6 +156,37 @@ def test_kmeans_entry_points(host, cpu_libs):
     assert 1 <= n < 50
 
 
+@pytest.mark.parametrize("N,D,K", [(60000, 4, 256), (30001, 8, 100), (60000, 8, 64), (20000, 16, 200), (5000, 5, 30)])
+def test_kmeans_tolerance_takes_the_same_iterations(host, N, D, K):
+    """A tolerance decides when the loop ends and nothing else: the same bits as that many iterations without one, ended where the two stopping rules
+    say, taken from the centroids and the inertia of every single iteration (one cluster stays empty)."""
+    rng = np.random.default_rng(N + D)
+    X = (rng.standard_normal((N, D)) * 0.02).astype(np.float32)
+    C0 = X[:K].copy(); C0[K // 2] = 1e6
+    ine = C.c_double()
+
+    def run(start, iters, tol):
+        c = start.copy(); idx = np.empty(N, np.int32)
+        n = host.ib_b200_kmeans_lloyd(p(X), N, D, K, iters, tol, p(c), p(idx), C.byref(ine))
+        return n, c, idx, ine.value
+
+    tol, now, prev, ends = 2e-3, C0, 0.0, 0
+    for it in range(30):
+        n, after, idx, inertia = run(now, 1, -1.0)
+        assert n == 1
+        shift = np.float32(0)
+        for move in (after - now)[np.bincount(idx, minlength=K) > 0].reshape(-1):
+            shift += move * move
+        now, ends = after, it + 1
+        if shift < np.float32(tol) or (it > 0 and abs(prev - inertia) < float(np.float32(tol)) * (prev + 1e-12)):
+            break
+        prev = inertia
+    got = run(C0, 30, tol)
+    assert got[0] == ends and np.array_equal(got[1], now) and np.array_equal(got[2], idx) and got[3] == inertia
+    for a, b in zip(run(C0, 4, 0.0), run(C0, 4, -1.0)):
+        assert np.array_equal(a, b)
+
+
 def _tiny_model(rng, cfg):
     H, I, kv, V = cfg.hidden, cfg.inter, cfg.n_kv_heads * cfg.head_dim, cfg.vocab
     shapes = [(H, H), (kv, H), (kv, H), (H, H), (I, H), (I, H), (H, I)]
