@@ -60,6 +60,7 @@ template <int D> struct Shape {
     static constexpr int copies = D == 16 ? 1 : 4;
     static constexpr int dim_stride = 8 * copies;                 // floats
     static constexpr int group_stride = dim_stride * D + (copies == 1 ? 4 : 0);
+    static constexpr int each_lane = D == 4 ? 10 : 16;            // undecided rows of a warp from which every lane does its own
     static constexpr int row_stride = D == 16 ? 20 : D;           // floats per cluster in a table of sums (16: skewed, or all clusters' pieces would share two places in the banks)
 };
 
@@ -455,8 +456,32 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                 const bool second = swap ? m4 == best : m0 != best;
                 win = g1 * 8 + (second ? at4 : at0) + (second != (swap != 0) ? 4 : 0);
             }
-            // rows the filter could not decide: the whole warp evaluates all centroids exactly
+            // Rows the filter could not decide: all centroids in the exact form, by the whole warp for one row after another, or, where they
+            // are many (equal centroids, points on a grid), by every lane for its own row. 1 Mi points that are all undecided, 256 centroids:
+            // 479 -> 178 us for 4 dimensions, 597 -> 287 for 8, 1239 -> 508 for 16 (assign_exact_kernel: 144, 256, 467). As turns of the
+            // loop that evaluates the best group it would save the code, but took 204 us instead of 183 per iteration without ties.
             unsigned todo = __ballot_sync(0xffffffffu, have && !sure);
+            if (__popc(todo) > S::each_lane) {
+                todo = 0u;
+                win = 0;
+                best = group_sqdist<D>(xr, cgrp, 0);                 // the reference's seed whatever its distance
+#pragma unroll 1
+                for (int k = 0; k < Kp; k += 4) {                    // four centroids at a time, the same for all lanes; padding is NaN
+                    const float* c4 = cgrp + (k >> 3) * S::group_stride + (k & 4);
+                    float dk[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+#pragma unroll
+                    for (int d = 0; d < D; d++) {
+                        const ulonglong2 c2 = *reinterpret_cast<const ulonglong2*>(c4 + d * S::dim_stride);
+                        const unsigned long long xx = pack2(xr[d], xr[d]), va = sub2(xx, c2.x), vb = sub2(xx, c2.y);
+                        float p0, p1, p2, p3;
+                        unpack2(mul2(va, va), p0, p1);
+                        unpack2(mul2(vb, vb), p2, p3);
+                        dk[0] = __fadd_rn(dk[0], p0); dk[1] = __fadd_rn(dk[1], p1); dk[2] = __fadd_rn(dk[2], p2); dk[3] = __fadd_rn(dk[3], p3);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) if (dk[j] < best) { best = dk[j]; win = k + j; }      // ascending and strict, as the reference goes
+                }
+            }
             while (todo) {
                 const int rl = __ffs(todo) - 1;
                 todo &= todo - 1;

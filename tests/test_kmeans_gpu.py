@@ -332,3 +332,26 @@ def test_fused_iteration_at_length(backend, cpu_libs, N, D, K, tables):
     assert np.array_equal(be.download(ds, np.float32, K * D).reshape(K, D), h[2]["sums"])
     for b in (dX, dC, di, dd, ds, dc, dn):
         b.free(); be._bufs.remove(b)
+
+
+@pytest.mark.parametrize("D,K", [(4, 256), (4, 130), (8, 250), (8, 33), (16, 256), (16, 49)])
+def test_many_points_the_filter_cannot_decide(backend, cpu_libs, D, K):
+    """Warps in which few, about the limit, or all rows are undecided: equal centroids, points on a grid (ties between any groups), with NaN and
+    Inf centroids among them, and a NaN centroid 0, from which the reference's scan never gets away."""
+    rng = np.random.default_rng(D * K)
+    N = 41000                                                # past 37888 points, where every one of these goes to the tensor cores
+    base = (rng.standard_normal((N, D)) * 0.02).astype(np.float32)
+    grid = (np.round(base / 0.02) * 0.02).astype(np.float32)
+    for name, X in [("zeros", np.zeros_like(base)), ("grid", grid)] + [(f, np.where(rng.random((N, 1)) < f, 0, base).astype(np.float32)) for f in (0.02, 0.3, 0.5, 0.7)]:
+        Cn = X[:K].copy()
+        Cn[K // 2] = 0; Cn[1] = 0                            # the same centroid in two groups
+        for bad in (None, (K - 1, np.nan), (2, np.inf), (0, np.nan)):
+            Cs = Cn.copy()
+            if bad:
+                Cs[bad[0], D - 1] = bad[1]
+            want, wd = oracle_assign(cpu_libs, X, Cs)
+            got, gd = backend.kmeans_assign(X, Cs, want_dist=True)
+            assert np.array_equal(got, want) and np.array_equal(gd, wd, equal_nan=True), (name, bad)
+            h = _lloyd_gpu(backend, X, Cs, 1)[0]
+            assert np.array_equal(h["idx"], want), (name, bad)
+            assert np.array_equal(h["counts"], np.bincount(want, minlength=K)), (name, bad)
