@@ -533,7 +533,7 @@ int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const floa
 }  // namespace
 
 // kmeans_tc.cu
-bool ibcu_kmeans_tc_takes(const float* X, long N, int D, const float* C, int K);
+bool ibcu_kmeans_tc_takes(const float* X, long N, int D, int K);
 long ibcu_kmeans_tc_blocks(long N);
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist);
 int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
@@ -629,7 +629,7 @@ extern "C" int ibcu_kmeans_lloyd_iter(ibcu_ctx* ctx, const float* X, long N, int
     // second read of X and no launch; only the per-block tables are left to add up
     bool fused = false;
     float* const move = ctx->world > 1 ? nullptr : C;       // one GPU: the kernel that adds up the tables moves the centroids
-    if (ctx->kmeans_path == IBCU_KMEANS_AUTO && ibcu_kmeans_tc_takes(X, N, D, C, K)) {
+    if (ctx->kmeans_path == IBCU_KMEANS_AUTO && ibcu_kmeans_tc_takes(X, N, D, K)) {
         const int nblocks = (int)ibcu_kmeans_tc_blocks(N);
         const size_t KD = (size_t)K * D;
         const size_t need = (size_t)nblocks * (KD * sizeof(float) + K * sizeof(int32_t) + sizeof(double)) + 64;

@@ -231,7 +231,11 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
     const int n = tid;
     float c[D], nn = 0.0f;
     if (n < Kp) {
-        load_row<D>(C, n, n < K, c);
+        if (((uintptr_t)C & 15) == 0) load_row<D>(C, n, n < K, c);
+        else {
+#pragma unroll
+            for (int d = 0; d < D; d++) c[d] = n < K ? __ldcg(C + n * D + d) : 0.0f;
+        }
 #pragma unroll
         for (int d = 0; d < D; d++) {
 #pragma unroll
@@ -603,10 +607,10 @@ constexpr size_t TC_SMEM_MAX = 227 * 1024;
 
 }  // namespace
 
-// The calls the tensor-memory kernel takes: 4, 8 or 16 dimensions, up to 256 centroids, 16-byte aligned arrays (their rows then are
+// The calls the tensor-memory kernel takes: 4, 8 or 16 dimensions, up to 256 centroids, points at 16 bytes (their rows then are
 // too). Tiles are counted in an int.
-bool ibcu_kmeans_tc_takes(const float* X, long N, int D, const float* C, int K) {
-    return (D == 4 || D == 8 || D == 16) && K >= 1 && K <= 256 && (((uintptr_t)X | (uintptr_t)C) & 15) == 0 && N <= (1L << 37);
+bool ibcu_kmeans_tc_takes(const float* X, long N, int D, int K) {
+    return (D == 4 || D == 8 || D == 16) && K >= 1 && K <= 256 && ((uintptr_t)X & 15) == 0 && N <= (1L << 37);
 }
 long ibcu_kmeans_tc_blocks(long N) {
     const long ntile = (N + TC_TILE - 1) / TC_TILE;
@@ -615,7 +619,7 @@ long ibcu_kmeans_tc_blocks(long N) {
 
 // Returns IBCU_DECLINED without touching the context's error when the call is not its own (the caller takes another kernel).
 int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist) {
-    if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
+    if (!ibcu_kmeans_tc_takes(X, N, D, K)) return IBCU_DECLINED;
     const long blocks = ibcu_kmeans_tc_blocks(N);
     switch (D) {
         case 4: return tc_launch<4, false, 12>(ctx, blocks, X, N, C, K, idx, dist, nullptr, nullptr, nullptr);
@@ -629,7 +633,7 @@ int ibcu_kmeans_assign_tc(ibcu_ctx* ctx, const float* X, long N, int D, const fl
 // and return convention as above.
 int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K, int32_t* idx, float* dist,
                                      float* part_sums, int32_t* part_counts, double* part_inertia) {
-    if (!ibcu_kmeans_tc_takes(X, N, D, C, K)) return IBCU_DECLINED;
+    if (!ibcu_kmeans_tc_takes(X, N, D, K)) return IBCU_DECLINED;
     const long blocks = ibcu_kmeans_tc_blocks(N);
     switch (D) {
         case 4: return tc_launch<4, true, 12>(ctx, blocks, X, N, C, K, idx, dist, part_sums, part_counts, part_inertia);
