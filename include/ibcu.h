@@ -262,8 +262,8 @@ int ibcu_int4g_matmul_fp32(ibcu_ctx* ctx, const ibcu_int4g_t* t, const float* x,
 int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K,
                        int32_t* idx, float* dist);
 /* Which assignment kernel ibcu_kmeans_assign may take; every one gives the same codes and distances. For tests
- * and comparisons: AUTO = the fastest the shape allows (D = 4, 8, 16 and K up to 256: tcgen05 tensor-core filter; D = 8 and
- * larger K in multiples of 8: the mma.sync filter; other shapes the exact kernel). */
+ * and comparisons: AUTO = the fastest the shape allows (D = 4, 8, 16 and K up to 256: tcgen05 tensor-core filter, except for few
+ * centroids or points; D = 8 and other K in multiples of 8 from 24: the mma.sync filter; else the exact kernel). */
 #define IBCU_KMEANS_AUTO     0
 #define IBCU_KMEANS_EXACT    1   /* every distance in the exact form on the CUDA cores */
 #define IBCU_KMEANS_MMA_SYNC 2   /* never the tcgen05 kernel */

@@ -541,6 +541,16 @@ int ibcu_kmeans_assign_accumulate_tc(ibcu_ctx* ctx, const float* X, long N, int 
 
 extern "C" void ibcu_kmeans_set_path(ibcu_ctx* ctx, int path) { if (ctx) ctx->kmeans_path = path; }
 
+// Whether an assignment without sums goes to the tcgen05 kernel. It takes 0.7 to 1.5 us longer to start than the others, and its time per point hardly
+// depends on the number of centroids below 64. Others / tcgen05, us: D = 4, 18944 points: 64 centroids 3.1 / 4.3, 100 4.3 / 4.8, 128 4.9 / 4.8;
+// 40000 points (past one block of 256 points per SM the exact kernel takes twice as long): 32 centroids 3.2 / 4.3, 48 5.8 / 4.7; 1 Mi: 32 21.6 / 20.4.
+// D = 8, 4096 points: 48 centroids 3.7 / 4.5, 64 3.8 / 4.5, 100 6.9 / 4.9, 128 4.7 / 4.9; 40000: 16 3.2 / 4.8, 24 4.7 / 4.8, 32 5.0 / 4.8. D = 16, 300 points:
+// 32 centroids 4.3 / 4.5, 48 5.6 / 4.6; 40000: 16 5.6 / 5.8, 24 7.2 / 6.1; 1 Mi: 16 35 / 42, 24 49 / 42. (An iteration with its sums is faster there at any size.)
+static bool tc_assign_pays(long N, int D, int K) {
+    if (K >= (D == 4 ? 128 : (D == 8 ? 72 : 48))) return true;
+    return K > (D == 4 ? 32 : 16) && N > 148 * 256;
+}
+
 extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K,
                                   int32_t* idx, float* dist) {
     IBCU_CHECK_CTX(ctx);
@@ -548,12 +558,13 @@ extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, 
     IBCU_REQUIRE(ctx, N > 0 && D >= 1 && D <= KM_MAX_D && K >= 1 && K <= 1024, "ibcu_kmeans_assign: N=%ld D=%d K=%d out of range", N, D, K);
     IBCU_REQUIRE(ctx, (size_t)K * D * sizeof(float) <= 128 * 1024, "ibcu_kmeans_assign: K*D=%d too large", K * D);
     // Scores on the tensor cores as a filter, exact re-evaluation of the candidates: the tcgen05 kernel for 4, 8 and 16 dimensions and
-    // up to 256 centroids; for D == 8 and more centroids, in multiples of 8, the register-operand (mma.sync) filter.
-    if (ctx->kmeans_path == IBCU_KMEANS_AUTO) {
+    // up to 256 centroids where it pays; for D == 8 and other numbers of centroids, in multiples of 8, the register-operand (mma.sync) filter.
+    if (ctx->kmeans_path == IBCU_KMEANS_AUTO && tc_assign_pays(N, D, K)) {
         const int rc = ibcu_kmeans_assign_tc(ctx, X, N, D, C, K, idx, dist);
         if (rc != IBCU_DECLINED) return rc;
     }
-    if (D == 8 && K % 8 == 0 && K >= 8 && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
+    // up to 16 centroids the exact form costs less (1 Mi points: 8 centroids 12.1 against 25.7 us, 16 19.7 against 29.4, 24 27.4 against 33.4)
+    if (D == 8 && K % 8 == 0 && (K > 16 || ctx->kmeans_path == IBCU_KMEANS_MMA_SYNC) && ctx->kmeans_path != IBCU_KMEANS_EXACT && ((uintptr_t)X & 15) == 0) {
         const size_t smem = ((size_t)K * 16 + K + (size_t)K * 8 + 4) * sizeof(float);
         static SmemOptIn opt;
         if (int rc = ibcu_allow_smem(ctx, opt, assign_filter_kernel, smem)) return rc;
