@@ -355,3 +355,32 @@ def test_many_points_the_filter_cannot_decide(backend, cpu_libs, D, K):
             h = _lloyd_gpu(backend, X, Cs, 1)[0]
             assert np.array_equal(h["idx"], want), (name, bad)
             assert np.array_equal(h["counts"], np.bincount(want, minlength=K)), (name, bad)
+
+
+@pytest.mark.parametrize("D", [4, 8, 16])
+def test_fused_iteration_on_what_the_filter_cannot_decide(backend, cpu_libs, D):
+    """Near ties across groups, NaN, Inf, squares that overflow or vanish, and points up to 2^20 times longer than every centroid, through an iteration,
+    which takes the tensor cores at every size: codes and distances are the checker's."""
+    rng = np.random.default_rng(300 + D)
+    be, K, N = backend, 72, 9000
+    Cn = (rng.standard_normal((K, D)) * 0.02).astype(np.float32)
+    d = Cn[60].astype(np.float64) - Cn[3]; d /= np.linalg.norm(d)
+    noise = rng.standard_normal((N, D)) * 0.002
+    near = ((Cn[3].astype(np.float64) + Cn[60]) / 2 + noise - (noise @ d)[:, None] * d).astype(np.float32)
+    near[5, 1] = np.nan; near[6, 0] = np.inf; near[7, 2] = -np.inf
+    near[8] *= np.float32(1e20); near[9] *= np.float32(1e-22); near[10] = 0
+    far = rng.standard_normal((N, D)).astype(np.float32) * np.exp2(rng.integers(-8, 14, (N, 1))).astype(np.float32)
+    cases = [(far, Cn[:41], 1.0, None)] + [(near, Cn, s, b) for s, b in ((1.0, None), (1.0, (0, np.nan)), (1.0, (70, np.nan)), (1.0, (9, np.inf)), (1e-20, None), (3e18, None), (2e19, None))]
+    for X, C0, scale, bad in cases:
+        Xs, Cs = X * np.float32(scale), C0 * np.float32(scale)
+        if bad:
+            Cs[bad[0], 1] = bad[1]
+        k = len(Cs)
+        bufs = [be.upload(Xs), be.upload(Cs), be.alloc(N * 4), be.alloc(N * 4), be.alloc(k * D * 4), be.alloc(k * 4), be.alloc(8)]
+        dX, dC, di, dd, ds, dc, dn = bufs
+        be._check(be.lib.ibcu_kmeans_lloyd_iter(be.ctx, dX.ptr, N, D, dC.ptr, k, di.ptr, dd.ptr, ds.ptr, dc.ptr, dn.ptr))
+        want, wd = oracle_assign(cpu_libs, Xs, Cs)
+        assert np.array_equal(be.download(di, np.int32, N), want), (scale, bad)
+        assert np.array_equal(be.download(dd, np.float32, N), wd, equal_nan=True), (scale, bad)
+        for b in bufs:
+            b.free(); be._bufs.remove(b)
