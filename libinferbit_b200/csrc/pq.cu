@@ -709,7 +709,7 @@ __device__ __forceinline__ unsigned topk_key(float v) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// One block (for more rows than the kernels below keep in registers, and where the quick choice finds too many). The K_top-th largest key by
+// One block (for more rows than the kernels below keep in registers). The K_top-th largest key by
 // passes of 8-bit digit counts over (key - smallest key), from its highest set bit down: counted from the smallest key
 // the first digit already spreads the rows over the table (logits themselves share their leading bits, and adds to a
 // few shared counters queue behind one another), and later passes only touch the rows of one digit. Then the rows above
@@ -717,9 +717,11 @@ __device__ __forceinline__ unsigned topk_key(float v) {
 // reference keeps the first row it met among equal first-level logits at the boundary too (a later row replaces the
 // heap's root only when strictly larger), but which equal rows survive inside its heap depends on the heap's shape;
 // equal logits at the boundary are a tie that callers cannot rely on either way.
-__device__ __forceinline__ void topk_by_digits(const float* coarse, int M, int K_top, int32_t* cand) {
+__global__ void __launch_bounds__(TOPK_THREADS) pq_topk_select_kernel(const float* __restrict__ coarse, int M, int K_top, int32_t* __restrict__ cand) {
     __shared__ unsigned hist[256], red_lo[TOPK_THREADS / 32], red_hi[TOPK_THREADS / 32];
     __shared__ unsigned s_prefix, s_need, s_gt, s_eq_before, warp_tot[TOPK_THREADS / 32];
+    pdl_launch_dependents();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nchunk = (M + TOPK_THREADS - 1) / TOPK_THREADS;
     auto key_at = [&](int j) -> unsigned {                    // key of row tid + 1024 j
@@ -790,25 +792,21 @@ __device__ __forceinline__ void topk_by_digits(const float* coarse, int M, int K
     }
 }
 
-__global__ void __launch_bounds__(TOPK_THREADS) pq_topk_select_kernel(const float* __restrict__ coarse, int M, int K_top, int32_t* __restrict__ cand) {
-    pdl_launch_dependents();
-    pdl_wait();
-    topk_by_digits(coarse, M, K_top, cand);
-}
-
-// The choice of up to 256 of at most 65536 rows, by one block whose threads hold NREG keys each (the rest is read twice). A key that at least K_top of the threads'
-// largest keys reach is no more than the K_top-th largest key; a bit-by-bit search over the 1024 largest keys finds a tight one with a
-// barrier per bit, and stops once few more than K_top reach it. The rows that reach it, a few more than K_top unless many are equal, are
-// ranked by counting those ahead of them: larger key, then smaller row. More than TOPK_FOUND of them: by digits over all rows.
+// The choice of up to 256 of at most 65536 rows, by one block whose threads hold TOPK_HELD keys each (the rest is read again). A key that at least
+// K_top of the threads' largest keys reach is no more than the K_top-th largest key; a bit-by-bit search over the 1024 largest keys finds
+// a tight one with a barrier per bit, and stops once few more than K_top reach it. The rows that reach it, a few more than K_top unless
+// many are equal or a few threads hold most of the largest, are ranked by counting those ahead of them: larger key, then smaller row.
+// Where they are more than TOPK_RANK, the K_top-th largest key itself is searched for, among the rows found or, beyond TOPK_FOUND, among
+// all, read again: halves of what is left between the bound and the largest key, either end moving on to the next key that there is (rows of a
+// few different logits take a step or two). Rows above it are taken, and of those equal to it the lowest.
 // 32000 rows, 64 chosen: the whole call 41.3 -> 32.6 us against the cluster below, whose rounds each cost two cluster barriers.
-constexpr int TOPK_QUICK = 256, TOPK_FOUND = 1024;
-template <int NREG>
+constexpr int TOPK_QUICK = 256, TOPK_HELD = 32, TOPK_RANK = 384, TOPK_FOUND = 2048;
 __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const float* coarse, int M, int K_top, int32_t* cand) {
-    __shared__ unsigned n_found;
+    __shared__ unsigned n_found, n_taken, warp_cnt[2][32], warp_low[2][32], warp_high[2][32];
     __shared__ uint2 found[TOPK_FOUND];                       // key, row
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto load4 = [&](int j, unsigned* k) {                    // rows 4 (1024 j + tid) .. + 3
         const int i = 4 * (j * TOPK_THREADS + tid);
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -818,19 +816,19 @@ __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const fl
 #pragma unroll
         for (int c = 0; c < 4; c++) k[c] = i + c < M ? topk_key(f[c]) : 0u;
     };
-    unsigned keys[NREG], top = 0u;
+    unsigned keys[TOPK_HELD], top = 0u;
 #pragma unroll
-    for (int j = 0; j < NREG / 4; j++) load4(j, keys + 4 * j);
+    for (int j = 0; j < TOPK_HELD / 4; j++) load4(j, keys + 4 * j);
 #pragma unroll
-    for (int j = 0; j < NREG; j++) top = max(top, keys[j]);
+    for (int j = 0; j < TOPK_HELD; j++) top = max(top, keys[j]);
     const int more = (M + 4 * TOPK_THREADS - 1) / (4 * TOPK_THREADS);
 #pragma unroll 4
-    for (int j = NREG / 4; j < more; j++) {                   // rows beyond those held are read again below
+    for (int j = TOPK_HELD / 4; j < more; j++) {              // rows beyond those held are read again below
         unsigned k[4];
         load4(j, k);
         top = max(max(max(top, k[0]), max(k[1], k[2])), k[3]);
     }
-    if (tid == 0) n_found = 0u;
+    if (tid == 0) n_found = n_taken = 0u;
     unsigned bound = 0u;
     for (unsigned bit = 0x80000000u; bit; bit >>= 1) {
         const int n = __syncthreads_count(top >= (bound | bit));
@@ -839,7 +837,7 @@ __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const fl
             if (n <= K_top + K_top / 8) break;
         }
     }
-    __syncthreads();                                          // n_found is zero for everyone, also where the loop ended at once
+    __syncthreads();                                          // the counters are zero for everyone, also where the loop ended at once
     auto take = [&](unsigned key, int i) {
         if (key >= bound && i < M) {
             const unsigned slot = atomicAdd(&n_found, 1u);
@@ -847,8 +845,8 @@ __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const fl
         }
     };
 #pragma unroll
-    for (int j = 0; j < NREG; j++) take(keys[j], 4 * ((j >> 2) * TOPK_THREADS + tid) + (j & 3));
-    for (int j = NREG / 4; j < more; j++) {
+    for (int j = 0; j < TOPK_HELD; j++) take(keys[j], 4 * ((j >> 2) * TOPK_THREADS + tid) + (j & 3));
+    for (int j = TOPK_HELD / 4; j < more; j++) {
         unsigned k[4];
         load4(j, k);
 #pragma unroll
@@ -856,18 +854,93 @@ __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const fl
     }
     __syncthreads();
     const int n = (int)n_found;
-    if (n > TOPK_FOUND) { topk_by_digits(coarse, M, K_top, cand); return; }      // uniform over the block
-    int per = 32;                                             // threads per row found
-    while (per > 1 && n * per > TOPK_THREADS) per >>= 1;
-    const int c = tid / per;
-    const uint2 me = found[c < n ? c : 0];
-    int ahead = 0;
-    for (int e = tid % per; e < n; e += per) {
-        const uint2 o = found[e];
-        ahead += o.x > me.x || (o.x == me.x && o.y < me.y);
+    if (n <= TOPK_RANK) {
+        int per = 32;                                         // threads per row found
+        while (per > 1 && n * per > TOPK_THREADS) per >>= 1;
+        const int c = tid / per;
+        const uint2 me = found[c < n ? c : 0];
+        int ahead = 0;
+        for (int e = tid % per; e < n; e += per) {
+            const uint2 o = found[e];
+            ahead += o.x > me.x || (o.x == me.x && o.y < me.y);
+        }
+        for (int o = per >> 1; o > 0; o >>= 1) ahead += __shfl_xor_sync(0xffffffffu, ahead, o);
+        if (c < n && tid % per == 0 && ahead < K_top) cand[ahead] = (int32_t)me.y;
+        return;
     }
-    for (int o = per >> 1; o > 0; o >>= 1) ahead += __shfl_xor_sync(0xffffffffu, ahead, o);
-    if (c < n && tid % per == 0 && ahead < K_top) cand[ahead] = (int32_t)me.y;
+    // ── the K_top-th largest key: at least K_top rows reach lo, n_gt < K_top rows lie above hi ──
+    const bool listed = n <= TOPK_FOUND;
+    int turn = 0;
+    // rows with a key of at least v, the smallest of those, and the largest key below v (a row that is not there has the key 0; v is never 0)
+    auto tally = [&](unsigned v, unsigned& below, unsigned& from) {
+        unsigned cnt = 0u, low = 0u, high = 0xffffffffu;
+        auto look = [&](unsigned k) { if (k >= v) { cnt++; high = min(high, k); } else low = max(low, k); };
+        if (listed) {
+            for (int e = tid; e < n; e += TOPK_THREADS) look(found[e].x);
+        } else {
+#pragma unroll 4
+            for (int j = 0; j < more; j++) {
+                unsigned k[4];
+                load4(j, k);
+#pragma unroll
+                for (int c = 0; c < 4; c++) look(k[c]);
+            }
+        }
+        cnt = __reduce_add_sync(0xffffffffu, cnt); low = __reduce_max_sync(0xffffffffu, low); high = __reduce_min_sync(0xffffffffu, high);
+        if (lane == 0) { warp_cnt[turn][warp] = cnt; warp_low[turn][warp] = low; warp_high[turn][warp] = high; }
+        __syncthreads();
+        cnt = __reduce_add_sync(0xffffffffu, warp_cnt[turn][lane]);
+        below = __reduce_max_sync(0xffffffffu, warp_low[turn][lane]); from = __reduce_min_sync(0xffffffffu, warp_high[turn][lane]);
+        turn ^= 1;                                            // the next call writes the other half: one barrier a call
+        return (int)cnt;
+    };
+    unsigned lo = bound, hi;
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) warp_low[1][warp] = top;                   // the first tally takes the other half
+    __syncthreads();
+    hi = __reduce_max_sync(0xffffffffu, warp_low[1][lane]);
+    int n_gt = 0;
+    while (lo < hi) {
+        const unsigned mid = lo + ((hi - lo) >> 1) + 1u;
+        unsigned below, from;
+        const int c = tally(mid, below, from);
+        if (c >= K_top) lo = from;
+        else { hi = below; n_gt = c; }
+    }
+    // ── rows above it in any order (the last launch orders by full logits), then the lowest of those equal to it ──
+    auto above = [&](unsigned key, int i) { if (key > hi) cand[atomicAdd(&n_taken, 1u)] = i; };
+    if (n_gt > 0) {
+        if (listed) {
+            for (int e = tid; e < n; e += TOPK_THREADS) above(found[e].x, (int)found[e].y);
+        } else {
+            for (int j = 0; j < more; j++) {
+                unsigned k[4];
+                load4(j, k);
+#pragma unroll
+                for (int c = 0; c < 4; c++) above(k[c], 4 * (j * TOPK_THREADS + tid) + c);
+            }
+        }
+    }
+    for (int j = 0, at = n_gt; j < more && at < K_top; j++) { // runs of 4096 rows, until enough are found
+        unsigned k[4];
+        load4(j, k);
+        const int i = 4 * (j * TOPK_THREADS + tid);
+        int mine = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) mine += k[c] == hi && i + c < M;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
+        if (lane == 31) warp_cnt[turn][warp] = (unsigned)incl;
+        __syncthreads();
+        const unsigned of_warp = warp_cnt[turn][lane];
+        int place = at + incl - mine + (int)__reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0u);
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (k[c] == hi && i + c < M) { if (place < K_top) cand[place] = i + c; place++; }
+        at += (int)__reduce_add_sync(0xffffffffu, of_warp);
+        turn ^= 1;
+    }
 }
 
 // The same selection by a cluster of eight blocks: a block keeps chunks rank, rank + 8, ... of 1024 rows (NREG keys per
@@ -1130,7 +1203,7 @@ extern "C" int ibcu_pq_lm_head_topk(ibcu_ctx* ctx, const ibcu_pq_t* t, const flo
     rc = pq_launch(ctx, t, x, coarse, t->M, 1, pl, (unsigned long long*)((char*)ctx->pq_acc + PQ_COUNTER_BYTES), (unsigned int*)ctx->pq_acc, true);
     if (rc) return rc;
     if (K_top <= TOPK_QUICK && t->M <= 64 * TOPK_THREADS)
-        rc = ibcu_launch(ctx, pq_topk_quick_kernel<32>, dim3(1), dim3(TOPK_THREADS), 0, 1, true, (const float*)coarse, t->M, K_top, cand);
+        rc = ibcu_launch(ctx, pq_topk_quick_kernel, dim3(1), dim3(TOPK_THREADS), 0, 1, true, (const float*)coarse, t->M, K_top, cand);
     else if (t->M <= 4 * TOPK_CL * TOPK_THREADS)
         rc = ibcu_launch(ctx, pq_topk_select_cluster_kernel<4>, dim3(TOPK_CL), dim3(TOPK_THREADS), 0, TOPK_CL, true, (const float*)coarse, t->M, K_top, cand);
     else if (t->M <= 32 * TOPK_CL * TOPK_THREADS)

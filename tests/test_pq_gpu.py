@@ -192,6 +192,28 @@ def test_pq_lm_head_topk_order_of_scaled_rows(backend, cpu_libs, M, k_top, step)
     assert np.all(np.diff(gl) <= 0)
 
 
+@pytest.mark.parametrize("M,k_top,layout", [(1000, 256, "equal"), (1023, 251, "falling"), (32000, 256, "falling"), (65536, 256, "falling"), (32768, 64, "comb"),
+                                            (65536, 128, "comb"), (40001, 200, "comb"), (33000, 200, "few threads"), (65535, 256, "few threads"),
+                                            (65536, 8, "two values"), (5000, 97, "two values"), (64000, 256, "equal")])
+def test_pq_lm_head_topk_where_many_rows_reach_the_bound(backend, cpu_libs, M, k_top, layout):
+    """More rows at the bound of the quick choice than it ranks: among those it has listed, among all rows, rows of a few logits, and the largest
+    rows with a few of its threads. Rows differ by their scale alone."""
+    rng = np.random.default_rng(M + k_top)
+    d = _cpu.make_pq_case_ex(rng, M, 32, 16, 256, 0, 0, 1)
+    for key in ("idx1_l", "idx1_r"):
+        d[key][:] = d[key][0]
+    row = np.arange(M)
+    level = {"equal": np.ones(M), "falling": np.linspace(2, 1, M), "comb": np.where(row % 4096 == 0, 3.0, np.where(row < 150, 2.0, 1.0)),
+             "few threads": np.where(row % 4096 < 160, 2 + rng.random(M), 1.0), "two values": np.where(rng.random(M) < 20 / M, 2.0, 1.0)}[layout].astype(np.float16)
+    d["rs"][:] = level.view(np.uint16)
+    x = d["x"][0].copy()
+    if _cpu.oracle_pq_topk(cpu_libs.oracle, d, x, 1)[0][0] < 0:
+        x = -x                                                # larger scales then have larger logits
+    gl, gi = backend.pq_lm_head_topk(backend.make_pq_ex(d), x, k_top)
+    assert gi.tolist() == np.argsort(-level.astype(np.float32), kind="stable")[:k_top].tolist()
+    assert np.all(np.diff(gl) <= 0)
+
+
 def test_pq_lm_head_topk_through_the_host_layer(cpu_libs):
     """ib_b200_pq_lm_head_topk takes the reference's own struct and host pointers."""
     from libinferbit_b200 import _ffi
