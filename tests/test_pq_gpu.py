@@ -214,6 +214,23 @@ def test_pq_lm_head_topk_where_many_rows_reach_the_bound(backend, cpu_libs, M, k
     assert np.all(np.diff(gl) <= 0)
 
 
+@pytest.mark.parametrize("M", [1, 127, 129, 257, 513, 1024])
+def test_pq_lm_head_topk_orders_zeros_infinities_and_nan(backend, cpu_libs, M):
+    """All rows chosen: descending logits, both zeros equal, NaN last, the lower row first among equals; one, two, four and eight rows per thread."""
+    rng = np.random.default_rng(M)
+    d = _cpu.make_pq_case_ex(rng, M, 32, 16, 256, 0, 0, 1)
+    for key in ("idx1_l", "idx1_r"):
+        d[key][:] = d[key][0]
+    level = rng.choice(np.array([0.0, -0.0, 1, -1, 2.5, np.inf, -np.inf, np.nan, 0.1], np.float16), M)
+    d["rs"][:] = level.view(np.uint16)
+    x = d["x"][0].copy()
+    if _cpu.oracle_pq_topk(cpu_libs.oracle, dict(d, rs=_cpu.fp16_bits(np.ones(M, np.float32))), x, 1)[0][0] < 0:
+        x = -x
+    gl, gi = backend.pq_lm_head_topk(backend.make_pq_ex(d), x, M)
+    assert gi.tolist() == sorted(range(M), key=lambda i: (np.isnan(level[i]), -float(level[i]) if not np.isnan(level[i]) else 0, i))
+    assert np.array_equal(np.isnan(gl), np.isnan(level[gi]))
+
+
 def test_pq_lm_head_topk_through_the_host_layer(cpu_libs):
     """ib_b200_pq_lm_head_topk takes the reference's own struct and host pointers."""
     from libinferbit_b200 import _ffi
