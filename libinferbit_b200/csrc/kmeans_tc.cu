@@ -239,8 +239,8 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
 #pragma unroll
         for (int d = 0; d < D; d++) {
 #pragma unroll
-            for (int j = 0; j < S::copies; j++)
-                cgrp[(n >> 3) * S::group_stride + d * S::dim_stride + j * 8 + (n & 7)] = n < K ? c[d] : __uint_as_float(0x7FFFFFFFu);
+            for (int j = 0; j < S::copies; j++)                          // neighbouring groups write different copies: no bank conflict
+                cgrp[(n >> 3) * S::group_stride + d * S::dim_stride + (j + (n >> 3)) % S::copies * 8 + (n & 7)] = n < K ? c[d] : __uint_as_float(0x7FFFFFFFu);
             nn = fmaf(c[d], c[d], nn);
         }
         cm_bits = __float_as_uint(nn);                       // nn >= 0 or NaN: NaN and Inf sort above everything finite
