@@ -26,8 +26,9 @@ namespace {
 
 constexpr int KM_MAX_D = 32;
 
-// One thread per point, centroids broadcast from shared memory.
-template <int DT>
+// One thread per point, centroids broadcast from shared memory. WIDE: rows are read 16 bytes at a time, else they may lie at any float (the other
+// kernels leave such arrays to this one). As a test inside the kernel the choice cost 1 Mi points of 16 against one centroid 1.5 of 10.2 us.
+template <int DT, bool WIDE>
 __global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restrict__ X, long N, int D, const float* __restrict__ C, int K,
                                                            int32_t* __restrict__ idx, float* __restrict__ dist,
                                                            const int32_t* __restrict__ todo, const int* __restrict__ n_todo) {
@@ -38,11 +39,11 @@ __global__ void __launch_bounds__(256) assign_exact_kernel(const float* __restri
     for (int i = threadIdx.x; i < K * d_all; i += blockDim.x) cs[i] = __ldcg(C + i);
     __syncthreads();
     const long total = todo ? (long)__ldcg(n_todo) : N;    // written by the kernel just ahead: read past L1, not as a read-only load
-    const bool wide = DT > 0 && DT % 4 == 0 && ((uintptr_t)X & 15) == 0;      // else rows lie at any float: the other kernels leave such arrays to this one
     for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long)gridDim.x * blockDim.x) {
         const long i = todo ? (long)todo[w] : w;
         float x[DT > 0 ? DT : KM_MAX_D];
-        if (wide) {
+        if constexpr (WIDE) {
+            static_assert(DT > 0 && DT % 4 == 0, "whole pieces of 16 bytes");
 #pragma unroll
             for (int d = 0; d < DT; d += 4) {
                 float4 v = *reinterpret_cast<const float4*>(X + (size_t)i * DT + d);
@@ -515,17 +516,18 @@ int assign_exact_launch(ibcu_ctx* ctx, const float* X, long N, int D, const floa
     long cap = (long)ctx->sm_count * 8;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-#define KM_LAUNCH(DT) do { \
+#define KM_LAUNCH(DT, WIDE) do { \
         static SmemOptIn opt; \
-        if (int rc = ibcu_allow_smem(ctx, opt, assign_exact_kernel<DT>, smem)) return rc; \
-        return ibcu_launch(ctx, assign_exact_kernel<DT>, dim3((unsigned)blocks), dim3(256), smem, 1, true, X, N, D, C, K, idx, dist, todo, n_todo); \
+        if (int rc = ibcu_allow_smem(ctx, opt, assign_exact_kernel<DT, WIDE>, smem)) return rc; \
+        return ibcu_launch(ctx, assign_exact_kernel<DT, WIDE>, dim3((unsigned)blocks), dim3(256), smem, 1, true, X, N, D, C, K, idx, dist, todo, n_todo); \
     } while (0)
+    const bool wide = ((uintptr_t)X & 15) == 0;
     switch (D) {
-        case 2: KM_LAUNCH(2);
-        case 4: KM_LAUNCH(4);
-        case 8: KM_LAUNCH(8);
-        case 16: KM_LAUNCH(16);
-        default: KM_LAUNCH(0);
+        case 2: KM_LAUNCH(2, false);
+        case 4: if (wide) KM_LAUNCH(4, true); KM_LAUNCH(4, false);
+        case 8: if (wide) KM_LAUNCH(8, true); KM_LAUNCH(8, false);
+        case 16: if (wide) KM_LAUNCH(16, true); KM_LAUNCH(16, false);
+        default: KM_LAUNCH(0, false);
     }
 #undef KM_LAUNCH
 }
@@ -544,11 +546,13 @@ extern "C" void ibcu_kmeans_set_path(ibcu_ctx* ctx, int path) { if (ctx) ctx->km
 // Whether an assignment without sums goes to the tcgen05 kernel. It takes 0.7 to 1.5 us longer to start than the others, and its time per point hardly
 // depends on the number of centroids below 64. Others / tcgen05, us: D = 4, 18944 points: 64 centroids 3.1 / 4.3, 100 4.3 / 4.8, 128 4.9 / 4.8;
 // 40000 points (past one block of 256 points per SM the exact kernel takes twice as long): 32 centroids 3.2 / 4.3, 48 5.8 / 4.7; 1 Mi: 32 21.6 / 20.4.
-// D = 8, 4096 points: 48 centroids 3.7 / 4.5, 64 3.8 / 4.5, 100 6.9 / 4.9, 128 4.7 / 4.9; 40000: 16 3.2 / 4.8, 24 4.7 / 4.8, 32 5.0 / 4.8. D = 16, 300 points:
+// D = 8, 4096 points: 48 centroids 3.7 / 4.5, 64 3.8 / 4.5, 100 6.9 / 4.9, 128 4.7 / 4.9; 40000: 16 3.2 / 4.8, 48 5.9 / 5.0; 65536: 24 4.7 / 5.5, 32 5.1 / 5.5;
+// 131072: 24 7.6 / 6.9, 32 8.1 / 6.9. D = 16, 300 points:
 // 32 centroids 4.3 / 4.5, 48 5.6 / 4.6; 40000: 16 5.6 / 5.8, 24 7.2 / 6.1; 1 Mi: 16 35 / 42, 24 49 / 42. (An iteration with its sums is faster there at any size.)
 static bool tc_assign_pays(long N, int D, int K) {
     if (K >= (D == 4 ? 128 : (D == 8 ? 72 : 48))) return true;
-    return K > (D == 4 ? 32 : 16) && N > 148 * 256;
+    if (D == 8 && K <= 32) return K > 16 && N > 98304;       // between the two measured sizes
+    return K > (D == 16 ? 16 : 32) && N > 148 * 256;
 }
 
 extern "C" int ibcu_kmeans_assign(ibcu_ctx* ctx, const float* X, long N, int D, const float* C, int K,
