@@ -6,7 +6,9 @@
 // with groups whose largest |x| is at most eps * max|x| left out when eps > 0 (build_skip_mask, :3854-3882; off by
 // default there). HBM-bound: N/2 bytes of weights and 2 N/G bytes of scales per row, read once.
 //
-// Fast kernel (N and G multiples of 32), integer arithmetic: the activation becomes 32-bit fixed point (2^sh max|x| in
+// Both kernels for N and G multiples of 32 use integer arithmetic; int4g_mma_kernel below takes the tensor cores and most calls, int4g_kernel dp4a: outlier
+// columns, the skip rule, groups of any other multiple of 32 columns, rows beyond 16384 columns, and what im_pays leaves it.
+// int4g_kernel: the activation becomes 32-bit fixed point (2^sh max|x| in
 // [2^29, 2^30)), split into four balanced base-256 digits per column ("limbs"), and a row's 32-column chunk is 32 dp4a
 // instructions: nibbles as bytes (even columns w & 0x0F0F0F0F, odd columns (w >> 4) & 0x0F0F0F0F) times the limb words of
 // the same columns, one int32 sum per limb, exact. The chunk's value sum_k 256^k a_k - 8 sum(X) goes to FP32, times the
@@ -19,6 +21,7 @@
 // reference's scalar loop and the activation is rounded to 2^-30 of its largest magnitude: equal to the reference within
 // the float bar, not bit for bit; f(2x) = 2 f(x) exactly.
 #include "common.cuh"
+#include <algorithm>
 #include <mutex>
 
 namespace {
@@ -308,7 +311,9 @@ __global__ void __launch_bounds__(I4G_THREADS) int4g_mma_kernel(const I4gMma p) 
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d + r * IM_LD + lane * 16),
                              "l"(p.q + (size_t)(pf_row + (on ? r : 0)) * rowbytes + (on ? col : 0)), "r"(on ? 16 : 0) : "memory");
             }
-            // the scales of group j of G columns; of a group longer than a k-block only once, at its place among the k-blocks
+            // The scales of group j of G columns; of a group longer than a k-block only once, at its place among the k-blocks. (Where the number of
+            // scales is odd the last word's other half lies behind them, in the same aligned word, and is not used; here and in int4g_kernel. Copies
+            // that stop before it took G = 32 3 to 8 % longer.)
             for (int e = tid; e < R * SW; e += I4G_THREADS) {
                 const int r = e / SW, w = e - r * SW;
                 const size_t first = (size_t)(pf_row + r) * p.ng + ((size_t)(pf_it * I4G_WARPS * SUB) >> p.gsh);
@@ -468,17 +473,30 @@ int im_launch(ibcu_ctx* ctx, const I4gMma& p, size_t smem) {
     return ibcu_launch(ctx, int4g_mma_kernel<G, RT, STAGES, 8>, grid, block, smem, 1, true, p);
 }
 
-// Rows in equal runs over two blocks per SM; tiles of 32 rows where a run is longer than 16 and three stages still fit beside the limbs.
+// Rows in equal runs over two blocks per SM, but at least a tile of 16 each: with fewer rows a block more blocks convert the whole activation, and
+// that is what they take their time for (256 x 16384, G = 128: 13.1 us with a row a block, 12.5 with 8, 8.8 with 16; 1024 x 4096 4.1 and 3.4).
+// Tiles of 32 rows where a run is longer than 16 and three stages still fit beside the limbs, else of 16, with as many stages as fit. Five
+// stages of 32 rows / three / eight stages of 16 / four, us, G = 128: 14336 x 4096 8.9 / 11.7 / 10.7 / 14.5; 14336 x 8192 - / 16.1 / 19.3 / 26.6;
+// 4096 x 4096 (14 rows a block) 5.2 / 7.0 / 4.3 / 6.5. Up to four groups of eight columns per thread held instead of eight: 16 to 35 registers.
 template <int G>
 int im_dispatch(ibcu_ctx* ctx, I4gMma& p) {
     const int nkb = (p.N + 127) / 128;
     const size_t tail = 4 * (size_t)p.xs_ld + 32 + (size_t)nkb * (128 / G) * 8, room = 112 * 1024;
-    p.rows_per = (p.M + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count);
+    p.rows_per = std::max(16, (p.M + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count));
     auto total = [&](int rt, int stages) { return stages * im_stage(rt, G) + tail + 2 * (size_t)I4G_WARPS * 16 * rt * sizeof(float); };
     if (p.rows_per > 16 && total(2, 5) <= room) return im_launch<G, 2, 5>(ctx, p, total(2, 5));
     if (p.rows_per > 16 && total(2, 3) <= room) return im_launch<G, 2, 3>(ctx, p, total(2, 3));
     if (total(1, 8) <= room) return im_launch<G, 1, 8>(ctx, p, total(1, 8));
     return im_launch<G, 1, 4>(ctx, p, total(1, 4));
+}
+
+// Whether such a call goes to the tensor cores. dp4a / tensor cores, us: few short rows are all launch, and dp4a's is the shorter: 4096 x 1024 3.0 / 3.3,
+// 8192 x 1024 4.1 / 3.4, 1024 x 2048 3.0 / 3.4, 2048 x 2048 3.6 / 3.3, 64 x 4096 4.1 / 3.3 (G = 32 to 256 alike). Groups of 32 in long rows leave room
+// for tiles of 16 rows only, and a run of 49 rows then pays for 64: 14336 x 14336 42.7 / 48.8, 8192 x 14336 (28 rows) 27.5 / 26.7.
+bool im_pays(const ibcu_ctx* ctx, int M, int N, int G) {
+    const int slots = 2 * ctx->sm_count;
+    if (N <= 1024 ? M <= 16 * slots : (N <= 2048 && M <= 4 * slots)) return false;
+    return !(G == 32 && N > 12288 && M > 48 * slots);
 }
 
 // Any N, G (even): a warp per row, lanes over the groups, columns in order inside a group; activations from global memory.
@@ -543,7 +561,7 @@ extern "C" int ibcu_int4g_matmul_fp32(ibcu_ctx* ctx, const ibcu_int4g_t* t, cons
     // groups of 32, 64 or a power-of-two multiple of 128 columns, nothing left out and nothing beside the groups: the tensor cores. Up to
     // 16384 columns are held in registers while they are converted.
     const int per128 = t->G / 128;
-    if (p.eps == 0.0f && t->K_out == 0 && (t->N & 31) == 0 && t->N <= 8 * 8 * I4G_THREADS && (t->G == 32 || t->G == 64 || (t->G % 128 == 0 && (per128 & (per128 - 1)) == 0)) &&
+    if (p.eps == 0.0f && t->K_out == 0 && (t->N & 31) == 0 && t->N <= 8 * 8 * I4G_THREADS && (t->G == 32 || t->G == 64 || (t->G % 128 == 0 && (per128 & (per128 - 1)) == 0)) && im_pays(ctx, t->M, t->N, t->G) &&
         (((uintptr_t)t->q | (uintptr_t)x) & 15) == 0 && ((uintptr_t)t->s & 3) == 0) {
         I4gMma m = { t->q, (const __half*)t->s, x, out, t->M, t->N, t->N / t->G, 0, 0, (t->N + 127) / 128 * 128 + 16 };
         while ((128 << m.gsh) < t->G) m.gsh++;

@@ -542,13 +542,42 @@ def test_group_scaled_int4_on_the_tensor_cores(backend, cpu_libs, M, N, G):
 @pytest.mark.gpu
 @pytest.mark.parametrize("N", [32, 2048, 2080, 8192, 8224, 16384, 16416])
 def test_group_scaled_int4_row_lengths(backend, cpu_libs, N):
-    """Where the fast kernel changes how it holds the activation: one and several groups of eight columns per thread, the last length of
-    each register instance and the first one of the next, the first that is read twice."""
+    """Where the kernels change how they hold the activation: one and several groups of eight columns per thread, the last length of each register
+    instance and the first one of the next; 2048 columns and fewer, and 16416, by dp4a, the others on the tensor cores."""
     rng = np.random.default_rng(N)
     q, s, x, oi, ov = _cpu.make_int4g_case(rng, 50, N, 32, 0)
     got = backend.int4g_matmul(q, s, 32, x, oi, ov, 0.0)
     want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, 32, x, oi, ov, 0.0)
     assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K_out,eps,G", [(3, 0.0, 32), (0, 0.02, 32), (3, 0.02, 32), (0, 0.0, 96), (5, 0.0, 96)])
+@pytest.mark.parametrize("N", [32, 2080, 8192, 8224, 12000, 16384, 16416])
+def test_group_scaled_int4_row_lengths_of_the_dp4a_kernel(backend, cpu_libs, N, K_out, eps, G):
+    """The same lengths with what keeps a call off the tensor cores: outlier columns, the skip rule, groups of 96."""
+    N = -(-N // 96) * 96 if G == 96 else N
+    rng = np.random.default_rng(N + K_out + G)
+    q, s, x, oi, ov = _cpu.make_int4g_case(rng, 51, N, G, K_out)
+    if eps:
+        x[: N // 4] *= 1e-3
+    got = backend.int4g_matmul(q, s, G, x, oi, ov, eps)
+    want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, G, x, oi, ov, eps)
+    assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
+    assert np.array_equal(backend.int4g_matmul(q, s, G, 2.0 * x, oi, ov, eps), 2.0 * got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,G", [(4736, 1024, 64), (4737, 1024, 64), (4750, 160, 32), (4737, 128, 128), (4800, 96, 32), (1184, 2048, 32), (1185, 2048, 32), (1184, 2080, 32),
+                                   (14208, 12320, 32), (14209, 12320, 32), (14209, 12288, 32), (15, 4096, 128), (16, 4096, 64), (2369, 4096, 256), (4753, 4096, 32)])
+def test_group_scaled_int4_kernel_by_size(backend, cpu_libs, M, N, G):
+    """Both sides of the lines between the two kernels, short rows on the tensor cores, and runs of 16 rows a block with a remainder."""
+    rng = np.random.default_rng(M + N + G)
+    q, s, x, oi, ov = _cpu.make_int4g_case(rng, M, N, G, 0)
+    got = backend.int4g_matmul(q, s, G, x, oi, ov, 0.0)
+    want = _cpu.oracle_int4g(cpu_libs.oracle, q, s, G, x, oi, ov, 0.0)
+    assert _cpu.close(got, want, RTOL, ATOL), float(np.max(np.abs(got - want)))
+    assert np.array_equal(backend.int4g_matmul(q, s, G, 2.0 * x, oi, ov, 0.0), 2.0 * got)
 
 
 @pytest.mark.parametrize("bits,Ms,N,B,tc", [
