@@ -462,11 +462,12 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
             }
             // Rows the filter could not decide: all centroids in the exact form, by the whole warp for one row after another, or, where they
             // are many (equal centroids, points on a grid), by every lane for its own row. 1 Mi points that are all undecided, 256 centroids:
-            // 479 -> 178 us for 4 dimensions, 597 -> 287 for 8, 1239 -> 508 for 16 (assign_exact_kernel: 144, 256, 467). As turns of the
+            // 479 -> 181 us for 4 dimensions, 595 -> 288 for 8, 1241 -> 508 for 16 (assign_exact_kernel: 144, 256, 467). As turns of the
             // loop that evaluates the best group it would save the code, but took 204 us instead of 183 per iteration without ties.
             unsigned todo = __ballot_sync(0xffffffffu, have && !sure);
-            if (__popc(todo) > S::each_lane) {
-                todo = 0u;
+            if (todo == 0u) {
+                // nearly always: one test on the way
+            } else if (__popc(todo) > S::each_lane) {
                 win = 0;
                 best = group_sqdist<D>(xr, cgrp, 0);                 // the reference's seed whatever its distance
 #pragma unroll 1
@@ -486,7 +487,7 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                     for (int j = 0; j < 4; j++) if (dk[j] < best) { best = dk[j]; win = k + j; }      // ascending and strict, as the reference goes
                 }
             }
-            while (todo) {
+            else do {
                 const int rl = __ffs(todo) - 1;
                 todo &= todo - 1;
                 float xq[D];
@@ -507,7 +508,7 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
                 bd = __shfl_sync(0xffffffffu, bd, 0);
                 bk = __shfl_sync(0xffffffffu, bk, 0);
                 if (lane == rl) { win = bk; best = bd; }
-            }
+            } while (todo);
             if (have) { idx[row] = win; if (dist) dist[row] = best; }
             if (ACC) {
                 // Points of the warp that share a cluster: the first of them fetches the others' rows, adds them behind its own, in index
