@@ -35,6 +35,7 @@ void* ib_b200_translate(const void* p, size_t bytes);
 int   ib_b200_stage(int slot, size_t bytes, void** host, void** dev);
 void  ib_b200_pq_release_all(void);
 void  ib_b200_kmeans_release(void);
+int   ib_b200_cores(void);
 void  ib_b200_lock(void);
 void  ib_b200_unlock(void);
 #endif

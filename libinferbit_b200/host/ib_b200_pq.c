@@ -6,10 +6,10 @@
 #include "ib_b200_internal.h"
 #include <pthread.h>
 #include <sched.h>
+#include <signal.h>
 #include <stdatomic.h>
 #include <stdlib.h>
 #include <string.h>
-#include <unistd.h>
 
 /* ── PQ tensors cached on the device, keyed by the address of the caller's struct ── */
 #define PQ_CACHE 64
@@ -222,6 +222,19 @@ static void* km_copy_helper(void* arg) {
     return NULL;
 }
 
+/* Helper threads of a copy: no more than the cores this thread may run on (a helper on the caller's core would only yield to it), and with all
+ * signals blocked, so that a handler of the program never runs on one. */
+static int km_helpers_start(pthread_t* helper, km_copy* c) {
+    const int cores = ib_b200_cores();
+    sigset_t all, caller;
+    sigfillset(&all);
+    if (pthread_sigmask(SIG_SETMASK, &all, &caller) != 0) return 0;
+    int n = 0;
+    while (n < KM_HELPERS && n + 1 < cores && pthread_create(&helper[n], NULL, km_copy_helper, c) == 0) n++;
+    pthread_sigmask(SIG_SETMASK, &caller, NULL);
+    return n;
+}
+
 static int km_upload(void* dst, const void* src, size_t bytes) {
     void *h, *d;
     int rc = ib_b200_stage(0, bytes < KM_STAGE ? bytes : KM_STAGE, &h, &d);
@@ -232,9 +245,7 @@ static int km_upload(void* dst, const void* src, size_t bytes) {
     c.done = (atomic_uchar*)calloc((size_t)c.n, sizeof *c.done);
     if (!c.done) return IBCU_ERR_NOMEM;
     pthread_t helper[KM_HELPERS];
-    int helpers = 0;
-    const long cores = sysconf(_SC_NPROCESSORS_ONLN);
-    while (bytes >= KM_SHARED && helpers < KM_HELPERS && helpers + 1 < cores && pthread_create(&helper[helpers], NULL, km_copy_helper, &c) == 0) helpers++;
+    const int helpers = bytes >= KM_SHARED ? km_helpers_start(helper, &c) : 0;
     for (int i = 0; i < c.n && !rc; i++) {
         while (!atomic_load_explicit(&c.done[i], memory_order_acquire)) km_copy_one(&c);
         const size_t off = (size_t)i * KM_PIECE, n = bytes - off < KM_PIECE ? bytes - off : KM_PIECE;

@@ -4,14 +4,24 @@
  * (activations, scales, outputs) through pinned staging buffers and runs the CUDA backend on the
  * device copy of the weights. No compute happens on the host.
  */
+#define _GNU_SOURCE                                /* sched_getaffinity */
 #include "ib_b200_internal.h"
+#include <sched.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 #include <pthread.h>
+#include <unistd.h>
 
 ib_b200_state g_ib;
+
+/* cores the calling thread may run on: its affinity, which is also a container's set of cores */
+int ib_b200_cores(void) {
+    cpu_set_t allowed;
+    CPU_ZERO(&allowed);
+    return sched_getaffinity(0, sizeof allowed, &allowed) == 0 ? CPU_COUNT(&allowed) : (int)sysconf(_SC_NPROCESSORS_ONLN);
+}
 
 /* The reference's pool workers call the table concurrently with row slices of one tensor
  * (src/threading.c:220-241). The staging buffers, the scale cache, the stream and the sticky error are

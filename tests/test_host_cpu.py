@@ -158,3 +158,64 @@ def test_a_stopped_kernel_does_not_run_out_of_time(tmp_path):
     assert r.returncode == 0, (r.returncode, r.stdout)
     code = open(os.path.join(LIB, "csrc", "tc_common.cuh")).read()
     assert "clock.spent(now)" in code
+
+
+HELPERS = r"""
+#define _GNU_SOURCE
+#include <pthread.h>
+#include <sched.h>
+#include <signal.h>
+#include <stdlib.h>
+#include <string.h>
+static int started, open_signals;
+static int counted_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* arg) {
+    sigset_t now;
+    pthread_sigmask(SIG_SETMASK, NULL, &now);                /* what the new thread inherits */
+    started++;
+    if (!sigismember(&now, SIGUSR1) || !sigismember(&now, SIGTERM)) open_signals++;
+    return pthread_create(t, a, f, arg);
+}
+#define pthread_create counted_create
+#include "ib_b200_internal.h"
+static char* area;
+static int fake_stage(int slot, size_t bytes, void** h, void** d) { (void)slot; area = realloc(area, bytes); *h = area; *d = NULL; return 0; }
+static int fake_sync(ibcu_ctx* c) { (void)c; return 0; }
+static int fake_h2d(ibcu_ctx* c, void* dst, const void* src, size_t n) { (void)c; memcpy(dst, src, n); return 0; }
+#define ib_b200_stage fake_stage
+#define ibcu_sync_spin fake_sync
+#define ibcu_memcpy_h2d fake_h2d
+#include "ib_b200_pq.c"
+#include <stdio.h>
+int main(void) {
+    const size_t n = 3 * KM_SHARED + 5;
+    char *src = malloc(n), *dst = malloc(n);
+    for (size_t i = 0; i < n; i++) src[i] = (char)(i * 31);
+    cpu_set_t all, one;
+    if (sched_getaffinity(0, sizeof all, &all)) return 1;
+    const int cores = CPU_COUNT(&all);
+    sigset_t now;
+    if (km_upload(dst, src, n) || memcmp(src, dst, n)) return 2;
+    if (started != (cores - 1 < KM_HELPERS ? cores - 1 : KM_HELPERS)) { printf("%d helpers on %d cores\n", started, cores); return 3; }
+    if (open_signals) { printf("%d helpers take signals\n", open_signals); return 4; }
+    pthread_sigmask(SIG_SETMASK, NULL, &now);
+    if (sigismember(&now, SIGUSR1)) return 5;                /* the caller's own mask is back */
+    int c = 0;
+    while (!CPU_ISSET(c, &all)) c++;
+    CPU_ZERO(&one); CPU_SET(c, &one);
+    if (sched_setaffinity(0, sizeof one, &one)) return 6;
+    started = 0;
+    memset(dst, 0, n);
+    if (km_upload(dst, src, n) || memcmp(src, dst, n)) return 7;
+    if (started) { printf("%d helpers beside the caller on its only core\n", started); return 8; }
+    return 0;
+}
+"""
+
+
+def test_copy_helpers_take_no_signals_and_no_core_that_is_not_there(tmp_path):
+    src, exe = tmp_path / "helpers.c", tmp_path / "helpers"
+    src.write_text(HELPERS)
+    subprocess.run(["gcc", "-std=gnu11", "-O2", "-w", f"-I{ROOT}/include", f"-I{LIB}/host", "-o", str(exe), str(src), f"{LIB}/host/ib_b200_table.c",
+                    f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}", "-lm", "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout)
