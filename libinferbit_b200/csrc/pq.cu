@@ -190,17 +190,17 @@ __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p
     pdl_wait();
     const bool vec_x = (p.N & 3) == 0 && ((uintptr_t)p.x & 15) == 0;
     auto fill_xs = [&](int s0) {                            // this slab's slices of x: subspace s covers x[s * half, (s + 1) * half)
-        if (half == 8) {
+        if constexpr (H8) {
             for (int e = tid; e < BT * 256; e += PQ_THREADS) {
                 const int t = e >> 8, l = (e >> 3) & 31, i = e & 7, s = s0 + l;
                 xs[t][l][i] = (t < nb && s < nsub) ? p.x[(size_t)(b0 + t) * p.N + ((EX && p.inner) ? p.inner[s * 8 + i] : s * 8 + i)] : 0.0f;
             }
-            return;
-        }
-        for (int e = tid; e < BT * 32 * half; e += PQ_THREADS) {
-            const int t = e / (32 * half), r = e - t * 32 * half, l = r / half, i = r - l * half;
-            const int s = s0 + l;
-            xs[t][l][i] = (t < nb && s < nsub) ? p.x[(size_t)(b0 + t) * p.N + ((EX && p.inner) ? p.inner[s * half + i] : s * half + i)] : 0.0f;
+        } else {
+            for (int e = tid; e < BT * 32 * half; e += PQ_THREADS) {
+                const int t = e / (32 * half), r = e - t * 32 * half, l = r / half, i = r - l * half;
+                const int s = s0 + l;
+                xs[t][l][i] = (t < nb && s < nsub) ? p.x[(size_t)(b0 + t) * p.N + ((EX && p.inner) ? p.inner[s * half + i] : s * half + i)] : 0.0f;
+            }
         }
     };
     // ── max |x| of each activation (the reference's 1 %-of-max rule and the fixed-point scale need it), as the
