@@ -3,6 +3,7 @@
 // residual add, softmax. They move O(hidden) or O(context) bytes per token; the design goal is few
 // launches and programmatic-dependent-launch friendliness, not bandwidth.
 #include "common.cuh"
+#include <algorithm>
 #include <type_traits>
 
 namespace {
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(32 * ATT_GMAX) attn_partial_kernel(const float
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    pdl_launch_dependents();                         // not earlier: the weights that the launches behind ask for would be ahead of this tile (decode step 1785 -> 1766 us)
+    pdl_launch_dependents();                         // not earlier: the weights that the launches behind ask for would be ahead of this tile (a decode step at 512 took 1785 us and 1766; since the linears lost their exchange code 1782 either way)
     const float scale = 1.0f / sqrtf((float)hd);
     const float4* q4 = reinterpret_cast<const float4*>(qs + g * hd);
     const int hd4 = hd / 4, ld4 = ld / 4;
@@ -688,6 +689,8 @@ static int attention_split(ibcu_ctx* ctx, const float* q, float* k_cache, float*
         att_plan(max_ctx, want, ATT_CHUNK, chunk, nsplit);     // longest context: most chunks, longest chunks
         grid_y = nsplit > n_lo ? nsplit : n_lo;
         if (want > grid_y) grid_y = want;
+        // few KV heads: no context has more chunks than of 32 positions, and the merge step may not hold as many as are wanted
+        if (combine_smem(head_dim, grid_y) > ATT_CMB_SMEM) grid_y = std::max(nsplit, std::max(n_lo, std::min(want, (max_ctx + 31) / 32)));
         chunk_cap = chunk;
         if (chunk_cap < 32) chunk_cap = 32;
     } else {

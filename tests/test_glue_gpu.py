@@ -173,6 +173,32 @@ def test_attention_of_a_long_context(backend, n_heads, n_kv, hd, pos0, B, entry)
         assert np.allclose(got[:, h], (p / p.sum(axis=1, keepdims=True)) @ vals[:, kv], rtol=RTOL, atol=ATOL)
 
 
+@pytest.mark.parametrize("n_heads,n_kv,hd,max_ctx", [(8, 2, 128, 1152), (4, 1, 64, 300), (2, 1, 256, 4000), (8, 1, 128, 6000)])
+@pytest.mark.parametrize("B", [1, 2, 3])
+def test_attention_of_few_kv_heads_at_a_device_position(backend, n_heads, n_kv, hd, max_ctx, B):
+    """Few KV heads want more blocks than there are chunks in any context, more than the merge step holds: the launch that serves every position is cut to
+    the chunks there can be, and gives what the launch for one position gives."""
+    be, lib, H, kv = backend, backend.lib, n_heads * hd, n_kv * hd
+    rng = np.random.default_rng(n_heads + hd + B)
+    draw = lambda *shape: rng.standard_normal(shape, dtype=np.float32)
+    q, k, v, kc, vc = draw(B, H), draw(B, kv), draw(B, kv), draw(max_ctx, kv), draw(max_ctx, kv)
+    for pos0 in (0, 60, max_ctx // 3, max_ctx - B):
+        got = []
+        for at in (True, False):
+            d = [be.upload(x) for x in (q, k, v, kc, vc)] + [be.alloc(B * H * 4), be.upload(np.array([pos0], np.int32))]
+            p = [b.ptr for b in d]
+            if at:
+                be._check(lib.ibcu_attention_decode_at(be.ctx, *p[:6], n_heads, n_kv, hd, p[6], max_ctx, B, 10000.0))
+            else:
+                be._check(lib.ibcu_attention_decode(be.ctx, *p[:6], n_heads, n_kv, hd, pos0, B, 10000.0))
+            be.sync()
+            got.append((be.download(d[5], np.float32, B * H), be.download(d[3], np.float32, max_ctx * kv)))
+            for b in d:
+                b.free(); be._bufs.remove(b)
+        assert np.allclose(got[0][0], got[1][0], rtol=RTOL, atol=ATOL), pos0
+        assert np.array_equal(got[0][1], got[1][1]), pos0
+
+
 @pytest.mark.parametrize("entry", ["attention", "decode"])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 @pytest.mark.parametrize("n_heads,n_kv,hd,pos0,B,at", [(8, 2, 64, 0, 6, 3), (4, 4, 128, 29, 9, 1), (4, 1, 256, 60, 8, 7), (8, 8, 64, 0, 40, 33),
