@@ -187,14 +187,15 @@ typedef struct { void *X, *C, *idx, *dist, *sums, *counts, *inertia, *shift; } k
 
 /* Pageable arrays go through the pinned staging area in pieces, so that pieces are on their way while others are copied
  * (the driver's own path for pageable memory copies and transfers one after the other). One core copies 17 GB/s, a third of
- * what the bus takes, so helper threads of the call share the copying of large arrays: one iteration over 262147 points of 16
- * 1572 -> 860 us. Starting and ending the three costs about 250 us, so arrays of less than 8 MB stay with the caller (262147
- * points of 4: 458 us, with helpers 709). CUDA calls are the caller's alone. The result area is separate. */
+ * what the bus takes, so helper threads of the call share the copying of large arrays. Starting and ending the three costs some
+ * 300 us, so arrays of less than 16 MB stay with the caller. One iteration over points of 16 and 64 clusters, alone / with helpers, us: 8 MB
+ * 612 / 914, 12 MB 892 / 1070, 16 MB 1168 / 823, 20 MB 1452 / 1429, 32 MB 2300 / 1571, 64 MB 5300 / 3195. CUDA calls are the
+ * caller's alone. The result area is separate. */
 #define KM_PIECE ((size_t)256 << 10)
 #define KM_STAGE ((size_t)16 << 20)
 #define KM_AREA ((int)(KM_STAGE / KM_PIECE))       /* pieces the staging area holds */
 #define KM_HELPERS 3
-#define KM_SHARED ((size_t)8 << 20)               /* arrays from here on are copied by several threads */
+#define KM_SHARED ((size_t)16 << 20)              /* arrays from here on are copied by several threads */
 
 typedef struct {
     char* stage; const char* src;
