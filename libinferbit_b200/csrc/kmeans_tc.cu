@@ -16,7 +16,7 @@
 //   finish (12 warps)      the best group in the exact form, results, and the point into its cluster's sums
 // A Lloyd iteration over 4 Mi points of 8 with 256 centroids: 183 us (285 with scan and finish in the same eight warps, whose chains of
 // TMEM loads, exact step and turns of equal clusters two warps per scheduler did not hide; 202 with eight finishing warps, 209 with votes
-// in place of match); 4 Mi of 4: 162 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 101 (582). What bounds it now
+// in place of match); 4 Mi of 4: 152 (652 on the CUDA cores, with a second pass to accumulate); 1 Mi of 16: 100 (582). What bounds it now
 // is the pipe for comparisons and logic, some 500 instructions per scheduler and tile, with issue slots close behind.
 //
 // The scores only FILTER. If the best group leads by more than 1.25 * 2^-16 (|x|^2 + max |c|^2), the reference's nearest centroid lies in
@@ -290,8 +290,9 @@ assign_tc_kernel(const float* X, long N, const float* C, int K, int32_t* __restr
     const uint32_t tmem_base = sh->tmem_base;
 
     if (warp >= LOAD0) {
-        // ── loaders: warp lw owns pipeline lw: raw rows by cp.async (one or two of its tiles ahead), the two FP16 terms into the operand stage, and the MMAs. (One warp issuing for
-        //    all accumulators was a chain of 1000 cycles per tile: two waits, two issues and three commits one after the other.) ──
+        // ── loaders: warp lw owns pipeline lw: raw rows by cp.async (one or two of its tiles ahead), the two FP16 terms into the operand
+        //    stage, and the MMAs. (One warp issuing for all accumulators was a chain of 1000 cycles per tile: two waits, two issues and
+        //    three commits one after the other.) ──
         const int lw = warp - LOAD0;
         const uint32_t a0 = smem_u32(sA + lw * S::a_stage), b0 = smem_u32(sB), aug = smem_u32(sAug), acc = tmem_base + (uint32_t)(lw * TC_ACC_COLS);
         bool ok = true;

@@ -123,7 +123,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // is enough (76 registers; the one with 8 takes 120): hidden size 4096, one token, 8-bit projections of 12 layers 171.8 -> 161.1 us; 2048:
 // 128.1 -> 115.6. Two blocks fill an SM's shared memory with either, so it is not room for a third; what else it is was not measured apart.
 // MG: the launch waits for rows of peers or pushes its own to them. Without that code, which a single GPU never runs, projections of a
-// 7B shape took 206 us instead of 216 (INT8, one activation, sixteen layers), a decode step 1812 instead of 1857.
+// 7B shape took 204 us instead of 214 (INT8, one activation, sixteen layers), a decode step 1779 instead of 1819.
 template <int BITS, int NCG, int RT, int W, int STAGES, int XV, bool MG>
 __global__ void __launch_bounds__(W * 32) linear_mma_kernel(const LinearParams p) {
     constexpr int R = RT * 16;                                // most rows per tile

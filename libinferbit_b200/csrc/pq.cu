@@ -800,7 +800,9 @@ __global__ void __launch_bounds__(TOPK_THREADS) pq_topk_select_kernel(const floa
 // Where they are more than TOPK_RANK, the K_top-th largest key itself is searched for, among the rows found or, beyond TOPK_FOUND, among
 // all, read again: halves of what is left between the bound and the largest key, either end moving on to the next key that there is (rows of a
 // few different logits take a step or two). Rows above it are taken, and of those equal to it the lowest.
-// 32000 rows, 64 chosen: the whole call 41.3 -> 32.6 us against the cluster below, whose rounds each cost two cluster barriers.
+// 32000 rows, 64 chosen: the whole call 41.3 -> 29.3 us against the cluster below, whose rounds each cost two cluster barriers (and with the
+// order by counting). Up to 65536 rows a thread reads at most twice what it holds: 64000 rows 69.9 -> 36.8; beyond, and for more rows chosen than 256,
+// which would leave a thread's largest key too coarse a bound, the cluster.
 constexpr int TOPK_QUICK = 256, TOPK_HELD = 32, TOPK_RANK = 384, TOPK_FOUND = 2048;
 __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const float* coarse, int M, int K_top, int32_t* cand) {
     __shared__ unsigned n_found, n_taken, warp_cnt[2][32], warp_low[2][32], warp_high[2][32];

@@ -23,7 +23,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 }
 // Bounded wait. Returns false when the block is giving up (this wait ran out, or another role's did). A phase that is complete
 // already is seen by the plain test in 65 cycles; the try takes 112 to say so. (Where phases are rarely complete the
-// test only delays the try: k-means takes the wait without it, 2864 against 2850 us.)
+// test only delays the try: k-means takes the wait without it, ten iterations 1844 against 1830 us.)
 template <bool TEST = true>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
     if (TEST && mbar_test(bar, parity)) return true;
