@@ -801,8 +801,7 @@ __global__ void __launch_bounds__(TOPK_THREADS) pq_topk_select_kernel(const floa
 // all, read again: halves of what is left between the bound and the largest key, either end moving on to the next key that there is (rows of a
 // few different logits take a step or two). Rows above it are taken, and of those equal to it the lowest.
 // 32000 rows, 64 chosen: the whole call 41.3 -> 29.3 us against the cluster below, whose rounds each cost two cluster barriers (and with the
-// order by counting). Up to 65536 rows a thread reads at most twice what it holds: 64000 rows 69.9 -> 36.8; beyond, and for more rows chosen than 256,
-// which would leave a thread's largest key too coarse a bound, the cluster.
+// order by counting).
 constexpr int TOPK_QUICK = 256, TOPK_HELD = 32, TOPK_RANK = 384, TOPK_FOUND = 2048;
 __global__ void __launch_bounds__(TOPK_THREADS, 1) pq_topk_quick_kernel(const float* coarse, int M, int K_top, int32_t* cand) {
     __shared__ unsigned n_found, n_taken, warp_cnt[2][32], warp_low[2][32], warp_high[2][32];
@@ -1199,6 +1198,10 @@ extern "C" int ibcu_pq_lm_head_topk(ibcu_ctx* ctx, const ibcu_pq_t* t, const flo
     float* refined = (float*)(cand + TOPK_MAX);
     rc = pq_launch(ctx, t, x, coarse, t->M, 1, pl, (unsigned long long*)((char*)ctx->pq_acc + PQ_COUNTER_BYTES), (unsigned int*)ctx->pq_acc, true);
     if (rc) return rc;
+    // Quick choice / cluster, whole call, us (one level, 1024 columns). Beyond 65536 rows what the one block reads again for every step of a search weighs:
+    // random logits, 64 chosen: 64000 rows 36 / 70, 128256 61 / 88, 262144 109 / 129; falling logits 43 / 58, 69 / 70, 117 / 98; the largest in a few threads
+    // 61 / 66, 107 / 95, 200 / 185. More rows chosen, 64000 rows, random / falling: 384 57 / 80 and 46 / 67, 512 59 / 78 and 92 / 65, 1000 180 / 102 and 142 / 88.
+    // The lines keep it to where no kind of logits takes much longer; rows that differ well would gain from it up to 262144 rows and 384 chosen.
     if (K_top <= TOPK_QUICK && t->M <= 64 * TOPK_THREADS)
         rc = ibcu_launch(ctx, pq_topk_quick_kernel, dim3(1), dim3(TOPK_THREADS), 0, 1, true, (const float*)coarse, t->M, K_top, cand);
     else if (t->M <= 4 * TOPK_CL * TOPK_THREADS)
