@@ -21,9 +21,7 @@
 // and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
 // activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4 (the INT4 instance of one tile spills 32 bytes a thread); at 32 the digits, which every SM reads from L2,
 // bound the kernel (26 us, 75 MB of them).
-// The weights do not depend on the kernel ahead: their ring fills before the dependency wait. With at most 128 rows per run a
-// block takes no more than half of an SM's shared memory and tensor memory, so that the next launch's blocks move in beside it
-// and have their weights under way while this launch ends.
+// The weights do not depend on the kernel ahead: their ring fills before the dependency wait.
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "xconvert.cuh"
@@ -506,11 +504,15 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     // up to 128 stay exact for 131071 (1118481) columns; rows with longer parts go to the kernel that cuts them into slices
     const long part_cols = (long)((p.nkb + S - 1) / S) * 128;
     if ((part_cols < N ? part_cols : N) * (bits == 8 ? 128L : 15L) * 128L > 0x7fffffffL) return IBCU_DECLINED;
-    // shared memory: half an SM's for runs of one tile, so that consecutive launches overlap; tensor memory likewise
+    // Shared memory: the rings take what an SM has. A block of runs of one tile used to keep to half, so that the next launch's blocks move in beside
+    // it, but what a block of columns costs is the way of its weights and digits from L2, and with twice the ring twice as many are on it:
+    // 4096 x 14336 INT4 at 4, 16 and 32 activations 15.0 -> 13.1, 18.1 -> 17.2, 25.3 -> 20.7 us, 6144 x 4096 INT8 at 4 and 32 9.9 -> 9.2,
+    // 17.6 -> 16.0. INT8 at 9 to 20 activations is where the overlap is worth as much (6144 x 4096 at 12 13.3 against 13.7, 4096 x 4096 at 16 9.4
+    // against 9.6) and keeps it.
     const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;
     while (p.tmem_cols < tcols) p.tmem_cols *= 2;
-    const size_t cap = (T == 1 ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
+    const size_t cap = (T == 1 && bits == 8 && p.NC > 32 && p.NC <= 80 ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
     const size_t b_block = (size_t)p.NC * 128;
     p.a_stage = R * (bits == 8 ? 128 : 64);
     const int nk = (p.nkb + S - 1) / S;
