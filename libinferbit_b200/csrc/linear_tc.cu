@@ -16,11 +16,12 @@
 // No warp polls a barrier while it would have to poll until the kernel ahead has ended: everyone sleeps in the dependency wait.
 // (When the warps of weights and MMAs polled their barriers meanwhile, with suspended tries, the end of the kernel ahead was in
 // rare cases - once in tens of thousands of launches - not delivered until they gave up.)
-// Workers (INT4 widening, then epilogue): eight warps per tile of 128 rows, in two teams that take the blocks of columns in turn;
+// Workers (INT4 widening, then epilogue): four warps per tile of 128 rows and team; the teams take the blocks of columns in turn;
 // then one warp each for the weights (TMA), the digits (bulk copies) and the MMAs. What a block of columns costs a warp is waits
 // and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
-// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4 (the INT4 instance of one tile spills 32 bytes a thread); at 32 the digits, which every SM reads from L2,
-// bound the kernel (26 us, 75 MB of them).
+// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4; at 32 the digits, which every SM reads from L2,
+// bound the kernel (26 us, 75 MB of them). Four teams where a run has one tile: 4096 x 4096 INT4 at 4, 16 and 32 activations 8.3 -> 7.5, 9.2 -> 8.9,
+// 12.4 -> 11.5, 2560 x 6400 at 32 14.3 -> 13.3, 4096 x 14336 at 32 20.7 -> 19.8.
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait.
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -32,8 +33,10 @@ void ibcu_push_fill(ibcu_ctx* ctx, GatherPush* gp, size_t bytes);
 
 namespace {
 
-// Warps of a block whose runs have T tiles: 8 T workers, then one each for the weights, the digits and the MMAs.
-template <int T> struct Tq { static constexpr int WORKERS = 8 * T, A_WARP = WORKERS, B_WARP = WORKERS + 1, MMA_WARP = WORKERS + 2, THREADS = (WORKERS + 3) * 32; };
+// Warps of a block whose runs have T tiles: Q teams of 4 T workers, then one each for the weights, the digits and the MMAs.
+template <int T, int Q> struct Tq { static constexpr int WORKERS = 4 * T * Q, A_WARP = WORKERS, B_WARP = WORKERS + 1, MMA_WARP = WORKERS + 2, THREADS = (WORKERS + 3) * 32; };
+// INT4 runs of one tile have room for four teams (16 workers); two tiles fill the block with two, and INT8 weights need none
+constexpr int tq_teams(int bits, int T) { return bits == 4 && T == 1 ? 4 : 2; }
 constexpr int TQ_MAX_STAGES = 12;
 constexpr int TQ_MAX_B = 32;
 
@@ -103,15 +106,16 @@ __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, i
     xconvert_any(src, N, b, c0, min(part_cols, all_cols - c0), dst, perm8, sc, xscale + b * gridDim.x + part, xsum + ((size_t)b * gridDim.x + part) * LIN_LIMBS);
 }
 
-// BITS 4 or 8; T: 128-row tiles per run; MG: see linear.cu
-template <int BITS, int T, bool MG>
-__global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
+// BITS 4 or 8; T: 128-row tiles per run; Q: teams of workers; MG: see linear.cu
+template <int BITS, int T, int Q, bool MG>
+__global__ void __launch_bounds__(Tq<T, Q>::THREADS, T * Q == 2 ? 2 : 1) linear_tc_kernel(const __grid_constant__ TqMaps maps, const __grid_constant__ TqParams p) {
     extern __shared__ __align__(1024) unsigned char tq_smem[];
     constexpr int NT = 4;                                      // INT4: widened blocks in tensor memory
-    constexpr int TQ_WORKERS = Tq<T>::WORKERS, TQ_A_WARP = Tq<T>::A_WARP, TQ_B_WARP = Tq<T>::B_WARP, TQ_MMA_WARP = Tq<T>::MMA_WARP, TQ_THREADS = Tq<T>::THREADS;
-    // INT4: two teams of workers, a warp per 32 rows, widen alternate blocks of columns. A warp's way from the nibbles to the MMA is
-    // a chain of waits and latencies (about 1300 cycles measured, a few hundred of them work), and two chains run side by side.
-    constexpr int TW = TQ_WORKERS / 2;
+    using W = Tq<T, Q>;
+    constexpr int TQ_WORKERS = W::WORKERS, TQ_A_WARP = W::A_WARP, TQ_B_WARP = W::B_WARP, TQ_MMA_WARP = W::MMA_WARP, TQ_THREADS = W::THREADS;
+    // INT4: Q teams of workers, a warp per 32 rows, widen every Q-th block of columns. A warp's way from the nibbles to the MMA is
+    // a chain of waits and latencies (about 1300 cycles measured, a few hundred of them work), and Q chains run side by side.
+    constexpr int TW = TQ_WORKERS / Q;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = p.S, rank = (int)blockIdx.x % S, cl = (int)blockIdx.x / S, ncl = (int)gridDim.x / S;
     const int nruns = p.run_start[p.n_tensors];
@@ -264,7 +268,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
             if (BITS == 4) {
                 const uint32_t rawrow = (uint32_t)rl * 64u, sw = (uint32_t)((rl >> 1) & 3);
                 const bool have = rt * 128 + q * 32 < p.R;                              // the box has rows for this warp
-                for (; next < nk; next += 2) {
+                for (; next < nk; next += Q) {
                     if (!waited && next >= NT) { pdl_wait(); waited = true; }           // the first widened blocks do not need the digits; the next wait for them to be used
                     if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_a[s]), phA, abort_flag, 8))) { alive = false; break; }
                     uint32_t o[32];
@@ -289,9 +293,9 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[sT]));
-                    s += 2;
+                    s += Q;
                     if (s >= p.sa) { s -= p.sa; phA ^= 1; }
-                    sT += 2;
+                    sT += Q;
                     if (sT >= NT) { sT -= NT; phT ^= 1; }
                 }
                 next -= nk;
@@ -317,7 +321,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
                 const unsigned tag = MG ? tag_current(p.gp) : 0u;
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_acc), (uint32_t)(j & 1), abort_flag, 10))) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int g = team; g * 4 < p.B; g += 2) {
+                for (int g = team; g * 4 < p.B; g += Q) {
                     uint32_t acc[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
                     float* o = W.out + (size_t)(g * 4) * W.out_stride + row;
@@ -363,7 +367,7 @@ __global__ void __launch_bounds__(Tq<T>::THREADS, T == 1 ? 2 : 1) linear_tc_kern
         if (warp < TQ_WORKERS && !*abort_flag) {
             const int q = warp & 3, rt = (warp >> 2) % T, team = warp / (4 * T), rl = rt * 128 + q * 32 + lane;
             if (rt * 128 + q * 32 < rows) {
-                for (int g = team; g * 4 < p.B; g += 2) {
+                for (int g = team; g * 4 < p.B; g += Q) {
                     uint32_t acc[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rt * p.NC + g * 16), acc);
 #pragma unroll
@@ -430,17 +434,18 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-template <int BITS, int T, bool MG>
+template <int BITS, int T, int Q, bool MG>
 int launch_tc_mg(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
-    auto kern = linear_tc_kernel<BITS, T, MG>;
+    auto kern = linear_tc_kernel<BITS, T, Q, MG>;
     static SmemOptIn opt;
     if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
-    return ibcu_launch(ctx, kern, dim3(grid), dim3(Tq<T>::THREADS), smem, p.S, true, maps, p);
+    return ibcu_launch(ctx, kern, dim3(grid), dim3(Tq<T, Q>::THREADS), smem, p.S, true, maps, p);
 }
 
 template <int BITS, int T>
 int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
-    return p.gp.world ? launch_tc_mg<BITS, T, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, false>(ctx, maps, p, grid, smem);
+    constexpr int Q = tq_teams(BITS, T);
+    return p.gp.world ? launch_tc_mg<BITS, T, Q, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, Q, false>(ctx, maps, p, grid, smem);
 }
 
 }  // namespace
@@ -547,11 +552,12 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
         if (recv > ring_of() || p.sa < 1) return IBCU_DECLINED;
         smem = ring_of();
     }
-    if (bits == 4 && p.sa < nk) {
-        // a ring that is used again: an even one, so that a stage always belongs to the same team of widening warps (a warp that
+    if (bits == 4 && (p.sa < nk || nruns > slots)) {
+        // a ring that is used again: a multiple of the teams, so that a stage always belongs to the same team of widening warps (a warp that
         // misses every other phase of a barrier cannot tell a phase from the next but one)
-        if (p.sa < 2) return IBCU_DECLINED;
-        p.sa &= ~1;
+        const int teams = tq_teams(bits, T);
+        if (p.sa < teams) return IBCU_DECLINED;
+        p.sa -= p.sa % teams;
         if (!p.recv_off && recv > ring_of()) return IBCU_DECLINED;
         smem = p.recv_off ? smem : ring_of();
     }
