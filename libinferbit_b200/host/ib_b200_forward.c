@@ -301,12 +301,13 @@ static int issue(ib_b200_model* m, int pos0, int B, int head_last) {
         lin* gu[2] = { &y->t[IB_B200_GATE], &y->t[IB_B200_UP] };
         float* gu_out[2] = { m->hg, m->hu };
         if (!rc) rc = linear_group(m, gu, gu_out, 2, m->x, H, B, &n2, IBCU_EPI_STORE);
-        /* silu(gate) * up (src/forward.c:637-640) in one small launch that also leaves max|h| for down_proj,
-         * whose blocks then turn h into their integer operand without a reduction of their own */
-        if (!rc) rc = ibcu_silu_mul_amax(ctx, m->hg, m->hg, m->hu, c->inter, B, m->amax, AMAX_PARTS);
-        ibcu_prologue_t km = { IBCU_PRO_KNOWN_MAX, NULL, NULL, 0.0f, m->amax, AMAX_PARTS };
+        /* silu(gate) * up (src/forward.c:637-640): with many positions, whose digits a launch of their own prepares anyway, in that launch; else
+         * in a small one that also leaves max|h|, so that down_proj's blocks turn h into their operand without a reduction of their own */
+        const int prepared = B > 16;
+        if (!rc && !prepared) rc = ibcu_silu_mul_amax(ctx, m->hg, m->hg, m->hu, c->inter, B, m->amax, AMAX_PARTS);
+        ibcu_prologue_t km = { IBCU_PRO_KNOWN_MAX, NULL, NULL, 0.0f, m->amax, AMAX_PARTS }, sm = { IBCU_PRO_SILU_MUL, m->hu, NULL, 0.0f, NULL, 0 };
         lin* dn[1] = { &y->t[IB_B200_DOWN] };
-        if (!rc) rc = linear_group(m, dn, xo, 1, m->hg, c->inter, B, &km, IBCU_EPI_ADD);
+        if (!rc) rc = linear_group(m, dn, xo, 1, m->hg, c->inter, B, prepared ? &sm : &km, IBCU_EPI_ADD);
     }
     ibcu_prologue_t nf = { IBCU_PRO_RMSNORM, NULL, (const uint16_t*)m->final_norm, c->eps, NULL, 0 };
     lin* hd[1] = { &m->head }; float* lg[1] = { m->logits };

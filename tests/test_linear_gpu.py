@@ -5,7 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from libinferbit_b200 import LinearT
+from libinferbit_b200 import LinearT, _ffi
 from tests import _cpu
 
 pytestmark = pytest.mark.gpu
@@ -614,3 +614,54 @@ def test_linear_kernel_by_cost(backend, bits, Ms, N, B, tc):
     assert n == want_n and np.array_equal(got, want)
     if tc:
         assert n == 2
+
+
+@pytest.mark.parametrize("M,N,B", [(130, 5 * 128, 2), (4096, 9 * 128, 7), (4000, 14336, 32), (2600, 6432, 12), (300, 23 * 128, 32), (40000, 11 * 128, 3)])
+def test_tcgen05_int4_four_teams(backend, M, N, B):
+    """Runs of one tile: blocks of columns that are not a multiple of the four teams of widening warps, rings shorter than a part of the
+    columns, clusters of one to eight blocks (the last shape: two tiles, two teams, several runs a block). Bound as above."""
+    rng = np.random.default_rng(M + N + B)
+    w, s16, x = _cpu.make_int4_case(rng, M, N, B)
+    backend.lib.ibcu_linear_use_tcgen05(backend.ctx, 2)
+    try:
+        got = backend.linear(w, s16, x, 4)
+    finally:
+        backend.lib.ibcu_linear_use_tcgen05(backend.ctx, 0)
+    sc = s16.view(np.float16).astype(np.float64)
+    v = np.stack([w & 15, w >> 4], axis=-1).reshape(M, N).astype(np.float32) - 8
+    want = (x.astype(np.float64) @ v.T.astype(np.float64)) * sc
+    bound = 2.0 ** -22 * np.abs(want) + 2.0 ** -30 * np.abs(x).max(axis=1, keepdims=True).astype(np.float64) * (np.abs(v).sum(axis=1, dtype=np.float64) * sc)
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("op", ["plain", "norm", "silu"])
+@pytest.mark.parametrize("N,B", [(32, 17), (2048, 32), (2080, 5), (4128, 17), (6176, 32), (8224, 18), (16384, 20), (16416, 17)])
+def test_tcgen05_digits_prepared_by_clusters(backend, bits, op, N, B):
+    """Digits by one to eight blocks per activation (the last length: one block): parts that end inside the last 128 columns or have none, every
+    prologue. Bound: the prologue rounds an activation to FP32 a few times (silu: exponential, division, product; the norm's sum of squares is a
+    tree of at most 8 + 5 + 3 + 3 additions), 32 units in the last place hold all of it; the rest as above."""
+    M, be = 70, backend
+    rng = np.random.default_rng(N + B + bits)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    x2 = rng.standard_normal((B, N)).astype(np.float32)
+    nw = _cpu.fp16_bits(rng.uniform(0.2, 3.0, N))
+    x64 = x.astype(np.float64)
+    act = {"plain": x64, "silu": x64 / (1.0 + np.exp(-x64)) * x2,
+           "norm": x64 / np.sqrt((x64 ** 2).mean(axis=1, keepdims=True) + float(np.float32(1e-5))) * nw.view(np.float16).astype(np.float64)}[op]
+    dw, ds, dx, dx2, dn, do = be.upload(w), be.upload(s16), be.upload(x), be.upload(x2), be.upload(nw), be.upload(np.zeros((B, M), np.float32))
+    t = LinearT(dw.ptr, ds.ptr, do.ptr, M, M, 0, 0)
+    pro = _ffi.PrologueT()
+    pro.op, pro.x2, pro.norm_w, pro.eps = {"plain": 0, "norm": 1, "silu": 2}[op], dx2.ptr, dn.ptr, 1e-5
+    be.lib.ibcu_linear_use_tcgen05(be.ctx, 2)
+    try:
+        be._check(be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.ptr, N, B, bits, C.byref(pro)))
+    finally:
+        be.lib.ibcu_linear_use_tcgen05(be.ctx, 0)
+    be.sync()
+    got = be.download(do, np.float32, B * M).reshape(B, M)
+    v = w.astype(np.float64) if bits == 8 else np.stack([w & 15, w >> 4], axis=-1).reshape(M, N).astype(np.float64) - 8
+    sc = s16.view(np.float16).astype(np.float64)
+    want = (act @ v.T) * sc
+    bound = 2.0 ** -22 * np.abs(want) + 2.0 ** -30 * np.abs(act).max(axis=1, keepdims=True) * (np.abs(v).sum(axis=1) * sc) + 32 * 2.0 ** -24 * (np.abs(act) @ np.abs(v).T) * sc
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
