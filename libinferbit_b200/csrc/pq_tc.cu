@@ -16,19 +16,33 @@
 //                64 columns at a time (four MMAs), joined in FP32 outside, and units are added with compensation. Parts of a row
 //                meet in the fixed-point accumulators of pq.cu. (Over 256 columns at a time the error was 3.4e-7 of the result's
 //                root mean square, over 128 1.9e-7, now 1.25e-7; the tables' 1.0e-7.)
-//   warps 24-26  codes (cp.async), operand image (bulk copies), MMA issue
+//   warps 24-26  codes (cp.async), operand image (bulk copies), MMA issue; a 28th warp fills their warpgroup
 // What bounds it: the latency of every role's chain of waits, not a pipe (a unit takes about 1300 cycles of which the entries
-// keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500; 864 threads leave 72 registers each, so every
-// instance spills, 36 to 364 bytes of stores: part of those waits), and about 7 us around the units: the preparation, staging the codebooks, and the meeting of the parts. 4096 x 14336, entries of eight, 24 tensors in turn: eight
-// activations 28.1 -> 21.2 us, sixteen 46 -> 27; 4096 x 8192 with entries of four at eight 49 -> 17.6, of sixteen 37 -> 23, with a
-// second level 45 -> 22.
+// keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500), and about 7 us around the units: the preparation, staging the codebooks, and the meeting of the parts. 4096 x 14336, entries of eight, 24 tensors in turn: eight
+// activations 28.1 -> 18 us, sixteen 46 -> 24; 4096 x 8192 with entries of four at eight 49 -> 17.3, of sixteen 37 -> 15, with a
+// second level 45 -> 19.
 #include "tc_common.cuh"
 #include "common.cuh"
 #include "pq_tc.cuh"
 
 namespace {
 
-constexpr int PT_TEAM = 8, PT_WORKERS = 2 * PT_TEAM, PT_SUMMERS = 8, PT_SUM_WARP = 16, PT_CODE_WARP = 24, PT_X_WARP = 25, PT_MMA_WARP = 26, PT_THREADS = 27 * 32;
+constexpr int PT_TEAM = 8, PT_WORKERS = 2 * PT_TEAM, PT_SUMMERS = 8, PT_SUM_WARP = 16, PT_CODE_WARP = 24, PT_X_WARP = 25, PT_MMA_WARP = 26, PT_THREADS = 28 * 32;       // the last warp only completes a warpgroup
+// Registers a thread by role (launched with PT_REGS each). With the same for all, every instance spilled 36 to 352 bytes of stores in its loops, and with
+// an SM's shared memory full there is little L1 to spill to. The helpers give up what the sums or, for entries of eight and up to eight
+// activations, the workers are short of (4 to 64 bytes are left): 4096 x 14336 at 3, 8 and 16 activations 18.4 -> 16.3, 20.4 -> 18.0, 26.7 -> 24.0 us, 4096 x 8192
+// with entries of sixteen at 1, 8 and 16 16.9 -> 12.3, 22.0 -> 15.1, 23.5 -> 19.0, with a second level 23.7 -> 19.1. Entries of four keep the even split (17.3;
+// 18.6 with 80 for workers and sums and 24 for the helpers).
+constexpr int PT_REGS = 72;
+template <int HALF, int NG> struct PtRegs {
+    static constexpr bool NARROW = HALF == 8 && NG == 1;
+    static constexpr int WORKER = HALF != 4 && NARROW ? 80 : 72, SUMMER = HALF == 4 ? 72 : (NARROW ? 64 : 88), HELPER = HALF == 4 ? 72 : (NARROW ? 56 : 40);
+    static_assert(PT_WORKERS * WORKER + PT_SUMMERS * SUMMER + 4 * HELPER == 28 * PT_REGS, "what the block is launched with");
+};
+template <int N> __device__ __forceinline__ void pt_set_regs() {
+    if constexpr (N > PT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N));
+    if constexpr (N < PT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N));
+}
 constexpr int PT_GROUP = 528;                                // bytes of a staged group of 16 rows x 32 codes: 16 more than it has, so that the two groups of a warp sit in different banks
 constexpr int PT_SLAB = 8 * PT_GROUP;
 constexpr int PT_MAX_X = 6, PT_MAX_C = 6, PT_MAXSEG = 8;
@@ -157,7 +171,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
     }
     __syncthreads();
 
-    if (warp == PT_CODE_WARP) {
+    if (warp >= PT_CODE_WARP) {
+        pt_set_regs<PtRegs<HALF, NG>::HELPER>();
+        if (warp == PT_CODE_WARP) {
         // the codes do not depend on the kernel ahead: the ring fills at once
         int s = 0; uint32_t ph = 1;
         for (int item = lo; item < hi; item++) {
@@ -176,26 +192,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
-    } else {
-        // the codebooks into the copies
-        const int t0 = warp < PT_CODE_WARP ? tid : tid - 32;
-        constexpr int NT = PT_THREADS - 32;
-        auto stage = [&](const __half* l, const __half* r, int k_have, int rows, int off) {
-            for (int e = t0; e < rows * 2 * PLANES; e += NT) {
-                const int k = e / (2 * PLANES), side = (e / PLANES) & 1, plane = e % PLANES;
-                const __half* src = (side ? r : l) + (size_t)k * HALF + plane * 8;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (k < k_have) {
-                    if constexpr (HALF == 4) { const uint2 w = *reinterpret_cast<const uint2*>(src); v = make_uint4(w.x, w.y, w.x, w.y); }
-                    else v = *reinterpret_cast<const uint4*>(src);
-                }
-                uint4* dst = reinterpret_cast<uint4*>(pt_smem + off + (size_t)k * ROW + side * 128 * PLANES + plane * 128);
-#pragma unroll
-                for (int c = 0; c < 8; c++) dst[(c + t0) & 7] = v;              // lanes start at different copies: 128 bytes apart they would share banks
-            }
-        };
-        stage(p.cb_l, p.cb_r, p.K, 256, p.tab_off);
-        if (p.rows2) stage(p.cb2_l, p.cb2_r, p.K2, p.rows2, p.tab2_off);
+        } else {
         if (warp == PT_MMA_WARP) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)p.tmem_cols) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -204,11 +201,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         asm volatile("bar.sync 1, %0;" :: "n"(PT_THREADS - 32) : "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-    const uint32_t tmem_base = warp == PT_CODE_WARP ? 0u : sh->tmem_base;
-    const uint32_t tmem_a = tmem_base + 2 * DC;                   // two units of CB / 2 columns
-
-    if (warp == PT_X_WARP) {
+            const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;
+        if (warp == PT_X_WARP) {
         pdl_wait();
         if (elect_one()) {
             int s = 0; uint32_t ph = 1;
@@ -226,7 +220,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
             }
         }
         __syncwarp();
-    } else if (warp == PT_MMA_WARP) {
+        } else if (warp == PT_MMA_WARP) {
         pdl_wait();
         if (elect_one()) {
             constexpr uint32_t idesc = (1u << 4) | (8u << 24);    // FP32 accumulators, FP16 operands, 128 rows
@@ -253,7 +247,34 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
             mbar_wait(smem_u32(&sh->drained), 0u, abort_flag, 5);
         }
         __syncwarp();
-    } else if (warp < PT_WORKERS) {
+        }
+        }
+    } else {
+        // the codebooks into the copies
+        const int t0 = tid;
+        constexpr int NT = PT_CODE_WARP * 32;
+        auto stage = [&](const __half* l, const __half* r, int k_have, int rows, int off) {
+            for (int e = t0; e < rows * 2 * PLANES; e += NT) {
+                const int k = e / (2 * PLANES), side = (e / PLANES) & 1, plane = e % PLANES;
+                const __half* src = (side ? r : l) + (size_t)k * HALF + plane * 8;
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if (k < k_have) {
+                    if constexpr (HALF == 4) { const uint2 w = *reinterpret_cast<const uint2*>(src); v = make_uint4(w.x, w.y, w.x, w.y); }
+                    else v = *reinterpret_cast<const uint4*>(src);
+                }
+                uint4* dst = reinterpret_cast<uint4*>(pt_smem + off + (size_t)k * ROW + side * 128 * PLANES + plane * 128);
+#pragma unroll
+                for (int c = 0; c < 8; c++) dst[(c + t0) & 7] = v;              // lanes start at different copies: 128 bytes apart they would share banks
+            }
+        };
+        stage(p.cb_l, p.cb_r, p.K, 256, p.tab_off);
+        if (p.rows2) stage(p.cb2_l, p.cb2_r, p.K2, p.rows2, p.tab2_off);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" :: "n"(PT_THREADS - 32) : "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;                   // two units of CB / 2 columns
+    if (warp < PT_WORKERS) {
+        pt_set_regs<PtRegs<HALF, NG>::WORKER>();
         // ── entries into tensor memory: the two teams take units in turn, each into its own half ──
         const int q = warp & 3, h = (warp >> 2) & 1, team = warp >> 3, rl = q * 32 + lane;
         const uint32_t at = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(team * (CB / 2) + h * (CB / 4));
@@ -318,6 +339,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
             if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[team]));
         }
     } else if (warp < PT_SUM_WARP + PT_SUMMERS) {
+        pt_set_regs<PtRegs<HALF, NG>::SUMMER>();
         // ── sums out of the accumulators ──
         const int q = warp & 3, rl = q * 32 + lane, st = tid - PT_SUM_WARP * 32, w = warp - PT_SUM_WARP, team = w >> 2;
         const uint32_t dq = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -429,11 +451,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
         if (alive) close_tile(cur);
         if (alive && nseg) settle();
     }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == PT_MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(sh->tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
     }
     if (tid == 0 && sh->abort_flag) {
         *p.err = IBCU_PQ_TC_ERR + sh->abort_flag;
