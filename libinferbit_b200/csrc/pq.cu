@@ -128,7 +128,10 @@ __device__ __forceinline__ void fold(float* v, int o) {
 // H8: entries of eight values, known at compile time (one activation through 4096 x 14336: 10.9 -> 10.75 us a call; its 64 registers spill less).
 template <int BT, bool EX, bool H8>
 __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p) {
-    constexpr int PQ_NG = BT == 1 ? 4 : 2;                   // groups of 16 rows whose codes a warp keeps in flight
+    // Groups of 16 rows whose codes a warp keeps in flight: as many as leave nothing to spill in 64 registers (four spilled 72 bytes for one level, us with
+    // four and three: 4096 x 14336 11.0 and 10.7, 1024 x 4096 7.5 and 7.2, 32000 x 4096 15.1 and 15.0; with a second level and four and two:
+    // 8000 x 8192 15.5 and 14.9, 2000 x 2048 8.0 and 7.5).
+    constexpr int PQ_NG = BT == 1 && !EX ? 3 : 2;
     extern __shared__ __align__(16) float lut[];            // [256][32][BT]
     __shared__ float xs[BT][32][17];                         // this slab's activation slices, one row per lane (half <= 16)
     __shared__ __align__(16) float4 cbf[256][2][2];          // [k][side][half of the entry]: the two shared codebooks (half == 8) widened to FP32, staged once;
@@ -559,12 +562,13 @@ constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;         // scratch of the a
 // activations, G / 2 weights each, and a preparation launch. So what is looked up (`work`: weights, over both levels) decides.
 // Both measured over M 1024 to 32000, N 1024 to 14336, one to eight activations, with second levels and outlier columns, direct and in
 // graphs; us, tables / tensor cores:
-//   entries of 4: from two activations on always ahead (8192 x 8192 31 / 23); one: 4096 x 8192 16.8 / 15.5, 14336 x 8192 29.5 / 32.7
-//   entries of 16: up to 62 M weights per activation; one: 4096 x 8192 22.0 / 17.5, 14336 x 8192 24.2 / 33.9, 14336 x 14336 27.3 / 50.7;
-//     eight: 32000 x 8192 103 / 70
-//   entries of 8: one never (4096 x 14336 10.8 / 17.9), three and more always (26.3 / 18.8); two where the rows are
-//     short or few: 14336 x 2048 17.0 / 13.5, 4096 x 4096 11.8 / 11.5, 4096 x 8192 13.4 / 14.9
-// The loss against the better of the two is 0.1 % on the mean and at most 30 %.
+//   entries of 4: from two activations on always ahead; one: 4096 x 8192 16.4 / 15.1, 14336 x 4096 19.5 / 20.2, 14336 x 14336 45.1 / 49.8
+//   entries of 16: one: 4096 x 8192 21.0 / 12.4, 8192 x 8192 22.5 / 15.5, 32000 x 4096 23.6 / 23.7, 14336 x 14336 26.2 / 30.8; eight: 59.8 / 26.8 for 32000 x 4096
+//   entries of 8: one never (4096 x 14336 10.8 / 15.5), three and more always; two: 14336 x 2048 14.9 / 12.2, 4096 x 4096 11.6 / 10.7, 4096 x 8192
+//     13.4 / 12.8, 14336 x 14336 33.3 / 33.9
+// The lines are where the two met before the tensor-core kernel had its registers by role, which put it ahead up to twice as much work (entries of 16, one
+// activation) and nearly everywhere (entries of 8, two). They were not moved: where both do, the tables' sums are the closer ones (1.0e-7 of the
+// result's root mean square against 1.25e-7).
 static bool pq_takes_tc(const ibcu_pq_t* t, int B) {
     const double cols = (double)(t->N - t->n_outlier) * (t->K_l2 > 0 ? 2 : 1), work = cols * t->M;
     if (t->G == 32) return work <= 62e6 * B;
