@@ -130,8 +130,9 @@ template <int BT, bool EX, bool H8>
 __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p) {
     // Groups of 16 rows whose codes a warp keeps in flight: as many as leave nothing to spill in 64 registers (four spilled 72 bytes for one level, us with
     // four and three: 4096 x 14336 11.0 and 10.7, 1024 x 4096 7.5 and 7.2, 32000 x 4096 15.1 and 15.0; with a second level and four and two:
-    // 8000 x 8192 15.5 and 14.9, 2000 x 2048 8.0 and 7.5).
-    constexpr int PQ_NG = BT == 1 && !EX ? 3 : 2;
+    // 8000 x 8192 15.5 and 14.9, 2000 x 2048 8.0 and 7.5; two activations, two and one: 4096 x 8192 13.1 and 12.4, 32000 x 4096 25.7 and 25.3, with a second
+    // level of 256 14336 x 4096 23.4 and 22.8, entries of sixteen with one 4096 x 4096 30.5 and 28.4).
+    constexpr int PQ_NG = BT == 1 ? (EX ? 2 : 3) : 1;
     extern __shared__ __align__(16) float lut[];            // [256][32][BT]
     __shared__ float xs[BT][32][17];                         // this slab's activation slices, one row per lane (half <= 16)
     __shared__ __align__(16) float4 cbf[256][2][2];          // [k][side][half of the entry]: the two shared codebooks (half == 8) widened to FP32, staged once;
@@ -565,9 +566,9 @@ constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;         // scratch of the a
 //   entries of 4: from two activations on always ahead; one: 4096 x 8192 16.4 / 15.1, 14336 x 4096 19.5 / 20.2, 14336 x 14336 45.1 / 49.8
 //   entries of 16: one: 4096 x 8192 21.0 / 12.4, 8192 x 8192 22.5 / 15.5, 32000 x 4096 23.6 / 23.7, 14336 x 14336 26.2 / 30.8; eight: 59.8 / 26.8 for 32000 x 4096
 //   entries of 8: one never (4096 x 14336 10.8 / 15.5), three and more always; two: 14336 x 2048 14.9 / 12.2, 4096 x 4096 11.6 / 10.7, 4096 x 8192
-//     13.4 / 12.8, 14336 x 14336 33.3 / 33.9
+//     12.4 / 12.8, 14336 x 14336 33 / 33.9
 // The lines are where the two met before the tensor-core kernel had its registers by role, which put it ahead up to twice as much work (entries of 16, one
-// activation) and nearly everywhere (entries of 8, two). They were not moved: where both do, the tables' sums are the closer ones (1.0e-7 of the
+// activation) and about level (entries of 8, two). They were not moved: where both do, the tables' sums are the closer ones (1.0e-7 of the
 // result's root mean square against 1.25e-7).
 static bool pq_takes_tc(const ibcu_pq_t* t, int B) {
     const double cols = (double)(t->N - t->n_outlier) * (t->K_l2 > 0 ? 2 : 1), work = cols * t->M;
