@@ -35,8 +35,9 @@ namespace {
 
 // Warps of a block whose runs have T tiles: Q teams of 4 T workers, then one each for the weights, the digits and the MMAs.
 template <int T, int Q> struct Tq { static constexpr int WORKERS = 4 * T * Q, A_WARP = WORKERS, B_WARP = WORKERS + 1, MMA_WARP = WORKERS + 2, THREADS = (WORKERS + 3) * 32; };
-// INT4 runs of one tile have room for four teams (16 workers); two tiles fill the block with two, and INT8 weights need none
-constexpr int tq_teams(int bits, int T) { return bits == 4 && T == 1 ? 4 : 2; }
+// INT4 runs of one tile have room for four teams (16 workers); two tiles fill the block with two, and INT8 weights need none. Clusters of eight keep to half an
+// SM a block: sixteen of them with an SM to each block do not find room at once (2048 x 6144 INT8 at 4 and 32 activations 7.3 and 12.6, 12.1 and 17.8 us).
+constexpr int tq_teams(int bits, int T, int S) { return bits == 4 && T == 1 && S < 8 ? 4 : 2; }
 constexpr int TQ_MAX_STAGES = 12;
 constexpr int TQ_MAX_B = 32;
 
@@ -530,7 +531,11 @@ int launch_tc_mg(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid,
 
 template <int BITS, int T>
 int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
-    constexpr int Q = tq_teams(BITS, T);
+    if constexpr (tq_teams(BITS, T, 1) != tq_teams(BITS, T, 8)) {
+        constexpr int H = tq_teams(BITS, T, 8);
+        if (p.S == 8) return p.gp.world ? launch_tc_mg<BITS, T, H, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, H, false>(ctx, maps, p, grid, smem);
+    }
+    constexpr int Q = tq_teams(BITS, T, 1);
     return p.gp.world ? launch_tc_mg<BITS, T, Q, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, Q, false>(ctx, maps, p, grid, smem);
 }
 
@@ -599,11 +604,11 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     // it, but what a block of columns costs is the way of its weights and digits from L2, and with twice the ring twice as many are on it:
     // 4096 x 14336 INT4 at 4, 16 and 32 activations 15.0 -> 13.1, 18.1 -> 17.2, 25.3 -> 20.7 us, 6144 x 4096 INT8 at 4 and 32 9.9 -> 9.2,
     // 17.6 -> 16.0. INT8 at 9 to 20 activations is where the overlap is worth as much (6144 x 4096 at 12 13.3 against 13.7, 4096 x 4096 at 16 9.4
-    // against 9.6) and keeps it.
+    // against 9.6) and keeps it, and clusters of eight (tq_teams).
     const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;
     while (p.tmem_cols < tcols) p.tmem_cols *= 2;
-    const size_t cap = (T == 1 && bits == 8 && p.NC > 32 && p.NC <= 80 ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
+    const size_t cap = (T == 1 && (S == 8 || (bits == 8 && p.NC > 32 && p.NC <= 80)) ? 111 : 200) * 1024 - sizeof(TqShared) - 2048;
     const size_t b_block = (size_t)p.NC * 128;
     p.a_stage = R * (bits == 8 ? 128 : 64);
     const int nk = (p.nkb + S - 1) / S;
@@ -641,7 +646,7 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     if (bits == 4 && (p.sa < nk || nruns > slots)) {
         // a ring that is used again: a multiple of the teams, so that a stage always belongs to the same team of widening warps (a warp that
         // misses every other phase of a barrier cannot tell a phase from the next but one)
-        const int teams = tq_teams(bits, T);
+        const int teams = tq_teams(bits, T, S);
         if (p.sa < teams) return IBCU_DECLINED;
         p.sa -= p.sa % teams;
         if (!p.recv_off && recv > ring_of()) return IBCU_DECLINED;
@@ -663,8 +668,9 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     // growing it may fail (under capture), and the call must then leave the gather to the next one.
     int parts = 1;
     // A cluster per activation where the kernel has something to add up, and beyond 16 activations: 4096 x 4096 INT8 with RMSNorm at 8, 16 and 32 8.8 -> 8.2,
-    // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2).
-    const bool clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || B > 16) && (long)p.nkb * 128 <= XCL_PARTS * XCL_COLS;
+    // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2),
+    // and 2048 x 6144 INT4, in clusters of eight, 11.5 -> 12.3 at 32.
+    const bool clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && S < 8)) && (long)p.nkb * 128 <= XCL_PARTS * XCL_COLS;
     if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
     if (clustered) while (parts * XCL_COLS < p.nkb * 128) parts *= 2;
     const int part_kb = (p.nkb + parts - 1) / parts;
