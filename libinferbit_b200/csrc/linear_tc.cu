@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(XCL_COLS / 8) xprep_tc_cluster_kernel(const XS
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = blockIdx.x, nparts = gridDim.x, b = blockIdx.y;
     const int col = part * part_cols + tid * 8;
     const bool mine = tid * 8 < part_cols && col < all_cols, have = mine && col < N;
+    cluster_arrive();                                         // waited for before the first store into a peer's shared memory: by then every block has started
     pdl_launch_dependents();
     float4 w0 = make_float4(1.0f, 1.0f, 1.0f, 1.0f), w1 = w0;
     if (src.op == IBCU_PRO_RMSNORM && have) {                 // weights: the kernel ahead does not write them
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(XCL_COLS / 8) xprep_tc_cluster_kernel(const XS
     mx = warp_max(fmaxf(mx, fmaxf(fmaxf(fabsf(v.x * w1.x), fabsf(v.y * w1.y)), fmaxf(fabsf(v.z * w1.z), fabsf(v.w * w1.w)))));
     if (lane == 0) warps[warp] = make_float2(mx, ss);
     __syncthreads();
+    cluster_wait();
     if (tid < nparts) {                                       // this part's into every block of the cluster
         float2 m = warps[0];
 #pragma unroll

@@ -47,3 +47,19 @@ def test_kmeans_kernels_read_the_launch_ahead_past_l1(kernel, arrays):
     for a in arrays:
         assert not re.search(rf"\b{a}\[", body[:end]), a
         assert re.search(rf"__ldcg\({a} \+", body[:end]), a
+
+
+def test_no_access_to_a_peers_shared_memory_before_it_has_started():
+    """Shared memory of another block of the cluster may be used once that block is known to run, which only a barrier of the cluster says: an
+    arrival and a wait stand before the first use. (A block's own barrier and the wait for the launch ahead say nothing about a peer.)"""
+    seen = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        for k in _code(path).split("__global__")[1:]:
+            body = k.split("\n}\n")[0]
+            use = re.search(r"st\.shared::cluster\.[uv]|map_shared_rank", body)
+            if not use:
+                continue
+            kernel, ahead = re.search(r"(\w+_kernel)\(", body).group(1), body[:use.start()]
+            seen.append(kernel)
+            assert "cluster.sync()" in ahead or 0 <= ahead.find("cluster_arrive()") < ahead.find("cluster_wait()"), kernel
+    assert seen == ["xprep_tc_cluster_kernel", "linear_tc_kernel", "pq_topk_select_cluster_kernel"]
