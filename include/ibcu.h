@@ -119,7 +119,9 @@ int ibcu_linear(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors,
  * (src/forward.c:566-572,625-636), or silu(x)*x2 ahead of down_proj (src/forward.c:637-640). */
 #define IBCU_PRO_NONE      0
 #define IBCU_PRO_RMSNORM   1  /* x <- x * rsqrt(mean(x^2) + eps) * fp16(norm_w) */
-#define IBCU_PRO_SILU_MUL  2  /* x <- x / (1 + exp(-x)) * x2 */
+#define IBCU_PRO_SILU_MUL  2  /* x <- x / (1 + exp(-x)) * x2. Several activations of up to IBCU_PREPARED_COLUMNS columns are prepared in one
+                               * pass; for longer rows ibcu_silu_mul_amax and IBCU_PRO_KNOWN_MAX are the faster way */
+#define IBCU_PREPARED_COLUMNS 16384
 #define IBCU_PRO_KNOWN_MAX 3  /* x as it is; the caller supplies max|x[b]| in pieces (ibcu_silu_mul_amax makes them), which
                                * spares every block of the kernel its own reduction over the activation */
 typedef struct {

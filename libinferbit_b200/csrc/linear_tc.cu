@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(T) xprep_tc_kernel(const XSource src, int N, i
 }
 
 // The same by a cluster of blocks per activation, a part of its columns each and eight columns a thread: one round trip to memory, and the parts' maxima and
-// sums of squares meet in shared memory. Rows of up to XCL_PARTS * XCL_COLS columns. src.op: none, RMSNorm or silu(x) * x2.
-constexpr int XCL_PARTS = 8, XCL_COLS = 2048;
+// sums of squares meet in shared memory. Rows of up to IBCU_PREPARED_COLUMNS columns. src.op: none, RMSNorm or silu(x) * x2.
+constexpr int XCL_PARTS = 8, XCL_COLS = IBCU_PREPARED_COLUMNS / XCL_PARTS;
 template <bool MG>       // MG: see linear.cu
 __global__ void __launch_bounds__(XCL_COLS / 8) xprep_tc_cluster_kernel(const XSource src, int N, int part_cols, int all_cols, int nc, int perm8, int8_t* __restrict__ xtiles,
                                                                         float* __restrict__ xscale, int* __restrict__ xsum, const GatherWait gw) {
@@ -672,7 +672,7 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     // A cluster per activation where the kernel has something to add up, and beyond 16 activations: 4096 x 4096 INT8 with RMSNorm at 8, 16 and 32 8.8 -> 8.2,
     // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2),
     // and 2048 x 6144 INT4, in clusters of eight, 11.5 -> 12.3 at 32.
-    const bool clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && S < 8)) && (long)p.nkb * 128 <= XCL_PARTS * XCL_COLS;
+    const bool clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && S < 8)) && p.nkb * 128L <= IBCU_PREPARED_COLUMNS;
     if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
     if (clustered) while (parts * XCL_COLS < p.nkb * 128) parts *= 2;
     const int part_kb = (p.nkb + parts - 1) / parts;

@@ -219,3 +219,46 @@ def test_copy_helpers_take_no_signals_and_no_core_that_is_not_there(tmp_path):
                     f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}", "-lm", "-lpthread"], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stdout)
+
+
+STEP = r"""
+#include "ibcu.h"
+#include <stdio.h>
+static int products, silu, known;
+static int fake_linear(ibcu_ctx* c, const ibcu_linear_t* t, int n, const float* x, int N, int B, int bits, const ibcu_prologue_t* p) {
+    (void)c; (void)t; (void)n; (void)x; (void)N; (void)B; (void)bits;
+    if (p) { silu += p->op == IBCU_PRO_SILU_MUL; known += p->op == IBCU_PRO_KNOWN_MAX; }
+    return 0;
+}
+static int fake_product(ibcu_ctx* c, float* o, const float* g, const float* u, int n, int B, float* a, int parts) { (void)c; (void)o; (void)g; (void)u; (void)n; (void)B; (void)a; (void)parts; products++; return 0; }
+#define ibcu_linear_ex fake_linear
+#define ibcu_silu_mul_amax fake_product
+#define ibcu_embed_rows(...) 0
+#define ibcu_attention_decode_at(...) 0
+#define ibcu_attention_decode(...) 0
+#include "ib_b200_forward.c"
+int main(void) {
+    layer y = { 0 };
+    ib_b200_model m = { 0 };
+    m.world = 1; m.L = &y; m.c.n_layers = 1; m.c.hidden = 4096;
+    const int wide[] = { 11008, IBCU_PREPARED_COLUMNS, IBCU_PREPARED_COLUMNS + 32, 28672 };
+    for (int w = 0; w < 4; w++)
+        for (int B = 1; B <= 32; B++) {
+            const int want = B >= 4 && w < 2;                /* the product where the digits are made, or in a launch with its maximum */
+            products = silu = known = 0;
+            m.c.inter = wide[w];
+            if (issue(&m, 0, B, 1) || silu != want || known != !want || products != !want) { printf("%d wide, %d positions: %d %d %d\n", wide[w], B, silu, known, products); return 1; }
+        }
+    return 0;
+}
+"""
+
+
+def test_where_a_step_forms_the_product_of_the_mlp(tmp_path):
+    """Rows that one pass of the preparation does not hold keep the launch of their own: many blocks form the product there, where the preparation would
+    have one block per position."""
+    src, exe = tmp_path / "step.c", tmp_path / "step"
+    src.write_text(STEP)
+    subprocess.run(["gcc", "-std=gnu11", "-O2", "-w", f"-I{ROOT}/include", f"-I{LIB}/host", "-o", str(exe), str(src), f"-L{LIB}", "-libcu", f"-Wl,-rpath,{LIB}"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout)
