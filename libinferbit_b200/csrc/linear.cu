@@ -595,8 +595,11 @@ extern "C" int ibcu_linear_ex(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n
     if (total_rows == 0) return IBCU_OK;
     const LinPlan pl = lin_plan(ctx, tensors, n_tensors, total_rows, N, B < 16 ? B : 16, bits, op);
     bool tc = ctx->linear_tc > 0 && (bits == 4 || ctx->linear_tc > 1);
-    if (ctx->linear_tc == 0)                                  // see lin_mma_us; beyond 16 activations the mma.sync kernel goes over the weights twice
-        tc = B > 16 || (B > 1 && lin_tc_us(ibcu_linear_tc_cut(ctx->sm_count, tensors, n_tensors, N, B), N, bits) < lin_mma_us(pl, N, B, bits));
+    // See lin_mma_us; beyond 16 activations the mma.sync kernel goes over the weights twice. The estimates know nothing of silu(x) * x2, which one block per
+    // activation forms ahead of the mma.sync kernel: 5.3 to 6.5 us more than digits of a known maximum, behind the tcgen05 kernel in all of 656 calls
+    // (1024 x 3072 INT8 at 4 activations 12.0 against 6.8 us, 4096 x 28672 48.6 against 41.0).
+    if (ctx->linear_tc == 0)
+        tc = B > 16 || (B > 1 && (op == IBCU_PRO_SILU_MUL || lin_tc_us(ibcu_linear_tc_cut(ctx->sm_count, tensors, n_tensors, N, B), N, bits) < lin_mma_us(pl, N, B, bits)));
     if (tc) {
         const int rc_tc = ibcu_linear_tc(ctx, tensors, n_tensors, x, N, B, bits, pro, op);
         if (rc_tc != IBCU_DECLINED) return rc_tc;

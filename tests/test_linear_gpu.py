@@ -5,7 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from libinferbit_b200 import LinearT, _ffi
+from libinferbit_b200 import Backend, LinearT, _ffi
 from tests import _cpu
 
 pytestmark = pytest.mark.gpu
@@ -112,7 +112,6 @@ def test_rows_longer_than_s32_sums_hold(backend, bits, N):
 def test_capture_without_room_for_the_digits(bits):
     """Under capture the digits of the tcgen05 kernel cannot be given more room: the call says so and launches nothing, it does not
     go on with another kernel under a context that holds an error. Afterwards the same call, run once outside, can be captured."""
-    from libinferbit_b200 import Backend
     rng = np.random.default_rng(bits)
     M, N, B = 64, 2048, 5
     w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
@@ -665,3 +664,29 @@ def test_tcgen05_digits_prepared_by_clusters(backend, bits, op, N, B):
     want = (act @ v.T) * sc
     bound = 2.0 ** -22 * np.abs(want) + 2.0 ** -30 * np.abs(act).max(axis=1, keepdims=True) * (np.abs(v).sum(axis=1) * sc) + 32 * 2.0 ** -24 * (np.abs(act) @ np.abs(v).T) * sc
     assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+
+
+@pytest.mark.parametrize("bits,M,N,B", [(8, 1024, 3072, 5), (4, 1024, 4096, 5), (8, 1024, 1024, 2)])
+def test_several_products_take_the_tcgen05_kernel(bits, M, N, B):
+    """silu(x) * x2 of several activations, where an estimate without it takes the mma.sync kernel. The digits of the tcgen05 kernel take more room than
+    those of the other: in a context that has run the other kernel, a capture of the call by itself has none and says so."""
+    rng = np.random.default_rng(N + B)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    with Backend(0) as be:
+        dw, ds, dx, do = be.upload(w), be.upload(s16), be.upload(x), be.alloc(B * M * 4)
+        t = LinearT(dw.ptr, ds.ptr, do.ptr, M, M, 0, 0)
+        pro = _ffi.PrologueT(); pro.op, pro.x2 = 2, dx.ptr
+
+        def captured(mode):
+            be.lib.ibcu_linear_use_tcgen05(be.ctx, mode)
+            gid = C.c_int(-1)
+            be._check(be.lib.ibcu_graph_begin(be.ctx))
+            rc = be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.ptr, N, B, bits, C.byref(pro))
+            rc_end = be.lib.ibcu_graph_end(be.ctx, C.byref(gid))
+            be.lib.ibcu_clear_error(be.ctx)
+            return rc or rc_end
+
+        be.lib.ibcu_linear_use_tcgen05(be.ctx, -1)
+        be._check(be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.ptr, N, B, bits, C.byref(pro))); be.sync()
+        assert captured(-1) == 0
+        assert captured(0) != 0
