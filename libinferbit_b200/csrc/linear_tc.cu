@@ -20,7 +20,7 @@
 // then one warp each for the weights (TMA), the digits (bulk copies) and the MMAs. What a block of columns costs a warp is waits
 // and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
 // activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4; at 32 the digits, which every SM reads from L2,
-// bound the kernel (26 us, 75 MB of them). Four teams where a run has one tile: 4096 x 4096 INT4 at 4, 16 and 32 activations 8.3 -> 7.5, 9.2 -> 8.9,
+// bound the kernel (26 us, 75 MB of them). Four teams for some runs of one tile (tq_teams): 4096 x 4096 INT4 at 4, 16 and 32 activations 8.3 -> 7.5, 9.2 -> 8.9,
 // 12.4 -> 11.5, 2560 x 6400 at 32 14.3 -> 13.3, 4096 x 14336 at 32 20.7 -> 19.8.
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait.
 #include "common.cuh"
@@ -35,9 +35,6 @@ namespace {
 
 // Warps of a block whose runs have T tiles: Q teams of 4 T workers, then one each for the weights, the digits and the MMAs.
 template <int T, int Q> struct Tq { static constexpr int WORKERS = 4 * T * Q, A_WARP = WORKERS, B_WARP = WORKERS + 1, MMA_WARP = WORKERS + 2, THREADS = (WORKERS + 3) * 32; };
-// INT4 runs of one tile have room for four teams (16 workers); two tiles fill the block with two, and INT8 weights need none. Clusters of eight keep to half an
-// SM a block: sixteen of them with an SM to each block do not find room at once (2048 x 6144 INT8 at 4 and 32 activations 7.3 and 12.6, 12.1 and 17.8 us).
-constexpr int tq_teams(int bits, int T, int S) { return bits == 4 && T == 1 && S < 8 ? 4 : 2; }
 constexpr int TQ_MAX_STAGES = 12;
 constexpr int TQ_MAX_B = 32;
 
@@ -523,6 +520,41 @@ EncodeFn encode_fn() {
     return fn;
 }
 
+// How a call's digits are prepared: parts blocks of part_kb blocks of columns each per activation, as a cluster or not.
+struct TqPrep { bool clustered; int parts, part_kb; };
+TqPrep tq_prep(const TqCut& cut, int B, int op) {
+    TqPrep x = { false, 1, cut.nkb };
+    // A cluster per activation where the kernel has something to add up, and beyond 16 activations: 4096 x 4096 INT8 with RMSNorm at 8, 16 and 32 8.8 -> 8.2,
+    // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2),
+    // and 2048 x 6144 INT4, in clusters of eight, 11.5 -> 12.3 at 32.
+    x.clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && cut.S < 8)) && cut.nkb * 128L <= IBCU_PREPARED_COLUMNS;
+    // otherwise a block per activation, or several when the maximum is known
+    if (op == IBCU_PRO_KNOWN_MAX) { x.parts = (cut.nkb + 15) / 16; if (x.parts > 8) x.parts = 8; }
+    if (x.clustered) while (x.parts * XCL_COLS < cut.nkb * 128) x.parts *= 2;
+    x.part_kb = (cut.nkb + x.parts - 1) / x.parts;
+    if (!x.clustered) x.parts = (cut.nkb + x.part_kb - 1) / x.part_kb;                 // a cluster may end with empty parts
+    return x;
+}
+
+// Teams of widening warps (INT4). Runs of one tile have room for four (16 workers); two tiles fill the block with two, and INT8 weights need none. Clusters of eight keep
+// to half an SM a block: sixteen of them with an SM to each block do not find room at once (2048 x 6144 at 4 and 32 activations 7.3 and 12.6, 12.1 and 17.8 us).
+// Beside a block of four teams, 19 warps of 96 registers, no block of the next call's preparation finds registers (with 72 or 80 it does, but the block
+// spills). Where that preparation does not fit on the SMs this launch leaves idle either, it starts late and two teams are the faster: us, two and four,
+// 8192 x 2048 (none idle) at 6 8.7 and 9.6, 2560 x 6400 with RMSNorm at 8 9.3 and 11.0, 16384 x 2048 at 8 9.3 and 10.2; where it fits, or finds no room beside two teams
+// either (rows of more than 2048 columns by one block), 4096 x 4096 with RMSNorm at 3 8.1 and 7.2, 8192 x 8192 at 4 16.9 and 15.8. Short parts of a row need more than eight
+// activations to have work for four in the epilogue (3072 + 3072 x 1024 at 4 5.8 and 6.2, at 16 8.4 and 7.3), and beyond 24 that work weighs more than the late start.
+// Against two teams with half an SM, 1296 calls: 0.854 of the time on the mean, 8 behind by more than 3 %, at most 10 %; four teams everywhere 0.871, 93, 14 %.
+int tq_teams(int sm_count, int bits, const TqCut& cut, int B, int op, const TqPrep& x) {
+    if (bits == 8 || cut.T == 2 || cut.S == 8) return 2;
+    const int nk = (cut.nkb + cut.S - 1) / cut.S, idle = sm_count - cut.S * (cut.nruns < cut.slots ? cut.nruns : cut.slots);
+    const int per_sm = x.clustered ? 5 : (x.part_kb * 128 <= 2048 ? 3 : 1);             // blocks of the preparation on an idle SM, by their registers
+    if (B > 24 || (per_sm == 1 && nk >= 5)) return 4;
+    if (op == IBCU_PRO_KNOWN_MAX && B > 4 && B <= 8) return 2;                          // at 8 3000 x 3008 6.5 and 7.2, 4096 x 4096 7.4 and 7.9
+    if (x.parts * B > idle * per_sm) return 2;
+    if (x.clustered && x.parts >= 4 && (x.parts > 4 || B > 4 || idle < 8)) return 2;    // clusters need their places in one group of SMs
+    return nk >= 5 || B > 8 ? 4 : 2;
+}
+
 template <int BITS, int T, int Q, bool MG>
 int launch_tc_mg(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
     auto kern = linear_tc_kernel<BITS, T, Q, MG>;
@@ -532,13 +564,11 @@ int launch_tc_mg(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid,
 }
 
 template <int BITS, int T>
-int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int grid, size_t smem) {
-    if constexpr (tq_teams(BITS, T, 1) != tq_teams(BITS, T, 8)) {
-        constexpr int H = tq_teams(BITS, T, 8);
-        if (p.S == 8) return p.gp.world ? launch_tc_mg<BITS, T, H, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, H, false>(ctx, maps, p, grid, smem);
+int launch_tc(ibcu_ctx* ctx, const TqMaps& maps, const TqParams& p, int teams, int grid, size_t smem) {
+    if constexpr (BITS == 4 && T == 1) {
+        if (teams == 4) return p.gp.world ? launch_tc_mg<4, 1, 4, true>(ctx, maps, p, grid, smem) : launch_tc_mg<4, 1, 4, false>(ctx, maps, p, grid, smem);
     }
-    constexpr int Q = tq_teams(BITS, T, 1);
-    return p.gp.world ? launch_tc_mg<BITS, T, Q, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, Q, false>(ctx, maps, p, grid, smem);
+    return p.gp.world ? launch_tc_mg<BITS, T, 2, true>(ctx, maps, p, grid, smem) : launch_tc_mg<BITS, T, 2, false>(ctx, maps, p, grid, smem);
 }
 
 }  // namespace
@@ -614,6 +644,8 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     const size_t b_block = (size_t)p.NC * 128;
     p.a_stage = R * (bits == 8 ? 128 : 64);
     const int nk = (p.nkb + S - 1) / S;
+    const TqPrep prep = tq_prep(cut, B, op);
+    const int teams = tq_teams(ctx->sm_count, bits, cut, B, op, prep);
     const size_t recv = S > 1 ? (size_t)S * ((B + S - 1) / S) * T * 128 * 8 : 0;
     const size_t spare = bits == 8 ? 16384 * T : 0;                                      // an MMA reads 128 rows whatever the run has
     // digit stages of at least 8 KB; the rings share the room in the proportion of what a block of columns takes of each
@@ -648,7 +680,6 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     if (bits == 4 && (p.sa < nk || nruns > slots)) {
         // a ring that is used again: a multiple of the teams, so that a stage always belongs to the same team of widening warps (a warp that
         // misses every other phase of a barrier cannot tell a phase from the next but one)
-        const int teams = tq_teams(bits, T, S);
         if (p.sa < teams) return IBCU_DECLINED;
         p.sa -= p.sa % teams;
         if (!p.recv_off && recv > ring_of()) return IBCU_DECLINED;
@@ -666,17 +697,8 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
                    bits == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return IBCU_DECLINED;
     }
-    // The digits: a block per activation, or several when the maximum is known. Their room is there before a pending gather is taken:
-    // growing it may fail (under capture), and the call must then leave the gather to the next one.
-    int parts = 1;
-    // A cluster per activation where the kernel has something to add up, and beyond 16 activations: 4096 x 4096 INT8 with RMSNorm at 8, 16 and 32 8.8 -> 8.2,
-    // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2),
-    // and 2048 x 6144 INT4, in clusters of eight, 11.5 -> 12.3 at 32.
-    const bool clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && S < 8)) && p.nkb * 128L <= IBCU_PREPARED_COLUMNS;
-    if (op == IBCU_PRO_KNOWN_MAX) { parts = (p.nkb + 15) / 16; if (parts > 8) parts = 8; }
-    if (clustered) while (parts * XCL_COLS < p.nkb * 128) parts *= 2;
-    const int part_kb = (p.nkb + parts - 1) / parts;
-    if (!clustered) parts = (p.nkb + part_kb - 1) / part_kb;                           // a cluster may end with empty parts
+    // The digits' room is there before a pending gather is taken: growing it may fail (under capture), and the call must then leave the gather to the next one.
+    const int parts = prep.parts;
     p.xparts = parts;
     const size_t tiles = (size_t)p.nkb * b_block, scales = (((size_t)B * parts * sizeof(float)) + 255) & ~(size_t)255;
     int rc = ibcu_reserve(ctx, &ctx->xpack, &ctx->xpack_bytes, tiles + scales + (size_t)B * parts * LIN_LIMBS * sizeof(int));
@@ -702,16 +724,16 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     const XSource xsrc = { x, pro ? pro->x2 : nullptr, pro ? (const __half*)pro->norm_w : nullptr, pro ? pro->eps : 0.0f, op,
                            op == IBCU_PRO_KNOWN_MAX ? pro->amax : nullptr, op == IBCU_PRO_KNOWN_MAX ? pro->n_amax : 0 };
     const dim3 xg(parts, B);
-    const int perm8 = bits == 4 ? 1 : 0, cols = part_kb * 128, all = p.nkb * 128;
+    const int perm8 = bits == 4 ? 1 : 0, cols = prep.part_kb * 128, all = p.nkb * 128;
     const bool mg = gw.flags || gw.tag.n;
-    if (clustered) {
+    if (prep.clustered) {
         rc = ibcu_launch(ctx, mg ? xprep_tc_cluster_kernel<true> : xprep_tc_cluster_kernel<false>, xg, dim3(XCL_COLS / 8), 0, parts, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
     } else {
-        auto prep = cols > 2048 ? (mg ? xprep_tc_kernel<512, true> : xprep_tc_kernel<512, false>) : (mg ? xprep_tc_kernel<256, true> : xprep_tc_kernel<256, false>);
-        rc = ibcu_launch(ctx, prep, xg, dim3(cols > 2048 ? 512 : 256), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
+        auto kern = cols > 2048 ? (mg ? xprep_tc_kernel<512, true> : xprep_tc_kernel<512, false>) : (mg ? xprep_tc_kernel<256, true> : xprep_tc_kernel<256, false>);
+        rc = ibcu_launch(ctx, kern, xg, dim3(cols > 2048 ? 512 : 256), 0, 1, true, xsrc, N, cols, all, p.NC, perm8, xtiles, xscale, xsum, gw);
     }
     if (rc) return rc;
     const int grid = S * (nruns < slots ? nruns : slots);
-    if (bits == 8) return T == 1 ? launch_tc<8, 1>(ctx, maps, p, grid, smem) : launch_tc<8, 2>(ctx, maps, p, grid, smem);
-    return T == 1 ? launch_tc<4, 1>(ctx, maps, p, grid, smem) : launch_tc<4, 2>(ctx, maps, p, grid, smem);
+    if (bits == 8) return T == 1 ? launch_tc<8, 1>(ctx, maps, p, teams, grid, smem) : launch_tc<8, 2>(ctx, maps, p, teams, grid, smem);
+    return T == 1 ? launch_tc<4, 1>(ctx, maps, p, teams, grid, smem) : launch_tc<4, 2>(ctx, maps, p, teams, grid, smem);
 }

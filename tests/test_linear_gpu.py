@@ -615,10 +615,12 @@ def test_linear_kernel_by_cost(backend, bits, Ms, N, B, tc):
         assert n == 2
 
 
-@pytest.mark.parametrize("M,N,B", [(130, 5 * 128, 2), (4096, 9 * 128, 7), (4000, 14336, 32), (2600, 6432, 12), (300, 23 * 128, 32), (40000, 11 * 128, 3)])
+@pytest.mark.parametrize("M,N,B", [(130, 5 * 128, 2), (4096, 9 * 128, 7), (4000, 14336, 32), (2600, 6432, 12), (300, 23 * 128, 32), (40000, 11 * 128, 3),
+                                   (16000, 2048, 4), (16000, 2048, 17), (9000, 15 * 128, 18), (9000, 15 * 128, 19), (6000, 1024, 8), (6000, 1024, 9), (4000, 14336, 3)])
 def test_tcgen05_int4_four_teams(backend, M, N, B):
-    """Runs of one tile: blocks of columns that are not a multiple of the four teams of widening warps, rings shorter than a part of the
-    columns, clusters of one to eight blocks (the last shape: two tiles, two teams, several runs a block). Bound as above."""
+    """Runs of one tile: blocks of columns that are not a multiple of the two or four teams of widening warps, rings shorter than a part of the
+    columns, clusters of one to eight blocks (40000 rows: two tiles, two teams, several runs a block); the last seven: both sides of the line between
+    two teams and four. Bound as above."""
     rng = np.random.default_rng(M + N + B)
     w, s16, x = _cpu.make_int4_case(rng, M, N, B)
     backend.lib.ibcu_linear_use_tcgen05(backend.ctx, 2)
