@@ -81,6 +81,7 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint
                  :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // the four digit sums of one (row, activation) as one integer
@@ -116,8 +117,10 @@ __global__ void __launch_bounds__(XCL_COLS / 8) xprep_tc_cluster_kernel(const XS
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = blockIdx.x, nparts = gridDim.x, b = blockIdx.y;
     const int col = part * part_cols + tid * 8;
     const bool mine = tid * 8 < part_cols && col < all_cols, have = mine && col < N;
-    cluster_arrive();                                         // waited for before the first store into a peer's shared memory: by then every block has started
     pdl_launch_dependents();
+    // Waited for before the first store into a peer's shared memory: by then every block has started. Nothing has been written yet, so nothing is
+    // released (with a release, ahead of the line above, 2048 x 5632 with silu at 6 activations took 8.7 us instead of 8.4).
+    cluster_arrive_relaxed();
     float4 w0 = make_float4(1.0f, 1.0f, 1.0f, 1.0f), w1 = w0;
     if (src.op == IBCU_PRO_RMSNORM && have) {                 // weights: the kernel ahead does not write them
         const __half2* h = reinterpret_cast<const __half2*>(src.norm_w + col);                          // 4-byte aligned at least
