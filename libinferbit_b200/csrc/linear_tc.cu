@@ -525,15 +525,25 @@ EncodeFn encode_fn() {
 
 // How a call's digits are prepared: parts blocks of part_kb blocks of columns each per activation, as a cluster or not.
 struct TqPrep { bool clustered; int parts, part_kb; };
-TqPrep tq_prep(const TqCut& cut, int B, int op) {
+TqPrep tq_prep(const TqCut& cut, int bits, int B, int op) {
     TqPrep x = { false, 1, cut.nkb };
-    // A cluster per activation where the kernel has something to add up, and beyond 16 activations: 4096 x 4096 INT8 with RMSNorm at 8, 16 and 32 8.8 -> 8.2,
-    // 10.5 -> 10.0, 12.9 -> 11.7 us, 4096 x 14336 at 32 22.1 -> 21.1; without a prologue 12.0 -> 11.6 at 32, but 9.6 -> 9.8 at 16 (6144 columns 11.8 -> 12.2),
-    // and 2048 x 6144 INT4, in clusters of eight, 11.5 -> 12.3 at 32.
-    x.clustered = op != IBCU_PRO_KNOWN_MAX && (op != IBCU_PRO_NONE || (B > 16 && cut.S < 8)) && cut.nkb * 128L <= IBCU_PREPARED_COLUMNS;
+    int blocks = 1;                                           // of a cluster
+    while (blocks * XCL_COLS < cut.nkb * 128) blocks *= 2;
+    // Clusters of INT4 runs of two tiles in clusters of four (19 warps of 96 registers on 132 SMs) leave clusters of four and eight blocks no room.
+    const bool crowded = bits == 4 && cut.T == 2 && cut.S == 4 && blocks >= 4;
+    // A cluster per activation, us, one block and a cluster. silu(x) * x2: always (936 calls: 0.73 of the time on the mean, 1.01 at most).
+    // RMSNorm: 4096 x 4096 INT8 at 8, 16 and 32 8.9 and 8.2, 10.5 and 10.1, 12.8 and 11.9, 4096 x 14336 at 32 22.1 and 21.1; crowded: 5120 x 5120 at 8, 20 and 32 10.1 and 11.3,
+    // 13.3 and 14.9, 16.7 and 16.6. Without a prologue there is no sum to wait for: beyond 16 activations, INT4 3072 + 1024 + 1024 x 3072 at 20 12.2 and 10.7,
+    // 3072 + 3072 x 1024 at 32 10.2 and 8.6, 4096 x 4096 INT8 at 20 and 32 10.7 and 11.1, 11.9 and 11.8; but INT4 2560 x 6400 at 17 11.3 and 13.0, INT8 6400 + 6400 x 2560 at 24
+    // 14.4 and 15.6, 10000 x 2560 at 24 15.4 and 16.2, 2048 x 6144 INT4, in clusters of eight, at 32 11.6 and 12.3.
+    if (cut.nkb * 128L <= IBCU_PREPARED_COLUMNS) {
+        if (op == IBCU_PRO_SILU_MUL) x.clustered = true;
+        if (op == IBCU_PRO_RMSNORM) x.clustered = !crowded || B > 20;
+        if (op == IBCU_PRO_NONE) x.clustered = B > 16 && ((cut.S == 4 && !crowded && (B > 20 || (bits == 4 && blocks <= 2))) || (cut.S == 2 && blocks == 1));
+    }
     // otherwise a block per activation, or several when the maximum is known
     if (op == IBCU_PRO_KNOWN_MAX) { x.parts = (cut.nkb + 15) / 16; if (x.parts > 8) x.parts = 8; }
-    if (x.clustered) while (x.parts * XCL_COLS < cut.nkb * 128) x.parts *= 2;
+    if (x.clustered) x.parts = blocks;
     x.part_kb = (cut.nkb + x.parts - 1) / x.parts;
     if (!x.clustered) x.parts = (cut.nkb + x.part_kb - 1) / x.part_kb;                 // a cluster may end with empty parts
     return x;
@@ -647,7 +657,7 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     const size_t b_block = (size_t)p.NC * 128;
     p.a_stage = R * (bits == 8 ? 128 : 64);
     const int nk = (p.nkb + S - 1) / S;
-    const TqPrep prep = tq_prep(cut, B, op);
+    const TqPrep prep = tq_prep(cut, bits, B, op);
     const int teams = tq_teams(ctx->sm_count, bits, cut, B, op, prep);
     const size_t recv = S > 1 ? (size_t)S * ((B + S - 1) / S) * T * 128 * 8 : 0;
     const size_t spare = bits == 8 ? 16384 * T : 0;                                      // an MMA reads 128 rows whatever the run has

@@ -640,9 +640,11 @@ def test_tcgen05_int4_four_teams(backend, M, N, B):
 @pytest.mark.parametrize("N,B", [(32, 17), (2048, 32), (2080, 5), (4128, 17), (6176, 32), (8224, 18), (16384, 20), (16416, 17)])
 def test_tcgen05_digits_prepared_by_clusters(backend, bits, op, N, B):
     """Digits by one to eight blocks per activation (the last length: one block): parts that end inside the last 128 columns or have none, every
-    prologue. Bound: the prologue rounds an activation to FP32 a few times (silu: exponential, division, product; the norm's sum of squares is a
+    prologue; without one, as many rows as leave runs to clusters of less than eight, which the preparation by clusters needs there. Bound: the prologue rounds an activation to FP32 a few times (silu: exponential, division, product; the norm's sum of squares is a
     tree of at most 8 + 5 + 3 + 3 additions), 32 units in the last place hold all of it; the rest as above."""
     M, be = 70, backend
+    if op == "plain":
+        M, B = 2700, max(B, 21)
     rng = np.random.default_rng(N + B + bits)
     w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
     x2 = rng.standard_normal((B, N)).astype(np.float32)
