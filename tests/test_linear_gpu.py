@@ -172,7 +172,7 @@ def test_tcgen05_rows_around_clusters_of_eight(backend, bits, Ms, N, B):
     assert np.allclose(outs[0], outs[1], rtol=2e-6, atol=1e-6 * float(np.abs(outs[1]).max()))
 
 
-@pytest.mark.parametrize("M,N,B", [(38000, 1664, 6), (25000, 1920, 32), (3000, 4224, 24)])
+@pytest.mark.parametrize("M,N,B", [(38000, 1664, 6), (25000, 1920, 32), (3000, 4224, 24), (40000, 1152, 8)])
 def test_tcgen05_int4_teams(backend, M, N, B):
     """Odd numbers of 128-column blocks through rings that are used again, over one and two runs of rows: the two teams of
     widening warps change places from run to run. Bound as above."""
@@ -694,3 +694,41 @@ def test_several_products_take_the_tcgen05_kernel(bits, M, N, B):
         be._check(be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.ptr, N, B, bits, C.byref(pro))); be.sync()
         assert captured(-1) == 0
         assert captured(0) != 0
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("op", ["plain", "norm", "silu"])
+@pytest.mark.parametrize("N", [2048, 5152])
+def test_rows_without_an_ordinary_maximum_through_clusters(backend, bits, op, N):
+    """Activations of zeros, with Inf, with NaN, and with magnitudes whose squares overflow: digits by clusters give what the other kernel's conversion
+    gives for them, to the bit (their maximum, scale and digits do not hang on the order of a sum; two activations a call, of which that kernel
+    cuts no row into slices), and leave the other activations alone: 32 units in the last place of the largest result, as above."""
+    M, B, be = 2700, 22, backend
+    rng = np.random.default_rng(N + bits)
+    w, s16, x = (_cpu.make_int8_case if bits == 8 else _cpu.make_int4_case)(rng, M, N, B)
+    x2 = rng.standard_normal((B, N)).astype(np.float32)
+    x[0] = 0.0
+    x[3, N - 1] = np.inf; x[4, 0] = -np.inf; x[5, N // 2] = np.nan; x[6, 5] = np.nan; x[6, N - 3] = np.inf
+    x[8] *= 1e25; x[9, 77] = 3e38; x[10] = np.nan; x[11] = np.inf
+    x2[13, 3] = np.inf; x2[14, N - 2] = np.nan; x2[15] = 0.0
+    odd = [0, 3, 4, 5, 6, 8, 9, 10, 11] + ([13, 14, 15] if op == "silu" else [])
+    dw, ds, dx, dx2 = be.upload(w), be.upload(s16), be.upload(x), be.upload(x2)
+    dn = be.upload(_cpu.fp16_bits(rng.uniform(0.2, 3.0, N)))
+    got = {}
+    for mode, group in ((-1, 2), (2, B)):
+        do = be.upload(np.full((B, M), 7.0, np.float32))
+        be.lib.ibcu_linear_use_tcgen05(be.ctx, mode)
+        try:
+            for b in range(0, B, group):
+                t = LinearT(dw.ptr, ds.ptr, do.at(4 * b * M), M, M, 0, 0)
+                pro = _ffi.PrologueT()
+                pro.op, pro.x2, pro.norm_w, pro.eps = {"plain": 0, "norm": 1, "silu": 2}[op], dx2.at(4 * b * N), dn.ptr, 1e-5
+                be._check(be.lib.ibcu_linear_ex(be.ctx, C.byref(t), 1, dx.at(4 * b * N), N, group, bits, C.byref(pro)))
+        finally:
+            be.lib.ibcu_linear_use_tcgen05(be.ctx, 0)
+        be.sync()
+        got[mode] = be.download(do, np.float32, B * M).reshape(B, M)
+    assert np.array_equal(got[2][odd], got[-1][odd], equal_nan=True)
+    rest = [b for b in range(B) if b not in odd]
+    scale = np.abs(got[-1][rest]).max(axis=1, keepdims=True)
+    assert np.all(np.abs(got[2][rest] - got[-1][rest]) <= 32 * 2.0 ** -24 * scale)
