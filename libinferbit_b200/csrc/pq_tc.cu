@@ -43,6 +43,12 @@ template <int N> __device__ __forceinline__ void pt_set_regs() {
     if constexpr (N > PT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N));
     if constexpr (N < PT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N));
 }
+// The codebooks' copies are written and tensor memory is allocated: every warp but that of the codes, which reads neither, comes here once.
+__device__ __forceinline__ void pt_staged() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" :: "n"(PT_THREADS - 32) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
 constexpr int PT_GROUP = 528;                                // bytes of a staged group of 16 rows x 32 codes: 16 more than it has, so that the two groups of a warp sit in different banks
 constexpr int PT_SLAB = 8 * PT_GROUP;
 constexpr int PT_MAX_X = 6, PT_MAX_C = 6, PT_MAXSEG = 8;
@@ -174,80 +180,78 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
     if (warp >= PT_CODE_WARP) {
         pt_set_regs<PtRegs<HALF, NG>::HELPER>();
         if (warp == PT_CODE_WARP) {
-        // the codes do not depend on the kernel ahead: the ring fills at once
-        int s = 0; uint32_t ph = 1;
-        for (int item = lo; item < hi; item++) {
-            if (item == lo + p.sc) pdl_wait();                // nobody polls a barrier for long while the kernel ahead runs
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_c[s]), ph, abort_flag, 1))) break;
-            const int tile = item / p.nslab, slab = item - tile * p.nslab;
-            const uint32_t dst = smem_u32(pt_smem + p.code_off + s * PT_SLAB) + lane * 16;
-            const unsigned char* src = p.idx_t + ((size_t)slab * G16 + (size_t)tile * 8) * 512 + lane * 16;
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const bool in = tile * 8 + u < G16;           // rows past the last group: zeros
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst + u * PT_GROUP), "l"(in ? src + u * 512 : p.idx_t), "r"(in ? 16 : 0) : "memory");
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&sh->full_c[s])) : "memory");
-            if (++s == p.sc) { s = 0; ph ^= 1; }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-        } else {
-        if (warp == PT_MMA_WARP) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)p.tmem_cols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-            pdl_launch_dependents();                          // not before: the blocks behind allocate too, and every block of this launch must hold its own first
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("bar.sync 1, %0;" :: "n"(PT_THREADS - 32) : "memory");
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;
-        if (warp == PT_X_WARP) {
-        pdl_wait();
-        if (elect_one()) {
+            // the codes do not depend on the kernel ahead: the ring fills at once
             int s = 0; uint32_t ph = 1;
-            bool ok = true;
-            for (int item = lo; item < hi && ok; item++) {
-                int slab = item % p.nslab;
-                if (slab >= p.nslab1) slab -= p.nslab1;       // the second level runs over the same activations
-                for (int hb = 0; hb < NB; hb++) {
-                    ok = mbar_wait(smem_u32(&sh->empty_x[s]), ph, abort_flag, 2);
-                    if (!ok) break;
-                    mbar_expect_tx(smem_u32(&sh->full_x[s]), x_stage);
-                    bulk_load(smem_u32(pt_smem + (size_t)s * x_stage), p.ximg + (size_t)(slab * NB + hb) * x_stage, x_stage, smem_u32(&sh->full_x[s]));
-                    if (++s == p.sx) { s = 0; ph ^= 1; }
-                }
-            }
-        }
-        __syncwarp();
-        } else if (warp == PT_MMA_WARP) {
-        pdl_wait();
-        if (elect_one()) {
-            constexpr uint32_t idesc = (1u << 4) | (8u << 24);    // FP32 accumulators, FP16 operands, 128 rows
-            constexpr uint32_t idesc_a = idesc | (2u << 17), idesc_b = idesc | ((uint32_t)(2 * NG) << 17);     // 16 columns; 16 NG columns
-            int s = 0; uint32_t ph = 0;
-            bool ok = true;
-            for (int n = 0; n < nunit; n++) {
-                ok = mbar_wait(smem_u32(&sh->full_x[s]), ph, abort_flag, 3) && mbar_wait(smem_u32(&sh->full_t[n & 1]), (uint32_t)(n >> 1) & 1u, abort_flag, 4);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t bd = smem_desc_sw128(smem_u32(pt_smem) + (uint32_t)s * x_stage);
-                const uint32_t a = tmem_a + (uint32_t)(n & 1) * (CB / 2), d = tmem_base + (uint32_t)((n & 1) * DC);
+            for (int item = lo; item < hi; item++) {
+                if (item == lo + p.sc) pdl_wait();                // nobody polls a barrier for long while the kernel ahead runs
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_c[s]), ph, abort_flag, 1))) break;
+                const int tile = item / p.nslab, slab = item - tile * p.nslab;
+                const uint32_t dst = smem_u32(pt_smem + p.code_off + s * PT_SLAB) + lane * 16;
+                const unsigned char* src = p.idx_t + ((size_t)slab * G16 + (size_t)tile * 8) * 512 + lane * 16;
 #pragma unroll
-                for (int m = 0; m < CB / 16; m++) {           // 16 columns each; the image has NC * 128 bytes per 64 columns
-                    const uint64_t b = bd + (uint64_t)((m >> 2) * (NC * 8) + (m & 3) * 2);
-                    mma_f16_ts(d + (m / (PT_CHAIN / 16)) * 16, a + m * 8, b, idesc_a, m % (PT_CHAIN / 16) ? 1u : 0u);
-                    mma_f16_ts(d + ND * 16, a + m * 8, b + 128, idesc_b, m ? 1u : 0u);
+                for (int u = 0; u < 8; u++) {
+                    const bool in = tile * 8 + u < G16;           // rows past the last group: zeros
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst + u * PT_GROUP), "l"(in ? src + u * 512 : p.idx_t), "r"(in ? 16 : 0) : "memory");
                 }
-                mma_commit(smem_u32(&sh->full_d[n & 1]));
-                mma_commit(smem_u32(&sh->empty_x[s]));
-                if (++s == p.sx) { s = 0; ph ^= 1; }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&sh->full_c[s])) : "memory");
+                if (++s == p.sc) { s = 0; ph ^= 1; }
             }
-            mma_commit(smem_u32(&sh->drained));
-            mbar_wait(smem_u32(&sh->drained), 0u, abort_flag, 5);
-        }
-        __syncwarp();
-        }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+        } else {
+            if (warp == PT_MMA_WARP) {
+                asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)p.tmem_cols) : "memory");
+                asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+                pdl_launch_dependents();                          // not before: the blocks behind allocate too, and every block of this launch must hold its own first
+            }
+            pt_staged();
+            const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;
+            if (warp == PT_X_WARP) {
+                pdl_wait();
+                if (elect_one()) {
+                    int s = 0; uint32_t ph = 1;
+                    bool ok = true;
+                    for (int item = lo; item < hi && ok; item++) {
+                        int slab = item % p.nslab;
+                        if (slab >= p.nslab1) slab -= p.nslab1;       // the second level runs over the same activations
+                        for (int hb = 0; hb < NB; hb++) {
+                            ok = mbar_wait(smem_u32(&sh->empty_x[s]), ph, abort_flag, 2);
+                            if (!ok) break;
+                            mbar_expect_tx(smem_u32(&sh->full_x[s]), x_stage);
+                            bulk_load(smem_u32(pt_smem + (size_t)s * x_stage), p.ximg + (size_t)(slab * NB + hb) * x_stage, x_stage, smem_u32(&sh->full_x[s]));
+                            if (++s == p.sx) { s = 0; ph ^= 1; }
+                        }
+                    }
+                }
+                __syncwarp();
+            } else if (warp == PT_MMA_WARP) {
+                pdl_wait();
+                if (elect_one()) {
+                    constexpr uint32_t idesc = (1u << 4) | (8u << 24);    // FP32 accumulators, FP16 operands, 128 rows
+                    constexpr uint32_t idesc_a = idesc | (2u << 17), idesc_b = idesc | ((uint32_t)(2 * NG) << 17);     // 16 columns; 16 NG columns
+                    int s = 0; uint32_t ph = 0;
+                    bool ok = true;
+                    for (int n = 0; n < nunit; n++) {
+                        ok = mbar_wait(smem_u32(&sh->full_x[s]), ph, abort_flag, 3) && mbar_wait(smem_u32(&sh->full_t[n & 1]), (uint32_t)(n >> 1) & 1u, abort_flag, 4);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t bd = smem_desc_sw128(smem_u32(pt_smem) + (uint32_t)s * x_stage);
+                        const uint32_t a = tmem_a + (uint32_t)(n & 1) * (CB / 2), d = tmem_base + (uint32_t)((n & 1) * DC);
+#pragma unroll
+                        for (int m = 0; m < CB / 16; m++) {           // 16 columns each; the image has NC * 128 bytes per 64 columns
+                            const uint64_t b = bd + (uint64_t)((m >> 2) * (NC * 8) + (m & 3) * 2);
+                            mma_f16_ts(d + (m / (PT_CHAIN / 16)) * 16, a + m * 8, b, idesc_a, m % (PT_CHAIN / 16) ? 1u : 0u);
+                            mma_f16_ts(d + ND * 16, a + m * 8, b + 128, idesc_b, m ? 1u : 0u);
+                        }
+                        mma_commit(smem_u32(&sh->full_d[n & 1]));
+                        mma_commit(smem_u32(&sh->empty_x[s]));
+                        if (++s == p.sx) { s = 0; ph ^= 1; }
+                    }
+                    mma_commit(smem_u32(&sh->drained));
+                    mbar_wait(smem_u32(&sh->drained), 0u, abort_flag, 5);
+                }
+                __syncwarp();
+            }
         }
     } else {
         // the codebooks into the copies
@@ -269,188 +273,186 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pq_tc_kernel(const __grid_const
         };
         stage(p.cb_l, p.cb_r, p.K, 256, p.tab_off);
         if (p.rows2) stage(p.cb2_l, p.cb2_r, p.K2, p.rows2, p.tab2_off);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("bar.sync 1, %0;" :: "n"(PT_THREADS - 32) : "memory");
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;                   // two units of CB / 2 columns
-    if (warp < PT_WORKERS) {
-        pt_set_regs<PtRegs<HALF, NG>::WORKER>();
-        // ── entries into tensor memory: the two teams take units in turn, each into its own half ──
-        const int q = warp & 3, h = (warp >> 2) & 1, team = warp >> 3, rl = q * 32 + lane;
-        const uint32_t at = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(team * (CB / 2) + h * (CB / 4));
-        const uint32_t lane_off = HALF == 4 ? (lane & 15) * 8 : (lane & 7) * 16;
-        const uint32_t tab1 = smem_u32(pt_smem + p.tab_off) + lane_off, tab2 = smem_u32(pt_smem + p.tab2_off) + lane_off;
-        // row i of a group keeps the code of subspace l at byte i ^ (l >> 1); the warp's subspaces: l0 .. l0 + SPW - 1 of the slab
-        const int l0 = (NB == 2 ? team * 2 * SPW : 0) + h * SPW;
-        const uint32_t crow = smem_u32(pt_smem + p.code_off) + (rl >> 4) * PT_GROUP + l0 * 16, ib = (uint32_t)((rl & 15) ^ (l0 >> 1));
-        uint32_t code[SPW];
-        int s = NB == 1 ? team : 0;
-        uint32_t ph = 0;
-        auto load_codes = [&]() {
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_c[s]), ph, abort_flag, 7))) return false;
+        pt_staged();
+        const uint32_t tmem_base = sh->tmem_base, tmem_a = tmem_base + 2 * DC;                   // two units of CB / 2 columns
+        if (warp < PT_WORKERS) {
+            pt_set_regs<PtRegs<HALF, NG>::WORKER>();
+            // ── entries into tensor memory: the two teams take units in turn, each into its own half ──
+            const int q = warp & 3, h = (warp >> 2) & 1, team = warp >> 3, rl = q * 32 + lane;
+            const uint32_t at = tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(team * (CB / 2) + h * (CB / 4));
+            const uint32_t lane_off = HALF == 4 ? (lane & 15) * 8 : (lane & 7) * 16;
+            const uint32_t tab1 = smem_u32(pt_smem + p.tab_off) + lane_off, tab2 = smem_u32(pt_smem + p.tab2_off) + lane_off;
+            // row i of a group keeps the code of subspace l at byte i ^ (l >> 1); the warp's subspaces: l0 .. l0 + SPW - 1 of the slab
+            const int l0 = (NB == 2 ? team * 2 * SPW : 0) + h * SPW;
+            const uint32_t crow = smem_u32(pt_smem + p.code_off) + (rl >> 4) * PT_GROUP + l0 * 16, ib = (uint32_t)((rl & 15) ^ (l0 >> 1));
+            uint32_t code[SPW];
+            int s = NB == 1 ? team : 0;
+            uint32_t ph = 0;
+            auto load_codes = [&]() {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_c[s]), ph, abort_flag, 7))) return false;
 #pragma unroll
-            for (int j = 0; j < SPW; j++) asm volatile("ld.shared.u8 %0, [%1];" : "=r"(code[j]) : "r"(crow + s * PT_SLAB + j * 16 + (ib ^ (j >> 1))) : "memory");
-            return true;
-        };
-        int slab = (lo + (NB == 1 ? team : 0)) % p.nslab;
-        uint32_t dph = 1;                                     // the first wait passes: nothing has used the team's half yet
-        bool alive = team < nunit && load_codes();
-        for (int n = team; n < nunit && alive; n += 2) {
-            const uint32_t tab = slab >= p.nslab1 ? tab2 : tab1;
-            // sixteen words at a time, the next ones on their way while these are stored: every warp's whole share at once kept the
-            // shared-memory pipe's queue so long that the other warps' barrier tests took 500 cycles
-            constexpr int CH = CB / 64, PER = SPW / CH;       // chunks; lookups of a chunk
-            uint32_t o[2][16];
-            auto lookup = [&](int c) {
-#pragma unroll
-                for (int i = 0; i < PER; i++) {
-                    const int j = c * PER + i;
-                    uint32_t* r = o[c & 1] + i * (16 / PER);
-                    const uint32_t e = tab + code[j] * ROW + (j & 1) * 128 * PLANES;
-                    if constexpr (HALF == 4) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(e) : "memory");
-                    else {
-#pragma unroll
-                        for (int pl = 0; pl < PLANES; pl++)
-                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r[4 * pl]), "=r"(r[4 * pl + 1]), "=r"(r[4 * pl + 2]), "=r"(r[4 * pl + 3]) : "r"(e + pl * 128) : "memory");
-                    }
-                }
+                for (int j = 0; j < SPW; j++) asm volatile("ld.shared.u8 %0, [%1];" : "=r"(code[j]) : "r"(crow + s * PT_SLAB + j * 16 + (ib ^ (j >> 1))) : "memory");
+                return true;
             };
-            lookup(0);
-            if (n >= 2 && n < 4) pdl_wait();                  // nobody polls a barrier for long while the kernel ahead runs
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_d[team]), dph, abort_flag, 6))) break;
-            dph ^= 1;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            int slab = (lo + (NB == 1 ? team : 0)) % p.nslab;
+            uint32_t dph = 1;                                     // the first wait passes: nothing has used the team's half yet
+            bool alive = team < nunit && load_codes();
+            for (int n = team; n < nunit && alive; n += 2) {
+                const uint32_t tab = slab >= p.nslab1 ? tab2 : tab1;
+                // sixteen words at a time, the next ones on their way while these are stored: every warp's whole share at once kept the
+                // shared-memory pipe's queue so long that the other warps' barrier tests took 500 cycles
+                constexpr int CH = CB / 64, PER = SPW / CH;       // chunks; lookups of a chunk
+                uint32_t o[2][16];
+                auto lookup = [&](int c) {
 #pragma unroll
-            for (int c = 0; c < CH; c++) {
-                if (c + 1 < CH) lookup(c + 1);
-                tmem_st16(at + 16 * c, o[c & 1]);
+                    for (int i = 0; i < PER; i++) {
+                        const int j = c * PER + i;
+                        uint32_t* r = o[c & 1] + i * (16 / PER);
+                        const uint32_t e = tab + code[j] * ROW + (j & 1) * 128 * PLANES;
+                        if constexpr (HALF == 4) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(e) : "memory");
+                        else {
+#pragma unroll
+                            for (int pl = 0; pl < PLANES; pl++)
+                                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r[4 * pl]), "=r"(r[4 * pl + 1]), "=r"(r[4 * pl + 2]), "=r"(r[4 * pl + 3]) : "r"(e + pl * 128) : "memory");
+                        }
+                    }
+                };
+                lookup(0);
+                if (n >= 2 && n < 4) pdl_wait();                  // nobody polls a barrier for long while the kernel ahead runs
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_d[team]), dph, abort_flag, 6))) break;
+                dph ^= 1;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    if (c + 1 < CH) lookup(c + 1);
+                    tmem_st16(at + 16 * c, o[c & 1]);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->empty_c[s]));              // the codes have become addresses
+                if (NB == 1) {
+                    s += 2; slab += 2;
+                    while (slab >= p.nslab) slab -= p.nslab;
+                } else { s++; if (++slab == p.nslab) slab = 0; }
+                if (s >= p.sc) { s -= p.sc; ph ^= 1; }
+                if (n + 2 < nunit) { alive = load_codes(); if (!alive) break; }    // the next unit's codes travel while this one's entries are stored
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[team]));
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->empty_c[s]));              // the codes have become addresses
-            if (NB == 1) {
-                s += 2; slab += 2;
-                while (slab >= p.nslab) slab -= p.nslab;
-            } else { s++; if (++slab == p.nslab) slab = 0; }
-            if (s >= p.sc) { s -= p.sc; ph ^= 1; }
-            if (n + 2 < nunit) { alive = load_codes(); if (!alive) break; }    // the next unit's codes travel while this one's entries are stored
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[team]));
-        }
-    } else if (warp < PT_SUM_WARP + PT_SUMMERS) {
-        pt_set_regs<PtRegs<HALF, NG>::SUMMER>();
-        // ── sums out of the accumulators ──
-        const int q = warp & 3, rl = q * 32 + lane, st = tid - PT_SUM_WARP * 32, w = warp - PT_SUM_WARP, team = w >> 2;
-        const uint32_t dq = tmem_base + ((uint32_t)(q * 32) << 16);
-        const float cbmax = *p.cbmax;
-        float acc[NG * 8], low[NG * 8];         // a sum and what its roundings lost
+        } else if (warp < PT_SUM_WARP + PT_SUMMERS) {
+            pt_set_regs<PtRegs<HALF, NG>::SUMMER>();
+            // ── sums out of the accumulators ──
+            const int q = warp & 3, rl = q * 32 + lane, st = tid - PT_SUM_WARP * 32, w = warp - PT_SUM_WARP, team = w >> 2;
+            const uint32_t dq = tmem_base + ((uint32_t)(q * 32) << 16);
+            const float cbmax = *p.cbmax;
+            float acc[NG * 8], low[NG * 8];         // a sum and what its roundings lost
 #pragma unroll
-        for (int i = 0; i < NG * 8; i++) acc[i] = low[i] = 0.0f;
-        bool alive = true;
-        int nseg = 0, seg_n = 0;
-        uint32_t met_ph = 0;
-        auto meet = [&]() {                                   // these warps' own barrier, bounded like every other wait
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->met));
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->met), met_ph, abort_flag, 8))) alive = false;
-            met_ph ^= 1;
-            return alive;
-        };
-        auto flush = [&](int tile) {                          // the sums of a tile into the fixed-point accumulators
-            const int r = tile * 128 + rl;
-#pragma unroll
-            for (int b = 0; b < NG * 8; b++) {
-                if (b < p.B && r < p.M) atomicAdd(p.acc + (size_t)b * p.M_pad + r, (unsigned long long)__double2ll_rn(((double)acc[b] + (double)low[b]) * sh->to_fix[b]));
-                acc[b] = low[b] = 0.0f;
-            }
-        };
-        // this warp's arrivals for the tiles met since the last time; 32 rows to which all parts have come become results
-        auto settle = [&]() {
-            __threadfence();
-            __syncwarp();
-            bool last = false;
-            if (lane < nseg) {
-                unsigned* cnt = p.arrive + sh->seg_tile[w][lane] * 4 + q;
-                const unsigned old = atomicAdd(cnt, (unsigned)sh->seg_n[w][lane]);
-                last = old + (unsigned)sh->seg_n[w][lane] == (unsigned)(p.nslab * NB);
-                if (last) *cnt = 0;
-            }
-            unsigned todo = __ballot_sync(0xffffffffu, last);
-            if (todo) __threadfence();                        // every part has arrived, each behind its warp's fence: loads past L1 read the sums
-            for (; todo; todo &= todo - 1) {
-                const int r = sh->seg_tile[w][__ffs(todo) - 1] * 128 + rl;
-                if (r >= p.M) continue;
-                const float sc = __half2float(p.row_scale[r]);
-                long long sum[NG * 8];
-#pragma unroll
-                for (int b = 0; b < NG * 8; b++) sum[b] = b < p.B ? (long long)__ldcg(p.acc + (size_t)b * p.M_pad + r) : 0;
+            for (int i = 0; i < NG * 8; i++) acc[i] = low[i] = 0.0f;
+            bool alive = true;
+            int nseg = 0, seg_n = 0;
+            uint32_t met_ph = 0;
+            auto meet = [&]() {                                   // these warps' own barrier, bounded like every other wait
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->met));
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->met), met_ph, abort_flag, 8))) alive = false;
+                met_ph ^= 1;
+                return alive;
+            };
+            auto flush = [&](int tile) {                          // the sums of a tile into the fixed-point accumulators
+                const int r = tile * 128 + rl;
 #pragma unroll
                 for (int b = 0; b < NG * 8; b++) {
-                    if (b >= p.B) break;
-                    p.acc[(size_t)b * p.M_pad + r] = 0ull;
-                    p.out[(size_t)b * p.out_stride + r] = (float)((double)sum[b] * sh->to_out[b]) * sc;
+                    if (b < p.B && r < p.M) atomicAdd(p.acc + (size_t)b * p.M_pad + r, (unsigned long long)__double2ll_rn(((double)acc[b] + (double)low[b]) * sh->to_fix[b]));
+                    acc[b] = low[b] = 0.0f;
                 }
+            };
+            // this warp's arrivals for the tiles met since the last time; 32 rows to which all parts have come become results
+            auto settle = [&]() {
+                __threadfence();
+                __syncwarp();
+                bool last = false;
+                if (lane < nseg) {
+                    unsigned* cnt = p.arrive + sh->seg_tile[w][lane] * 4 + q;
+                    const unsigned old = atomicAdd(cnt, (unsigned)sh->seg_n[w][lane]);
+                    last = old + (unsigned)sh->seg_n[w][lane] == (unsigned)(p.nslab * NB);
+                    if (last) *cnt = 0;
+                }
+                unsigned todo = __ballot_sync(0xffffffffu, last);
+                if (todo) __threadfence();                        // every part has arrived, each behind its warp's fence: loads past L1 read the sums
+                for (; todo; todo &= todo - 1) {
+                    const int r = sh->seg_tile[w][__ffs(todo) - 1] * 128 + rl;
+                    if (r >= p.M) continue;
+                    const float sc = __half2float(p.row_scale[r]);
+                    long long sum[NG * 8];
+#pragma unroll
+                    for (int b = 0; b < NG * 8; b++) sum[b] = b < p.B ? (long long)__ldcg(p.acc + (size_t)b * p.M_pad + r) : 0;
+#pragma unroll
+                    for (int b = 0; b < NG * 8; b++) {
+                        if (b >= p.B) break;
+                        p.acc[(size_t)b * p.M_pad + r] = 0ull;
+                        p.out[(size_t)b * p.out_stride + r] = (float)((double)sum[b] * sh->to_out[b]) * sc;
+                    }
+                }
+                __syncwarp();
+                nseg = 0;
+            };
+            auto close_tile = [&](int tile) {
+                if (!seg_n) return;                               // all of it was the other team's
+                flush(tile);
+                if (lane == 0) { sh->seg_tile[w][nseg] = tile; sh->seg_n[w][nseg] = seg_n; }
+                seg_n = 0;
+                if (++nseg == PT_MAXSEG) settle();
+            };
+            if (lane == 0)
+                mbar_arrive(smem_u32(&sh->full_t[team]));         // the accumulators start free
+            pdl_wait();
+            if (st < p.B) {
+                const unsigned ab = __ldcg(p.amax_bits + st);
+                sh->to_fix[st] = pt_pow2(62 - pt_bound(p.N, cbmax, ab) - pt_shift(ab));
+                sh->to_out[st] = ab > 0x7f7fffffu ? __longlong_as_double(0x7ff8000000000000ll) : pt_pow2(pt_bound(p.N, cbmax, ab) - 62);
             }
-            __syncwarp();
-            nseg = 0;
-        };
-        auto close_tile = [&](int tile) {
-            if (!seg_n) return;                               // all of it was the other team's
-            flush(tile);
-            if (lane == 0) { sh->seg_tile[w][nseg] = tile; sh->seg_n[w][nseg] = seg_n; }
-            seg_n = 0;
-            if (++nseg == PT_MAXSEG) settle();
-        };
-        if (lane == 0)
-            mbar_arrive(smem_u32(&sh->full_t[team]));         // the accumulators start free
-        pdl_wait();
-        if (st < p.B) {
-            const unsigned ab = __ldcg(p.amax_bits + st);
-            sh->to_fix[st] = pt_pow2(62 - pt_bound(p.N, cbmax, ab) - pt_shift(ab));
-            sh->to_out[st] = ab > 0x7f7fffffu ? __longlong_as_double(0x7ff8000000000000ll) : pt_pow2(pt_bound(p.N, cbmax, ab) - 62);
+            meet();
+            int cur = lo / p.nslab, left = (cur + 1) * p.nslab - lo;           // left: slabs of the tile from this piece's first on
+            uint32_t ph = 0;
+            for (int n = team; n < nunit && alive; n += 2, ph ^= 1) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_d[team]), ph, abort_flag, 9))) { alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                while (n / NB >= left) { close_tile(cur); cur++; left += p.nslab; }
+                const uint32_t d = dq + (uint32_t)(team * DC);
+                float f[16];
+                {
+                    uint32_t u[16], v[16];
+                    tmem_ld16(d, u); tmem_ld16(d + 16, v);
+#pragma unroll
+                    for (int b = 0; b < NG * 8; b++) f[b] = __uint_as_float(u[b]) + __uint_as_float(v[b]);
+                    if constexpr (ND == 4) {
+                        tmem_ld16(d + 32, u); tmem_ld16(d + 48, v);
+#pragma unroll
+                        for (int b = 0; b < NG * 8; b++) f[b] += __uint_as_float(u[b]) + __uint_as_float(v[b]);
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < NG; g++) {
+                    uint32_t u[16];
+                    tmem_ld16(d + ND * 16 + 16 * g, u);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {                 // piece p counts 2^(-11 p)
+                        const int b = 8 * g + i;
+                        const float v = fmaf(__uint_as_float(u[2 * i + 1]), 0x1p-22f, fmaf(__uint_as_float(u[2 * i]), 0x1p-11f, f[b]));
+                        const float a = acc[b], sum = __fadd_rn(a, v), fr = __fsub_rn(sum, a);
+                        low[b] += __fadd_rn(__fsub_rn(a, __fsub_rn(sum, fr)), __fsub_rn(v, fr));
+                        acc[b] = sum;
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[team]));
+                seg_n++;
+            }
+            if (alive) close_tile(cur);
+            if (alive && nseg) settle();
         }
-        meet();
-        int cur = lo / p.nslab, left = (cur + 1) * p.nslab - lo;           // left: slabs of the tile from this piece's first on
-        uint32_t ph = 0;
-        for (int n = team; n < nunit && alive; n += 2, ph ^= 1) {
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->full_d[team]), ph, abort_flag, 9))) { alive = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            while (n / NB >= left) { close_tile(cur); cur++; left += p.nslab; }
-            const uint32_t d = dq + (uint32_t)(team * DC);
-            float f[16];
-            {
-                uint32_t u[16], v[16];
-                tmem_ld16(d, u); tmem_ld16(d + 16, v);
-#pragma unroll
-                for (int b = 0; b < NG * 8; b++) f[b] = __uint_as_float(u[b]) + __uint_as_float(v[b]);
-                if constexpr (ND == 4) {
-                    tmem_ld16(d + 32, u); tmem_ld16(d + 48, v);
-#pragma unroll
-                    for (int b = 0; b < NG * 8; b++) f[b] += __uint_as_float(u[b]) + __uint_as_float(v[b]);
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < NG; g++) {
-                uint32_t u[16];
-                tmem_ld16(d + ND * 16 + 16 * g, u);
-#pragma unroll
-                for (int i = 0; i < 8; i++) {                 // piece p counts 2^(-11 p)
-                    const int b = 8 * g + i;
-                    const float v = fmaf(__uint_as_float(u[2 * i + 1]), 0x1p-22f, fmaf(__uint_as_float(u[2 * i]), 0x1p-11f, f[b]));
-                    const float a = acc[b], sum = __fadd_rn(a, v), fr = __fsub_rn(sum, a);
-                    low[b] += __fadd_rn(__fsub_rn(a, __fsub_rn(sum, fr)), __fsub_rn(v, fr));
-                    acc[b] = sum;
-                }
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->full_t[team]));
-            seg_n++;
-        }
-        if (alive) close_tile(cur);
-        if (alive && nseg) settle();
-    }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
