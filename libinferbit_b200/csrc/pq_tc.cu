@@ -473,6 +473,15 @@ int launch_pt(ibcu_ctx* ctx, const PtParams& p, int grid, size_t smem) {
     if (int rc = ibcu_allow_smem(ctx, opt, kern, smem)) return rc;
     return ibcu_launch(ctx, kern, dim3(grid), dim3(PT_THREADS), smem, 1, true, p);
 }
+// setmaxnreg.inc waits for registers out of those that the block was launched with. A build that gives a thread fewer than PT_REGS (a debug build, a register
+// limit) would wait for good: its calls take the tables.
+template <int HALF, int NG>
+bool pt_regs_suffice() {
+    static const bool ok = [] { cudaFuncAttributes a; return cudaFuncGetAttributes(&a, pq_tc_kernel<HALF, NG>) == cudaSuccess ? a.numRegs >= PT_REGS : (cudaGetLastError(), false); }();
+    return ok;
+}
+template <int HALF>
+bool pt_regs_suffice(int B) { return B <= 8 ? pt_regs_suffice<HALF, 1>() : pt_regs_suffice<HALF, 2>(); }
 template <int HALF>
 int launch_half(ibcu_ctx* ctx, const PtParams& p, int grid, size_t smem) {
     return p.B <= 8 ? launch_pt<HALF, 1>(ctx, p, grid, smem) : launch_pt<HALF, 2>(ctx, p, grid, smem);
@@ -494,6 +503,8 @@ int ibcu_pq_tc(ibcu_ctx* ctx, const ibcu_pq_t* t, const float* x, float* out, in
     const uintptr_t align = half == 4 ? 7 : 15;
     if ((half != 4 && half != 8 && half != 16) || t->cb_chunk_stride || B > 32 || (((uintptr_t)t->codebook_l | (uintptr_t)t->codebook_r) & align)) return IBCU_DECLINED;
     if (two && (((uintptr_t)t->codebook2_l | (uintptr_t)t->codebook2_r) & align)) return IBCU_DECLINED;
+    const int b_launch = B > PT_MAXB ? (B + 1) / 2 : B;
+    if (!(half == 4 ? pt_regs_suffice<4>(b_launch) : half == 8 ? pt_regs_suffice<8>(b_launch) : pt_regs_suffice<16>(b_launch))) return IBCU_DECLINED;
     if (B > PT_MAXB) {
         const int b0 = (B + 1) / 2;
         const int rc = ibcu_pq_tc(ctx, t, x, out, out_stride, b0, l1_only, acc, arrive, max_counters, amax_bits, image);
