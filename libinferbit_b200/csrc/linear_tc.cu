@@ -533,12 +533,12 @@ TqPrep tq_prep(const TqCut& cut, int bits, int B, int op) {
     const bool crowded = bits == 4 && cut.T == 2 && cut.S == 4 && blocks >= 4;
     // A cluster per activation, us, one block and a cluster. silu(x) * x2: always (936 calls: 0.73 of the time on the mean, 1.01 at most).
     // RMSNorm: 4096 x 4096 INT8 at 8, 16 and 32 8.9 and 8.2, 10.5 and 10.1, 12.8 and 11.9, 4096 x 14336 at 32 22.1 and 21.1; crowded: 5120 x 5120 at 8, 20 and 32 10.1 and 11.3,
-    // 13.3 and 14.9, 16.7 and 16.6. Without a prologue there is no sum to wait for: beyond 16 activations, INT4 3072 + 1024 + 1024 x 3072 at 20 12.2 and 10.7,
+    // 13.3 and 14.9, 16.7 and 16.6; clusters of eight ahead of runs of two tiles: 935 + 8677 x 10848 INT4 at 4 and 8 20.7 and 22.4, 23.4 and 22.7, 4463 + 279 x 13120 INT8 at 4 17.2 and 18.5, 4500 x 9600 INT8 at 6 14.5 and 13.8. Without a prologue there is no sum to wait for: beyond 16 activations, INT4 3072 + 1024 + 1024 x 3072 at 20 12.2 and 10.7,
     // 3072 + 3072 x 1024 at 32 10.2 and 8.6, 4096 x 4096 INT8 at 20 and 32 10.7 and 11.1, 11.9 and 11.8; but INT4 2560 x 6400 at 17 11.3 and 13.0, INT8 6400 + 6400 x 2560 at 24
     // 14.4 and 15.6, 10000 x 2560 at 24 15.4 and 16.2, 2048 x 6144 INT4, in clusters of eight, at 32 11.6 and 12.3.
     if (cut.nkb * 128L <= IBCU_PREPARED_COLUMNS) {
         if (op == IBCU_PRO_SILU_MUL) x.clustered = true;
-        if (op == IBCU_PRO_RMSNORM) x.clustered = !crowded || B > 20;
+        if (op == IBCU_PRO_RMSNORM) x.clustered = (!crowded || B > 20) && (cut.T == 1 || cut.S == 1 || blocks < 8 || B >= (bits == 8 ? 5 : 8));
         if (op == IBCU_PRO_NONE) x.clustered = B > 16 && ((cut.S == 4 && !crowded && (B > 20 || (bits == 4 && blocks <= 2))) || (cut.S == 2 && blocks == 1));
     }
     // otherwise a block per activation, or several when the maximum is known
