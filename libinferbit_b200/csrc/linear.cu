@@ -519,9 +519,11 @@ LinPlan lin_plan(const ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensor
 
 // Which kernel takes a call of 2 to 16 activations: the time of either, in us, from what it does. The coefficients are least squares
 // (relative error 6 %) over 2296 calls on a B200, direct and in graphs: 2, 3, 4, 5, 6, 8, 12 and 16 activations, 512 to 14336 columns, 512
-// to 32000 rows in one to three tensors, 4 and 8 bits. The choice is 0.2 % behind the better kernel on the mean and more than 5 % behind
+// to 32000 rows in one to three tensors, 4 and 8 bits. The choice was 0.2 % behind the better kernel on the mean and more than 5 % behind
 // it in one call of 60; choosing by the number of activations and the bytes of the weights was 2.2 % behind, up to 95 %.
-// (Fitted before the tcgen05 kernel's rings took an SM and clusters prepared its digits, which is 2 to 20 % off its times: calls near the line could go over now.)
+// The fit is older than the tcgen05 kernel's full rings and its digits by clusters, which took 2 to 20 % off its times: now the choice is 1.1 % behind the better kernel on the mean
+// of 2592 calls (0.4 % without a prologue, 1.7 % with RMSNorm), more than 5 % in one of 15, up to 60 % (INT4 856 x 1440 with RMSNorm at 4 activations 8.9 against 5.5),
+// nearly always by staying with mma.sync.
 // mma.sync kernel: per block the MMAs of its tiles, the weights, and a reduction per tile; the conversion in the block, or a launch ahead.
 double lin_mma_us(const LinPlan& pl, int N, int B, int bits) {
     const int R = 16 * pl.rt, tiles = (pl.rows_per_block + R - 1) / R, stages = ((pl.slice_kb < pl.nkb ? pl.slice_kb : pl.nkb) + 7) / 8;

@@ -2,8 +2,8 @@
 // tensor memory): the exact integer arithmetic of linear.cu as a GEMM, weights [rows x columns] times the four base-256
 // digits ("limbs") of every activation, 4 B columns.
 //
-// xprep_tc_kernel turns the activations into digits once, with one power-of-two scale per activation, and lays them out as
-// the operand image: per block of 128 columns NC rows of 128 bytes, swizzled. linear_tc_kernel is a cluster of S blocks per
+// xprep_tc_kernel, or xprep_tc_cluster_kernel with a cluster of blocks per activation (tq_prep), turns the activations into digits once, with one
+// power-of-two scale per activation, and lays them out as the operand image: per block of 128 columns NC rows of 128 bytes, swizzled. linear_tc_kernel is a cluster of S blocks per
 // run of up to 256 weight rows; block r of the cluster takes the r-th part of the columns. Per 128-column block of its part
 // TMA brings the weights of all rows of the run (one box, rows the tensor lacks are not fetched) and one bulk copy the
 // digits. INT8 weights are the A operand as they land. INT4 nibbles go to tensor memory as bytes (worker warps: four
@@ -19,8 +19,8 @@
 // Workers (INT4 widening, then epilogue): four warps per tile of 128 rows and team; the teams take the blocks of columns in turn;
 // then one warp each for the weights (TMA), the digits (bulk copies) and the MMAs. What a block of columns costs a warp is waits
 // and latencies one behind the other, not work: with two teams instead of one, gate and up of 14336 x 4096 INT4 at eight
-// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4; at 32 the digits, which every SM reads from L2,
-// bound the kernel (26 us, 75 MB of them). Four teams for some runs of one tile (tq_teams): 4096 x 4096 INT4 at 4, 16 and 32 activations 8.3 -> 7.5, 9.2 -> 8.9,
+// activations went from 22.0 to 18.0 us and 4096 x 14336 from 19.3 to 16.4. No single pipe bounds it: 4096 x 14336 at 32 activations took 19.9 us, 19.8 without the
+// transfer of the digits (which every SM reads from L2, 56 MB of them), 19.1 without three of four MMAs, 19.2 without the weights, 9.9 with one block of columns. Four teams for some runs of one tile (tq_teams): 4096 x 4096 INT4 at 4, 16 and 32 activations 8.3 -> 7.5, 9.2 -> 8.9,
 // 12.4 -> 11.5, 2560 x 6400 at 32 14.3 -> 13.3, 4096 x 14336 at 32 20.7 -> 19.8.
 // The weights do not depend on the kernel ahead: their ring fills before the dependency wait.
 #include "common.cuh"
@@ -550,7 +550,8 @@ TqPrep tq_prep(const TqCut& cut, int bits, int B, int op) {
 }
 
 // Teams of widening warps (INT4). Runs of one tile have room for four (16 workers); two tiles fill the block with two, and INT8 weights need none. Clusters of eight keep
-// to half an SM a block: sixteen of them with an SM to each block do not find room at once (2048 x 6144 at 4 and 32 activations 7.3 and 12.6, 12.1 and 17.8 us).
+// to half an SM a block: sixteen of them with an SM to each block do not find room at once (2048 x 6144 INT8 at 4 and 32 activations 7.3 and 12.6, 12.1 and 17.8 us); that is two
+// teams, with 80 registers, of which 32 bytes spill.
 // Beside a block of four teams, 19 warps of 96 registers, no block of the next call's preparation finds registers (with 72 or 80 it does, but the block
 // spills). Where that preparation does not fit on the SMs this launch leaves idle either, it starts late and two teams are the faster: us, two and four,
 // 8192 x 2048 (none idle) at 6 8.7 and 9.6, 2560 x 6400 with RMSNorm at 8 9.3 and 11.0, 16384 x 2048 at 8 9.3 and 10.2; where it fits, or finds no room beside two teams
@@ -648,8 +649,8 @@ int ibcu_linear_tc(ibcu_ctx* ctx, const ibcu_linear_t* tensors, int n_tensors, c
     // Shared memory: the rings take what an SM has. A block of runs of one tile used to keep to half, so that the next launch's blocks move in beside
     // it, but what a block of columns costs is the way of its weights and digits from L2, and with twice the ring twice as many are on it:
     // 4096 x 14336 INT4 at 4, 16 and 32 activations 15.0 -> 13.1, 18.1 -> 17.2, 25.3 -> 20.7 us, 6144 x 4096 INT8 at 4 and 32 9.9 -> 9.2,
-    // 17.6 -> 16.0. INT8 at 9 to 20 activations is where the overlap is worth as much (6144 x 4096 at 12 13.3 against 13.7, 4096 x 4096 at 16 9.4
-    // against 9.6) and keeps it, and clusters of eight (tq_teams).
+    // 17.6 -> 16.0. INT8 at 9 to 20 activations keeps the overlap: an SM's ring against half of one, without a prologue, runs alone, in clusters of two and of four: at 8 0.98, 0.99, 0.96,
+    // at 9 1.02, 1.00, 0.99, at 12 1.00, 1.00, 0.98, at 16 1.00, 0.99, 0.98, at 20 0.99, 1.00, 0.97, at 24 0.98, 0.95, 0.94 (22 shapes). So do clusters of eight (tq_teams).
     const int tcols = T * (p.NC + (bits == 4 ? 128 : 0));
     p.tmem_cols = 32;
     while (p.tmem_cols < tcols) p.tmem_cols *= 2;

@@ -125,12 +125,12 @@ __device__ __forceinline__ void fold(float* v, int o) {
 // BT activations (1 or 2) share a pass over the codes: table entries are BT floats wide. grid = (blocks of rows,
 // blocks of slabs, passes); pass z serves activations BT z .. BT z + BT - 1.
 // EX: the tensor has a second level or outlier columns; plain tensors take the instance without that code.
-// H8: entries of eight values, known at compile time (one activation through 4096 x 14336: 10.9 -> 10.75 us a call; its 64 registers spill less).
+// H8: entries of eight values, known at compile time (one activation through 4096 x 14336: 10.9 -> 10.75 us a call).
 template <int BT, bool EX, bool H8>
 __global__ void __launch_bounds__(PQ_THREADS, 2) pq_slab_kernel(const PqParams p) {
-    // Groups of 16 rows whose codes a warp keeps in flight: as many as leave nothing to spill in 64 registers (four spilled 72 bytes for one level, us with
-    // four and three: 4096 x 14336 11.0 and 10.7, 1024 x 4096 7.5 and 7.2, 32000 x 4096 15.1 and 15.0; with a second level and four and two:
-    // 8000 x 8192 15.5 and 14.9, 2000 x 2048 8.0 and 7.5; two activations, two and one: 4096 x 8192 13.1 and 12.4, 32000 x 4096 25.7 and 25.3, with a second
+    // Groups of 16 rows whose codes a warp keeps in flight: as many as leave nothing to spill in 64 registers (but for 28 bytes of entries of any width with one level and
+    // one activation). Four spilled 72 bytes for one level (us with four and three: 4096 x 14336 11.0 and 10.7, 1024 x 4096 7.5 and 7.2, 32000 x 4096 15.1 and 15.0; with a
+    // second level and four and two: 8000 x 8192 15.5 and 14.9, 2000 x 2048 8.0 and 7.5; two activations, two and one: 4096 x 8192 13.1 and 12.4, 32000 x 4096 25.7 and 25.3, with a second
     // level of 256 14336 x 4096 23.4 and 22.8, entries of sixteen with one 4096 x 4096 30.5 and 28.4).
     constexpr int PQ_NG = BT == 1 ? (EX ? 2 : 3) : 1;
     extern __shared__ __align__(16) float lut[];            // [256][32][BT]
@@ -568,8 +568,9 @@ constexpr size_t PQ_STATIC_FLOATS = (size_t)1 << 20;         // scratch of the a
 //   entries of 8: one never (4096 x 14336 10.8 / 15.5), three and more always; two: 14336 x 2048 14.9 / 12.2, 4096 x 4096 11.6 / 10.7, 4096 x 8192
 //     12.4 / 12.8, 14336 x 14336 33 / 33.9
 // The lines are where the two met before the tensor-core kernel had its registers by role, which put it ahead up to twice as much work (entries of 16, one
-// activation) and about level (entries of 8, two). They were not moved: where both do, the tables' sums are the closer ones (1.0e-7 of the
-// result's root mean square against 1.25e-7).
+// activation) and about level (entries of 8, two). They are those lines still, so that no call changed over to the sums that are less close (1.25e-7 of the
+// result's root mean square against the tables' 1.0e-7); what that costs: against the faster of the two over 437 calls 0.9 % on the mean, more than 5 % in 11, most for entries of 16
+// (32000 x 4096 at two 40.7 / 24.2, 8192 x 8192 at one 21.6 / 15.2) and, the other way, small tensors beyond 16 activations, two launches there (1024 x 2048 at 32 13.1 / 18.8).
 static bool pq_takes_tc(const ibcu_pq_t* t, int B) {
     const double cols = (double)(t->N - t->n_outlier) * (t->K_l2 > 0 ? 2 : 1), work = cols * t->M;
     if (t->G == 32) return work <= 62e6 * B;

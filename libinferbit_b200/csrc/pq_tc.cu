@@ -17,10 +17,11 @@
 //                meet in the fixed-point accumulators of pq.cu. (Over 256 columns at a time the error was 3.4e-7 of the result's
 //                root mean square, over 128 1.9e-7, now 1.25e-7; the tables' 1.0e-7.)
 //   warps 24-26  codes (cp.async), operand image (bulk copies), MMA issue; a 28th warp fills their warpgroup
-// What bounds it: the latency of every role's chain of waits, not a pipe (a unit takes about 1300 cycles of which the entries
-// keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500), and about 7 us around the units: the preparation, staging the codebooks, and the meeting of the parts. 4096 x 14336, entries of eight, 24 tensors in turn: eight
-// activations 28.1 -> 18 us, sixteen 46 -> 24; 4096 x 8192 with entries of four at eight 49 -> 17.3, of sixteen 37 -> 15, with a
-// second level 45 -> 19.
+// What bounds it: the latency of every role's chain of waits, not a pipe, and what lies around the units: launches, the preparation, staging the codebooks, and the
+// meeting of the parts. 4096 rows of entries of eight, 4096, 8192 and 14336 columns (4, 7 and 13 units a block at most): eight activations 12.8, 14.8 and 18.1 us, sixteen 16.8, 19.4
+// and 23.7, so a unit takes about 0.58 us (1150 cycles, of which the entries keep the shared-memory pipe busy for 740 and the MMAs the tensor cores for 500) and all
+// around the units 10.5. 4096 x 14336, entries of eight, 24 tensors in turn: eight activations 28.1 -> 18 us, sixteen 46 -> 24; 4096 x 8192 with entries
+// of four at eight 49 -> 17, of sixteen 37 -> 15, with a second level 45 -> 19.
 #include "tc_common.cuh"
 #include "common.cuh"
 #include "pq_tc.cuh"
@@ -28,9 +29,9 @@
 namespace {
 
 constexpr int PT_TEAM = 8, PT_WORKERS = 2 * PT_TEAM, PT_SUMMERS = 8, PT_SUM_WARP = 16, PT_CODE_WARP = 24, PT_X_WARP = 25, PT_MMA_WARP = 26, PT_THREADS = 28 * 32;       // the last warp only completes a warpgroup
-// Registers a thread by role (launched with PT_REGS each). With the same for all, every instance spilled 36 to 352 bytes of stores in its loops, and with
+// Registers a thread by role (launched with PT_REGS each). With the same for all, every instance spilled 36 to 364 bytes of stores in its loops, and with
 // an SM's shared memory full there is little L1 to spill to. The helpers give up what the sums or, for entries of eight and up to eight
-// activations, the workers are short of (4 to 64 bytes are left): 4096 x 14336 at 3, 8 and 16 activations 18.4 -> 16.3, 20.4 -> 18.0, 26.7 -> 24.0 us, 4096 x 8192
+// activations, the workers are short of (4 to 72 bytes are left, the most in entries of four): 4096 x 14336 at 3, 8 and 16 activations 18.4 -> 16.3, 20.4 -> 18.0, 26.7 -> 24.0 us, 4096 x 8192
 // with entries of sixteen at 1, 8 and 16 16.9 -> 12.3, 22.0 -> 15.1, 23.5 -> 19.0, with a second level 23.7 -> 19.1. Entries of four keep the even split (17.3;
 // 18.6 with 80 for workers and sums and 24 for the helpers).
 constexpr int PT_REGS = 72;

@@ -304,7 +304,7 @@ static int issue(ib_b200_model* m, int pos0, int B, int head_last) {
         /* silu(gate) * up (src/forward.c:637-640): with several positions, whose digits a launch of their own prepares anyway, in that launch; else
          * in a small one that also leaves max|h|, so that down_proj's blocks turn h into their operand without a reduction of their own. (Six layers, us, either
          * way: 2560 wide INT4 MLP at 4 and 16 positions 342 and 330, 428 and 416, 4096 wide 426 and 417, 545 and 540.) Rows that one pass does not prepare
-         * keep the launch: four layers of 28672 wide INT8 MLP at 5 and 16 positions 499 -> 455, 586 -> 552, of 17408 wide INT4 at 5 340 -> 321. */
+         * keep the launch: four layers of 28672 wide INT8 MLP at 5 and 16 positions 499 -> 450, 586 -> 537, of 17408 wide INT4 at 5 340 -> 314. */
         const int prepared = B >= 4 && c->inter <= IBCU_PREPARED_COLUMNS;
         if (!rc && !prepared) rc = ibcu_silu_mul_amax(ctx, m->hg, m->hg, m->hu, c->inter, B, m->amax, AMAX_PARTS);
         ibcu_prologue_t km = { IBCU_PRO_KNOWN_MAX, NULL, NULL, 0.0f, m->amax, AMAX_PARTS }, sm = { IBCU_PRO_SILU_MUL, m->hu, NULL, 0.0f, NULL, 0 };
