@@ -145,7 +145,7 @@ void ibcu_linear_force_generic(ibcu_ctx* ctx, int on);
 /* A second kernel for calls with several activations (up to 32): the same exact arithmetic on the tcgen05 tensor cores, weights
  * as the A operand (INT8 from shared memory, INT4 widened into tensor memory), limbs as the B operand, s32 accumulators in
  * tensor memory. on = 0 (the default): where an estimate of both kernels' times says that it is faster (2 to 16 activations;
- * more than 16: always); 1: every INT4 call whatever the number of activations; 2: INT8 calls as well; -1: never. The choice
+ * more than 16, and several with IBCU_PRO_SILU_MUL: always); 1: every INT4 call whatever the number of activations; 2: INT8 calls as well; -1: never. The choice
  * depends on the shapes of the call only: ranks with equal shards of a model take the same kernel, a rank with other rows, or a
  * single GPU with all of them, may take the other. Both kernels' sums are exact; they differ in the last place where the mma.sync
  * kernel cuts a row into slices with scales of their own, or through the order in which RMSNorm's squares are added. */
